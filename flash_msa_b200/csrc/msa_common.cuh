@@ -25,31 +25,46 @@ __host__ __device__ __forceinline__ int64_t dense_row_offset(int j, int S) {
 //
 // A reverse-index row (batch, proxy head, key block j) can hold anything from one chunk of 128
 // query rows to all S - 128*j later rows (a "sink" block).  To keep the persistent CTAs balanced a
-// row is cut into sub-units of at most kChunksPerSubUnit chunks.  The number of rows is only known
+// row is cut into sub-units of at most C chunks (chunks_per_subunit below).  The number of rows is only known
 // on the device, so the sub-units are enumerated for the worst case (NB - j chunks) and a CTA that
 // draws a sub-unit beyond the real end of its row simply skips it.
 //
-// Order: (batch, KV head) group major, then sub-unit index s (chunks 8s .. 8s+7 of a row), then key
+// Order: (batch, KV head) group major, then sub-unit index s (chunks C*s .. C*s+C-1 of a row), then key
 // block ascending, then proxy head of the group.  Group-major order keeps the rows that the active
 // CTAs gather from and reduce into (a few heads of Q, dO) resident in L2.  Inside a group, putting s
 // outermost makes neighbouring sub-units alike in size (for a given s the rows of neighbouring key
 // blocks are about equally long, and the sub-units that lie beyond the end of their row cluster
 // together), so both a dynamic work counter and a static round-robin deal stay balanced.
 // -------------------------------------------------------------------------------------------
-constexpr int kChunksPerSubUnit = 8;
+constexpr int kMaxChunksPerSubUnit = 8;
 
 // Key blocks j that can have a sub-unit s: NB - j > C*s, i.e. j < NB - C*s.
 __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int ppk, int C) {
-    int64_t total = 0;
-    for (int s = 0; s * C < NB; ++s) total += NB - s * C;
-    return total * ppk;
+    // sum over s = 0 .. n-1 of (NB - C*s), n = ceil(NB / C)
+    const int64_t n = (NB + C - 1) / C;
+    return (n * NB - C * (n * (n - 1) / 2)) * ppk;
+}
+
+// C for a launch: the largest power of two up to 8 that still leaves every CTA `kSubUnitsPerCta` sub-units on average.  A
+// sub-unit loads K and V once and flushes dV and dK once, so long ones save traffic; short ones fill the SMs and bound the
+// tail of the launch: a problem of a few dozen chunks otherwise runs on a handful of SMs (B=1, S=1024, Hq=8, top-k 4 blocks:
+// 64 chunks on 16 CTAs).  `edges` is an upper bound of the selected (row, block) pairs; a row of the reverse index is on
+// average half a chunk longer than its edges.  Drawing and passing over a sub-unit beyond the end of its row costs about a
+// microsecond, so C does not go below what keeps the enumeration at `kDrawsPerCta` per CTA.
+constexpr int kSubUnitsPerCta = 6, kDrawsPerCta = 32;
+inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int ppk, int sms) {
+    const int64_t chunks = (edges + kBlock - 1) / kBlock + groups * ppk * NB / 2;
+    int c = kMaxChunksPerSubUnit;
+    while (c > 1 && chunks < static_cast<int64_t>(c) * kSubUnitsPerCta * sms &&
+           groups * subunits_per_group(NB, ppk, c / 2) <= static_cast<int64_t>(kDrawsPerCta) * sms)
+        c >>= 1;
+    return c;
 }
 
 struct SubUnit {
     int g, j, pp, chunk0;
 };
-__device__ __forceinline__ SubUnit decode_subunit(int64_t u, int NB, int ppk) {
-    constexpr int C = kChunksPerSubUnit;
+__device__ __forceinline__ SubUnit decode_subunit(int64_t u, int NB, int ppk, int C) {
     const int64_t per_group = subunits_per_group(NB, ppk, C);
     SubUnit su;
     su.g = static_cast<int>(u / per_group);

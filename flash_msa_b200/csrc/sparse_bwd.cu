@@ -63,6 +63,7 @@ struct BwdParams {
     int S, NB, Hq, Hkv, Hp, Hpkv, mpp, ppk, pg;
     int g_begin, G;
     int64_t n_subunits;
+    int chunks;             // chunks per sub-unit
     int with_kl, dense;
     float scale_log2e;
     float* kl_value;        // optional: += KL(teacher || proxy) summed over this launch's rows, / (B*Hp*S)
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
             for (;;) {
                 const int64_t u = atomicAdd(P.counter, 1);
                 if (u >= P.n_subunits) break;
-                const SubUnit su = decode_subunit(u, P.NB, P.ppk);
+                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks);
                 const int g = P.g_begin + su.g;
                 const int b = g / P.Hkv, kvh = g % P.Hkv, p = kvh * P.ppk + su.pp;
                 const int64_t bp = static_cast<int64_t>(b) * P.Hp + p;
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     nu.j = static_cast<uint16_t>(su.j); nu.b = static_cast<uint16_t>(b); nu.kvh = static_cast<uint16_t>(kvh);
                     nu.p = static_cast<uint16_t>(p); nu.n = n; nu.e0 = e0;
                     nu.chunk0 = static_cast<uint16_t>(su.chunk0);
-                    nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + kChunksPerSubUnit));
+                    nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + P.chunks));
                     break;
                 }
             }
@@ -1200,7 +1201,8 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
                            : (varlen ? reinterpret_cast<const void*>(sparse_bwd_kernel<false, true>) : reinterpret_cast<const void*>(sparse_bwd_kernel<false, false>));
     if (sms <= 0 || !ensure_smem_attr(kfn, kBwdSmemBytes)) return FMSA_ERR_CUDA;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
-    P.n_subunits = g_count * subunits_per_group(P.NB, P.ppk, kChunksPerSubUnit);
+    P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
+    P.n_subunits = g_count * subunits_per_group(P.NB, P.ppk, P.chunks);
     FMSA_REQUIRE(P.n_subunits < 0x7fffffffLL);
     const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
     if (fp16 && varlen) sparse_bwd_kernel<true, true><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);

@@ -57,6 +57,7 @@ struct FwdParams {
     int g_begin, G;
     int with_proxy, dense;
     int64_t n_subunits;
+    int chunks;             // chunks per sub-unit
     float scale_log2e;
 };
 
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
             for (;;) {
                 const int64_t u = atomicAdd(P.counter, 1);
                 if (u >= P.n_subunits) break;
-                const SubUnit su = decode_subunit(u, P.NB, P.ppk);
+                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks);
                 const int g = P.g_begin + su.g;
                 const int b = g / P.Hkv, kvh = g % P.Hkv, p = kvh * P.ppk + su.pp;
                 const int64_t bp = static_cast<int64_t>(b) * P.Hp + p;
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                 if (su.chunk0 * kBlock < n) {
                     nu.j = su.j; nu.b = b; nu.kvh = kvh; nu.p = p; nu.n = n; nu.e0 = e0;
                     nu.chunk0 = su.chunk0;
-                    nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + kChunksPerSubUnit);
+                    nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + P.chunks);
                     break;
                 }
             }
@@ -959,7 +960,8 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
                            : (varlen ? reinterpret_cast<const void*>(sparse_fwd_kernel<false, true>) : reinterpret_cast<const void*>(sparse_fwd_kernel<false, false>));
     if (sms <= 0 || !ensure_smem_attr(kfn, kFwdSmemBytes)) return FMSA_ERR_CUDA;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
-    P.n_subunits = g_count * subunits_per_group(P.NB, P.ppk, kChunksPerSubUnit);
+    P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
+    P.n_subunits = g_count * subunits_per_group(P.NB, P.ppk, P.chunks);
     FMSA_REQUIRE(P.n_subunits < 0x7fffffffLL);
     const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
     if (fp16 && varlen) sparse_fwd_kernel<true, true><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
