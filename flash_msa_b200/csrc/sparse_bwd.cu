@@ -802,12 +802,16 @@ struct BwdCombineParams {
     float scale, kl_out_scale; // factors the backward kernel left out of its partial rows
     int S, NB, Hq, Hp, mpp, ppk, Kb;
     int g_begin, G, dense;
+    int hgroup;             // main heads per blockIdx.y
     int split;              // the partial buffers hold a second plane (rounding remainders) part_slots slots further on
     int64_t part_slots;
 };
 
-template <bool FP16>
-__global__ void __launch_bounds__(256) bwd_combine_kernel(const BwdCombineParams P) {
+// One sweep over the contiguous mpp*256-byte record of each edge; with more than eight main heads per proxy head blockIdx.y
+// takes groups of heads, each a contiguous piece of the record (and group 0 the proxy row): at Hq/Hp = 12, 96 edges per row,
+// two planes, B=1 S=16384 Hq=24, one head at a time with 8-byte loads took 4.26 ms, groups of six heads 2.48 ms.
+template <int KITER, bool SPLIT, bool FP16, bool GROUPED>   // heads of a group <= 2*KITER: few accumulators, high occupancy (latency bound)
+__global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_kernel(const BwdCombineParams P) {
     const int lane = threadIdx.x & 31;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     const int64_t bp0 = static_cast<int64_t>(P.g_begin) * P.ppk;
@@ -824,64 +828,8 @@ __global__ void __launch_bounds__(256) bwd_combine_kernel(const BwdCombineParams
         const int e = erow[s];
         return e < 0 ? -1 : static_cast<int64_t>(e) - edge_base;
     };
-    const float gk = ((P.dqp && P.grad_kl) ? *P.grad_kl : 1.f) * P.kl_out_scale;
-    const int nheads = P.mpp + (P.dqp ? 1 : 0);
-    for (int hh = 0; hh < nheads; ++hh) {
-        const bool proxy = hh == P.mpp;
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-        for (int s0 = 0; s0 < nslots; s0 += 32) {
-            const int64_t sl = slot_of(s0 + lane);
-            const int cnt = min(32, nslots - s0);
-#pragma unroll 4
-            for (int i = 0; i < cnt; ++i) {
-                const int64_t si = __shfl_sync(0xffffffffu, sl, i);
-                if (si < 0) continue;
-                for (int part = 0; part <= P.split; ++part) {
-                    const int64_t sp = si + part * P.part_slots;
-                    const __nv_bfloat16* src = proxy ? P.dqp_part + sp * kHeadDim : P.dq_part + (sp * P.mpp + hh) * kHeadDim;
-                    const uint2 raw = *reinterpret_cast<const uint2*>(src + lane * 4);
-                    const uint32_t lo = raw.x;
-                    const uint32_t hi = raw.y;
-                    a0 += act_lo<FP16>(lo);
-                    a1 += act_hi<FP16>(lo);
-                    a2 += act_lo<FP16>(hi);
-                    a3 += act_hi<FP16>(hi);
-                }
-            }
-        }
-        uint2 o;
-        if (proxy) {
-            o.x = pack_act<FP16>(a0 * gk, a1 * gk);
-            o.y = pack_act<FP16>(a2 * gk, a3 * gk);
-            *reinterpret_cast<uint2*>(P.dqp + (static_cast<int64_t>(b) * P.dqp_sb + static_cast<int64_t>(p) * P.dqp_sh + static_cast<int64_t>(q) * P.dqp_ss) + lane * 4) = o;
-        } else {
-            o.x = pack_act<FP16>(a0 * P.scale, a1 * P.scale);
-            o.y = pack_act<FP16>(a2 * P.scale, a3 * P.scale);
-            *reinterpret_cast<uint2*>(P.dq + (static_cast<int64_t>(b) * P.dq_sb + static_cast<int64_t>(p * P.mpp + hh) * P.dq_sh + static_cast<int64_t>(q) * P.dq_ss) + lane * 4) = o;
-        }
-    }
-}
-
-// Wide variant for Hq/Hp <= 8: one sweep over the contiguous mpp*256-byte record of each edge.
-template <int KITER, bool SPLIT, bool FP16>   // Hq/Hp <= 2*KITER: few accumulators, high occupancy (latency bound)
-__global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_wide_kernel(const BwdCombineParams P) {
-    const int lane = threadIdx.x & 31;
-    const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const int64_t bp0 = static_cast<int64_t>(P.g_begin) * P.ppk;
-    if (w >= static_cast<int64_t>(P.G) * P.ppk * P.S) return;
-    const int64_t bp = bp0 + w / P.S;
-    const int q = static_cast<int>(w % P.S);
-    const int b = static_cast<int>(bp / P.Hp), p = static_cast<int>(bp % P.Hp);
-    const int64_t edge_base = P.dense ? dense_edge_base(bp0, P.S, P.NB) : static_cast<int64_t>(P.row_ptr[bp0 * P.NB]);
-    const int nslots = P.dense ? (q >> 7) + 1 : P.Kb;
-    const int32_t* erow = P.dense ? nullptr : P.edge_pos + (bp * P.S + q) * P.Kb;
-    auto slot_of = [&](int s) -> int64_t {
-        if (s >= nslots) return -1;
-        if (P.dense) return dense_edge_base(bp, P.S, P.NB) + dense_row_offset(s, P.S) + (q - s * kBlock) - edge_base;
-        const int e = erow[s];
-        return e < 0 ? -1 : static_cast<int64_t>(e) - edge_base;
-    };
-    const int nchunk = P.mpp * 16;
+    const int h0 = GROUPED ? blockIdx.y * P.hgroup : 0, hn = GROUPED ? min(P.hgroup, P.mpp - h0) : P.mpp;   // this block's main heads
+    const int nchunk = hn * 16;
     float acc[KITER][8];
 #pragma unroll
     for (int k = 0; k < KITER; ++k)
@@ -890,7 +838,7 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_wide_ke
     float pa0 = 0.f, pa1 = 0.f, pa2 = 0.f, pa3 = 0.f;   // proxy row: lane owns columns 4*lane..+3
     // Four edges at a time: every load of the group is issued before the first sum (the kernel is bound by memory
     // latency; left to itself the compiler batches the loads only when the register budget happens to allow it).
-    const bool has_proxy = P.dqp != nullptr;
+    const bool has_proxy = P.dqp != nullptr && (!GROUPED || blockIdx.y == 0);
     for (int s0 = 0; s0 < nslots; s0 += 32) {
         const int sl = static_cast<int>(slot_of(s0 + lane));   // slot numbers of a pass fit 31 bits
         const int cnt = min(32, nslots - s0);
@@ -908,7 +856,7 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_wide_ke
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int64_t sp = static_cast<int64_t>(si[u]) + part * P.part_slots;
-                    const __nv_bfloat16* rec = P.dq_part + sp * P.mpp * kHeadDim;
+                    const __nv_bfloat16* rec = P.dq_part + (sp * P.mpp + h0) * kHeadDim;
 #pragma unroll
                     for (int k = 0; k < KITER; ++k) {
                         const int ck = k * 32 + lane;
@@ -950,7 +898,7 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_wide_ke
     for (int k = 0; k < KITER; ++k) {
         const int ck = k * 32 + lane;
         if (ck < nchunk) {
-            const int hh = ck >> 4, col = (ck & 15) * 8;
+            const int hh = h0 + (ck >> 4), col = (ck & 15) * 8;
             uint4 o;
             o.x = pack_act<FP16>(acc[k][0] * P.scale, acc[k][1] * P.scale);
             o.y = pack_act<FP16>(acc[k][2] * P.scale, acc[k][3] * P.scale);
@@ -959,7 +907,7 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_wide_ke
             *reinterpret_cast<uint4*>(P.dq + (static_cast<int64_t>(b) * P.dq_sb + static_cast<int64_t>(p * P.mpp + hh) * P.dq_sh + static_cast<int64_t>(q) * P.dq_ss) + col) = o;
         }
     }
-    if (P.dqp) {
+    if (has_proxy) {
         const float gk = (P.grad_kl ? *P.grad_kl : 1.f) * P.kl_out_scale;
         uint2 o;
         o.x = pack_act<FP16>(pa0 * gk, pa1 * gk);
@@ -1246,31 +1194,26 @@ extern "C" int fmsa_sparse_bwd_combine(const fmsa_problem* pb, const void* dq_pa
     const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * P.S;
     const int64_t grid = (rows + 7) / 8;
     FMSA_REQUIRE(grid <= 0x7fffffffLL);
-    const dim3 cg(static_cast<unsigned>(grid));
+    const int groups = P.mpp <= 8 ? 1 : (P.mpp + 5) / 6;   // as in the forward combine
+    P.hgroup = (P.mpp + groups - 1) / groups;
+    const dim3 cg(static_cast<unsigned>(grid), static_cast<unsigned>(groups));
     cudaStream_t cst = static_cast<cudaStream_t>(stream);
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
-#define FMSA_BWD_COMBINE(K)                                                                          \
+#define FMSA_BWD_COMBINE(K, G)                                                                          \
     do {                                                                                             \
         if (fp16) {                                                                                  \
-            if (P.split) bwd_combine_wide_kernel<K, true, true><<<cg, 256, 0, cst>>>(P);             \
-            else bwd_combine_wide_kernel<K, false, true><<<cg, 256, 0, cst>>>(P);                    \
+            if (P.split) bwd_combine_kernel<K, true, true, G><<<cg, 256, 0, cst>>>(P);             \
+            else bwd_combine_kernel<K, false, true, G><<<cg, 256, 0, cst>>>(P);                    \
         } else {                                                                                     \
-            if (P.split) bwd_combine_wide_kernel<K, true, false><<<cg, 256, 0, cst>>>(P);            \
-            else bwd_combine_wide_kernel<K, false, false><<<cg, 256, 0, cst>>>(P);                   \
+            if (P.split) bwd_combine_kernel<K, true, false, G><<<cg, 256, 0, cst>>>(P);            \
+            else bwd_combine_kernel<K, false, false, G><<<cg, 256, 0, cst>>>(P);                   \
         }                                                                                            \
     } while (0)
-    if (P.mpp > 8) {
-        if (fp16) bwd_combine_kernel<true><<<cg, 256, 0, cst>>>(P);
-        else bwd_combine_kernel<false><<<cg, 256, 0, cst>>>(P);
-    } else if (P.mpp <= 2) {
-        FMSA_BWD_COMBINE(1);
-    } else if (P.mpp <= 4) {
-        FMSA_BWD_COMBINE(2);
-    } else if (P.mpp <= 6) {
-        FMSA_BWD_COMBINE(3);
-    } else {
-        FMSA_BWD_COMBINE(4);
-    }
+    if (groups > 1) FMSA_BWD_COMBINE(3, true);
+    else if (P.mpp <= 2) FMSA_BWD_COMBINE(1, false);
+    else if (P.mpp <= 4) FMSA_BWD_COMBINE(2, false);
+    else if (P.mpp <= 6) FMSA_BWD_COMBINE(3, false);
+    else FMSA_BWD_COMBINE(4, false);
 #undef FMSA_BWD_COMBINE
     return check_launch();
 }

@@ -635,92 +635,13 @@ struct CombineParams {
     float* lse_proxy;          // [B, Hp, S] or null
     int S, NB, Hq, Hp, mpp, ppk, Kb;
     int g_begin, G, dense;
+    int hgroup;                // main heads per blockIdx.y of the row kernel
 };
 
-template <bool FP16>
-__global__ void __launch_bounds__(256) combine_kernel(const CombineParams P) {
-    const int lane = threadIdx.x & 31;
-    const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const int64_t bp0 = static_cast<int64_t>(P.g_begin) * P.ppk;
-    const int64_t nrows = static_cast<int64_t>(P.G) * P.ppk * P.S;
-    if (w >= nrows) return;
-    const int64_t bp = bp0 + w / P.S;
-    const int q = static_cast<int>(w % P.S);
-    const int b = static_cast<int>(bp / P.Hp), p = static_cast<int>(bp % P.Hp);
-    const int64_t edge_base = P.dense ? dense_edge_base(bp0, P.S, P.NB) : static_cast<int64_t>(P.row_ptr[bp0 * P.NB]);
-    const int nslots = P.dense ? (q >> 7) + 1 : P.Kb;
-    const int lse_stride = P.mpp + 1;
-    const int32_t* erow = P.dense ? nullptr : P.edge_pos + (bp * P.S + q) * P.Kb;
-
-    auto slot_of = [&](int s) -> int64_t {
-        if (s >= nslots) return -1;
-        if (P.dense) return dense_edge_base(bp, P.S, P.NB) + dense_row_offset(s, P.S) + (q - s * kBlock) - edge_base;
-        const int e = erow[s];
-        return e < 0 ? -1 : static_cast<int64_t>(e) - edge_base;
-    };
-
-    const float2* stats = reinterpret_cast<const float2*>(P.lse_part);
-    const int nheads = P.mpp + (P.lse_proxy ? 1 : 0);
-    for (int hh = 0; hh < nheads; ++hh) {
-        // pass A: every partial carries (row max m in the log2 domain, row sum l); merge them
-        float m = -INFINITY, sum = 0.f;
-        for (int s0 = 0; s0 < nslots; s0 += 32) {
-            const int64_t sl = slot_of(s0 + lane);
-            if (sl >= 0) {
-                const float2 st = stats[sl * lse_stride + hh];
-                const float mn = fmaxf(m, st.x);
-                sum = sum * fast_exp2(m - mn) + st.y * fast_exp2(st.x - mn);
-                m = mn;
-            }
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float mo = __shfl_xor_sync(0xffffffffu, m, off);
-            const float so = __shfl_xor_sync(0xffffffffu, sum, off);
-            const float mn = fmaxf(m, mo);
-            const float a = (m == -INFINITY) ? 0.f : sum * fast_exp2(m - mn);
-            const float c = (mo == -INFINITY) ? 0.f : so * fast_exp2(mo - mn);
-            sum = a + c;
-            m = mn;
-        }
-        const float total = (m + __log2f(sum)) * kLn2;   // natural-log LSE of the whole row
-        if (hh == P.mpp) {
-            if (lane == 0) P.lse_proxy[bp * P.S + q] = total;
-            continue;
-        }
-        const int h = p * P.mpp + hh;
-        if (lane == 0) P.lse[(static_cast<int64_t>(b) * P.Hq + h) * P.S + q] = total;
-        // pass B: weighted sum of the unnormalised partial outputs; lane owns columns 4*lane..4*lane+3
-        const float inv = 1.f / sum;
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-        for (int s0 = 0; s0 < nslots; s0 += 32) {
-            const int64_t sl = slot_of(s0 + lane);
-            const float wgt = sl >= 0 ? fast_exp2(stats[sl * lse_stride + hh].x - m) * inv : 0.f;
-            const int cnt = min(32, nslots - s0);
-#pragma unroll 4
-            for (int i = 0; i < cnt; ++i) {
-                const int64_t si = __shfl_sync(0xffffffffu, sl, i);
-                const float wi = __shfl_sync(0xffffffffu, wgt, i);
-                if (si < 0) continue;
-                const uint2 raw = *reinterpret_cast<const uint2*>(P.o_part + (si * P.mpp + hh) * kHeadDim + lane * 4);
-                const uint32_t lo = raw.x;
-                const uint32_t hi = raw.y;
-                a0 += wi * act_lo<FP16>(lo);
-                a1 += wi * act_hi<FP16>(lo);
-                a2 += wi * act_lo<FP16>(hi);
-                a3 += wi * act_hi<FP16>(hi);
-            }
-        }
-        uint2 o;
-        o.x = pack_act<FP16>(a0, a1);
-        o.y = pack_act<FP16>(a2, a3);
-        *reinterpret_cast<uint2*>(P.out + (static_cast<int64_t>(b) * P.S + q) * (static_cast<int64_t>(P.Hq) * kHeadDim) +
-                                  static_cast<int64_t>(h) * kHeadDim + lane * 4) = o;
-    }
-}
-
-// Wide form for Hq/Hp <= 8, two kernels.  The partial rows of all main heads of one edge are contiguous (mpp * 256
-// bytes), so a warp reads them with 16-byte loads per lane in sweeps of 512 bytes.
+// Two kernels.  The partial rows of all main heads of one edge are contiguous (mpp * 256 bytes), so a warp reads them with
+// 16-byte loads per lane in sweeps of 512 bytes.  With more than eight main heads per proxy head blockIdx.y takes groups of
+// heads, each a contiguous piece of the record, so that the loads stay as wide and as deep as below (one head at a time with
+// 8-byte loads, Hq/Hp = 12, 96 edges per row, B=1 S=16384 Hq=24: 3.26 ms; groups of six heads: 1.31 + 0.13 ms).
 //   combine_lse_kernel   one thread per (query row, edge): loads the (max, sum) pairs of all heads of its edge at once,
 //                        merges them across the row's lanes and writes the row's log-sum-exp per head (and the proxy's).
 //   combine_rows_kernel  one warp per query row: an edge's weight exp2(m_edge - m_row) / l_row equals
@@ -729,7 +650,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineParams P) {
 //                        edges are in flight before the first sum.
 // As one kernel (statistics, then weights through shared memory, then the rows) the same work took 0.443 ms at B=2,
 // S=8192, Hq=32, top-k 16 blocks on a B200; the two kernels take 0.062 + 0.338 ms.
-constexpr int kWideMaxHeads = 8;
+constexpr int kWideMaxHeads = 8;   // largest Hq/Hp one block of the row kernel takes
 
 // Slot (record number inside the partial buffers of this pass) of edge `s` of query row (bp, q), or -1.
 template <bool DENSE>
@@ -766,7 +687,8 @@ __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P)
     const CombineRow<DENSE> row(P, valid ? w0 : nrows - 1);
     const int lse_stride = P.mpp + 1;
     const float2* stats = reinterpret_cast<const float2*>(P.lse_part);
-    const int nheads = P.mpp + (P.lse_proxy ? 1 : 0);
+    const int h0 = blockIdx.y * kMaxHeads;   // first head of this block's group; head number mpp is the proxy
+    const int nheads = min(kMaxHeads, P.mpp + (P.lse_proxy ? 1 : 0) - h0);
     float hm[kMaxHeads], hs[kMaxHeads];
 #pragma unroll
     for (int hh = 0; hh < kMaxHeads; ++hh) {
@@ -775,7 +697,7 @@ __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P)
     }
     for (int s0 = 0; s0 < row.nslots; s0 += LPR) {
         const int sl = valid ? row.slot_of(P, s0 + l) : -1;
-        const float2* rec = stats + static_cast<int64_t>(sl) * lse_stride;
+        const float2* rec = stats + static_cast<int64_t>(sl) * lse_stride + h0;
 #pragma unroll
         for (int hh = 0; hh < kMaxHeads; ++hh) {
             if (hh < nheads && sl >= 0) {
@@ -799,14 +721,16 @@ __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P)
             for (int off = LPR / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
             if (l == 0 && valid) {
                 const float total = (m + __log2f(sum)) * kLn2;   // natural-log LSE of the whole row
-                if (hh == P.mpp) P.lse_proxy[row.bp * P.S + row.q] = total;
-                else P.lse[(static_cast<int64_t>(row.b) * P.Hq + row.p * P.mpp + hh) * P.S + row.q] = total;
+                if (h0 + hh == P.mpp) P.lse_proxy[row.bp * P.S + row.q] = total;
+                else P.lse[(static_cast<int64_t>(row.b) * P.Hq + row.p * P.mpp + h0 + hh) * P.S + row.q] = total;
             }
         }
     }
 }
 
-template <int KITER, bool FP16, bool DENSE>   // Hq/Hp <= 2*KITER: few accumulators, high occupancy (the kernel is bound by memory latency)
+// heads of a group <= 2*KITER: few accumulators, high occupancy (the kernel is bound by memory latency).  Without GROUPED the
+// 64-register budget of four CTAs per SM just holds; the group's offsets would spill there (0.34 -> 0.77 ms at Hq/Hp = 4).
+template <int KITER, bool FP16, bool DENSE, bool GROUPED>
 __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) combine_rows_kernel(const CombineParams P) {
     const int lane = threadIdx.x & 31;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
@@ -814,14 +738,15 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) combine_rows_kernel
     const CombineRow<DENSE> row(P, w);
     const int lse_stride = P.mpp + 1;
     const float2* stats = reinterpret_cast<const float2*>(P.lse_part);
-    const int nchunk = P.mpp * 16;   // lane owns the 16-byte chunks ck = k*32 + lane of the mpp*128-element edge record
+    const int h0 = GROUPED ? blockIdx.y * P.hgroup : 0, hn = GROUPED ? min(P.hgroup, P.mpp - h0) : P.mpp;   // this block's main heads
+    const int nchunk = hn * 16;   // lane owns the 16-byte chunks ck = k*32 + lane of the group's piece of the edge record
     float acc[KITER][8];
     float row_lse2[KITER];   // the row's log-sum-exp of the lane's head in each sweep, in the log2 domain
 #pragma unroll
     for (int k = 0; k < KITER; ++k) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[k][e] = 0.f;
-        const int hh = min((k * 32 + lane) >> 4, P.mpp - 1);
+        const int hh = h0 + min((k * 32 + lane) >> 4, hn - 1);
         row_lse2[k] = P.lse[(static_cast<int64_t>(row.b) * P.Hq + row.p * P.mpp + hh) * P.S + row.q] * kLog2e;
     }
     for (int s0 = 0; s0 < row.nslots; s0 += 32) {
@@ -838,13 +763,13 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) combine_rows_kernel
             float em[4][KITER];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const __nv_bfloat16* rec = P.o_part + static_cast<int64_t>(si[u]) * P.mpp * kHeadDim;
+                const __nv_bfloat16* rec = P.o_part + (static_cast<int64_t>(si[u]) * P.mpp + h0) * kHeadDim;
 #pragma unroll
                 for (int k = 0; k < KITER; ++k) {
                     const int ck = k * 32 + lane;
                     const bool ok = si[u] >= 0 && ck < nchunk;
                     raw[u][k] = ok ? *reinterpret_cast<const uint4*>(rec + ck * 8) : make_uint4(0, 0, 0, 0);
-                    em[u][k] = ok ? stats[static_cast<int64_t>(si[u]) * lse_stride + (ck >> 4)].x : -INFINITY;
+                    em[u][k] = ok ? stats[static_cast<int64_t>(si[u]) * lse_stride + h0 + (ck >> 4)].x : -INFINITY;
                 }
             }
 #pragma unroll
@@ -877,7 +802,7 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) combine_rows_kernel
         }
     }
     __nv_bfloat16* orow = P.out + (static_cast<int64_t>(row.b) * P.S + row.q) * (static_cast<int64_t>(P.Hq) * kHeadDim) +
-                          static_cast<int64_t>(row.p) * P.mpp * kHeadDim;
+                          (static_cast<int64_t>(row.p) * P.mpp + h0) * kHeadDim;
 #pragma unroll
     for (int k = 0; k < KITER; ++k) {
         const int ck = k * 32 + lane;
@@ -987,24 +912,26 @@ extern "C" int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_par
     const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * P.S;
     const int64_t grid = (rows + 7) / 8;
     FMSA_REQUIRE(grid <= 0x7fffffffLL);
-    const dim3 cg(static_cast<unsigned>(grid));
     cudaStream_t cst = static_cast<cudaStream_t>(stream);
     const bool f16 = pb->dtype == FMSA_DTYPE_FP16;
-    if (P.mpp > kWideMaxHeads) {
-        if (f16) combine_kernel<true><<<cg, 256, 0, cst>>>(P);
-        else combine_kernel<false><<<cg, 256, 0, cst>>>(P);
-        return check_launch();
-    }
-    if (dense) combine_lse_kernel<32, true><<<cg, 256, 0, cst>>>(P);
-    else if (P.Kb <= 16) combine_lse_kernel<16, false><<<dim3(static_cast<unsigned>((rows + 15) / 16)), 256, 0, cst>>>(P);
-    else combine_lse_kernel<32, false><<<cg, 256, 0, cst>>>(P);
-#define FMSA_ROWS2(K, F) (dense ? combine_rows_kernel<K, F, true><<<cg, 256, 0, cst>>>(P) : combine_rows_kernel<K, F, false><<<cg, 256, 0, cst>>>(P))
-#define FMSA_ROWS(K) (f16 ? FMSA_ROWS2(K, true) : FMSA_ROWS2(K, false))
-    if (P.mpp <= 2) FMSA_ROWS(1);
-    else if (P.mpp <= 4) FMSA_ROWS(2);
-    else if (P.mpp <= 6) FMSA_ROWS(3);
-    else FMSA_ROWS(4);
-#undef FMSA_ROWS2
+    // Up to eight main heads per proxy head one block takes them all; beyond, groups of (nearly) equal size of at most six
+    // heads: the three-sweep form has its loads in flight without spilling.
+    const int row_groups = P.mpp <= kWideMaxHeads ? 1 : (P.mpp + 5) / 6;
+    P.hgroup = (P.mpp + row_groups - 1) / row_groups;
+    const int lse_groups = (P.mpp + (lse_proxy ? 1 : 0) + kWideMaxHeads) / (kWideMaxHeads + 1);
+    const dim3 cg(static_cast<unsigned>(grid), static_cast<unsigned>(row_groups));
+    const dim3 lg(static_cast<unsigned>(grid), static_cast<unsigned>(lse_groups));
+    if (dense) combine_lse_kernel<32, true><<<lg, 256, 0, cst>>>(P);
+    else if (P.Kb <= 16) combine_lse_kernel<16, false><<<dim3(static_cast<unsigned>((rows + 15) / 16), static_cast<unsigned>(lse_groups)), 256, 0, cst>>>(P);
+    else combine_lse_kernel<32, false><<<lg, 256, 0, cst>>>(P);
+#define FMSA_ROWS3(K, F, G) (dense ? combine_rows_kernel<K, F, true, G><<<cg, 256, 0, cst>>>(P) : combine_rows_kernel<K, F, false, G><<<cg, 256, 0, cst>>>(P))
+#define FMSA_ROWS(K, G) (f16 ? FMSA_ROWS3(K, true, G) : FMSA_ROWS3(K, false, G))
+    if (row_groups > 1) FMSA_ROWS(3, true);
+    else if (P.mpp <= 2) FMSA_ROWS(1, false);
+    else if (P.mpp <= 4) FMSA_ROWS(2, false);
+    else if (P.mpp <= 6) FMSA_ROWS(3, false);
+    else FMSA_ROWS(4, false);
+#undef FMSA_ROWS3
 #undef FMSA_ROWS
     return check_launch();
 }
