@@ -64,20 +64,21 @@ inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int ppk, in
 struct SubUnit {
     int g, j, pp, chunk0;
 };
-__device__ __forceinline__ SubUnit decode_subunit(int64_t u, int NB, int ppk, int C) {
-    const int64_t per_group = subunits_per_group(NB, ppk, C);
+// (32-bit arithmetic: the entry points require fewer than 2^31 sub-units; 64-bit divisions cost kilobytes of code here.)
+__device__ __forceinline__ SubUnit decode_subunit(uint32_t u, int NB, uint32_t ppk, int C, uint32_t per_group) {
     SubUnit su;
     su.g = static_cast<int>(u / per_group);
-    const int64_t r = u % per_group;
+    const uint32_t r = u % per_group;
     su.pp = static_cast<int>(r % ppk);
-    int64_t x = r / ppk;
-    int s = 0;
-    while (x >= NB - s * C) {   // at most NB/C iterations
-        x -= NB - s * C;
-        ++s;
+    int x = static_cast<int>(r / ppk);
+    int left = NB, s = 0;   // key blocks that have a sub-unit s
+    while (x >= left) {   // at most NB/C iterations
+        x -= left;
+        left -= C;
+        s += C;
     }
-    su.j = static_cast<int>(x);
-    su.chunk0 = s * C;
+    su.j = x;
+    su.chunk0 = s;
     return su;
 }
 

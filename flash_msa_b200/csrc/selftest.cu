@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(128) pipeline_selftest_kernel(const __grid_con
     __syncthreads();
     if (ok && tid == 0) {
         tc_fence_after_sync();
-        umma_tile_128_ts<true>(t_d2, t_a2lo, t_a2hi, tile_b, false);
+        umma_ts<4, 8, false>(t_d2, t_a2lo, tile_b, false);
+        umma_ts<4, 8, false>(t_d2, t_a2hi, tile_b + 64 * 128, true);
         if (!withhold) umma_commit(bar_m2);
         tma_store_3d(&tmap_part, tile_st, 0, 1, 0);
         tma_store_3d(&tmap_part, tile_st + kPanelBytes, 64, 1, 0);

@@ -29,6 +29,7 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 // Status words written by kernels into the caller's status buffer (0 = ok).
 constexpr int kStatusWaitTimeout = 1;    // a bounded mbarrier wait gave up
+constexpr int kStatusBadSmem = 3;        // shared or tensor memory does not start where a kernel needs it to
 constexpr int kStatusBadIndex = 2;       // an index read from metadata was out of range
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -101,31 +102,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_
     if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_poll(bar, parity, limit_ns);
 }
-// (Inlined: a kernel that re-divides its registers between warpgroups with setmaxnreg cannot make calls.)
-// Variant for kernels whose roles run decoupled: `abort_flag` is a word in shared memory that any thread sets
-// when one of its waits ran out.  Every other waiter sees it within one parking period and gives up as well,
-// so the whole CTA leaves its loops together instead of each role waiting out its own limit in turn.
-static __device__ __forceinline__ bool mbar_wait_poll_abortable(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    // Kept as small as possible: this loop is inlined at every wait site of the warp-specialised kernels, whose
-    // code has to fit the instruction cache.  The clock and the abort flag are looked at once per 64 parked tries
-    // (a parked try returns after kParkNs at the latest), the time limit is counted in such rounds.
-    uint32_t tries = 0;
-    uint64_t t0 = 0;
-    for (;;) {
-        if (mbar_try_wait_parked(bar, parity, kParkNs)) return true;
-        if ((++tries & 63u) != 0) continue;
-        if (*abort_flag) return false;
-        const uint64_t now = global_timer_ns();
-        if (t0 == 0) t0 = now;
-        if (now - t0 > kWaitLimitNs) {
-            *abort_flag = 1;
-            return false;
-        }
-    }
-}
-__device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+// Variant for the warp-specialised kernels, whose code has to fit the instruction cache: the whole wait is one short loop of
+// parked tries (a kernel that re-divides its registers with setmaxnreg cannot make calls, so every wait site carries it).
+// Bounded by the number of tries, at most kRoleWaitTries * kRoleParkNs = 2 s of waiting; false when it gives up.  A role
+// whose wait gave up stops taking work and signalling, so the others give up in the same way and the CTA leaves together.
+// (With the clock and a CTA-wide flag looked at in the loop the waits of the backward kernel took 27 KB of code.)
+constexpr uint32_t kRoleParkNs = 20000, kRoleWaitTries = 100000;
+__device__ __forceinline__ bool mbar_wait_role(uint32_t bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
-    return mbar_wait_poll_abortable(bar, parity, abort_flag);
+#pragma unroll 1
+    for (uint32_t n = 0; n < kRoleWaitTries; ++n)
+        if (mbar_try_wait_parked(bar, parity, kRoleParkNs)) return true;
+    return false;
 }
 
 // Re-division of the register file between the warpgroups of a CTA (all four warps of a warpgroup execute it).
@@ -193,73 +181,84 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile, int ks) {
     return umma_desc(tile + ks * 2048, kPanelBytes, 1024);
 }
 
-// `elect` != 0 selects the lane that really issues.  The predicate sits inside the instruction so
-// that a whole warp can run the issue sequence without diverging: a lone lane that branches away
-// from its warp after a block barrier was measured to be scheduled thousands of cycles late.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate, uint32_t elect = 1u) {
+// True in one lane of a converged warp.  The issuing warp runs its loop with all lanes and enters a branch on this around
+// every product: the compiler then knows that one thread issues, and moves the descriptors to the uniform registers that
+// tcgen05.mma takes them from once.  (With the whole warp executing instructions predicated on `lane == 0` it cannot know
+// that the operands of the active lanes agree: measured alone 55-60 issue cycles per instruction against the 48 that a
+// 128 x 64 x 16 step occupies the tensor core, and several times that beside busy warps of the same scheduler.)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
     asm volatile(
         "{\n"
-        ".reg .pred p, q;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "setp.ne.b32 q, %5, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elect)
-        : "memory");
+        ".reg .pred P;\n"
+        "elect.sync _|P, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, P;\n"
+        "}\n"
+        : "=r"(p));
+    return p != 0;
 }
 // Arrives once on `bar` when every tcgen05.mma issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t elect = 1u) {
-    asm volatile(
-        "{\n"
-        ".reg .pred q;\n"
-        "setp.ne.b32 q, %1, 0;\n"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-        "}\n" ::"r"(bar),
-        "r"(elect)
-        : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// One full 128x128x128 product D (+)= A * B^T issued by the calling thread (8 instructions).
-// The descriptors of the eight reduction steps differ from the first one only in the 14-bit
+// The descriptors of the reduction steps (16 elements each) of a tile differ from the first one only in the 14-bit
 // address field (a tile lies below 256 KB, so the field never carries): K-major steps advance by
 // 32 bytes inside a panel and jump to the second panel after four steps; MN-major steps advance
-// by 16 rows = 2048 bytes.  Adding the encoded step to the low word keeps the issue loop at a few
-// instructions per MMA, which matters because a single thread feeds the tensor core.
+// by 16 rows = 2048 bytes.
 __host__ __device__ constexpr uint32_t umma_kstep(bool mn_major, int ks) {
     return mn_major ? static_cast<uint32_t>(ks) * (2048u >> 4)
                     : static_cast<uint32_t>(ks >> 2) * (kPanelBytes >> 4) + static_cast<uint32_t>(ks & 3) * 2u;
 }
-// The eight instructions sit in ONE asm block (two predicate set-ups and two 64-bit adds per step with
-// immediate step sizes), so the issuing warp spends as few issue slots per MMA as possible.
-template <bool A_MN, bool B_MN, bool FP16 = false>
-__device__ __forceinline__ void umma_tile_128(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, bool accumulate,
-                                              uint32_t elect = 1u) {
-    constexpr uint32_t idesc = umma_idesc(128, A_MN, B_MN, FP16);
+// D[128 x N] (+)= A[128 x 16*STEPS] * B^T, both operands in shared memory; issued by the calling thread.  A half tile as B:
+// 64 rows of a K-major tile (N = 64), 64 columns (one panel) of an MN-major one (N = 64), given by the address of the half.
+template <int N, int STEPS, bool A_MN, bool B_MN, bool FP16>
+__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, bool accumulate) {
+    constexpr uint32_t idesc = umma_idesc(N, A_MN, B_MN, FP16);
     const uint64_t a0 = A_MN ? desc_mnmajor(a_tile, 0) : desc_kmajor(a_tile, 0);
     const uint64_t b0 = B_MN ? desc_mnmajor(b_tile, 0) : desc_kmajor(b_tile, 0);
-#define FMSA_UMMA_STEP(AI, BI)                                                  \
-    "add.s64 a, %1, " #AI ";\n"                                                 \
-    "add.s64 b, %2, " #BI ";\n"                                                 \
-    "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n"
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q, t;\n"
-        ".reg .b64 a, b;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "setp.ne.b32 q, %5, 0;\n"
-        "setp.eq.b32 t, %5, %5;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        FMSA_UMMA_STEP(%6, %13) FMSA_UMMA_STEP(%7, %14) FMSA_UMMA_STEP(%8, %15) FMSA_UMMA_STEP(%9, %16)
-        FMSA_UMMA_STEP(%10, %17) FMSA_UMMA_STEP(%11, %18) FMSA_UMMA_STEP(%12, %19)
-        "}\n" ::"r"(d_tmem),
-        "l"(a0), "l"(b0), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(elect),
-        "n"(umma_kstep(A_MN, 1)), "n"(umma_kstep(A_MN, 2)), "n"(umma_kstep(A_MN, 3)), "n"(umma_kstep(A_MN, 4)),
-        "n"(umma_kstep(A_MN, 5)), "n"(umma_kstep(A_MN, 6)), "n"(umma_kstep(A_MN, 7)),
-        "n"(umma_kstep(B_MN, 1)), "n"(umma_kstep(B_MN, 2)), "n"(umma_kstep(B_MN, 3)), "n"(umma_kstep(B_MN, 4)),
-        "n"(umma_kstep(B_MN, 5)), "n"(umma_kstep(B_MN, 6)), "n"(umma_kstep(B_MN, 7))
-        : "memory");
-#undef FMSA_UMMA_STEP
+    const uint32_t a_lo = static_cast<uint32_t>(a0), b_lo = static_cast<uint32_t>(b0), a_hi = static_cast<uint32_t>(a0 >> 32), b_hi = static_cast<uint32_t>(b0 >> 32);
+#pragma unroll
+    for (int ks = 0; ks < STEPS; ++ks)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            ".reg .b64 a, b;\n"
+            "mov.b64 a, {%1, %2};\n"
+            "mov.b64 b, {%3, %4};\n"
+            "setp.ne.b32 p, %6, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n"
+            "}\n" ::"r"(d_tmem),
+            "r"(a_lo + umma_kstep(A_MN, ks)), "r"(a_hi), "r"(b_lo + umma_kstep(B_MN, ks)), "r"(b_hi), "r"(idesc),
+            "r"(ks > 0 || accumulate ? 1u : 0u)
+            : "memory");
+}
+template <bool A_MN, bool B_MN, bool FP16 = false>
+__device__ __forceinline__ void umma_tile_128(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, bool accumulate) {
+    umma_ss<128, 8, A_MN, B_MN, FP16>(d_tmem, a_tile, b_tile, accumulate);
+}
+
+// The A operand in TMEM ("TS" form): D[128 x 128] (+)= A[128 x 16*STEPS] * B.  Row m of A lives in TMEM lane m; a 32-bit
+// column holds two consecutive reduction elements (the even one in the low half), so a step reads 8 columns; step i of A
+// starts at column a + ASTRIDE * i (8: contiguous; 16: interleaved with another operand).  B is used MN-major: its rows are
+// the reduction index.
+template <int STEPS, int ASTRIDE, bool FP16>
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a, uint32_t b_tile, bool accumulate) {
+    constexpr uint32_t idesc = umma_idesc(128, false, true, FP16);
+    const uint64_t b0 = desc_mnmajor(b_tile, 0);
+    const uint32_t b_lo = static_cast<uint32_t>(b0), b_hi = static_cast<uint32_t>(b0 >> 32);
+#pragma unroll
+    for (int ks = 0; ks < STEPS; ++ks)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            ".reg .b64 b;\n"
+            "mov.b64 b, {%2, %3};\n"
+            "setp.ne.b32 p, %5, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n"
+            "}\n" ::"r"(d_tmem),
+            "r"(a + ASTRIDE * ks), "r"(b_lo + umma_kstep(true, ks)), "r"(b_hi), "r"(idesc), "r"(ks > 0 || accumulate ? 1u : 0u)
+            : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -319,41 +318,25 @@ __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// ---------------------------------------------------------------------------------------------
-// tcgen05.mma with the A operand in TMEM ("TS" form): D[128 x 128] (+)= A[128 x 128] * B^T.
-// A is a 128 x 128 bf16 matrix whose row m lives in TMEM lane m; a 32-bit column holds the two
-// consecutive reduction elements (2c, 2c+1), the even one in the low half, so the whole operand
-// takes 64 columns and one instruction (16 reduction elements) reads 8 of them.  The operand may
-// be split: `a_lo` is the TMEM address of reduction elements 0..63 (32 columns), `a_hi` that of
-// elements 64..127.  B is a shared-memory tile as in umma_tile_128.
-// ---------------------------------------------------------------------------------------------
-template <bool B_MN, bool FP16 = false>
-__device__ __forceinline__ void umma_tile_128_ts(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_tile,
-                                                 bool accumulate, uint32_t elect = 1u) {
-    constexpr uint32_t idesc = umma_idesc(128, false, B_MN, FP16);
-    const uint64_t b0 = B_MN ? desc_mnmajor(b_tile, 0) : desc_kmajor(b_tile, 0);
-#define FMSA_UMMA_TS_STEP(AREG, AOFF, BI)                                       \
-    "add.u32 a, " #AREG ", " #AOFF ";\n"                                        \
-    "add.s64 b, %3, " #BI ";\n"                                                 \
-    "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
+// Transposing read-out of an accumulator: tcgen05.ld.16x256b gives thread i of the warp, for 16 lanes starting at the
+// address's lane and 64 columns, the values of lane i/4 (registers 4j, 4j+1) and of lane i/4 + 8 (4j+2, 4j+3) in columns
+// 8j + 2*(i%4) and the next one: the layout in which stmatrix stores 8x8 blocks of 16-bit pairs, transposed if asked to.
+__device__ __forceinline__ void tmem_ld_16x256_x8(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
-        "{\n"
-        ".reg .pred p, q, t;\n"
-        ".reg .b64 b;\n"
-        ".reg .b32 a;\n"
-        "setp.ne.b32 p, %5, 0;\n"
-        "setp.ne.b32 q, %6, 0;\n"
-        "setp.eq.b32 t, %6, %6;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %3, %4, p;\n"
-        FMSA_UMMA_TS_STEP(%1, 8, %7) FMSA_UMMA_TS_STEP(%1, 16, %8) FMSA_UMMA_TS_STEP(%1, 24, %9)
-        FMSA_UMMA_TS_STEP(%2, 0, %10) FMSA_UMMA_TS_STEP(%2, 8, %11) FMSA_UMMA_TS_STEP(%2, 16, %12)
-        FMSA_UMMA_TS_STEP(%2, 24, %13)
-        "}\n" ::"r"(d_tmem),
-        "r"(a_lo), "r"(a_hi), "l"(b0), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(elect),
-        "n"(umma_kstep(B_MN, 1)), "n"(umma_kstep(B_MN, 2)), "n"(umma_kstep(B_MN, 3)), "n"(umma_kstep(B_MN, 4)),
-        "n"(umma_kstep(B_MN, 5)), "n"(umma_kstep(B_MN, 6)), "n"(umma_kstep(B_MN, 7))
+        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
         : "memory");
-#undef FMSA_UMMA_TS_STEP
+}
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
+                 "r"(d)
+                 : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -565,6 +548,11 @@ __device__ __forceinline__ void store_transposed_bf16_16(__nv_bfloat16* dst, int
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");

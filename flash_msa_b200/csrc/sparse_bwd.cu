@@ -44,9 +44,9 @@ __device__ unsigned long long g_bwd_trace[20][8];
 
 struct BwdParams {
     // Row-gather views: element row (b, h, s) of q / d_out / q_proxy is matrix row b*row_b + h*row_h + s*row_s.
-    int64_t q_row_b, q_row_h, q_row_s;
-    int64_t do_row_b, do_row_h, do_row_s;
-    int64_t qp_row_b, qp_row_h, qp_row_s;
+    int32_t q_row_b, q_row_h, q_row_s;
+    int32_t do_row_b, do_row_h, do_row_s;
+    int32_t qp_row_b, qp_row_h, qp_row_s;
     int32_t q_rows_total, do_rows_total, qp_rows_total;   // first row index outside each view (reads as zeros)
     const float *lse, *lse_proxy, *delta;   // [B,Hq,S], [B,Hp,S], [B,Hq,S]
     const int32_t* row_ptr;
@@ -62,9 +62,10 @@ struct BwdParams {
     int32_t* status;
     int S, NB, Hq, Hkv, Hp, Hpkv, mpp, ppk, pg;
     int g_begin, G;
-    int64_t n_subunits;
+    int32_t n_subunits;
+    uint32_t units_per_group;
     int chunks;             // chunks per sub-unit
-    int with_kl, dense;
+    int dense;
     float scale_log2e;
     float* kl_value;        // optional: += KL(teacher || proxy) summed over this launch's rows, / (B*Hp*S)
     float kl_value_scale;   // ln(2) / (B*Hp*S)
@@ -78,6 +79,7 @@ struct BwdUnit {   // (kept small: the control block shares the last 3 KB of sha
 };
 
 constexpr int kBwdUnitRing = 8;
+constexpr int kReads = 0, kDraws = 1, kOneThread = 2;   // how a role takes part in the common sequence of sub-units
 
 // Per-tile facts about the 128 gathered query rows (= TMEM columns), staged for the compute groups.
 struct alignas(16) BwdRowStats {   // (filled and read with 16-byte vector accesses)
@@ -85,18 +87,19 @@ struct alignas(16) BwdRowStats {   // (filled and read with 16-byte vector acces
     float neg_delta[128];  // -delta
     uint8_t limit[128];    // last visible key of the row inside this key block (127 = all)
     uint8_t low[128];      // first visible key (0 = all, 128 = none): document masking; written only with documents
-    int32_t any_low;       // some row of the tile has low > 0
 };
 
 struct BwdCtrl {
-    uint64_t k_full, v_full, kv_empty, acc_full, acc_free;
-    uint64_t q_full[2], q_empty[2], do_full[2], do_empty[2], st_full[2], st_empty[2];
-    uint64_t sdp_full, pds_full, dq_full, r0_free, ds_free, dkp_full, r1_free;
+    uint64_t kv_full, kv_empty, acc_full, acc_free;
+    uint64_t qdo_full[2][2], qdo_empty[2][2];    // [stage][half]
+    uint64_t st_full[2], st_empty[2];
+    uint64_t sdp_full[2], pds_full[2], dq_full[2], dq_free[2], ds_free[2];   // [half]
+    uint64_t dkp_full, dkp_free;
     uint64_t unit_full[kBwdUnitRing];
     BwdUnit units[kBwdUnitRing];
     BwdRowStats stats[2];
+    int32_t any_low[2];          // some row of the tile has low > 0 (document masking)
     uint32_t tmem_slot;
-    int32_t abort_flag;
 };
 
 // Roles (warp index): 0-3 compute group A (queries 0..63 of a tile), 4-7 compute group B (queries 64..127),
@@ -116,24 +119,28 @@ static_assert(kBwdRegsLaunch == (65536 / kBwdThreads) / 8 * 8, "registers per th
 constexpr size_t kBwdTileBytes = 7 * static_cast<size_t>(kTileBytes);   // K, V, Q x2, dO x2, dS^T
 constexpr size_t kBwdSmemBytes = 232448;                                 // everything a CTA can have
 static_assert(kBwdTileBytes + sizeof(BwdCtrl) <= kBwdSmemBytes, "shared memory budget of one CTA");
-constexpr int kStatusBadSmem = 3;   // the dynamic shared memory window does not start on a 1024-byte boundary
+constexpr uint32_t kHalfRowBytes = 64 * 128;   // rows 64.. of a panel: where half 1 of a gathered tile starts
 
 // Warp-specialised backward.  Every role walks the same sequence of sub-units (published by the gather warp in a
-// ring) and of tiles.  TMEM (512 columns):
-//   R0 [0,128)   S^T, overwritten in place by P^T (bf16: queries 0..63 in columns 0..31, queries 64..127 in columns
-//                64..95), then dQ (lane = query).  Proxy tile: Sp^T, dSp^T parked in place, then dQp.
-//   R1 [128,256) dP^T, overwritten by dS^T in the same split.  Proxy tile: dKp^T (lane = head dimension).
+// ring) and of tiles.  A tile is worked on as two halves of 64 queries, x = 0 and 1, that take turns on the tensor core:
+// while the compute group of one half turns S^T, dP^T into P^T, dS^T, the products of the other half run.  TMEM (512 columns):
+//   Rx [128x, 128x+128), x = 0, 1: columns 0..63 S^T of the half, overwritten in place by P^T and dS^T (16 bit; 16 queries
+//                at a time: 8 columns of P^T, then 8 of dS^T); columns 64..127 dP^T, then dQ^T (lane = head dimension).
 //   R2 [256,384) dV, R3 [384,512) dK (lane = key), accumulated over the sub-unit.
-// Issue order of a main tile t (one full product always lies between a product that reads a TMEM operand and a
-// later one that overwrites those columns):
-//   [compute(t) done]  dV += P^T dO,  dK += dS^T Q,  dQ = dS K -> R0,  dP^T(t+1) -> R1,  [dQ read out]  S^T(t+1) -> R0.
-// Hand-offs (mbarriers; one arrival per warp or per tcgen05.commit): q_full/do_full (TMA bytes) <- q_empty/do_empty;
-// st_full <- st_empty (row statistics); sdp_full (S^T and dP^T of a tile), pds_full (P^T, dS^T written), dq_full,
-// r0_free (dQ read out), ds_free (the dS^T tile, which doubles as the staging tile of the dQ store, is reusable),
-// dkp_full / r1_free (proxy tile), acc_full / acc_free (dV, dK flushed at the end of a sub-unit).
+//   Proxy tile: Sp^T in columns 0..63 of both Rx; then dKp^T (lane = head dimension) takes R0, dQp^T of the halves R1.
+// A step of the issuing warp (half x of main tile t), behind P^T / dS^T of that half:
+//   dQ^T = K^T dS^T -> Rx+64,  dV += P^T dO,  dK += dS^T Q,  S^T(t+1) = K Q^T -> Rx,  [dQ^T read out]  dP^T(t+1) = V dO^T -> Rx+64
+// so dQ^T is read out under three products, and everything half x needs for tile t+1 is under way before the step of the
+// other half begins.  (As one 128-query tile whose products, arithmetic and hand-offs followed one another, a tile took 8.1 k
+// cycles, 4.0 k of them products: S^T, dP^T, dV and dK of 128 queries fill the 512 columns, and nothing of the next tile
+// could start before dQ had been read out.)
+// Hand-offs (mbarriers; one arrival per warp or per tcgen05.commit): qdo_full (TMA bytes) <- qdo_empty; st_full <- st_empty
+// (row statistics); sdp_full (S^T and dP^T of a half), pds_full (P^T, dS^T written), dq_full -> dq_free (dQ^T read out),
+// ds_free (the half's panel of the dS^T tile, which doubles as the staging tile of its dQ store, is reusable),
+// dkp_full / dkp_free (proxy tile), acc_full / acc_free (dV, dK flushed at the end of a sub-unit).
 // VARLEN: document masking of packed sequences (P.doc_start given).  A separate instantiation, so that the plain kernel
 // carries none of its registers or code.
-template <bool FP16, bool VARLEN>
+template <bool FP16, bool VARLEN, bool KL>
 __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
                                                                     const __grid_constant__ CUtensorMap tmap_do,
                                                                     const __grid_constant__ CUtensorMap tmap_qp,
@@ -156,39 +163,36 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;   // TMEM lane of this thread: key (compute, dKp/dV/dK read-out) or query (dQ read-out)
-    const uint32_t elect = (lane == 0) ? 1u : 0u;
     auto BAR = [&](uint64_t& b) { return smem_u32(&b); };
 
     if (tid == 0) {
-        mbar_init(BAR(sm->k_full), 1);
-        mbar_init(BAR(sm->v_full), 1);
+        mbar_init(BAR(sm->kv_full), 1);
         mbar_init(BAR(sm->kv_empty), 1);
         mbar_init(BAR(sm->acc_full), 1);
         mbar_init(BAR(sm->acc_free), 4);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(BAR(sm->q_full[i]), kBwdGatherWarps);
-            mbar_init(BAR(sm->q_empty[i]), 1);
-            mbar_init(BAR(sm->do_full[i]), kBwdGatherWarps);
-            mbar_init(BAR(sm->do_empty[i]), 1);
+            for (int x = 0; x < 2; ++x) {
+                mbar_init(BAR(sm->qdo_full[i][x]), kBwdGatherWarps / 2);
+                mbar_init(BAR(sm->qdo_empty[i][x]), 1);
+            }
             mbar_init(BAR(sm->st_full[i]), 1);
             mbar_init(BAR(sm->st_empty[i]), 8);
+            mbar_init(BAR(sm->sdp_full[i]), 1);
+            mbar_init(BAR(sm->pds_full[i]), 8);
+            mbar_init(BAR(sm->dq_full[i]), 1);
+            mbar_init(BAR(sm->dq_free[i]), 4);
+            mbar_init(BAR(sm->ds_free[i]), 1);
         }
-        mbar_init(BAR(sm->sdp_full), 1);
-        mbar_init(BAR(sm->pds_full), 8);
-        mbar_init(BAR(sm->dq_full), 1);
-        mbar_init(BAR(sm->r0_free), 4);
-        mbar_init(BAR(sm->ds_free), 1);
         mbar_init(BAR(sm->dkp_full), 1);
-        mbar_init(BAR(sm->r1_free), 4);
+        mbar_init(BAR(sm->dkp_free), 4);
         for (int i = 0; i < kBwdUnitRing; ++i) mbar_init(BAR(sm->unit_full[i]), 1);
-        sm->abort_flag = 0;
         fence_mbar_init();
         prefetch_tmap(&tmap_q);
         prefetch_tmap(&tmap_do);
         prefetch_tmap(&tmap_k);
         prefetch_tmap(&tmap_v);
         prefetch_tmap(&tmap_dq);
-        if (P.with_kl) {
+        if (KL) {
             prefetch_tmap(&tmap_qp);
             prefetch_tmap(&tmap_kp);
             prefetch_tmap(&tmap_dqp);
@@ -201,13 +205,19 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = sm->tmem_slot;
-    const uint32_t r0 = tmem, r1 = tmem + 128, r2 = tmem + 256, r3 = tmem + 384;
+    // All 512 columns are this CTA's, so the allocation starts at column 0 and every TMEM address is a constant.
+    constexpr uint32_t tmem = 0;
+    if (sm->tmem_slot != tmem) {
+        if (tid == 0) atomicMax(P.status, kStatusBadSmem);
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);
+        return;
+    }
+    const uint32_t r0 = tmem, r1 = tmem + 128, r2 = tmem + 256, r3 = tmem + 384;   // (Rx = tmem + 128 * x)
 
-    const int hpc = P.mpp + (P.with_kl ? 1 : 0);   // tiles per chunk
+    const int hpc = P.mpp + (KL ? 1 : 0);   // tiles per chunk
     const int64_t edge_base = P.dense ? dense_edge_base(static_cast<int64_t>(P.g_begin) * P.ppk, P.S, P.NB)
                                       : static_cast<int64_t>(P.row_ptr[static_cast<int64_t>(P.g_begin) * P.ppk * P.NB]);
-    volatile int* abort_flag = &sm->abort_flag;
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
 #ifdef FMSA_TRACE
     unsigned long long trace_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -217,11 +227,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
 #ifdef FMSA_TRACE
         const long long w0 = clock64();
 #endif
-        if (!bad) bad = __any_sync(0xffffffffu, !mbar_wait_abortable(bar, parity, abort_flag));
+        if (!bad) bad = __any_sync(0xffffffffu, !mbar_wait_role(bar, parity));
 #ifdef FMSA_TRACE
         trace_acc[kind & 7] += static_cast<unsigned long long>(clock64() - w0);
 #endif
         (void)kind;
+    };
+    auto wait1 = [&](uint32_t bar, uint32_t parity) {   // the same in a role that a single thread runs
+        if (!bad) bad = !mbar_wait_role(bar, parity);
     };
     auto group_or = [&](int id, bool flag) -> bool {   // 128-thread barrier that also ORs a flag
         uint32_t r;
@@ -251,17 +264,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     // work and publishes the decoded sub-unit; it passes over sub-units that lie beyond the end of their row, so
     // every published entry has work (or is the end marker).  The roles are at most a few tiles apart, fewer than the
     // ring has entries.
-    auto next_unit = [&](uint32_t draw, BwdUnit& ud, auto may_draw) -> bool {
+    auto next_unit = [&](uint32_t draw, BwdUnit& ud, auto mode) -> bool {
         const uint32_t uslot = draw & (kBwdUnitRing - 1);
-        if (decltype(may_draw)::value && warp == 12 && lane == 0) {
+        if (decltype(mode)::value == kDraws && warp == 12 && lane == 0) {
             BwdUnit nu;
             nu.chunk1 = -1;
             for (;;) {
-                const int64_t u = atomicAdd(P.counter, 1);
-                if (u >= P.n_subunits) break;
-                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks);
-                const int g = P.g_begin + su.g;
-                const int b = g / P.Hkv, kvh = g % P.Hkv, p = kvh * P.ppk + su.pp;
+                const uint32_t u = static_cast<uint32_t>(atomicAdd(P.counter, 1));
+                if (u >= static_cast<uint32_t>(P.n_subunits)) break;
+                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks, P.units_per_group);
+                const uint32_t g = P.g_begin + su.g;
+                const int b = g / static_cast<uint32_t>(P.Hkv), kvh = g % static_cast<uint32_t>(P.Hkv), p = kvh * P.ppk + su.pp;
                 const int64_t bp = static_cast<int64_t>(b) * P.Hp + p;
                 int64_t e0;
                 int n;
@@ -283,7 +296,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
             sm->units[uslot] = nu;
             mbar_arrive(BAR(sm->unit_full[uslot]));
         }
-        wait(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1, 7);
+        if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1);
+        else wait(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1, 7);
         if (warp >= 8 && warp < 12) bad = group_or(1, bad);
         if (bad) return false;
         ud = sm->units[uslot];
@@ -304,83 +318,119 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     // allocation of one role from being charged with the live values of the others).
     if (warp >= 16) {
         reg_dec<kBwdRegsMisc>();
-        if (warp == 17) {
+        if (warp == 17 && elect_one()) {
             // =========================== MMA issue ===========================
+            // One thread runs the whole role.  The tensor core holds a handful of instructions that have not started, i.e.
+            // about 200 cycles of work: whatever the issuing thread does between two products in more than that is time the
+            // tensor core stands still, so barriers are looked at before the product that precedes their use is issued.
             BwdUnit ud;
-            for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
+            for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kOneThread>{}); ++draw, ++nsub) {
                 const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
-                wait(BAR(sm->k_full), nsub & 1, 6);
-                wait(BAR(sm->v_full), nsub & 1, 6);
-                // S^T and dP^T of tile g (running index), whose predecessor was tile g-1
-                auto issue_front = [&](uint32_t g, bool proxy, bool prev_proxy) {
-                    const uint32_t s = g & 1, ph = (g >> 1) & 1;
-                    const uint32_t tq = tile_q0 + s * kTileBytes, tdo = tile_do0 + s * kTileBytes;
-                    wait(BAR(sm->do_full[s]), ph, 1);
-                    if (!proxy) {
-                        if (g >= 1 && prev_proxy) wait(BAR(sm->r1_free), (pt - 1) & 1, 4);   // dKp has been read out of R1
+                const int last_main = 2 * (ntiles - (KL ? 1 : 0)) - 1;   // step of the last half that uses K and V
+                wait1(BAR(sm->kv_full), nsub & 1);
+                // One step per half tile: the products of (tile t, half x), then the front of the next tile (S^T and dP^T) for
+                // the halves whose regions they free: that half after a main tile, both at once behind the second step of a
+                // proxy tile and at the start (u = -1).
+                int hh = KL ? P.mpp : 0;      // head of tile t; before the first tile the last head of the previous sub-unit
+                int hh1 = 0;                         // head of tile t + 1
+                bool pds_ready = false;              // the next step's operands have been seen written
+#pragma unroll 1
+                for (int u = -1; u < 2 * ntiles && !bad; ++u) {
+                    const int x = u & 1;
+                    const bool is_proxy = KL && hh == P.mpp;
+                    const uint32_t rx = tmem + 128 * x;
+                    if (u >= 0) {
+                        const uint32_t s = gt & 1;
+                        const uint32_t tq = tile_q0 + s * kTileBytes, tdo = tile_do0 + s * kTileBytes;
+                        if (is_proxy && x == 0) {
+                            // (the front of a proxy tile does not wait for the dQ^T of the main tile before it)
+                            wait1(BAR(sm->dq_free[0]), (gt - 1) & 1);
+                            wait1(BAR(sm->dq_free[1]), (gt - 1) & 1);
+                            wait1(BAR(sm->pds_full[1]), gt & 1);
+                        }
+                        if (!pds_ready && (!is_proxy || x == 0)) wait1(BAR(sm->pds_full[x]), gt & 1);
+                        if (bad) break;
                         tc_fence_after_sync();
-                        if (!bad) umma_tile_128<false, false, FP16>(r1, tile_v, tdo, false, elect);   // dP^T = V_j dO_g^T
-                    }
-                    wait(BAR(sm->q_full[s]), ph, 2);
-                    if (g >= 1) wait(BAR(sm->r0_free), (g - 1) & 1, 3);                       // dQ / dQp has been read out of R0
-                    tc_fence_after_sync();
-                    if (!bad) {
-                        umma_tile_128<false, false, FP16>(r0, proxy ? tdo : tile_k, tq, false, elect);   // S^T = K_j Q_g^T  (Sp^T = Kp_j Qp_g^T)
-                        umma_commit(BAR(sm->sdp_full), elect);
-                    }
-                };
-                issue_front(gt, false, P.with_kl != 0);   // (a sub-unit ends with a proxy tile when there are any)
-                int hh = 0;
-                for (int t = 0; t < ntiles && !bad; ++t, ++gt) {
-                    const bool is_proxy = hh == P.mpp;
-                    const uint32_t s = gt & 1;
-                    const uint32_t tq = tile_q0 + s * kTileBytes, tdo = tile_do0 + s * kTileBytes;
-                    int hh1 = hh + 1;
-                    if (hh1 == hpc) hh1 = 0;
-                    wait(BAR(sm->pds_full), gt & 1, 5);
-                    tc_fence_after_sync();
-                    if (!is_proxy) {
-                        if (t == 0 && nsub > 0) wait(BAR(sm->acc_free), (nsub - 1) & 1, 6);   // dV, dK of the previous sub-unit flushed
-                        if (!bad) {
-                            umma_tile_128_ts<true, FP16>(r2, r0, r0 + 64, tdo, t != 0, elect);    // dV += P^T dO_g
-                            umma_commit(BAR(sm->do_empty[s]), elect);
-                            umma_tile_128_ts<true, FP16>(r3, r1, r1 + 64, tq, t != 0, elect);     // dK += dS^T Q_g
-                            umma_commit(BAR(sm->q_empty[s]), elect);
-                            umma_tile_128<true, true, FP16>(r0, tile_ds, tile_k, false, elect);   // dQ = dS K_j
-                            umma_commit(BAR(sm->dq_full), elect);
+                        if (is_proxy && x == 0) {
+                            umma_ss<128, 8, true, false, FP16>(r0, tq, tile_ds, false);   // dKp^T = Qp_g^T dSp
+                            umma_commit(BAR(sm->dkp_full));
                         }
-                    } else {
-                        if (!bad) {
-                            umma_tile_128<true, false, FP16>(r1, tq, tile_ds, false, elect);      // dKp^T = Qp_g^T dSp  (lane = head dim)
-                            umma_commit(BAR(sm->dkp_full), elect);
-                            umma_tile_128<true, true, FP16>(r0, tile_ds, tdo, false, elect);      // dQp = dSp Kp_j
-                            umma_commit(BAR(sm->dq_full), elect);
-                            umma_commit(BAR(sm->q_empty[s]), elect);
-                            umma_commit(BAR(sm->do_empty[s]), elect);
+                        // dQ^T = K_j^T dS^T, dQp^T = Kp_j^T dSp^T
+                        umma_ss<64, 8, true, true, FP16>(is_proxy ? r1 + 64 * x : rx + 64, is_proxy ? tdo : tile_k, tile_ds + x * kPanelBytes, false);
+                        umma_commit(BAR(sm->dq_full[x]));
+                        if (!is_proxy) {
+                            if (u == 0 && nsub > 0) {
+                                wait1(BAR(sm->acc_free), (nsub - 1) & 1);   // dV, dK of the previous sub-unit flushed
+                                if (bad) break;
+                                tc_fence_after_sync();
+                            }
+                            umma_ts<4, 16, FP16>(r2, rx, tdo + x * kHalfRowBytes, u != 0);       // dV += P^T dO_g
+                            umma_ts<4, 16, FP16>(r3, rx + 8, tq + x * kHalfRowBytes, u != 0);    // dK += dS^T Q_g
+                            umma_commit(BAR(sm->qdo_empty[s][x]));
+                            // K and V are done with after the last main tile: they are fetched anew under the proxy tile
+                            if (u == last_main) umma_commit(BAR(sm->kv_empty));
+                        } else if (x == 1) {
+                            umma_commit(BAR(sm->qdo_empty[s][0]));
+                            umma_commit(BAR(sm->qdo_empty[s][1]));
+                            ++pt;
                         }
-                        ++pt;
                     }
-                    if (t + 1 < ntiles) issue_front(gt + 1, hh1 == P.mpp, is_proxy);
-                    hh = hh1;
+                    pds_ready = false;
+                    if (u + 2 < 2 * ntiles) {
+                        // (The waits for a free Rx follow the order in which the output group hands the regions back, so no phase
+                        // of a barrier is passed over.)
+                        const bool both = u < 0 || is_proxy, proxy1 = KL && hh1 == P.mpp;
+                        const uint32_t g = u < 0 ? gt : gt + 1, s = g & 1;
+                        const uint32_t tdo = tile_do0 + s * kTileBytes;
+#pragma unroll 1
+                        for (int fx = both ? 0 : x; fx < (both ? 2 * x : x + 1); ++fx) {
+                            const uint32_t rf = tmem + 128 * fx;
+                            wait1(BAR(sm->qdo_full[s][fx]), (g >> 1) & 1);
+                            if (g >= 1 && is_proxy) {   // R0 held dKp^T, R1 the dQp^T of both halves
+                                wait1(fx == 0 ? BAR(sm->dkp_free) : BAR(sm->dq_free[0]), fx == 0 ? (pt - 1) & 1 : (g - 1) & 1);
+                                if (fx == 1) wait1(BAR(sm->dq_free[1]), (g - 1) & 1);
+                            }
+                            if (bad) break;
+                            tc_fence_after_sync();
+                            // S^T = K_j Q_g^T  (Sp^T = Kp_j Qp_g^T: the proxy keys sit in the dO stage)
+                            umma_ss<64, 8, false, false, FP16>(rf, proxy1 ? tdo : tile_k, tile_q0 + s * kTileBytes + fx * kHalfRowBytes, false);
+                            // the next step is that of the other half (of this tile, or of the next one after a second half)
+                            if (!both && !is_proxy && !(x == 1 && proxy1)) pds_ready = mbar_try_wait(BAR(sm->pds_full[x ^ 1]), (gt + x) & 1);
+                            if (!proxy1) {
+                                if (g >= 1 && !is_proxy) {
+                                    wait1(BAR(sm->dq_free[fx]), (g - 1) & 1);   // dQ^T has been read out
+                                    if (bad) break;
+                                    tc_fence_after_sync();
+                                }
+                                umma_ss<64, 8, false, false, FP16>(rf + 64, tile_v, tdo + fx * kHalfRowBytes, false);   // dP^T = V_j dO_g^T
+                            }
+                            umma_commit(BAR(sm->sdp_full[fx]));
+                        }
+                    }
+                    if (x == 1) {
+                        if (u >= 0) ++gt;
+                        hh = hh1;
+                        if (++hh1 == hpc) hh1 = 0;
+                    }
                 }
-                if (!bad) {
-                    umma_commit(BAR(sm->kv_empty), elect);
-                    umma_commit(BAR(sm->acc_full), elect);
-                }
+                if (!bad) umma_commit(BAR(sm->acc_full));
             }
         } else if (warp == 16) {
             // =========================== K / V loads, row statistics ===========================
             BwdUnit ud;
-            for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
-                const int64_t bp = static_cast<int64_t>(ud.b) * P.Hp + ud.p;
+            for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
                 if (nsub > 0) wait(BAR(sm->kv_empty), (nsub - 1) & 1, 1);
-                if (!bad && lane == 0) {
-                    mbar_arrive_expect_tx(BAR(sm->k_full), kTileBytes);
-                    tma_load_tile(tile_k, &tmap_k, ud.j * kBlock, ud.kvh, ud.b, BAR(sm->k_full));
-                    mbar_arrive_expect_tx(BAR(sm->v_full), kTileBytes);
-                    tma_load_tile(tile_v, &tmap_v, ud.j * kBlock, ud.kvh, ud.b, BAR(sm->v_full));
+                if (!bad && elect_one()) {
+                    mbar_arrive_expect_tx(BAR(sm->kv_full), 2 * kTileBytes);
+#pragma unroll 1
+                    for (int i = 0; i < 4; ++i)   // two panels of K_j, two of V_j
+                        tma_load_4d(tile_k + i * kPanelBytes, i < 2 ? &tmap_k : &tmap_v, (i & 1) * 64, ud.j * kBlock, ud.kvh, ud.b, BAR(sm->kv_full));
                 }
                 __syncwarp();
+                // per main head: -lse * log2 e and -delta of the 128 rows; for the proxy head its -lse * log2 e
+                const int64_t head0 = (static_cast<int64_t>(ud.b) * P.Hq + ud.p * P.mpp) * P.S;
+                const float* proxy_lse = P.lse_proxy + (static_cast<int64_t>(ud.b) * P.Hp + ud.p) * P.S;
+#pragma unroll 1
                 for (int chunk = ud.chunk0; chunk < ud.chunk1 && !bad; ++chunk) {
                     int qid[4];
                     uint32_t lim4 = 0, low4 = 0;
@@ -396,24 +446,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                         }
                     }
                     const bool any_low = VARLEN && __any_sync(0xffffffffu, low4 != 0);
-                    for (int hh = 0; hh < hpc && !bad; ++hh, ++gt) {
+                    const float *lse_row = P.lse + head0, *delta_row = P.delta + head0;
+#pragma unroll 1
+                    for (int hh = 0; hh < hpc; ++hh, ++gt) {
                         const uint32_t s = gt & 1;
-                        const bool proxy = hh == P.mpp;
+                        const bool proxy = KL && hh == P.mpp;
+                        if (proxy) lse_row = proxy_lse;
                         float nl[4], dl[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            nl[i] = -INFINITY;
-                            dl[i] = 0.f;
-                            if (qid[i] >= 0) {
-                                if (proxy) {
-                                    nl[i] = -P.lse_proxy[bp * P.S + qid[i]] * kLog2e;
-                                } else {
-                                    const int64_t at = (static_cast<int64_t>(ud.b) * P.Hq + ud.p * P.mpp + hh) * P.S + qid[i];
-                                    nl[i] = -P.lse[at] * kLog2e;
-                                    dl[i] = -P.delta[at];
-                                }
-                            }
+                            nl[i] = qid[i] >= 0 ? -kLog2e * lse_row[qid[i]] : -INFINITY;
+                            dl[i] = qid[i] >= 0 && !proxy ? -delta_row[qid[i]] : 0.f;
                         }
+                        lse_row += P.S;
+                        delta_row += P.S;
                         if (gt >= 2) wait(BAR(sm->st_empty[s]), ((gt >> 1) - 1) & 1, 2);
                         if (bad) break;
                         BwdRowStats* st = &sm->stats[s];
@@ -422,7 +468,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                         reinterpret_cast<uint32_t*>(st->limit)[lane] = lim4;
                         if (VARLEN) {
                             reinterpret_cast<uint32_t*>(st->low)[lane] = low4;
-                            if (lane == 0) st->any_low = any_low ? 1 : 0;
+                            if (lane == 0) sm->any_low[s] = any_low ? 1 : 0;
                         }
                         warp_arrive(BAR(sm->st_full[s]));
                     }
@@ -432,18 +478,22 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     } else if (warp >= 12) {
         reg_dec<kBwdRegsGather>();
         // =========================== row gather ===========================
-        // Gather warp g fetches rows 32g .. 32g+31 of every tile: lanes 0..15 issue the dO rows (dP^T is issued before
-        // S^T), lanes 16..31 the Q rows; a lane takes row quad (lane/2)%8 and 64-column panel lane%2.  Lane r holds the
-        // query position of row 32g + r.  In a proxy tile the Q stage takes the Qp rows and the dO stage the proxy keys
-        // of the block (one ordinary tile load by the first gather warp).
-        const int g = warp - 12;
+        // Gather warp g fetches rows 32g .. 32g+31 of every tile, i.e. warps 0, 1 half 0 and warps 2, 3 half 1: lanes 0..15
+        // issue the dO rows, lanes 16..31 the Q rows; a lane takes row quad (lane/2)%8 and 64-column panel lane%2.  Lane r
+        // holds the query position of row 32g + r.  In a proxy tile the Q stage takes the Qp rows and the dO stage the proxy
+        // keys of the block (one ordinary tile load by the first gather warp, whose half is consumed first).
+        const int g = warp - 12, half = g >> 1;
         const int quad = (lane >> 1) & 7, panel = lane & 1;
         const bool q_lane = lane >= 16;
+        const int main_row_h = q_lane ? P.q_row_h : P.do_row_h, main_row_s = q_lane ? P.q_row_s : P.do_row_s;
+        const int main_rows_total = q_lane ? P.q_rows_total : P.do_rows_total;
+        const void* main_tmap = q_lane ? static_cast<const void*>(&tmap_q) : static_cast<const void*>(&tmap_do);
         BwdUnit ud;
-        for (uint32_t draw = 0; next_unit(draw, ud, std::true_type{}); ++draw, ++nsub) {
-            const int64_t q_base = static_cast<int64_t>(ud.b) * P.q_row_b + static_cast<int64_t>(ud.p) * P.mpp * P.q_row_h;
-            const int64_t do_base = static_cast<int64_t>(ud.b) * P.do_row_b + static_cast<int64_t>(ud.p) * P.mpp * P.do_row_h;
-            const int64_t qp_base = static_cast<int64_t>(ud.b) * P.qp_row_b + static_cast<int64_t>(ud.p) * P.qp_row_h;
+        for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kDraws>{}); ++draw, ++nsub) {
+            // matrix row of (this lane's tensor, first main head, position 0); row numbers fit 31 bits
+            const int main_base = q_lane ? ud.b * P.q_row_b + ud.p * P.mpp * P.q_row_h : ud.b * P.do_row_b + ud.p * P.mpp * P.do_row_h;
+            const int qp_base = ud.b * P.qp_row_b + ud.p * P.qp_row_h;
+            const int kph = ud.p / P.pg;
             for (int chunk = ud.chunk0; chunk < ud.chunk1 && !bad; ++chunk) {
                 const int q = row_qid(ud, chunk * kBlock + 32 * g + lane);
                 int qr[4];
@@ -451,47 +501,38 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                 for (int i = 0; i < 4; ++i) qr[i] = __shfl_sync(0xffffffffu, q, 4 * quad + i);
                 for (int hh = 0; hh < hpc && !bad; ++hh, ++gt) {
                     const uint32_t s = gt & 1, ph = (gt >> 1) & 1;
-                    const bool proxy = hh == P.mpp;
-                    const uint32_t qf = BAR(sm->q_full[s]), df = BAR(sm->do_full[s]);
+                    const bool proxy = KL && hh == P.mpp;
+                    const uint32_t full = BAR(sm->qdo_full[s][half]);
                     const uint32_t off = panel * kPanelBytes + (32 * g + 4 * quad) * 128;
                     if (gt >= 2) {
-                        wait(BAR(sm->do_empty[s]), ph ^ 1, 1);
-                        wait(BAR(sm->q_empty[s]), ph ^ 1, 2);
+                        wait(BAR(sm->qdo_empty[s][half]), ph ^ 1, 1);
+                        if (proxy && g == 0) wait(BAR(sm->qdo_empty[s][1]), ph ^ 1, 2);   // the keys fill both halves of the stage
                     }
                     if (bad) break;
-                    if (lane == 0) {
-                        mbar_arrive_expect_tx(qf, kTileBytes / kBwdGatherWarps);
+                    if (elect_one()) {
+                        constexpr uint32_t kShare = kTileBytes / kBwdGatherWarps;   // this warp's rows of one tile
                         if (!proxy) {
-                            mbar_arrive_expect_tx(df, kTileBytes / kBwdGatherWarps);
+                            mbar_arrive_expect_tx(full, 2 * kShare);
                         } else if (g == 0) {
-                            mbar_arrive_expect_tx(df, kTileBytes);
-                            tma_load_tile(tile_do0 + s * kTileBytes, &tmap_kp, ud.j * kBlock, ud.p / P.pg, ud.b, df);
+                            mbar_arrive_expect_tx(full, kShare + kTileBytes);
+#pragma unroll 1
+                            for (int i = 0; i < 2; ++i)
+                                tma_load_4d(tile_do0 + s * kTileBytes + i * kPanelBytes, &tmap_kp, i * 64, ud.j * kBlock, kph, ud.b, full);
                         } else {
-                            mbar_arrive(df);
+                            mbar_arrive_expect_tx(full, kShare);
                         }
                     }
                     __syncwarp();
+                    // One issue site for the three tensors: every lane's gather4 goes through the uniform registers by itself, so
+                    // each site is a loop of its own in the code.
+                    const int base = proxy ? qp_base : main_base + hh * main_row_h;
+                    const int rs = proxy ? P.qp_row_s : main_row_s, oob = proxy ? P.qp_rows_total : main_rows_total;
                     int r[4];
-                    if (!q_lane) {
-                        if (!proxy) {
-                            const int64_t base = do_base + static_cast<int64_t>(hh) * P.do_row_h;
 #pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                r[i] = qr[i] >= 0 ? static_cast<int>(base + qr[i] * P.do_row_s) : P.do_rows_total;
-                            tma_gather4(tile_do0 + s * kTileBytes + off, &tmap_do, panel * 64, r[0], r[1], r[2], r[3], df);
-                        }
-                    } else if (proxy) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            r[i] = qr[i] >= 0 ? static_cast<int>(qp_base + qr[i] * P.qp_row_s) : P.qp_rows_total;
-                        tma_gather4(tile_q0 + s * kTileBytes + off, &tmap_qp, panel * 64, r[0], r[1], r[2], r[3], qf);
-                    } else {
-                        const int64_t base = q_base + static_cast<int64_t>(hh) * P.q_row_h;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            r[i] = qr[i] >= 0 ? static_cast<int>(base + qr[i] * P.q_row_s) : P.q_rows_total;
-                        tma_gather4(tile_q0 + s * kTileBytes + off, &tmap_q, panel * 64, r[0], r[1], r[2], r[3], qf);
-                    }
+                    for (int i = 0; i < 4; ++i) r[i] = qr[i] >= 0 ? base + qr[i] * rs : oob;
+                    const uint32_t dst = (q_lane ? tile_q0 : tile_do0) + s * kTileBytes + off;
+                    const void* tm = proxy ? static_cast<const void*>(&tmap_qp) : main_tmap;
+                    if (q_lane || !proxy) tma_gather4(dst, tm, panel * 64, r[0], r[1], r[2], r[3], full);
                 }
             }
         }
@@ -499,111 +540,104 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         reg_dec<kBwdRegsOutput>();
         // =========================== output group ===========================
         const int otid = tid - 8 * 32;
-        // Reads accumulator `acc` (lane = key row of the block) and adds it to the fp32 rows starting at `dst`.
-        auto flush_rows = [&](uint32_t acc, float* dst) {
-            float* drow = dst + static_cast<int64_t>(row) * kHeadDim;
-#pragma unroll 1
-            for (int c = 0; c < 128; c += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem_addr(acc, quarter, c), v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                    red_add_v4(drow + c + i, __uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
-                               __uint_as_float(v[i + 3]));
-            }
-        };
         BwdUnit ud;
-        for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
+        for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
             const int64_t slot_base = ud.e0 - edge_base;
             const int kph = ud.p / P.pg;
             int hh = 0, chunk = ud.chunk0;
             for (int t = 0; t < ntiles && !bad; ++t, ++gt) {
-                const bool is_proxy = hh == P.mpp;
-                const int nrows = min(kBlock, ud.n - chunk * kBlock);
+                const bool is_proxy = KL && hh == P.mpp;
                 const int64_t slot0 = slot_base + static_cast<int64_t>(chunk) * kBlock;
-                const bool full = nrows == kBlock;
                 if (is_proxy) {
                     wait(BAR(sm->dkp_full), pt & 1, 1);
                     if (!bad) {
                         tc_fence_after_sync();
-                        {
-                            // dKp^T: lane = head-dimension index, column = key row: the 32 lanes of a warp add to 32
-                            // consecutive floats of one row per instruction
-                            float* kbase = P.dkp_acc + ((static_cast<int64_t>(ud.b) * P.Hpkv + kph) * P.S + ud.j * kBlock) * kHeadDim + row;
+                        // dKp^T: lane = head-dimension index, column = key row: the 32 lanes of a warp add to 32
+                        // consecutive floats of one row per instruction
+                        float* kbase = P.dkp_acc + ((static_cast<int64_t>(ud.b) * P.Hpkv + kph) * P.S + ud.j * kBlock) * kHeadDim + row;
 #pragma unroll 1
-                            for (int c = 0; c < 128; c += 32) {
-                                uint32_t v[32];
-                                tmem_ld32(tmem_addr(r1, quarter, c), v);
-                                tmem_ld_wait();
+                        for (int c = 0; c < 128; c += 32) {
+                            uint32_t v[32];
+                            tmem_ld32(tmem_addr(r0, quarter, c), v);
+                            tmem_ld_wait();
 #pragma unroll
-                                for (int i = 0; i < 32; ++i) atomicAdd(kbase + static_cast<int64_t>(c + i) * kHeadDim, __uint_as_float(v[i]));
-                            }
+                            for (int i = 0; i < 32; ++i) atomicAdd(kbase + static_cast<int64_t>(c + i) * kHeadDim, __uint_as_float(v[i]));
                         }
                         tc_fence_before_sync();
-                        warp_arrive(BAR(sm->r1_free));
+                        warp_arrive(BAR(sm->dkp_free));
                     }
                     ++pt;
                 }
-                wait(BAR(sm->dq_full), gt & 1, 2);
-                bad = group_or(1, bad);
-                if (bad) break;
-                tc_fence_after_sync();
-                // With `split` the row leaves twice: rounded to bf16, and the remainder of that rounding (a second plane of
-                // the partial buffers, `part_slots` slots further on), so that the sum over many edges keeps fp32-like accuracy.
-                const int nparts = P.split ? 2 : 1;
-                for (int part = 0; part < nparts; ++part) {
-                    if (part > 0 && full) named_barrier_sync(1, 128);   // the staging tile's first store has read it
-                    const int64_t pslot0 = slot0 + part * P.part_slots;
-                    __nv_bfloat16* grow = is_proxy ? P.dqp_part + (pslot0 + row) * kHeadDim
-                                                   : P.dq_part + ((pslot0 + row) * P.mpp + hh) * kHeadDim;
 #pragma unroll 1
-                    for (int c = 0; c < 128; c += 32) {
-                        uint32_t v[32];
-                        tmem_ld32(tmem_addr(r0, quarter, c), v);
-                        tmem_ld_wait();
-                        uint32_t pk[16];
-                        if (part == 0) {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) pk[i] = pack_act<FP16>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                const float x0 = __uint_as_float(v[2 * i]), x1 = __uint_as_float(v[2 * i + 1]);
-                                pk[i] = pack_act<FP16>(x0 - act_round<FP16>(x0), x1 - act_round<FP16>(x1));
+                for (int x = 0; x < 2; ++x) {
+                    wait(BAR(sm->dq_full[x]), gt & 1, 2);
+                    bad = group_or(1, bad);
+                    if (bad) break;
+                    tc_fence_after_sync();
+                    // dQ^T (lane = head dimension, column = query of the half) -> 16 bit -> transposed into the half's panel of
+                    // the dS^T tile (its products are done): 64 rows of one query each, two 64-column panels in the swizzle of
+                    // the TMA tile store.  With `split` the rows leave twice: rounded, and the remainder of that rounding (a second
+                    // plane of the partial buffers, `part_slots` slots further on), so that the sum over many edges keeps
+                    // fp32-like accuracy.
+                    const uint32_t src = is_proxy ? r1 + 64 * x : tmem + 128 * x + 64;
+                    const uint32_t stage = tile_ds + x * kPanelBytes;
+                    const int nrows = min(64, ud.n - chunk * kBlock - 64 * x);   // <= 0: nothing to write
+                    const int nparts = P.split ? 2 : 1;
+                    for (int part = 0; part < nparts; ++part) {
+                        if (part > 0) named_barrier_sync(1, 128);   // the staging tile's first part has been read
+#pragma unroll 1
+                        for (int i = 0; i < 2; ++i) {   // 16 head-dimension lanes of the warp's 32 at a time
+                            uint32_t v[32];
+                            tmem_ld_16x256_x8(src + (static_cast<uint32_t>(quarter * 32 + 16 * i) << 16), v);
+                            tmem_ld_wait();
+                            if (i == 1 && part == nparts - 1) {
+                                tc_fence_before_sync();
+                                warp_arrive(BAR(sm->dq_free[x]));
                             }
-                        }
-                        if (full) {
-                            // the dS^T tile is free (dQ has been computed): it stages the rows for one TMA tile store
+                            uint32_t pk[16];
+                            if (part == 0) {
 #pragma unroll
-                            for (int k8 = 0; k8 < 4; ++k8)
-                                st_shared_v4(tile_ds + swz_offset(row, (c >> 3) + k8), pk[4 * k8], pk[4 * k8 + 1], pk[4 * k8 + 2],
-                                             pk[4 * k8 + 3]);
-                        } else if (row < nrows) {
+                                for (int k = 0; k < 16; ++k) pk[k] = pack_act<FP16>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+                            } else {
 #pragma unroll
-                            for (int k8 = 0; k8 < 4; ++k8)
-                                *reinterpret_cast<uint4*>(grow + c + 8 * k8) =
-                                    make_uint4(pk[4 * k8], pk[4 * k8 + 1], pk[4 * k8 + 2], pk[4 * k8 + 3]);
+                                for (int k = 0; k < 16; ++k) {
+                                    const float x0 = __uint_as_float(v[2 * k]), x1 = __uint_as_float(v[2 * k + 1]);
+                                    pk[k] = pack_act<FP16>(x0 - act_round<FP16>(x0), x1 - act_round<FP16>(x1));
+                                }
+                            }
+                            // stmatrix: lane l addresses row l%8 of block l/8; blocks are (queries +0, dims +0), (+0, +8), (+8, +0), (+8, +8)
+                            const int cd = quarter * 4 + 2 * i + ((lane >> 3) & 1);   // 16-byte chunk of the 256-byte row
+                            const int q8 = (lane >> 4) * 8 + (lane & 7);
+                            const uint32_t at = stage + (cd >> 3) * (kPanelBytes / 2) + q8 * 128 + (((cd & 7) ^ (lane & 7)) << 4);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) stmatrix_x4_trans(at + j * 16 * 128, pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
                         }
-                    }
-                    if (part == nparts - 1) {
-                        tc_fence_before_sync();
-                        warp_arrive(BAR(sm->r0_free));
-                    }
-                    if (full) {
+                        const int64_t pslot0 = slot0 + 64 * x + part * P.part_slots;
                         fence_async_smem();
                         named_barrier_sync(1, 128);
-                        if (otid == 0) {
-                            const void* tm = is_proxy ? static_cast<const void*>(&tmap_dqp) : static_cast<const void*>(&tmap_dq);
-                            tma_store_3d(tm, tile_ds, 0, is_proxy ? 0 : hh, static_cast<int>(pslot0));
-                            tma_store_3d(tm, tile_ds + kPanelBytes, 64, is_proxy ? 0 : hh, static_cast<int>(pslot0));
-                            tma_store_commit();
-                            tma_store_wait_read();
+                        if (nrows == 64) {
+                            if (warp == 8 && elect_one()) {
+                                const void* tm = is_proxy ? static_cast<const void*>(&tmap_dqp) : static_cast<const void*>(&tmap_dq);
+#pragma unroll 1
+                                for (int c = 0; c < 2; ++c)
+                                    tma_store_3d(tm, stage + c * (kPanelBytes / 2), 64 * c, is_proxy ? 0 : hh, static_cast<int>(pslot0));
+                                tma_store_commit();
+                                tma_store_wait_read();
+                            }
+                        } else if (nrows > 0) {
+                            // the ragged end of a reverse-index row (its slots end where the next row's begin)
+                            for (int e = otid; e < nrows * 16; e += 128) {
+                                const int r = e >> 4, c = e & 15;
+                                __nv_bfloat16* grow = is_proxy ? P.dqp_part + (pslot0 + r) * kHeadDim : P.dq_part + ((pslot0 + r) * P.mpp + hh) * kHeadDim;
+                                *reinterpret_cast<uint4*>(grow + 8 * c) =
+                                    ld_shared_v4(stage + (c >> 3) * (kPanelBytes / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+                            }
+                            named_barrier_sync(1, 128);
                         }
                     }
+                    if (warp == 8) warp_arrive(BAR(sm->ds_free[x]));
                 }
-                if (otid == 0) mbar_arrive(BAR(sm->ds_free));
                 if (++hh == hpc) {
                     hh = 0;
                     ++chunk;
@@ -615,148 +649,160 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                 if (!bad) {
                     tc_fence_after_sync();
                     const int64_t at = ((static_cast<int64_t>(ud.b) * P.Hkv + ud.kvh) * P.S + ud.j * kBlock) * kHeadDim;
-                    flush_rows(r2, P.dv_acc + at);
-                    flush_rows(r3, P.dk_acc + at);
+#pragma unroll 1
+                    for (int c = 0; c < 256; c += 32) {   // lane = key row of the block; columns 0..127 dV, 128..255 dK
+                        float* drow = (c < 128 ? P.dv_acc : P.dk_acc) + at + static_cast<int64_t>(row) * kHeadDim + (c & 127);
+                        uint32_t v[32];
+                        tmem_ld32(tmem_addr(r2, quarter, c), v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4)
+                            red_add_v4(drow + i, __uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+                    }
                     tc_fence_before_sync();
                     warp_arrive(BAR(sm->acc_free));
                 }
             }
         }
-        if (otid == 0) tma_store_wait_all();
+        if (warp == 8 && elect_one()) tma_store_wait_all();
     } else {
         reg_inc<kBwdRegsCompute>();
         // =========================== compute groups ===========================
-        // Thread = (key `row`, the 64 queries of its group).  Reads S^T and dP^T, writes P^T and dS^T back into
-        // TMEM over them (bf16) and dS^T into the shared tile that feeds dQ = dS K.
-        const int hf = warp >> 2;          // which half of the queries
-        const int cbase = hf * 64;
+        // Both groups work on the same half tile, 32 queries each (group A 0..31, B 32..63 of the half): what counts is how soon
+        // the operands of the half are written, because the products of the other half run meanwhile and no longer.
+        // Thread = (key `row`, 32 queries of the half).  Reads S^T and dP^T, writes P^T and dS^T back into TMEM over S^T
+        // (16 bit) and dS^T into the shared tile that feeds dQ^T = K^T dS^T.
+        const int qoff = (warp >> 2) * 32;   // first query of the group inside a half
         const float2 sc2 = make_float2(P.scale_log2e, P.scale_log2e);
         const float inv_mpp = 1.f / static_cast<float>(P.mpp);
-        const bool with_kl = P.with_kl != 0;
         // sum over the main heads of P for this thread's 64 queries: the KL teacher, as packed fp16 pairs
         // (values in [0,1], at most Hq/Hp addends; the result is rounded to bf16 anyway)
-        __half2 teacher[32];
+        __half2 teacher[16], teacher_other[16];   // queries of this half, and of the other one: they change places after each
 #pragma unroll
-        for (int i = 0; i < 32; ++i) teacher[i] = __floats2half2_rn(0.f, 0.f);
+        for (int i = 0; i < 16; ++i) teacher[i] = teacher_other[i] = __floats2half2_rn(0.f, 0.f);
         BwdUnit ud;
-        for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
+        for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
             int hh = 0, chunk = ud.chunk0;
             for (int t = 0; t < ntiles && !bad; ++t, ++gt) {
-                const bool is_proxy = hh == P.mpp;
+                const bool is_proxy = KL && hh == P.mpp;
                 const uint32_t s = gt & 1;
                 wait(BAR(sm->st_full[s]), (gt >> 1) & 1, 1);
-                wait(BAR(sm->sdp_full), gt & 1, 3);
-                if (bad) break;
-                tc_fence_after_sync();
                 const BwdRowStats* st = &sm->stats[s];
                 // only the first chunk of a reverse-index row can hold rows of the key block itself
                 const bool own = (chunk == 0);
-                const bool masked = own || (VARLEN && st->any_low != 0);
-                // The body is instantiated per (masked, proxy) combination: the common tile (neither) must not pay for
-                // predicated-off mask arithmetic or per-element branches in its inner loop, which is bound by instruction issue.
-                auto compute_tile = [&](auto masked_c, auto proxy_c) __attribute__((always_inline)) {
-                    constexpr bool kMasked = decltype(masked_c)::value;
-                    constexpr bool kProxy = decltype(proxy_c)::value;
-                    // Software pipeline over four 16-column pieces: the TMEM loads of piece c+1 are in flight while piece c
-                    // is worked on (tcgen05.wait::ld waits for every load issued so far, hence the order wait, issue, compute).
-                    uint32_t sv[2][16], dv[2][16];
-                    tmem_ld16(tmem_addr(r0, quarter, cbase), sv[0]);
-                    if (!kProxy) tmem_ld16(tmem_addr(r1, quarter, cbase), dv[0]);
-#pragma unroll
-                    for (int c = 0; c < 64; c += 16) {
-                        const int cur = (c >> 4) & 1;
+#pragma unroll 1
+                for (int x = 0; x < 2; ++x) {
+                    const int q0 = 64 * x + qoff;                     // first query of this thread inside the tile
+                    const uint32_t rc = tmem + 128 * x + qoff;        // its first S^T column; dP^T is 64 columns on
+                    const uint32_t ds_row = tile_ds + x * kPanelBytes + row * 128;
+                    wait(BAR(sm->sdp_full[x]), gt & 1, 3);
+                    // the half's panel of the dS^T tile doubles as the staging buffer of the previous tile's dQ store
+                    if (gt >= 1) wait(BAR(sm->ds_free[x]), (gt - 1) & 1, 2);
+                    if (bad) break;
+                    tc_fence_after_sync();
+                    const bool masked = own || (VARLEN && sm->any_low[s] != 0);
+                    // KL(teacher || proxy) = sum t (ln t - ln p), when its value is asked for; t = 0 contributes nothing
+                    if (KL && is_proxy && P.kl_value) {
+                        uint32_t sv[32];
+                        tmem_ld32(tmem_addr(rc, quarter, 0), sv);
                         tmem_ld_wait();
-                        if (c + 16 < 64) {
-                            tmem_ld16(tmem_addr(r0, quarter, cbase + c + 16), sv[cur ^ 1]);
-                            if (!kProxy) tmem_ld16(tmem_addr(r1, quarter, cbase + c + 16), dv[cur ^ 1]);
-                        }
-                        uint32_t lim[4] = {0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu};
-                        uint32_t lw[4] = {0u, 0u, 0u, 0u};
-                        if (kMasked) {
-                            if (own) {
-                                const uint4 l4 = *reinterpret_cast<const uint4*>(&st->limit[cbase + c]);
-                                lim[0] = l4.x; lim[1] = l4.y; lim[2] = l4.z; lim[3] = l4.w;
-                            }
-                            if (VARLEN) {
-                                const uint4 w4 = *reinterpret_cast<const uint4*>(&st->low[cbase + c]);
-                                lw[0] = w4.x; lw[1] = w4.y; lw[2] = w4.z; lw[3] = w4.w;
-                            }
-                        }
-                        uint32_t pk[8], dk[8];
 #pragma unroll
-                        for (int i = 0; i < 16; i += 2) {
-                            const float2 nl2 = *reinterpret_cast<const float2*>(&st->neg_lse[cbase + c + i]);
-                            const float2 a = f2_fma(f2_from_bits(sv[cur][i], sv[cur][i + 1]), sc2, nl2);   // log2 of the probability
-                            float p0 = fast_exp2(a.x);
-                            float p1 = fast_exp2(a.y);
-                            if (kMasked) {
-                                const int l0 = static_cast<int>((lim[i >> 2] >> (8 * (i & 3))) & 0xffu);
-                                const int l1 = static_cast<int>((lim[i >> 2] >> (8 * ((i + 1) & 3))) & 0xffu);
-                                if (VARLEN) {
-                                    const int w0 = static_cast<int>((lw[i >> 2] >> (8 * (i & 3))) & 0xffu);
-                                    const int w1 = static_cast<int>((lw[i >> 2] >> (8 * ((i + 1) & 3))) & 0xffu);
-                                    p0 = (row <= l0 && row >= w0) ? p0 : 0.f;
-                                    p1 = (row <= l1 && row >= w1) ? p1 : 0.f;
-                                } else {
-                                    p0 = (row <= l0) ? p0 : 0.f;
-                                    p1 = (row <= l1) ? p1 : 0.f;
-                                }
-                            }
-                            const int ti = (c + i) >> 1;
-                            if (!kProxy) {
-                                // dS = P o (dP - delta)
-                                const float2 nd2 = *reinterpret_cast<const float2*>(&st->neg_delta[cbase + c + i]);
-                                const float2 d = f2_mul(make_float2(p0, p1), f2_add(f2_from_bits(dv[cur][i], dv[cur][i + 1]), nd2));
-                                pk[i >> 1] = pack_act<FP16>(p0, p1);
-                                dk[i >> 1] = pack_act<FP16>(d.x, d.y);
-                                if (with_kl) teacher[ti] = __hadd2(teacher[ti], __floats2half2_rn(p0, p1));
-                            } else {
-                                const float2 tt = __half22float2(teacher[ti]);
-                                const float t0 = tt.x * inv_mpp, t1 = tt.y * inv_mpp;
-                                dk[i >> 1] = pack_act<FP16>(p0 - t0, p1 - t1);
-                                if (P.kl_value) {   // KL(teacher || proxy) = sum t (ln t - ln p); t = 0 contributes nothing
-                                    kl_acc += (t0 > 0.f) ? t0 * (fast_log2(t0) - a.x) : 0.f;
-                                    kl_acc += (t1 > 0.f) ? t1 * (fast_log2(t1) - a.y) : 0.f;
-                                }
-                                teacher[ti] = __floats2half2_rn(0.f, 0.f);
-                            }
-                        }
-                        // bf16 operands back into TMEM over the columns this thread has consumed: two queries per column.
-                        // (In a proxy tile dSp^T is only parked in R0 until it can go to shared memory, see below.)
-                        if (!kProxy) {
-                            tmem_st8(tmem_addr(r0, quarter, cbase + (c >> 1)), pk);
-                            tmem_st8(tmem_addr(r1, quarter, cbase + (c >> 1)), dk);
-                        } else {
-                            tmem_st8(tmem_addr(r0, quarter, cbase + (c >> 1)), dk);
+                        for (int i = 0; i < 32; ++i) {
+                            const float2 tt = __half22float2(teacher[i >> 1]);
+                            const float tv = ((i & 1) ? tt.y : tt.x) * inv_mpp;
+                            const float a = __uint_as_float(sv[i]) * P.scale_log2e + st->neg_lse[q0 + i];
+                            kl_acc += (tv > 0.f) ? tv * (fast_log2(tv) - a) : 0.f;
                         }
                     }
-                };
-                if (masked) {
-                    if (is_proxy) compute_tile(std::true_type{}, std::true_type{});
-                    else compute_tile(std::true_type{}, std::false_type{});
-                } else {
-                    if (is_proxy) compute_tile(std::false_type{}, std::true_type{});
-                    else compute_tile(std::false_type{}, std::false_type{});
-                }
-                tmem_st_wait();
-                // dS^T also goes to the shared tile that feeds dQ = dS K (row = key, columns = queries).  That tile doubles
-                // as the staging buffer of the previous tile's dQ store, so it is the last thing this tile touches: the
-                // arithmetic above overlaps the previous tile's read-out.
-                if (gt >= 1) wait(BAR(sm->ds_free), (gt - 1) & 1, 2);
-                if (bad) break;
-                {
-                    uint32_t ds[32];
-                    tmem_ld32(tmem_addr(is_proxy ? r0 : r1, quarter, cbase), ds);
-                    tmem_ld_wait();
+                    // The body is instantiated per (masked, proxy) combination: the common tile (neither) must not pay for
+                    // predicated-off mask arithmetic or per-element branches in its inner loop.
+                    auto compute_half = [&](auto masked_c, auto proxy_c) __attribute__((always_inline)) {
+                        constexpr bool kMasked = decltype(masked_c)::value;
+                        constexpr bool kProxy = decltype(proxy_c)::value;
+                        // Two pieces of 16 columns: the TMEM loads of the second are in flight while the first is worked on
+                        // (tcgen05.wait::ld waits for every load issued so far, hence the order wait, issue, compute).
+                        uint32_t sv[2][16], dv[2][16];
+                        tmem_ld16(tmem_addr(rc, quarter, 0), sv[0]);
+                        if (!kProxy) tmem_ld16(tmem_addr(rc, quarter, 64), dv[0]);
 #pragma unroll
-                    for (int k8 = 0; k8 < 8; ++k8)
-                        st_shared_v4(tile_ds + swz_offset(row, (cbase >> 3) + k8), ds[4 * k8], ds[4 * k8 + 1], ds[4 * k8 + 2],
-                                     ds[4 * k8 + 3]);
+                        for (int cc = 0; cc < 2; ++cc) {
+                            const int c = 16 * cc;
+                            tmem_ld_wait();
+                            if (cc == 0) {
+                                tmem_ld16(tmem_addr(rc, quarter, 16), sv[1]);
+                                if (!kProxy) tmem_ld16(tmem_addr(rc, quarter, 64 + 16), dv[1]);
+                            }
+                            uint32_t pk[8], dk[8];
+#pragma unroll
+                            for (int i4 = 0; i4 < 16; i4 += 4) {
+                                const float4 nl4 = *reinterpret_cast<const float4*>(&st->neg_lse[q0 + c + i4]);
+                                float4 nd4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                                if (!kProxy) nd4 = *reinterpret_cast<const float4*>(&st->neg_delta[q0 + c + i4]);
+                                uint32_t lim = 0x7f7f7f7fu, lw = 0u;
+                                if (kMasked) {
+                                    if (own) lim = *reinterpret_cast<const uint32_t*>(&st->limit[q0 + c + i4]);
+                                    if (VARLEN) lw = *reinterpret_cast<const uint32_t*>(&st->low[q0 + c + i4]);
+                                }
+#pragma unroll
+                                for (int i2 = 0; i2 < 4; i2 += 2) {
+                                    const int i = i4 + i2;
+                                    const float2 nl2 = i2 ? make_float2(nl4.z, nl4.w) : make_float2(nl4.x, nl4.y);
+                                    const float2 a = f2_fma(f2_from_bits(sv[cc][i], sv[cc][i + 1]), sc2, nl2);   // log2 of the probability
+                                    float p0 = fast_exp2(a.x);
+                                    float p1 = fast_exp2(a.y);
+                                    if (kMasked) {
+                                        const int l0 = static_cast<int>((lim >> (8 * i2)) & 0xffu), l1 = static_cast<int>((lim >> (8 * i2 + 8)) & 0xffu);
+                                        const int w0 = static_cast<int>((lw >> (8 * i2)) & 0xffu), w1 = static_cast<int>((lw >> (8 * i2 + 8)) & 0xffu);
+                                        p0 = (row <= l0 && (!VARLEN || row >= w0)) ? p0 : 0.f;
+                                        p1 = (row <= l1 && (!VARLEN || row >= w1)) ? p1 : 0.f;
+                                    }
+                                    const int ti = 8 * cc + (i >> 1);
+                                    if (!kProxy) {
+                                        // dS = P o (dP - delta)
+                                        const float2 nd2 = i2 ? make_float2(nd4.z, nd4.w) : make_float2(nd4.x, nd4.y);
+                                        const float2 d = f2_mul(make_float2(p0, p1), f2_add(f2_from_bits(dv[cc][i], dv[cc][i + 1]), nd2));
+                                        pk[i >> 1] = pack_act<FP16>(p0, p1);
+                                        dk[i >> 1] = pack_act<FP16>(d.x, d.y);
+                                        if (KL) teacher[ti] = __hadd2(teacher[ti], __floats2half2_rn(p0, p1));
+                                    } else {
+                                        const float2 tt = __half22float2(teacher[ti]);
+                                        dk[i >> 1] = pack_act<FP16>(p0 - tt.x * inv_mpp, p1 - tt.y * inv_mpp);
+                                        teacher[ti] = __floats2half2_rn(0.f, 0.f);
+                                    }
+                                }
+                            }
+                            // 16-bit operands back into TMEM over the 16 score columns this thread has consumed: P^T, then dS^T,
+                            // two queries per column.  dS^T also goes to the half's panel of the shared tile that feeds
+                            // dQ^T = K^T dS^T (row = key, columns = queries); of a proxy tile nothing else is needed.
+                            if (!kProxy) {
+                                tmem_st8(tmem_addr(rc, quarter, c), pk);
+                                tmem_st8(tmem_addr(rc, quarter, c + 8), dk);
+                            }
+                            st_shared_v4(ds_row + ((2 * (qoff + c)) ^ ((row & 7) << 4)), dk[0], dk[1], dk[2], dk[3]);
+                            st_shared_v4(ds_row + ((2 * (qoff + c) + 16) ^ ((row & 7) << 4)), dk[4], dk[5], dk[6], dk[7]);
+                        }
+                    };
+                    if (KL && is_proxy) {
+                        compute_half(std::true_type{}, std::true_type{});
+                    } else {
+                        if (masked) compute_half(std::true_type{}, std::false_type{});
+                        else compute_half(std::false_type{}, std::false_type{});
+                        tmem_st_wait();
+                    }
+                    fence_async_smem();
+                    tc_fence_before_sync();
+                    warp_arrive(BAR(sm->pds_full[x]));
+                    if (KL) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const __half2 other = teacher[i];
+                            teacher[i] = teacher_other[i];
+                            teacher_other[i] = other;
+                        }
+                    }
                 }
-                fence_async_smem();
-                tc_fence_before_sync();
-                warp_arrive(BAR(sm->pds_full));
+                if (bad) break;
                 warp_arrive(BAR(sm->st_empty[s]));
                 if (++hh == hpc) {
                     hh = 0;
@@ -781,6 +827,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 200000) __nanosleep(1000);
     }
+    __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
@@ -1117,14 +1164,14 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
         !make_tmap_bhsd(&tv, v->ptr, pb->B, pb->Hkv, pb->S, v->stride_b, v->stride_h, v->stride_s, 128) ||
         !make_tmap_bhsd(&tkp, kpx->ptr, pb->B, h_kpx, pb->S, kpx->stride_b, kpx->stride_h, kpx->stride_s, 128) ||
         !make_tmap_partials_swz(&tdq, dq_part, static_cast<uint64_t>(part_slots) * (split ? 2 : 1),
-                                static_cast<uint64_t>(pb->Hq / pb->Hp)) ||
-        !make_tmap_partials_swz(&tdqp, with_kl ? dqp_part : dq_part, static_cast<uint64_t>(part_slots) * (split ? 2 : 1), 1))
+                                static_cast<uint64_t>(pb->Hq / pb->Hp), 64) ||
+        !make_tmap_partials_swz(&tdqp, with_kl ? dqp_part : dq_part, static_cast<uint64_t>(part_slots) * (split ? 2 : 1), 1, 64))
         return FMSA_ERR_CUDA;
 
     BwdParams P;
-    P.q_row_b = q->stride_b / 128; P.q_row_h = q->stride_h / 128; P.q_row_s = q->stride_s / 128;
-    P.do_row_b = d_out->stride_b / 128; P.do_row_h = d_out->stride_h / 128; P.do_row_s = d_out->stride_s / 128;
-    P.qp_row_b = qpx->stride_b / 128; P.qp_row_h = qpx->stride_h / 128; P.qp_row_s = qpx->stride_s / 128;
+    P.q_row_b = static_cast<int32_t>(q->stride_b / 128); P.q_row_h = static_cast<int32_t>(q->stride_h / 128); P.q_row_s = static_cast<int32_t>(q->stride_s / 128);
+    P.do_row_b = static_cast<int32_t>(d_out->stride_b / 128); P.do_row_h = static_cast<int32_t>(d_out->stride_h / 128); P.do_row_s = static_cast<int32_t>(d_out->stride_s / 128);
+    P.qp_row_b = static_cast<int32_t>(qpx->stride_b / 128); P.qp_row_h = static_cast<int32_t>(qpx->stride_h / 128); P.qp_row_s = static_cast<int32_t>(qpx->stride_s / 128);
     P.q_rows_total = static_cast<int32_t>(q_rows); P.do_rows_total = static_cast<int32_t>(do_rows);
     P.qp_rows_total = static_cast<int32_t>(qp_rows);
     P.lse = lse; P.lse_proxy = lse_proxy; P.delta = delta;
@@ -1136,7 +1183,7 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     P.S = pb->S; P.NB = pb->S / kBlock; P.Hq = pb->Hq; P.Hkv = pb->Hkv; P.Hp = pb->Hp; P.Hpkv = pb->Hpkv;
     P.mpp = pb->Hq / pb->Hp; P.ppk = pb->Hp / pb->Hkv; P.pg = pb->Hp / pb->Hpkv;
     P.g_begin = g_begin; P.G = g_count;
-    P.with_kl = with_kl ? 1 : 0; P.dense = dense ? 1 : 0;
+    P.dense = dense ? 1 : 0;
     P.scale_log2e = pb->scale * kLog2e;
     P.kl_value = with_kl ? kl_value : nullptr;
     P.kl_value_scale = kLn2 / (static_cast<float>(pb->B) * pb->Hp * pb->S);
@@ -1145,18 +1192,22 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     const int sms = device_sm_count();
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
     const bool varlen = P.doc_start != nullptr;
-    const void* kfn = fp16 ? (varlen ? reinterpret_cast<const void*>(sparse_bwd_kernel<true, true>) : reinterpret_cast<const void*>(sparse_bwd_kernel<true, false>))
-                           : (varlen ? reinterpret_cast<const void*>(sparse_bwd_kernel<false, true>) : reinterpret_cast<const void*>(sparse_bwd_kernel<false, false>));
+    using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
+    static const KernelFn kernels[8] = {sparse_bwd_kernel<false, false, false>, sparse_bwd_kernel<false, false, true>,
+                                        sparse_bwd_kernel<false, true, false>,  sparse_bwd_kernel<false, true, true>,
+                                        sparse_bwd_kernel<true, false, false>,  sparse_bwd_kernel<true, false, true>,
+                                        sparse_bwd_kernel<true, true, false>,   sparse_bwd_kernel<true, true, true>};
+    const KernelFn kernel = kernels[(fp16 ? 4 : 0) + (varlen ? 2 : 0) + (with_kl ? 1 : 0)];
+    const void* kfn = reinterpret_cast<const void*>(kernel);
     if (sms <= 0 || !ensure_smem_attr(kfn, kBwdSmemBytes)) return FMSA_ERR_CUDA;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
     P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
-    P.n_subunits = g_count * subunits_per_group(P.NB, P.ppk, P.chunks);
-    FMSA_REQUIRE(P.n_subunits < 0x7fffffffLL);
+    const int64_t per_group = subunits_per_group(P.NB, P.ppk, P.chunks);
+    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA)
+    P.units_per_group = static_cast<uint32_t>(per_group);
+    P.n_subunits = static_cast<int32_t>(per_group * g_count);
     const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
-    if (fp16 && varlen) sparse_bwd_kernel<true, true><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);
-    else if (fp16) sparse_bwd_kernel<true, false><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);
-    else if (varlen) sparse_bwd_kernel<false, true><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);
-    else sparse_bwd_kernel<false, false><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);
+    kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);
     return check_launch();
 }
 

@@ -56,7 +56,8 @@ struct FwdParams {
     int S, NB, Hq, Hkv, Hp, mpp, ppk, pg;
     int g_begin, G;
     int with_proxy, dense;
-    int64_t n_subunits;
+    int32_t n_subunits;
+    uint32_t units_per_group;
     int chunks;             // chunks per sub-unit
     float scale_log2e;
 };
@@ -80,7 +81,6 @@ struct FwdCtrl {
     UnitDesc units[kUnitRing];
     alignas(16) uint8_t limits[kLimitRing][128];   // per chunk in flight: last visible key of each row (127 = all)
     uint32_t tmem_slot;
-    int32_t abort_flag;
 };
 
 // Roles (warp index): 0-3 softmax group A (tiles with an even running index), 4-7 softmax group B
@@ -134,7 +134,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int quarter = warp & 3;              // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;       // softmax / output: tile row of this thread
-    const uint32_t elect = (lane == 0) ? 1u : 0u;
     auto BAR = [&](uint64_t& b) { return smem_u32(&b); };
 
     if (tid == 0) {
@@ -156,7 +155,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
         mbar_init(BAR(sm->o_full), 1);
         mbar_init(BAR(sm->o_empty), 4);
         for (int i = 0; i < kUnitRing; ++i) mbar_init(BAR(sm->unit_full[i]), 1);
-        sm->abort_flag = 0;
         fence_mbar_init();
         prefetch_tmap(&tmap_q);
         prefetch_tmap(&tmap_qp);
@@ -172,14 +170,20 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = sm->tmem_slot;
+    // All 512 columns are this CTA's, so the allocation starts at column 0 and every TMEM address is a constant.
+    constexpr uint32_t tmem = 0;
+    if (sm->tmem_slot != tmem) {
+        if (tid == 0) atomicMax(P.status, kStatusBadSmem);
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);
+        return;
+    }
     const uint32_t tmem_s0 = tmem, tmem_o0 = tmem + 384;
 
     const int hpc = P.mpp + (P.with_proxy ? 1 : 0);   // tiles per chunk
     const int lse_stride = P.mpp + 1;
     const int64_t edge_base = P.dense ? dense_edge_base(static_cast<int64_t>(P.g_begin) * P.ppk, P.S, P.NB)
                                       : static_cast<int64_t>(P.row_ptr[static_cast<int64_t>(P.g_begin) * P.ppk * P.NB]);
-    volatile int* abort_flag = &sm->abort_flag;
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
 #ifdef FMSA_TRACE
     unsigned long long trace_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
 #ifdef FMSA_TRACE
         const long long w0 = clock64();
 #endif
-        if (!bad) bad = __any_sync(0xffffffffu, !mbar_wait_abortable(bar, parity, abort_flag));
+        if (!bad) bad = __any_sync(0xffffffffu, !mbar_wait_role(bar, parity));
 #ifdef FMSA_TRACE
         trace_acc[kind & 7] += static_cast<unsigned long long>(clock64() - w0);
 #endif
@@ -234,11 +238,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
             UnitDesc nu;
             nu.chunk1 = -1;
             for (;;) {
-                const int64_t u = atomicAdd(P.counter, 1);
-                if (u >= P.n_subunits) break;
-                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks);
-                const int g = P.g_begin + su.g;
-                const int b = g / P.Hkv, kvh = g % P.Hkv, p = kvh * P.ppk + su.pp;
+                const uint32_t u = static_cast<uint32_t>(atomicAdd(P.counter, 1));
+                if (u >= static_cast<uint32_t>(P.n_subunits)) break;
+                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks, P.units_per_group);
+                const uint32_t g = P.g_begin + su.g;
+                const int b = g / static_cast<uint32_t>(P.Hkv), kvh = g % static_cast<uint32_t>(P.Hkv), p = kvh * P.ppk + su.pp;
                 const int64_t bp = static_cast<int64_t>(b) * P.Hp + p;
                 int64_t e0;
                 int n;
@@ -273,7 +277,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
             // =========================== MMA issue ===========================
             UnitDesc ud;
             for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
-                const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
+                const int ntiles = __shfl_sync(0xffffffffu, (ud.chunk1 - ud.chunk0) * hpc, 0);   // (known to be uniform)
                 wait(BAR(sm->k_full), nsub & 1, 5);
                 bool kp_ready = false, v_ready = false;
                 uint32_t gts = gt;            // running index of the next S to issue, its accumulator and phase bit
@@ -290,11 +294,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     wait(BAR(sm->q_full[qs]), qph, 1);
                     if (gts >= 3) wait(BAR(sm->s_free[ssb]), ssph ^ 1, 2);
                     tc_fence_after_sync();
-                    if (!bad) {
-                        umma_tile_128<false, false, FP16>(tmem_s0 + ssb * 128, tile_q0 + qs * kTileBytes, proxy ? tile_kp : tile_k, false,
-                                                    elect);
-                        umma_commit(BAR(sm->s_full[ssb]), elect);
-                        umma_commit(BAR(sm->q_empty[qs]), elect);
+                    if (!bad && elect_one()) {
+                        umma_tile_128<false, false, FP16>(tmem_s0 + ssb * 128, tile_q0 + qs * kTileBytes, proxy ? tile_kp : tile_k, false);
+                        umma_commit(BAR(sm->s_full[ssb]));
+                        umma_commit(BAR(sm->q_empty[qs]));
                     }
                     if (++qs == kFwdQStages) {
                         qs = 0;
@@ -306,9 +309,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     }
                     ++gts;
                     if (++hs == hpc) hs = 0;
-                    if (++s_issued == ntiles && !bad) {
-                        umma_commit(BAR(sm->k_empty), elect);    // every S of this sub-unit has been issued
-                        umma_commit(BAR(sm->kp_empty), elect);
+                    if (++s_issued == ntiles && !bad && elect_one()) {
+                        umma_commit(BAR(sm->k_empty));    // every S of this sub-unit has been issued
+                        umma_commit(BAR(sm->kp_empty));
                     }
                 };
                 next_s();
@@ -325,21 +328,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                         }
                         if (mt >= 1) wait(BAR(sm->o_empty), (mt - 1) & 1, 4);
                         tc_fence_after_sync();
-                        if (!bad) {
+                        if (!bad && elect_one()) {
                             const uint32_t ts = tmem_s0 + sb * 128;
-                            umma_tile_128_ts<true, FP16>(tmem_o0, ts, ts + 32, tile_v, false, elect);   // O = P V_j
-                            umma_commit(BAR(sm->o_full), elect);
+                            umma_ts<8, 8, FP16>(tmem_o0, ts, tile_v, false);   // O = P V_j
+                            umma_commit(BAR(sm->o_full));
                         }
                         ++mt;
                     }
-                    if (!bad) umma_commit(BAR(sm->s_free[sb]), elect);
+                    if (!bad && elect_one()) umma_commit(BAR(sm->s_free[sb]));
                     if (++sb == 3) {
                         sb = 0;
                         sph ^= 1;
                     }
                     if (++hh == hpc) hh = 0;
                 }
-                if (!bad) umma_commit(BAR(sm->v_empty), elect);
+                if (!bad && elect_one()) umma_commit(BAR(sm->v_empty));
             }
         } else if (warp == 20) {
             // =========================== K / V / Kp loads ===========================
@@ -886,8 +889,10 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     if (sms <= 0 || !ensure_smem_attr(kfn, kFwdSmemBytes)) return FMSA_ERR_CUDA;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
     P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
-    P.n_subunits = g_count * subunits_per_group(P.NB, P.ppk, P.chunks);
-    FMSA_REQUIRE(P.n_subunits < 0x7fffffffLL);
+    const int64_t per_group = subunits_per_group(P.NB, P.ppk, P.chunks);
+    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA)
+    P.units_per_group = static_cast<uint32_t>(per_group);
+    P.n_subunits = static_cast<int32_t>(per_group * g_count);
     const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
     if (fp16 && varlen) sparse_fwd_kernel<true, true><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
     else if (fp16) sparse_fwd_kernel<true, false><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
