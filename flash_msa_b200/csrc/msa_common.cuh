@@ -82,4 +82,57 @@ __device__ __forceinline__ SubUnit decode_subunit(uint32_t u, int NB, uint32_t p
     return su;
 }
 
+// What a launch needs to enumerate its sub-units; a member of the parameters of the backward kernels.
+struct UnitSpace {
+    const int32_t* row_ptr;
+    int32_t* counter;
+    int32_t n_subunits;
+    uint32_t per_group;
+    int S, NB, Hkv, Hp, ppk, g_begin, chunks, dense;
+};
+
+// A sub-unit as the drawing thread publishes it to the other roles (kept small: it shares the last 3 KB of shared memory).
+struct UnitRec {
+    int64_t e0;                      // position of the reverse-index row in col_q / the slot space
+    int32_t n;                       // its length
+    uint16_t j, b, kvh, p, chunk0;   // (B*Hp < 65536 and S/128 <= 2048 are required by the entry points)
+    int16_t chunk1;                  // < 0: no more work
+};
+
+// Next sub-unit with work; sub-units that lie beyond the end of their row are passed over.
+__device__ __forceinline__ UnitRec draw_subunit(const UnitSpace& U) {
+    UnitRec nu;
+    nu.chunk1 = -1;
+    for (;;) {
+        const uint32_t u = static_cast<uint32_t>(atomicAdd(U.counter, 1));
+        if (u >= static_cast<uint32_t>(U.n_subunits)) break;
+        const SubUnit su = decode_subunit(u, U.NB, U.ppk, U.chunks, U.per_group);
+        const uint32_t g = U.g_begin + su.g;
+        const int b = g / static_cast<uint32_t>(U.Hkv), kvh = g % static_cast<uint32_t>(U.Hkv), p = kvh * U.ppk + su.pp;
+        const int64_t bp = static_cast<int64_t>(b) * U.Hp + p;
+        int64_t e0;
+        int n;
+        if (U.dense) {
+            e0 = dense_edge_base(bp, U.S, U.NB) + dense_row_offset(su.j, U.S);
+            n = U.S - su.j * kBlock;
+        } else {
+            e0 = U.row_ptr[bp * U.NB + su.j];
+            n = U.row_ptr[bp * U.NB + su.j + 1] - static_cast<int>(e0);
+        }
+        if (su.chunk0 * kBlock < n) {
+            nu.j = static_cast<uint16_t>(su.j); nu.b = static_cast<uint16_t>(b); nu.kvh = static_cast<uint16_t>(kvh);
+            nu.p = static_cast<uint16_t>(p); nu.n = n; nu.e0 = e0;
+            nu.chunk0 = static_cast<uint16_t>(su.chunk0);
+            nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + U.chunks));
+            break;
+        }
+    }
+    return nu;
+}
+// CSR position of the first slot of a pass over the groups from g_begin on.
+__device__ __forceinline__ int64_t first_slot(const UnitSpace& U) {
+    return U.dense ? dense_edge_base(static_cast<int64_t>(U.g_begin) * U.ppk, U.S, U.NB)
+                   : static_cast<int64_t>(U.row_ptr[static_cast<int64_t>(U.g_begin) * U.ppk * U.NB]);
+}
+
 }  // namespace fmsa

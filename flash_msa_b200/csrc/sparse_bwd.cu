@@ -4,19 +4,22 @@
 // memory, the unit walks the reverse-index row of every proxy head of its group in chunks of 128
 // gathered query rows.  For each chunk the main heads of the proxy head run one after another.  Scores
 // are computed TRANSPOSED (TMEM lane = key, column = query) so that P^T and dS^T, written back into TMEM
-// as bf16 over the columns S^T and dP^T occupied, are the TMEM operands of the dV and dK products:
+// as 16-bit operands over the columns S^T occupied, are the TMEM operands of the dV and dK products:
 //     S^T = K_j Q_g^T           dP^T = V_j dO_g^T                   (both operands in shared memory)
-//     P^T = exp2(S^T*c - lse)   dS^T = P^T o (dP^T - delta)         (fp32, rounded to bf16)
+//     P^T = exp2(S^T*c - lse)   dS^T = P^T o (dP^T - delta)         (fp32, rounded to 16 bit)
 //     dV += P^T dO_g            dK += dS^T Q_g                      (A operand in TMEM; accumulators stay in
 //                                                                    TMEM for the whole sub-unit)
-//     dQ  = dS K_j                                                  (dS^T also goes to shared memory)
-// while every thread sums the P of its (key, queries) over the heads: the KL teacher.
-// Then one proxy tile:
+//     dQ^T = K_j^T dS^T                                             (dS^T also goes to shared memory)
+// while every thread sums the P of its (key, queries) over the heads: the KL teacher, which is stored once per chunk.
+// The proxy head's part runs as a kernel of its own behind this one (proxy_bwd.cu), from the teacher:
 //     Sp^T = Kp_j Qp_g^T        p_px = exp2(Sp^T*c - lse_proxy)     dSp^T = p_px - teacher/mpp
 //     dKp = dSp^T Qp_g, dQp = dSp Kp_j.
-// dQ and dQp leave as bf16 per-edge partial rows (a combine kernel sums them per query row, applying
-// scale and scale/(B*Hp*S)); dK, dV (once per sub-unit) and dKp (once per proxy tile) are added to fp32
-// accumulators with vector reductions and cast afterwards.
+// As one more tile of every chunk it took twice the time of a main tile (its two halves need each other, its dKp does
+// not fit TMEM beside dV and dK and left as 64 KB of fp32 reductions per chunk) and its code displaced the main tile's from
+// the instruction cache.
+// dQ and dQp leave as 16-bit per-edge partial rows (a combine kernel sums them per query row, applying
+// scale and scale/(B*Hp*S)); dK and dV are added to fp32 accumulators with vector reductions once per sub-unit and
+// cast afterwards.
 //
 // Formulas and rounding points follow the reference kernel
 // (flash_msa/msa_backward_cutedsl.py:456-733: P and dS rounded to the input type before the
@@ -31,6 +34,7 @@
 
 #include "host_common.h"
 #include "msa_common.cuh"
+#include "proxy_bwd.h"
 #include "sm100.cuh"
 #include "tma_host.h"
 
@@ -46,36 +50,19 @@ struct BwdParams {
     // Row-gather views: element row (b, h, s) of q / d_out / q_proxy is matrix row b*row_b + h*row_h + s*row_s.
     int32_t q_row_b, q_row_h, q_row_s;
     int32_t do_row_b, do_row_h, do_row_s;
-    int32_t qp_row_b, qp_row_h, qp_row_s;
-    int32_t q_rows_total, do_rows_total, qp_rows_total;   // first row index outside each view (reads as zeros)
-    const float *lse, *lse_proxy, *delta;   // [B,Hq,S], [B,Hp,S], [B,Hq,S]
-    const int32_t* row_ptr;
+    int32_t q_rows_total, do_rows_total;   // first row index outside each view (reads as zeros)
+    const float *lse, *delta;   // [B,Hq,S]
+    UnitSpace units;
     const int32_t* col_q;
     const int32_t* doc_start;   // [B,S] first token of each token's document (packed sequences), or null
     __nv_bfloat16* dq_part;    // [(edge - edge_base) * mpp + head][128]: per-edge dQ contributions (unscaled)
-    __nv_bfloat16* dqp_part;   // [(edge - edge_base)][128]: per-edge dQp contributions (unscaled)
-    int64_t part_slots;        // slots per plane of the two buffers above
+    uint32_t* teacher;         // KL kernels: per edge 256 bytes (the dqp_part buffer), filled by the compute groups below
+    int64_t part_slots;        // slots per plane of dq_part
     int split;                 // 1: every contribution is stored as a bf16 pair (value, rounding remainder) in two planes
-    // fp32, zero-initialised: [B,Hpkv,S,128], [B,Hkv,S,128] x2
-    float *dkp_acc, *dk_acc, *dv_acc;
-    int32_t* counter;
+    float *dk_acc, *dv_acc;    // fp32, zero-initialised, [B,Hkv,S,128]
     int32_t* status;
-    int S, NB, Hq, Hkv, Hp, Hpkv, mpp, ppk, pg;
-    int g_begin, G;
-    int32_t n_subunits;
-    uint32_t units_per_group;
-    int chunks;             // chunks per sub-unit
-    int dense;
+    int S, Hq, Hkv, mpp;
     float scale_log2e;
-    float* kl_value;        // optional: += KL(teacher || proxy) summed over this launch's rows, / (B*Hp*S)
-    float kl_value_scale;   // ln(2) / (B*Hp*S)
-};
-
-struct BwdUnit {   // (kept small: the control block shares the last 3 KB of shared memory with the row statistics)
-    int64_t e0;
-    int32_t n;
-    uint16_t j, b, kvh, p, chunk0;   // (B*Hp < 65536 and S/128 <= 2048 are required by the entry point)
-    int16_t chunk1;                  // < 0: no more work
 };
 
 constexpr int kBwdUnitRing = 8;
@@ -94,16 +81,15 @@ struct BwdCtrl {
     uint64_t qdo_full[2][2], qdo_empty[2][2];    // [stage][half]
     uint64_t st_full[2], st_empty[2];
     uint64_t sdp_full[2], pds_full[2], dq_full[2], dq_free[2], ds_free[2];   // [half]
-    uint64_t dkp_full, dkp_free;
     uint64_t unit_full[kBwdUnitRing];
-    BwdUnit units[kBwdUnitRing];
+    UnitRec units[kBwdUnitRing];
     BwdRowStats stats[2];
     int32_t any_low[2];          // some row of the tile has low > 0 (document masking)
     uint32_t tmem_slot;
 };
 
-// Roles (warp index): 0-3 compute group A (queries 0..63 of a tile), 4-7 compute group B (queries 64..127),
-// 8-11 output group, 12-15 row gather (Q, dO, Qp; Kp_j), 16 K/V loads and row statistics, 17 MMA issue (18, 19 only
+// Roles (warp index): 0-3 compute group A (queries 0..31 of a half tile), 4-7 compute group B (queries 32..63),
+// 8-11 output group, 12-15 row gather (Q, dO), 16 K/V loads and row statistics, 17 MMA issue (18, 19 only
 // take part in the block-wide steps).  A TMA row gather costs the issuing warp ~65 cycles whatever its size, so the
 // 128 gathers of a tile are spread over four warps.
 constexpr int kBwdGatherWarps = 4;
@@ -123,11 +109,10 @@ constexpr uint32_t kHalfRowBytes = 64 * 128;   // rows 64.. of a panel: where ha
 
 // Warp-specialised backward.  Every role walks the same sequence of sub-units (published by the gather warp in a
 // ring) and of tiles.  A tile is worked on as two halves of 64 queries, x = 0 and 1, that take turns on the tensor core:
-// while the compute group of one half turns S^T, dP^T into P^T, dS^T, the products of the other half run.  TMEM (512 columns):
+// while the compute groups turn S^T, dP^T of one half into P^T, dS^T, the products of the other half run.  TMEM (512 columns):
 //   Rx [128x, 128x+128), x = 0, 1: columns 0..63 S^T of the half, overwritten in place by P^T and dS^T (16 bit; 16 queries
 //                at a time: 8 columns of P^T, then 8 of dS^T); columns 64..127 dP^T, then dQ^T (lane = head dimension).
 //   R2 [256,384) dV, R3 [384,512) dK (lane = key), accumulated over the sub-unit.
-//   Proxy tile: Sp^T in columns 0..63 of both Rx; then dKp^T (lane = head dimension) takes R0, dQp^T of the halves R1.
 // A step of the issuing warp (half x of main tile t), behind P^T / dS^T of that half:
 //   dQ^T = K^T dS^T -> Rx+64,  dV += P^T dO,  dK += dS^T Q,  S^T(t+1) = K Q^T -> Rx,  [dQ^T read out]  dP^T(t+1) = V dO^T -> Rx+64
 // so dQ^T is read out under three products, and everything half x needs for tile t+1 is under way before the step of the
@@ -137,18 +122,15 @@ constexpr uint32_t kHalfRowBytes = 64 * 128;   // rows 64.. of a panel: where ha
 // Hand-offs (mbarriers; one arrival per warp or per tcgen05.commit): qdo_full (TMA bytes) <- qdo_empty; st_full <- st_empty
 // (row statistics); sdp_full (S^T and dP^T of a half), pds_full (P^T, dS^T written), dq_full -> dq_free (dQ^T read out),
 // ds_free (the half's panel of the dS^T tile, which doubles as the staging tile of its dQ store, is reusable),
-// dkp_full / dkp_free (proxy tile), acc_full / acc_free (dV, dK flushed at the end of a sub-unit).
+// acc_full / acc_free (dV, dK flushed at the end of a sub-unit).
 // VARLEN: document masking of packed sequences (P.doc_start given).  A separate instantiation, so that the plain kernel
 // carries none of its registers or code.
 template <bool FP16, bool VARLEN, bool KL>
 __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
                                                                     const __grid_constant__ CUtensorMap tmap_do,
-                                                                    const __grid_constant__ CUtensorMap tmap_qp,
                                                                     const __grid_constant__ CUtensorMap tmap_k,
                                                                     const __grid_constant__ CUtensorMap tmap_v,
-                                                                    const __grid_constant__ CUtensorMap tmap_kp,
                                                                     const __grid_constant__ CUtensorMap tmap_dq,
-                                                                    const __grid_constant__ CUtensorMap tmap_dqp,
                                                                     const BwdParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -162,7 +144,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;   // TMEM lane of this thread: key (compute, dKp/dV/dK read-out) or query (dQ read-out)
+    const int row = quarter * 32 + lane;   // TMEM lane of this thread: key (compute, dV/dK read-out)
     auto BAR = [&](uint64_t& b) { return smem_u32(&b); };
 
     if (tid == 0) {
@@ -183,8 +165,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
             mbar_init(BAR(sm->dq_free[i]), 4);
             mbar_init(BAR(sm->ds_free[i]), 1);
         }
-        mbar_init(BAR(sm->dkp_full), 1);
-        mbar_init(BAR(sm->dkp_free), 4);
         for (int i = 0; i < kBwdUnitRing; ++i) mbar_init(BAR(sm->unit_full[i]), 1);
         fence_mbar_init();
         prefetch_tmap(&tmap_q);
@@ -192,11 +172,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         prefetch_tmap(&tmap_k);
         prefetch_tmap(&tmap_v);
         prefetch_tmap(&tmap_dq);
-        if (KL) {
-            prefetch_tmap(&tmap_qp);
-            prefetch_tmap(&tmap_kp);
-            prefetch_tmap(&tmap_dqp);
-        }
     }
     if (warp == 0) {
         tmem_alloc(smem_u32(&sm->tmem_slot), 512);
@@ -213,11 +188,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);
         return;
     }
-    const uint32_t r0 = tmem, r1 = tmem + 128, r2 = tmem + 256, r3 = tmem + 384;   // (Rx = tmem + 128 * x)
+    const uint32_t r2 = tmem + 256, r3 = tmem + 384;   // (Rx = tmem + 128 * x)
 
-    const int hpc = P.mpp + (KL ? 1 : 0);   // tiles per chunk
-    const int64_t edge_base = P.dense ? dense_edge_base(static_cast<int64_t>(P.g_begin) * P.ppk, P.S, P.NB)
-                                      : static_cast<int64_t>(P.row_ptr[static_cast<int64_t>(P.g_begin) * P.ppk * P.NB]);
+    const int hpc = P.mpp;   // tiles per chunk
+    const int64_t edge_base = first_slot(P.units);
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
 #ifdef FMSA_TRACE
     unsigned long long trace_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -256,44 +230,16 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     };
 
     uint32_t gt = 0;     // tiles seen so far by this CTA (every role counts the same sequence)
-    uint32_t pt = 0;     // proxy tiles seen so far
     uint32_t nsub = 0;   // sub-units seen so far
-    float kl_acc = 0.f;  // compute groups: this thread's share of sum t * (log2 t - log2 p_proxy)
 
     // Next sub-unit of the common sequence (false: no more work, or the CTA is giving up).  The gather warp draws the
     // work and publishes the decoded sub-unit; it passes over sub-units that lie beyond the end of their row, so
     // every published entry has work (or is the end marker).  The roles are at most a few tiles apart, fewer than the
     // ring has entries.
-    auto next_unit = [&](uint32_t draw, BwdUnit& ud, auto mode) -> bool {
+    auto next_unit = [&](uint32_t draw, UnitRec& ud, auto mode) -> bool {
         const uint32_t uslot = draw & (kBwdUnitRing - 1);
         if (decltype(mode)::value == kDraws && warp == 12 && lane == 0) {
-            BwdUnit nu;
-            nu.chunk1 = -1;
-            for (;;) {
-                const uint32_t u = static_cast<uint32_t>(atomicAdd(P.counter, 1));
-                if (u >= static_cast<uint32_t>(P.n_subunits)) break;
-                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks, P.units_per_group);
-                const uint32_t g = P.g_begin + su.g;
-                const int b = g / static_cast<uint32_t>(P.Hkv), kvh = g % static_cast<uint32_t>(P.Hkv), p = kvh * P.ppk + su.pp;
-                const int64_t bp = static_cast<int64_t>(b) * P.Hp + p;
-                int64_t e0;
-                int n;
-                if (P.dense) {
-                    e0 = dense_edge_base(bp, P.S, P.NB) + dense_row_offset(su.j, P.S);
-                    n = P.S - su.j * kBlock;
-                } else {
-                    e0 = P.row_ptr[bp * P.NB + su.j];
-                    n = P.row_ptr[bp * P.NB + su.j + 1] - static_cast<int>(e0);
-                }
-                if (su.chunk0 * kBlock < n) {
-                    nu.j = static_cast<uint16_t>(su.j); nu.b = static_cast<uint16_t>(b); nu.kvh = static_cast<uint16_t>(kvh);
-                    nu.p = static_cast<uint16_t>(p); nu.n = n; nu.e0 = e0;
-                    nu.chunk0 = static_cast<uint16_t>(su.chunk0);
-                    nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + P.chunks));
-                    break;
-                }
-            }
-            sm->units[uslot] = nu;
+            sm->units[uslot] = draw_subunit(P.units);
             mbar_arrive(BAR(sm->unit_full[uslot]));
         }
         if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1);
@@ -304,9 +250,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         return ud.chunk1 >= 0;
     };
     // query position of row `at` of a reverse-index row, -1 when there is none (or the index is bad)
-    auto row_qid = [&](const BwdUnit& ud, int at) -> int {
+    auto row_qid = [&](const UnitRec& ud, int at) -> int {
         if (at >= ud.n) return -1;
-        const int q = P.dense ? (ud.j * kBlock + at) : P.col_q[ud.e0 + at];
+        const int q = P.units.dense ? (ud.j * kBlock + at) : P.col_q[ud.e0 + at];
         if (static_cast<unsigned>(q) >= static_cast<unsigned>(P.S) || (q >> 7) < ud.j) {
             atomicMax(P.status, kStatusBadIndex);
             return -1;
@@ -323,101 +269,62 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
             // One thread runs the whole role.  The tensor core holds a handful of instructions that have not started, i.e.
             // about 200 cycles of work: whatever the issuing thread does between two products in more than that is time the
             // tensor core stands still, so barriers are looked at before the product that precedes their use is issued.
-            BwdUnit ud;
+            UnitRec ud;
             for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kOneThread>{}); ++draw, ++nsub) {
                 const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
-                const int last_main = 2 * (ntiles - (KL ? 1 : 0)) - 1;   // step of the last half that uses K and V
                 wait1(BAR(sm->kv_full), nsub & 1);
-                // One step per half tile: the products of (tile t, half x), then the front of the next tile (S^T and dP^T) for
-                // the halves whose regions they free: that half after a main tile, both at once behind the second step of a
-                // proxy tile and at the start (u = -1).
-                int hh = KL ? P.mpp : 0;      // head of tile t; before the first tile the last head of the previous sub-unit
-                int hh1 = 0;                         // head of tile t + 1
+                // One step per half tile: the products of (tile t, half x), then the front (S^T and dP^T) of that half of the next
+                // tile; at the start (u = -1) the front of both halves.
                 bool pds_ready = false;              // the next step's operands have been seen written
 #pragma unroll 1
                 for (int u = -1; u < 2 * ntiles && !bad; ++u) {
                     const int x = u & 1;
-                    const bool is_proxy = KL && hh == P.mpp;
                     const uint32_t rx = tmem + 128 * x;
                     if (u >= 0) {
                         const uint32_t s = gt & 1;
-                        const uint32_t tq = tile_q0 + s * kTileBytes, tdo = tile_do0 + s * kTileBytes;
-                        if (is_proxy && x == 0) {
-                            // (the front of a proxy tile does not wait for the dQ^T of the main tile before it)
-                            wait1(BAR(sm->dq_free[0]), (gt - 1) & 1);
-                            wait1(BAR(sm->dq_free[1]), (gt - 1) & 1);
-                            wait1(BAR(sm->pds_full[1]), gt & 1);
-                        }
-                        if (!pds_ready && (!is_proxy || x == 0)) wait1(BAR(sm->pds_full[x]), gt & 1);
+                        const uint32_t tq = tile_q0 + s * kTileBytes + x * kHalfRowBytes, tdo = tile_do0 + s * kTileBytes + x * kHalfRowBytes;
+                        if (!pds_ready) wait1(BAR(sm->pds_full[x]), gt & 1);
                         if (bad) break;
                         tc_fence_after_sync();
-                        if (is_proxy && x == 0) {
-                            umma_ss<128, 8, true, false, FP16>(r0, tq, tile_ds, false);   // dKp^T = Qp_g^T dSp
-                            umma_commit(BAR(sm->dkp_full));
-                        }
-                        // dQ^T = K_j^T dS^T, dQp^T = Kp_j^T dSp^T
-                        umma_ss<64, 8, true, true, FP16>(is_proxy ? r1 + 64 * x : rx + 64, is_proxy ? tdo : tile_k, tile_ds + x * kPanelBytes, false);
+                        umma_ss<64, 8, true, true, FP16>(rx + 64, tile_k, tile_ds + x * kPanelBytes, false);   // dQ^T = K_j^T dS^T
                         umma_commit(BAR(sm->dq_full[x]));
-                        if (!is_proxy) {
-                            if (u == 0 && nsub > 0) {
-                                wait1(BAR(sm->acc_free), (nsub - 1) & 1);   // dV, dK of the previous sub-unit flushed
-                                if (bad) break;
-                                tc_fence_after_sync();
-                            }
-                            umma_ts<4, 16, FP16>(r2, rx, tdo + x * kHalfRowBytes, u != 0);       // dV += P^T dO_g
-                            umma_ts<4, 16, FP16>(r3, rx + 8, tq + x * kHalfRowBytes, u != 0);    // dK += dS^T Q_g
-                            umma_commit(BAR(sm->qdo_empty[s][x]));
-                            // K and V are done with after the last main tile: they are fetched anew under the proxy tile
-                            if (u == last_main) umma_commit(BAR(sm->kv_empty));
-                        } else if (x == 1) {
-                            umma_commit(BAR(sm->qdo_empty[s][0]));
-                            umma_commit(BAR(sm->qdo_empty[s][1]));
-                            ++pt;
+                        if (u == 0 && nsub > 0) {
+                            wait1(BAR(sm->acc_free), (nsub - 1) & 1);   // dV, dK of the previous sub-unit flushed
+                            if (bad) break;
+                            tc_fence_after_sync();
                         }
+                        umma_ts<4, 16, FP16>(r2, rx, tdo, u != 0);       // dV += P^T dO_g
+                        umma_ts<4, 16, FP16>(r3, rx + 8, tq, u != 0);    // dK += dS^T Q_g
+                        umma_commit(BAR(sm->qdo_empty[s][x]));
                     }
                     pds_ready = false;
                     if (u + 2 < 2 * ntiles) {
-                        // (The waits for a free Rx follow the order in which the output group hands the regions back, so no phase
-                        // of a barrier is passed over.)
-                        const bool both = u < 0 || is_proxy, proxy1 = KL && hh1 == P.mpp;
                         const uint32_t g = u < 0 ? gt : gt + 1, s = g & 1;
-                        const uint32_t tdo = tile_do0 + s * kTileBytes;
 #pragma unroll 1
-                        for (int fx = both ? 0 : x; fx < (both ? 2 * x : x + 1); ++fx) {
+                        for (int fx = u < 0 ? 0 : x; fx <= x; ++fx) {
                             const uint32_t rf = tmem + 128 * fx;
                             wait1(BAR(sm->qdo_full[s][fx]), (g >> 1) & 1);
-                            if (g >= 1 && is_proxy) {   // R0 held dKp^T, R1 the dQp^T of both halves
-                                wait1(fx == 0 ? BAR(sm->dkp_free) : BAR(sm->dq_free[0]), fx == 0 ? (pt - 1) & 1 : (g - 1) & 1);
-                                if (fx == 1) wait1(BAR(sm->dq_free[1]), (g - 1) & 1);
-                            }
                             if (bad) break;
                             tc_fence_after_sync();
-                            // S^T = K_j Q_g^T  (Sp^T = Kp_j Qp_g^T: the proxy keys sit in the dO stage)
-                            umma_ss<64, 8, false, false, FP16>(rf, proxy1 ? tdo : tile_k, tile_q0 + s * kTileBytes + fx * kHalfRowBytes, false);
-                            // the next step is that of the other half (of this tile, or of the next one after a second half)
-                            if (!both && !is_proxy && !(x == 1 && proxy1)) pds_ready = mbar_try_wait(BAR(sm->pds_full[x ^ 1]), (gt + x) & 1);
-                            if (!proxy1) {
-                                if (g >= 1 && !is_proxy) {
-                                    wait1(BAR(sm->dq_free[fx]), (g - 1) & 1);   // dQ^T has been read out
-                                    if (bad) break;
-                                    tc_fence_after_sync();
-                                }
-                                umma_ss<64, 8, false, false, FP16>(rf + 64, tile_v, tdo + fx * kHalfRowBytes, false);   // dP^T = V_j dO_g^T
+                            umma_ss<64, 8, false, false, FP16>(rf, tile_k, tile_q0 + s * kTileBytes + fx * kHalfRowBytes, false);   // S^T = K_j Q_g^T
+                            if (u >= 0) pds_ready = mbar_try_wait(BAR(sm->pds_full[x ^ 1]), (gt + x) & 1);
+                            if (g >= 1) {
+                                wait1(BAR(sm->dq_free[fx]), (g - 1) & 1);   // dQ^T has been read out
+                                if (bad) break;
+                                tc_fence_after_sync();
                             }
+                            umma_ss<64, 8, false, false, FP16>(rf + 64, tile_v, tile_do0 + s * kTileBytes + fx * kHalfRowBytes, false);   // dP^T = V_j dO_g^T
                             umma_commit(BAR(sm->sdp_full[fx]));
                         }
                     }
-                    if (x == 1) {
-                        if (u >= 0) ++gt;
-                        hh = hh1;
-                        if (++hh1 == hpc) hh1 = 0;
-                    }
+                    if (u >= 0 && x == 1) ++gt;
                 }
+                if (!bad) umma_commit(BAR(sm->kv_empty));
                 if (!bad) umma_commit(BAR(sm->acc_full));
             }
         } else if (warp == 16) {
             // =========================== K / V loads, row statistics ===========================
-            BwdUnit ud;
+            UnitRec ud;
             for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
                 if (nsub > 0) wait(BAR(sm->kv_empty), (nsub - 1) & 1, 1);
                 if (!bad && elect_one()) {
@@ -427,9 +334,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                         tma_load_4d(tile_k + i * kPanelBytes, i < 2 ? &tmap_k : &tmap_v, (i & 1) * 64, ud.j * kBlock, ud.kvh, ud.b, BAR(sm->kv_full));
                 }
                 __syncwarp();
-                // per main head: -lse * log2 e and -delta of the 128 rows; for the proxy head its -lse * log2 e
+                // per head: -lse * log2 e and -delta of the 128 rows
                 const int64_t head0 = (static_cast<int64_t>(ud.b) * P.Hq + ud.p * P.mpp) * P.S;
-                const float* proxy_lse = P.lse_proxy + (static_cast<int64_t>(ud.b) * P.Hp + ud.p) * P.S;
 #pragma unroll 1
                 for (int chunk = ud.chunk0; chunk < ud.chunk1 && !bad; ++chunk) {
                     int qid[4];
@@ -450,13 +356,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
 #pragma unroll 1
                     for (int hh = 0; hh < hpc; ++hh, ++gt) {
                         const uint32_t s = gt & 1;
-                        const bool proxy = KL && hh == P.mpp;
-                        if (proxy) lse_row = proxy_lse;
                         float nl[4], dl[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             nl[i] = qid[i] >= 0 ? -kLog2e * lse_row[qid[i]] : -INFINITY;
-                            dl[i] = qid[i] >= 0 && !proxy ? -delta_row[qid[i]] : 0.f;
+                            dl[i] = qid[i] >= 0 ? -delta_row[qid[i]] : 0.f;
                         }
                         lse_row += P.S;
                         delta_row += P.S;
@@ -480,20 +384,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         // =========================== row gather ===========================
         // Gather warp g fetches rows 32g .. 32g+31 of every tile, i.e. warps 0, 1 half 0 and warps 2, 3 half 1: lanes 0..15
         // issue the dO rows, lanes 16..31 the Q rows; a lane takes row quad (lane/2)%8 and 64-column panel lane%2.  Lane r
-        // holds the query position of row 32g + r.  In a proxy tile the Q stage takes the Qp rows and the dO stage the proxy
-        // keys of the block (one ordinary tile load by the first gather warp, whose half is consumed first).
+        // holds the query position of row 32g + r.
         const int g = warp - 12, half = g >> 1;
         const int quad = (lane >> 1) & 7, panel = lane & 1;
         const bool q_lane = lane >= 16;
         const int main_row_h = q_lane ? P.q_row_h : P.do_row_h, main_row_s = q_lane ? P.q_row_s : P.do_row_s;
         const int main_rows_total = q_lane ? P.q_rows_total : P.do_rows_total;
         const void* main_tmap = q_lane ? static_cast<const void*>(&tmap_q) : static_cast<const void*>(&tmap_do);
-        BwdUnit ud;
+        UnitRec ud;
         for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kDraws>{}); ++draw, ++nsub) {
             // matrix row of (this lane's tensor, first main head, position 0); row numbers fit 31 bits
             const int main_base = q_lane ? ud.b * P.q_row_b + ud.p * P.mpp * P.q_row_h : ud.b * P.do_row_b + ud.p * P.mpp * P.do_row_h;
-            const int qp_base = ud.b * P.qp_row_b + ud.p * P.qp_row_h;
-            const int kph = ud.p / P.pg;
             for (int chunk = ud.chunk0; chunk < ud.chunk1 && !bad; ++chunk) {
                 const int q = row_qid(ud, chunk * kBlock + 32 * g + lane);
                 int qr[4];
@@ -501,38 +402,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                 for (int i = 0; i < 4; ++i) qr[i] = __shfl_sync(0xffffffffu, q, 4 * quad + i);
                 for (int hh = 0; hh < hpc && !bad; ++hh, ++gt) {
                     const uint32_t s = gt & 1, ph = (gt >> 1) & 1;
-                    const bool proxy = KL && hh == P.mpp;
                     const uint32_t full = BAR(sm->qdo_full[s][half]);
                     const uint32_t off = panel * kPanelBytes + (32 * g + 4 * quad) * 128;
-                    if (gt >= 2) {
-                        wait(BAR(sm->qdo_empty[s][half]), ph ^ 1, 1);
-                        if (proxy && g == 0) wait(BAR(sm->qdo_empty[s][1]), ph ^ 1, 2);   // the keys fill both halves of the stage
-                    }
+                    if (gt >= 2) wait(BAR(sm->qdo_empty[s][half]), ph ^ 1, 1);
                     if (bad) break;
-                    if (elect_one()) {
-                        constexpr uint32_t kShare = kTileBytes / kBwdGatherWarps;   // this warp's rows of one tile
-                        if (!proxy) {
-                            mbar_arrive_expect_tx(full, 2 * kShare);
-                        } else if (g == 0) {
-                            mbar_arrive_expect_tx(full, kShare + kTileBytes);
-#pragma unroll 1
-                            for (int i = 0; i < 2; ++i)
-                                tma_load_4d(tile_do0 + s * kTileBytes + i * kPanelBytes, &tmap_kp, i * 64, ud.j * kBlock, kph, ud.b, full);
-                        } else {
-                            mbar_arrive_expect_tx(full, kShare);
-                        }
-                    }
+                    if (elect_one()) mbar_arrive_expect_tx(full, 2 * kTileBytes / kBwdGatherWarps);   // this warp's rows of both tiles
                     __syncwarp();
-                    // One issue site for the three tensors: every lane's gather4 goes through the uniform registers by itself, so
-                    // each site is a loop of its own in the code.
-                    const int base = proxy ? qp_base : main_base + hh * main_row_h;
-                    const int rs = proxy ? P.qp_row_s : main_row_s, oob = proxy ? P.qp_rows_total : main_rows_total;
+                    // One issue site for both tensors: every lane's gather4 goes through the uniform registers by itself, so each
+                    // site is a loop of its own in the code.
+                    const int base = main_base + hh * main_row_h;
                     int r[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) r[i] = qr[i] >= 0 ? base + qr[i] * rs : oob;
+                    for (int i = 0; i < 4; ++i) r[i] = qr[i] >= 0 ? base + qr[i] * main_row_s : main_rows_total;
                     const uint32_t dst = (q_lane ? tile_q0 : tile_do0) + s * kTileBytes + off;
-                    const void* tm = proxy ? static_cast<const void*>(&tmap_qp) : main_tmap;
-                    if (q_lane || !proxy) tma_gather4(dst, tm, panel * 64, r[0], r[1], r[2], r[3], full);
+                    tma_gather4(dst, main_tmap, panel * 64, r[0], r[1], r[2], r[3], full);
                 }
             }
         }
@@ -540,35 +423,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         reg_dec<kBwdRegsOutput>();
         // =========================== output group ===========================
         const int otid = tid - 8 * 32;
-        BwdUnit ud;
+        UnitRec ud;
         for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
             const int64_t slot_base = ud.e0 - edge_base;
-            const int kph = ud.p / P.pg;
             int hh = 0, chunk = ud.chunk0;
             for (int t = 0; t < ntiles && !bad; ++t, ++gt) {
-                const bool is_proxy = KL && hh == P.mpp;
                 const int64_t slot0 = slot_base + static_cast<int64_t>(chunk) * kBlock;
-                if (is_proxy) {
-                    wait(BAR(sm->dkp_full), pt & 1, 1);
-                    if (!bad) {
-                        tc_fence_after_sync();
-                        // dKp^T: lane = head-dimension index, column = key row: the 32 lanes of a warp add to 32
-                        // consecutive floats of one row per instruction
-                        float* kbase = P.dkp_acc + ((static_cast<int64_t>(ud.b) * P.Hpkv + kph) * P.S + ud.j * kBlock) * kHeadDim + row;
-#pragma unroll 1
-                        for (int c = 0; c < 128; c += 32) {
-                            uint32_t v[32];
-                            tmem_ld32(tmem_addr(r0, quarter, c), v);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) atomicAdd(kbase + static_cast<int64_t>(c + i) * kHeadDim, __uint_as_float(v[i]));
-                        }
-                        tc_fence_before_sync();
-                        warp_arrive(BAR(sm->dkp_free));
-                    }
-                    ++pt;
-                }
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
                     wait(BAR(sm->dq_full[x]), gt & 1, 2);
@@ -580,7 +441,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     // the TMA tile store.  With `split` the rows leave twice: rounded, and the remainder of that rounding (a second
                     // plane of the partial buffers, `part_slots` slots further on), so that the sum over many edges keeps
                     // fp32-like accuracy.
-                    const uint32_t src = is_proxy ? r1 + 64 * x : tmem + 128 * x + 64;
+                    const uint32_t src = tmem + 128 * x + 64;
                     const uint32_t stage = tile_ds + x * kPanelBytes;
                     const int nrows = min(64, ud.n - chunk * kBlock - 64 * x);   // <= 0: nothing to write
                     const int nparts = P.split ? 2 : 1;
@@ -618,10 +479,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                         named_barrier_sync(1, 128);
                         if (nrows == 64) {
                             if (warp == 8 && elect_one()) {
-                                const void* tm = is_proxy ? static_cast<const void*>(&tmap_dqp) : static_cast<const void*>(&tmap_dq);
 #pragma unroll 1
                                 for (int c = 0; c < 2; ++c)
-                                    tma_store_3d(tm, stage + c * (kPanelBytes / 2), 64 * c, is_proxy ? 0 : hh, static_cast<int>(pslot0));
+                                    tma_store_3d(&tmap_dq, stage + c * (kPanelBytes / 2), 64 * c, hh, static_cast<int>(pslot0));
                                 tma_store_commit();
                                 tma_store_wait_read();
                             }
@@ -629,7 +489,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                             // the ragged end of a reverse-index row (its slots end where the next row's begin)
                             for (int e = otid; e < nrows * 16; e += 128) {
                                 const int r = e >> 4, c = e & 15;
-                                __nv_bfloat16* grow = is_proxy ? P.dqp_part + (pslot0 + r) * kHeadDim : P.dq_part + ((pslot0 + r) * P.mpp + hh) * kHeadDim;
+                                __nv_bfloat16* grow = P.dq_part + ((pslot0 + r) * P.mpp + hh) * kHeadDim;
                                 *reinterpret_cast<uint4*>(grow + 8 * c) =
                                     ld_shared_v4(stage + (c >> 3) * (kPanelBytes / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
                             }
@@ -674,18 +534,16 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         // (16 bit) and dS^T into the shared tile that feeds dQ^T = K^T dS^T.
         const int qoff = (warp >> 2) * 32;   // first query of the group inside a half
         const float2 sc2 = make_float2(P.scale_log2e, P.scale_log2e);
-        const float inv_mpp = 1.f / static_cast<float>(P.mpp);
-        // sum over the main heads of P for this thread's 64 queries: the KL teacher, as packed fp16 pairs
-        // (values in [0,1], at most Hq/Hp addends; the result is rounded to bf16 anyway)
+        // Sum over the main heads of P for this thread's 64 queries: the KL teacher, as packed fp16 pairs (values in [0,1], at
+        // most Hq/Hp addends; what is formed from it is rounded to 16 bit anyway).  It goes to memory once per chunk.
         __half2 teacher[16], teacher_other[16];   // queries of this half, and of the other one: they change places after each
 #pragma unroll
         for (int i = 0; i < 16; ++i) teacher[i] = teacher_other[i] = __floats2half2_rn(0.f, 0.f);
-        BwdUnit ud;
+        UnitRec ud;
         for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
             int hh = 0, chunk = ud.chunk0;
             for (int t = 0; t < ntiles && !bad; ++t, ++gt) {
-                const bool is_proxy = KL && hh == P.mpp;
                 const uint32_t s = gt & 1;
                 wait(BAR(sm->st_full[s]), (gt >> 1) & 1, 1);
                 const BwdRowStats* st = &sm->stats[s];
@@ -702,43 +560,27 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     if (bad) break;
                     tc_fence_after_sync();
                     const bool masked = own || (VARLEN && sm->any_low[s] != 0);
-                    // KL(teacher || proxy) = sum t (ln t - ln p), when its value is asked for; t = 0 contributes nothing
-                    if (KL && is_proxy && P.kl_value) {
-                        uint32_t sv[32];
-                        tmem_ld32(tmem_addr(rc, quarter, 0), sv);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const float2 tt = __half22float2(teacher[i >> 1]);
-                            const float tv = ((i & 1) ? tt.y : tt.x) * inv_mpp;
-                            const float a = __uint_as_float(sv[i]) * P.scale_log2e + st->neg_lse[q0 + i];
-                            kl_acc += (tv > 0.f) ? tv * (fast_log2(tv) - a) : 0.f;
-                        }
-                    }
-                    // The body is instantiated per (masked, proxy) combination: the common tile (neither) must not pay for
-                    // predicated-off mask arithmetic or per-element branches in its inner loop.
-                    auto compute_half = [&](auto masked_c, auto proxy_c) __attribute__((always_inline)) {
+                    // Two instances of the body: the common tile must not pay for mask arithmetic.
+                    auto compute_half = [&](auto masked_c) __attribute__((always_inline)) {
                         constexpr bool kMasked = decltype(masked_c)::value;
-                        constexpr bool kProxy = decltype(proxy_c)::value;
                         // Two pieces of 16 columns: the TMEM loads of the second are in flight while the first is worked on
                         // (tcgen05.wait::ld waits for every load issued so far, hence the order wait, issue, compute).
                         uint32_t sv[2][16], dv[2][16];
                         tmem_ld16(tmem_addr(rc, quarter, 0), sv[0]);
-                        if (!kProxy) tmem_ld16(tmem_addr(rc, quarter, 64), dv[0]);
+                        tmem_ld16(tmem_addr(rc, quarter, 64), dv[0]);
 #pragma unroll
                         for (int cc = 0; cc < 2; ++cc) {
                             const int c = 16 * cc;
                             tmem_ld_wait();
                             if (cc == 0) {
                                 tmem_ld16(tmem_addr(rc, quarter, 16), sv[1]);
-                                if (!kProxy) tmem_ld16(tmem_addr(rc, quarter, 64 + 16), dv[1]);
+                                tmem_ld16(tmem_addr(rc, quarter, 64 + 16), dv[1]);
                             }
                             uint32_t pk[8], dk[8];
 #pragma unroll
                             for (int i4 = 0; i4 < 16; i4 += 4) {
                                 const float4 nl4 = *reinterpret_cast<const float4*>(&st->neg_lse[q0 + c + i4]);
-                                float4 nd4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                                if (!kProxy) nd4 = *reinterpret_cast<const float4*>(&st->neg_delta[q0 + c + i4]);
+                                const float4 nd4 = *reinterpret_cast<const float4*>(&st->neg_delta[q0 + c + i4]);
                                 uint32_t lim = 0x7f7f7f7fu, lw = 0u;
                                 if (kMasked) {
                                     if (own) lim = *reinterpret_cast<const uint32_t*>(&st->limit[q0 + c + i4]);
@@ -757,43 +599,44 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                                         p0 = (row <= l0 && (!VARLEN || row >= w0)) ? p0 : 0.f;
                                         p1 = (row <= l1 && (!VARLEN || row >= w1)) ? p1 : 0.f;
                                     }
-                                    const int ti = 8 * cc + (i >> 1);
-                                    if (!kProxy) {
-                                        // dS = P o (dP - delta)
-                                        const float2 nd2 = i2 ? make_float2(nd4.z, nd4.w) : make_float2(nd4.x, nd4.y);
-                                        const float2 d = f2_mul(make_float2(p0, p1), f2_add(f2_from_bits(dv[cc][i], dv[cc][i + 1]), nd2));
-                                        pk[i >> 1] = pack_act<FP16>(p0, p1);
-                                        dk[i >> 1] = pack_act<FP16>(d.x, d.y);
-                                        if (KL) teacher[ti] = __hadd2(teacher[ti], __floats2half2_rn(p0, p1));
-                                    } else {
-                                        const float2 tt = __half22float2(teacher[ti]);
-                                        dk[i >> 1] = pack_act<FP16>(p0 - tt.x * inv_mpp, p1 - tt.y * inv_mpp);
-                                        teacher[ti] = __floats2half2_rn(0.f, 0.f);
-                                    }
+                                    // dS = P o (dP - delta)
+                                    const float2 nd2 = i2 ? make_float2(nd4.z, nd4.w) : make_float2(nd4.x, nd4.y);
+                                    const float2 d = f2_mul(make_float2(p0, p1), f2_add(f2_from_bits(dv[cc][i], dv[cc][i + 1]), nd2));
+                                    pk[i >> 1] = pack_act<FP16>(p0, p1);
+                                    dk[i >> 1] = pack_act<FP16>(d.x, d.y);
+                                    if (KL) teacher[8 * cc + (i >> 1)] = __hadd2(teacher[8 * cc + (i >> 1)], __floats2half2_rn(p0, p1));
                                 }
                             }
                             // 16-bit operands back into TMEM over the 16 score columns this thread has consumed: P^T, then dS^T,
                             // two queries per column.  dS^T also goes to the half's panel of the shared tile that feeds
-                            // dQ^T = K^T dS^T (row = key, columns = queries); of a proxy tile nothing else is needed.
-                            if (!kProxy) {
-                                tmem_st8(tmem_addr(rc, quarter, c), pk);
-                                tmem_st8(tmem_addr(rc, quarter, c + 8), dk);
-                            }
+                            // dQ^T = K^T dS^T (row = key, columns = queries).
+                            tmem_st8(tmem_addr(rc, quarter, c), pk);
+                            tmem_st8(tmem_addr(rc, quarter, c + 8), dk);
                             st_shared_v4(ds_row + ((2 * (qoff + c)) ^ ((row & 7) << 4)), dk[0], dk[1], dk[2], dk[3]);
                             st_shared_v4(ds_row + ((2 * (qoff + c) + 16) ^ ((row & 7) << 4)), dk[4], dk[5], dk[6], dk[7]);
                         }
                     };
-                    if (KL && is_proxy) {
-                        compute_half(std::true_type{}, std::true_type{});
-                    } else {
-                        if (masked) compute_half(std::true_type{}, std::false_type{});
-                        else compute_half(std::false_type{}, std::false_type{});
-                        tmem_st_wait();
-                    }
+                    if (masked) compute_half(std::true_type{});
+                    else compute_half(std::false_type{});
+                    tmem_st_wait();
                     fence_async_smem();
                     tc_fence_before_sync();
                     warp_arrive(BAR(sm->pds_full[x]));
                     if (KL) {
+                        if (hh == hpc - 1) {
+                            // Teacher of the chunk: queries 2i, 2i+1 of the tile as one word per key, so that a pair of edges is 512
+                            // bytes [key][2] and a warp writes 128 consecutive ones; an odd last row of the reverse-index row
+                            // is 256 bytes [key].
+                            const int64_t slot = ud.e0 - edge_base + static_cast<int64_t>(chunk) * kBlock + q0;
+                            const int left = ud.n - chunk * kBlock - q0;   // rows from this thread's first query on
+                            uint32_t* dst = P.teacher + slot * 64 + row;
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                if (2 * i + 1 < left) dst[i * 128] = *reinterpret_cast<const uint32_t*>(&teacher[i]);
+                                else if (2 * i < left) reinterpret_cast<__half*>(dst - row + i * 128)[row] = __low2half(teacher[i]);
+                                teacher[i] = __floats2half2_rn(0.f, 0.f);
+                            }
+                        }
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const __half2 other = teacher[i];
@@ -817,10 +660,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         for (int i = 0; i < 8; ++i) g_bwd_trace[warp][i] = trace_acc[i];
     }
 #endif
-    if (P.kl_value && warp < 8) {
-        for (int o = 16; o > 0; o >>= 1) kl_acc += __shfl_xor_sync(0xffffffffu, kl_acc, o);
-        if (lane == 0) atomicAdd(P.kl_value, kl_acc * P.kl_value_scale);
-    }
     if (bad) {
         atomicMax(P.status, kStatusWaitTimeout);
         // Give loads and products that are still in flight time to finish before shared memory and TMEM are released.
@@ -1151,48 +990,34 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     FMSA_REQUIRE(gather_compatible(d_out->ptr, d_out->stride_b, d_out->stride_h, d_out->stride_s));
     if (with_kl) FMSA_REQUIRE(gather_compatible(q_proxy->ptr, q_proxy->stride_b, q_proxy->stride_h, q_proxy->stride_s));
     FMSA_REQUIRE(part_slots > 0 && part_slots * (split ? 2 : 1) < 0x7fffffffLL);
-    const fmsa_tensor* qpx = with_kl ? q_proxy : q;
-    const fmsa_tensor* kpx = with_kl ? k_proxy : k;
-    const int h_qpx = with_kl ? pb->Hp : pb->Hq, h_kpx = with_kl ? pb->Hpkv : pb->Hkv;
     const uint64_t q_rows = gather_rows(pb->B, pb->Hq, pb->S, q->stride_b, q->stride_h, q->stride_s);
     const uint64_t do_rows = gather_rows(pb->B, pb->Hq, pb->S, d_out->stride_b, d_out->stride_h, d_out->stride_s);
-    const uint64_t qp_rows = gather_rows(pb->B, h_qpx, pb->S, qpx->stride_b, qpx->stride_h, qpx->stride_s);
-    CUtensorMap tq, tdo, tqp, tk, tv, tkp, tdq, tdqp;
+    CUtensorMap tq, tdo, tk, tv, tdq;
     if (!make_tmap_gather(&tq, q->ptr, q_rows) || !make_tmap_gather(&tdo, d_out->ptr, do_rows) ||
-        !make_tmap_gather(&tqp, qpx->ptr, qp_rows) ||
         !make_tmap_bhsd(&tk, k->ptr, pb->B, pb->Hkv, pb->S, k->stride_b, k->stride_h, k->stride_s, 128) ||
         !make_tmap_bhsd(&tv, v->ptr, pb->B, pb->Hkv, pb->S, v->stride_b, v->stride_h, v->stride_s, 128) ||
-        !make_tmap_bhsd(&tkp, kpx->ptr, pb->B, h_kpx, pb->S, kpx->stride_b, kpx->stride_h, kpx->stride_s, 128) ||
         !make_tmap_partials_swz(&tdq, dq_part, static_cast<uint64_t>(part_slots) * (split ? 2 : 1),
-                                static_cast<uint64_t>(pb->Hq / pb->Hp), 64) ||
-        !make_tmap_partials_swz(&tdqp, with_kl ? dqp_part : dq_part, static_cast<uint64_t>(part_slots) * (split ? 2 : 1), 1, 64))
+                                static_cast<uint64_t>(pb->Hq / pb->Hp), 64))
         return FMSA_ERR_CUDA;
 
     BwdParams P;
     P.q_row_b = static_cast<int32_t>(q->stride_b / 128); P.q_row_h = static_cast<int32_t>(q->stride_h / 128); P.q_row_s = static_cast<int32_t>(q->stride_s / 128);
     P.do_row_b = static_cast<int32_t>(d_out->stride_b / 128); P.do_row_h = static_cast<int32_t>(d_out->stride_h / 128); P.do_row_s = static_cast<int32_t>(d_out->stride_s / 128);
-    P.qp_row_b = static_cast<int32_t>(qpx->stride_b / 128); P.qp_row_h = static_cast<int32_t>(qpx->stride_h / 128); P.qp_row_s = static_cast<int32_t>(qpx->stride_s / 128);
     P.q_rows_total = static_cast<int32_t>(q_rows); P.do_rows_total = static_cast<int32_t>(do_rows);
-    P.qp_rows_total = static_cast<int32_t>(qp_rows);
-    P.lse = lse; P.lse_proxy = lse_proxy; P.delta = delta;
-    P.row_ptr = row_ptr; P.col_q = col_q; P.doc_start = pb->doc_start;
-    P.dq_part = static_cast<__nv_bfloat16*>(dq_part); P.dqp_part = static_cast<__nv_bfloat16*>(dqp_part);
+    P.lse = lse; P.delta = delta;
+    P.col_q = col_q; P.doc_start = pb->doc_start;
+    P.dq_part = static_cast<__nv_bfloat16*>(dq_part); P.teacher = static_cast<uint32_t*>(dqp_part);
     P.part_slots = part_slots; P.split = split ? 1 : 0;
-    P.dkp_acc = dkp_acc; P.dk_acc = dk_acc; P.dv_acc = dv_acc;
-    P.counter = counter; P.status = status;
-    P.S = pb->S; P.NB = pb->S / kBlock; P.Hq = pb->Hq; P.Hkv = pb->Hkv; P.Hp = pb->Hp; P.Hpkv = pb->Hpkv;
-    P.mpp = pb->Hq / pb->Hp; P.ppk = pb->Hp / pb->Hkv; P.pg = pb->Hp / pb->Hpkv;
-    P.g_begin = g_begin; P.G = g_count;
-    P.dense = dense ? 1 : 0;
+    P.dk_acc = dk_acc; P.dv_acc = dv_acc;
+    P.status = status;
+    P.S = pb->S; P.Hq = pb->Hq; P.Hkv = pb->Hkv; P.mpp = pb->Hq / pb->Hp;
     P.scale_log2e = pb->scale * kLog2e;
-    P.kl_value = with_kl ? kl_value : nullptr;
-    P.kl_value_scale = kLn2 / (static_cast<float>(pb->B) * pb->Hp * pb->S);
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = device_sm_count();
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
     const bool varlen = P.doc_start != nullptr;
-    using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
+    using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
     static const KernelFn kernels[8] = {sparse_bwd_kernel<false, false, false>, sparse_bwd_kernel<false, false, true>,
                                         sparse_bwd_kernel<false, true, false>,  sparse_bwd_kernel<false, true, true>,
                                         sparse_bwd_kernel<true, false, false>,  sparse_bwd_kernel<true, false, true>,
@@ -1201,13 +1026,21 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     const void* kfn = reinterpret_cast<const void*>(kernel);
     if (sms <= 0 || !ensure_smem_attr(kfn, kBwdSmemBytes)) return FMSA_ERR_CUDA;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
-    P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
-    const int64_t per_group = subunits_per_group(P.NB, P.ppk, P.chunks);
+    UnitSpace& U = P.units;
+    U.row_ptr = row_ptr; U.counter = counter;
+    U.S = pb->S; U.NB = pb->S / kBlock; U.Hkv = pb->Hkv; U.Hp = pb->Hp; U.ppk = pb->Hp / pb->Hkv;
+    U.g_begin = g_begin; U.dense = dense ? 1 : 0;
+    U.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, U.NB, U.ppk, sms);
+    const int64_t per_group = subunits_per_group(U.NB, U.ppk, U.chunks);
     FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA)
-    P.units_per_group = static_cast<uint32_t>(per_group);
-    P.n_subunits = static_cast<int32_t>(per_group * g_count);
-    const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
-    kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tqp, tk, tv, tkp, tdq, tdqp, P);
+    U.per_group = static_cast<uint32_t>(per_group);
+    U.n_subunits = static_cast<int32_t>(per_group * g_count);
+    const int grid = U.n_subunits < sms ? U.n_subunits : sms;
+    kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tk, tv, tdq, P);
+    if (with_kl) {
+        const int rc = launch_proxy_bwd(pb, *q_proxy, *k_proxy, lse_proxy, U, col_q, dqp_part, part_slots, split, dkp_acc, kl_value, grid, status, st);
+        if (rc != FMSA_OK) return rc;
+    }
     return check_launch();
 }
 

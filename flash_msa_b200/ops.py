@@ -510,7 +510,7 @@ def attention_backward(q, k, v, q_proxy, k_proxy, out, grad_out, lse, lse_proxy,
     for g0 in range(0, groups, gstep):
         gc = min(gstep, groups - g0)
         with _Timed("attn_bwd", dev):
-            _launch("fmsa_sparse_bwd", 1, lib.fmsa_sparse_bwd(
+            _launch("fmsa_sparse_bwd", 2 if with_kl else 1, lib.fmsa_sparse_bwd(   # main kernel, proxy kernel
                 ctypes_byref(pb), _tensor_arg(q), _tensor_arg(k), _tensor_arg(v), _tensor_arg(qp), _tensor_arg(kp),
                 _tensor_arg(go), lse.data_ptr(), lse_proxy.data_ptr() if with_kl else 0, delta.data_ptr(), row_ptr, col_q,
                 dq_part.data_ptr(), dqp_part.data_ptr() if with_kl else 0, slots, split,

@@ -188,6 +188,8 @@ int fmsa_bwd_delta(const void* out, const fmsa_tensor* d_out, float* delta, int3
  *   dq_part    bf16 [slots, Hq/Hp, 128], dqp_part bf16 [slots, 128]: per-edge contributions to dQ and
  *              dQp (part_slots = slots >= fmsa_fwd_partial_slots); fmsa_sparse_bwd_combine sums them per row.
  *              Both are unscaled; the combine applies scale and scale/(B*Hp*S).
+ *              With with_kl = 1 a second kernel does the proxy head's part; dqp_part carries the KL teacher of every
+ *              edge between the two.
  *   split      0: one bf16 value per element, as above.  1: both buffers hold TWO planes of part_slots slots
  *              (so twice the size): plane 0 the contribution rounded to bf16, plane 1 the remainder of that
  *              rounding, and the combine adds both.  The sum over the edges of a row then keeps fp32-like
