@@ -89,6 +89,16 @@ def _declare(lib):
     lib.fmsa_cast_scaled.argtypes = [P, P, c_int64, P, c_float, c_int32, P]
     lib.fmsa_cast_scaled_rows.restype = c_int
     lib.fmsa_cast_scaled_rows.argtypes = [P, T, c_int32, c_int32, c_int32, P, c_float, c_int32, P]
+    lib.fmsa_forward_workspace_bytes.restype = c_int64
+    lib.fmsa_forward_workspace_bytes.argtypes = [PB, c_int32, c_int64]
+    lib.fmsa_backward_workspace_bytes.restype = c_int64
+    lib.fmsa_backward_workspace_bytes.argtypes = [PB, c_int32, c_int32, c_int32, c_int64]
+    lib.fmsa_forward.restype = c_int
+    lib.fmsa_forward.argtypes = [P, P, P, P]
+    lib.fmsa_backward.restype = c_int
+    lib.fmsa_backward.argtypes = [P, P, P, P]
+    lib.fmsa_doc_start.restype = c_int
+    lib.fmsa_doc_start.argtypes = [P, c_int32, c_int32, c_int32, c_int32, P, P]
     lib.fmsa_copy2d_async.restype = c_int
     lib.fmsa_copy2d_async.argtypes = [P, ctypes.c_size_t, P, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t, P]
 

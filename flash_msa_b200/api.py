@@ -5,15 +5,15 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import ops, passes
 
 BLOCK_SIZE = 128
 MAX_TOP_K_BLOCKS = 128
 
-# The device status word of every call (a bounded wait that ran out, a bad index in metadata) is checked
-# without synchronising: it is copied to pinned memory behind the call and looked at by the next call of the
-# library, which raises RuntimeError then; `check_pending_status()` waits for everything queued so far.
-# DEBUG_CHECK_STATUS = True reads the word right after every call instead (synchronises; for debugging).
+# The device status word of every call (a bounded wait that ran out, a bad index in metadata) is looked at
+# without synchronising: the kernels write it to pinned host memory, and the next call of the library raises
+# RuntimeError; `check_pending_status()` waits for everything queued so far.
+# DEBUG_CHECK_STATUS = True reads a word of the call's own right after every call instead (synchronises; for debugging).
 DEBUG_CHECK_STATUS = False
 
 
@@ -90,46 +90,26 @@ def _publish_kl(buf):
         _last_kl_value = buf.reshape(())
 
 
-def _maybe_check(status, what):
-    if DEBUG_CHECK_STATUS:
-        ops.check_status(status, what)
-    else:
-        ops.deferred_status.push(status, what)
+class _Status:
+    """Status word of one call."""
+
+    def __init__(self, kind, device):
+        self.kind = kind
+        if DEBUG_CHECK_STATUS:
+            self.word = torch.zeros(1, dtype=torch.int32, device=device)
+            self.ptr = self.word.data_ptr()
+        else:
+            self.word = None
+            self.ptr = passes.status_board.pointer(kind, device)
+
+    def check(self):
+        if self.word is not None:
+            ops.check_status(self.word, passes.StatusBoard.KINDS[self.kind])
 
 
 def check_pending_status():
-    """Waits for the status words of all calls issued so far and raises RuntimeError for a non-zero one."""
-    ops.deferred_status.drain()
-
-
-# Softmax bias ("attention sink": one learnable logit per main head that joins the softmax denominator and takes
-# probability mass without contributing a value; the reference lists it as missing).  It changes nothing but the
-# normaliser of a row, so it is applied around the kernels: lse' = logaddexp(lse, sink) and out' = out * exp(lse - lse')
-# after the forward; the backward runs on (out', lse') unchanged, because P = exp(s - lse') and delta = rowsum(out' dO)
-# are exactly what it needs.  The KL teacher (mean of the main probabilities) then has rows that sum to
-# T = mean_h exp(lse_h - lse'_h) < 1, and the gradient of -sum_k t_k log p_k becomes T p - t: the proxy log-sum-exp handed
-# to the backward is lowered by log T, which scales the proxy probabilities by T.  The sink's own gradient is
-# -sum over rows of exp(sink - lse') * delta.
-def _apply_sinks(out, lse_main, lse_proxy, sinks, hp):
-    b, hq, s = lse_main.shape
-    sk = sinks.detach().float().view(1, hq, 1)
-    lse2 = torch.logaddexp(lse_main, sk)
-    keep = torch.exp(lse_main - lse2)                                      # 1 - probability of the sink, [B,Hq,S]
-    out2 = (out.view(b, s, hq, -1).float() * keep.transpose(1, 2).unsqueeze(-1)).to(out.dtype).view(out.shape)
-    lse_proxy2 = None
-    if lse_proxy is not None:
-        lse_proxy2 = lse_proxy - torch.log(keep.view(b, hp, hq // hp, s).mean(dim=2))
-    return out2, lse2, lse_proxy2
-
-
-def _sink_grad(out_kernel, grad_out, lse_main, sinks):
-    """`out_kernel` is the output as the kernels wrote it (before the sink rescaling), `lse_main` the log-sum-exp WITH the
-    sink.  delta is formed from out_kernel * (1 - p_sink) in fp32: the rescaled output that the backward kernels read
-    has been rounded a second time, and the sum over all rows of a head amplifies that (measured: twice the error)."""
-    b, hq, s = lse_main.shape
-    p_sink = torch.exp(sinks.detach().float().view(1, hq, 1) - lse_main)                                       # [B,Hq,S]
-    delta = (out_kernel.view(b, s, hq, -1).float() * grad_out.reshape(b, s, hq, -1).float()).sum(-1).transpose(1, 2) * (1.0 - p_sink)
-    return (-(p_sink * delta).sum(dim=(0, 2))).to(sinks.dtype)
+    """Waits for all calls issued so far and raises RuntimeError if one of them reported trouble."""
+    passes.status_board.drain()
 
 
 def _check_sinks(sinks, q):
@@ -140,97 +120,61 @@ def _check_sinks(sinks, q):
     return sinks
 
 
-class _SparseAttentionFunction(torch.autograd.Function):
+def _sink_logits(sinks):
+    """fp32 contiguous logits as the kernels read them (a softmax bias, "attention sink": see fmsa_forward_args)."""
+    return None if sinks is None else sinks.detach().to(torch.float32).contiguous()
+
+
+class _AttentionFunction(torch.autograd.Function):
+    """Sparse (plan.dense False) or dense warmup attention behind autograd.  kl_loss is a placeholder whose gradient
+    switches the KL branch of the backward on (reference: flash_msa/msa_forward_cutedsl.py:69)."""
+
     @staticmethod
-    def forward(ctx, q_proxy, k_proxy, q, k, v, top_k, scale, doc_start=None, sinks=None):
-        num_blocks, top_k_blocks = _validate_inputs(q_proxy, k_proxy, q, k, v, int(top_k), True)
-        _require_cuda(q)
-        sinks = _check_sinks(sinks, q)
-        status = torch.zeros(1, dtype=torch.int32, device=q.device)
-        if top_k_blocks <= ops.FUSED_SELECT_MAX_BLOCKS:
-            block_indices = ops.select_blocks_fused(q_proxy, k_proxy, float(scale), top_k_blocks, status=status,
-                                                    doc_start=doc_start)
-        else:
-            scores = ops.proxy_block_scores(q_proxy, k_proxy, float(scale), status=status, doc_start=doc_start)
-            block_indices = ops.select_topk(scores, top_k_blocks)
-            del scores
-        rix = ops.build_reverse_index(block_indices)
-        out, lse_main, lse_proxy = ops.attention_forward(q, k, v, q_proxy, k_proxy, float(scale), rix, status=status,
-                                                         doc_start=doc_start)
-        _maybe_check(status, "flash_msa_func forward")
-        ctx.out_kernel = None
-        if sinks is not None:
-            ctx.out_kernel = out
-            out, lse_main, lse_proxy = _apply_sinks(out, lse_main, lse_proxy, sinks, q_proxy.shape[1])
-        ctx.sinks = sinks
-        # kl_loss is a placeholder whose gradient switches the KL branch of the backward on
-        # (reference: flash_msa/msa_forward_cutedsl.py:69)
-        kl_loss = torch.zeros((), dtype=torch.float32, device=q.device)
-        ctx.save_for_backward(q_proxy, k_proxy, q, k, v, out, lse_main, lse_proxy, rix.row_ptr, rix.col_q, rix.edge_pos)
+    def forward(ctx, q_proxy, k_proxy, q, k, v, sinks, doc_start, plan):
+        status = _Status(2 if plan.dense else 0, plan.device)
+        logits = _sink_logits(sinks)
+        out, kl_loss, saved = passes.forward(plan, (q_proxy, k_proxy, q, k, v), doc_start, logits, status.ptr, True)
+        status.check()
+        ctx.save_for_backward(q_proxy, k_proxy, q, k, v, out, saved)
         # an output that does not feed the loss arrives as None in backward (not as zeros): no gradient for
         # kl_loss then really skips the proxy work, as the reference intends (flash_msa/flash_msa.py:104-106)
         ctx.set_materialize_grads(False)
-        ctx.scale = float(scale)
-        ctx.top_k_blocks = top_k_blocks
-        ctx.doc_start = doc_start
+        ctx.plan, ctx.doc_start, ctx.logits = plan, doc_start, logits
+        ctx.sinks_dtype = None if sinks is None else sinks.dtype
         return out, kl_loss
 
     @staticmethod
     def backward(ctx, grad_out, grad_kl):
-        q_proxy, k_proxy, q, k, v, out, lse_main, lse_proxy, row_ptr, col_q, edge_pos = ctx.saved_tensors
-        b, _, s, _ = q.shape
+        q_proxy, k_proxy, q, k, v, out, saved = ctx.saved_tensors
+        plan = ctx.plan
         if grad_out is None:
             grad_out = torch.zeros_like(out)
-        rix = ops.ReverseIndex(row_ptr, col_q, edge_pos, b, q_proxy.shape[1], s, ctx.top_k_blocks)
-        status = torch.zeros(1, dtype=torch.int32, device=q.device)
-        klv = _kl_buffer(grad_kl, q.device)
-        dqp, dkp, dq, dk, dv = ops.attention_backward(q, k, v, q_proxy, k_proxy, out, grad_out, lse_main, lse_proxy,
-                                                      ctx.scale, rix, grad_kl, status=status, kl_value=klv,
-                                                      doc_start=ctx.doc_start)
+        status = _Status(3 if plan.dense else 1, plan.device)
+        klv = _kl_buffer(grad_kl, plan.device)
+        dqp, dkp, dq, dk, dv, dsinks = passes.backward(plan, (q_proxy, k_proxy, q, k, v), out, grad_out, saved, grad_kl, klv, ctx.doc_start,
+                                                       ctx.logits, status.ptr)
         _publish_kl(klv)
-        _maybe_check(status, "flash_msa_func backward")
-        dsinks = _sink_grad(ctx.out_kernel, grad_out, lse_main, ctx.sinks) if ctx.sinks is not None else None
-        return dqp, dkp, dq, dk, dv, None, None, None, dsinks
+        status.check()
+        return dqp, dkp, dq, dk, dv, None if dsinks is None else dsinks.to(ctx.sinks_dtype), None, None
 
 
-class _WarmupSparseAttentionFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q_proxy, k_proxy, q, k, v, top_k, scale, doc_start=None, sinks=None):
-        _ = int(top_k)                         # accepted and ignored, as in the reference
-        _validate_inputs(q_proxy, k_proxy, q, k, v, 0, False)
-        sinks = _check_sinks(sinks, q)
-        if q.device.type != "cuda":
-            raise RuntimeError("warmup MSA forward requires CUDA tensors")
-        status = torch.zeros(1, dtype=torch.int32, device=q.device)
-        out, lse_main, lse_proxy = ops.attention_forward(q, k, v, q_proxy, k_proxy, float(scale), None, dense=True,
-                                                         status=status, doc_start=doc_start)
-        _maybe_check(status, "flash_msa_warmup_func forward")
-        ctx.out_kernel = None
-        if sinks is not None:
-            ctx.out_kernel = out
-            out, lse_main, lse_proxy = _apply_sinks(out, lse_main, lse_proxy, sinks, q_proxy.shape[1])
-        ctx.sinks = sinks
-        kl_loss = torch.zeros((), dtype=torch.float32, device=q.device)
-        ctx.save_for_backward(q_proxy, k_proxy, q, k, v, out, lse_main, lse_proxy)
-        ctx.set_materialize_grads(False)
-        ctx.scale = float(scale)
-        ctx.doc_start = doc_start
-        return out, kl_loss
-
-    @staticmethod
-    def backward(ctx, grad_out, grad_kl):
-        q_proxy, k_proxy, q, k, v, out, lse_main, lse_proxy = ctx.saved_tensors
-        if grad_out is None:
-            grad_out = torch.zeros_like(out)
-        status = torch.zeros(1, dtype=torch.int32, device=q.device)
-        klv = _kl_buffer(grad_kl, q.device)
-        dqp, dkp, dq, dk, dv = ops.attention_backward(q, k, v, q_proxy, k_proxy, out, grad_out, lse_main, lse_proxy,
-                                                      ctx.scale, None, grad_kl, dense=True, status=status, kl_value=klv,
-                                                      doc_start=ctx.doc_start)
-        _publish_kl(klv)
-        _maybe_check(status, "flash_msa_warmup_func backward")
-        dsinks = _sink_grad(ctx.out_kernel, grad_out, lse_main, ctx.sinks) if ctx.sinks is not None else None
-        return dqp, dkp, dq, dk, dv, None, None, None, dsinks
+def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks):
+    q_proxy = _spread_proxy_heads(q_proxy, k_proxy, q, k)
+    _, top_k_blocks = _validate_inputs(q_proxy, k_proxy, q, k, v, top_k if sparse else 0, sparse)
+    if sparse:
+        _require_cuda(q)
+    sinks = _check_sinks(sinks, q)
+    if q.device.type != "cuda":
+        raise RuntimeError("warmup MSA forward requires CUDA tensors")
+    inputs = (q_proxy, k_proxy, q, k, v)
+    plan = passes.plan(inputs, top_k_blocks, scale, not sparse)
+    if torch.is_grad_enabled() and (any(t.requires_grad for t in inputs) or (sinks is not None and sinks.requires_grad)):
+        return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, plan)
+    # no backward will follow: the proxy log-sum-exp, which only the backward needs, is left out
+    status = _Status(0 if sparse else 2, plan.device)
+    out, kl_loss, _ = passes.forward(plan, inputs, doc_start, _sink_logits(sinks), status.ptr, False)
+    status.check()
+    return out, kl_loss
 
 
 def _spread_proxy_heads(q_proxy, k_proxy, q, k):
@@ -249,11 +193,18 @@ def _spread_proxy_heads(q_proxy, k_proxy, q, k):
     return q_proxy   # (anything else is judged by the shape checks of the call)
 
 
+def _doc_start(q, cu_seqlens):
+    if q.ndim != 4:
+        raise ValueError("all attention tensors must have shape (B, H, S, D)")
+    _require_cuda(q)
+    return ops.doc_start_from_cu_seqlens(cu_seqlens, q.shape[0], q.shape[2], q.device)
+
+
 def sparse_attention(q_proxy, k_proxy, q, k, v, top_k: int, scale: float, sinks=None):
     """Block-sparse top-k GQA attention.  Returns ``(attn_out [B,S,Hq*D], kl_loss placeholder)``.
-    ``sinks`` (optional, beyond the reference): one softmax-bias logit per main query head, see `_apply_sinks`."""
-    return _SparseAttentionFunction.apply(_spread_proxy_heads(q_proxy, k_proxy, q, k), k_proxy, q, k, v, int(top_k), float(scale), None,
-                                          sinks)
+    ``sinks`` (optional, beyond the reference): one softmax-bias logit per main query head that joins the softmax
+    denominator and contributes no value."""
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, None, sinks)
 
 
 def sparse_attention_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, scale: float, sinks=None):
@@ -262,28 +213,18 @@ def sparse_attention_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, s
     varlen convention) gives their boundaries, and a query sees only the keys of its own document - in the block scores
     and the selection, in the attention and in every gradient.  Blocks stay 128 positions of the PACKED sequence, so S
     must still be a multiple of 128 (pad the last document).  The reference has no such path (its README lists
-    variable-length batches as missing)."""
-    if q.ndim != 4:
-        raise ValueError("all attention tensors must have shape (B, H, S, D)")
-    _require_cuda(q)
-    doc_start = ops.doc_start_from_cu_seqlens(cu_seqlens, q.shape[0], q.shape[2], q.device)
-    return _SparseAttentionFunction.apply(_spread_proxy_heads(q_proxy, k_proxy, q, k), k_proxy, q, k, v, int(top_k), float(scale), doc_start,
-                                          sinks)
+    variable-length batches as missing).  Boundaries in host memory (a list, a CPU tensor) spare the call a wait."""
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, _doc_start(q, cu_seqlens), sinks)
 
 
 def sparse_attention_warmup(q_proxy, k_proxy, q, k, v, top_k: int, scale: float, sinks=None):
-    """Dense causal warmup attention with full-sequence proxy KL gradients."""
-    return _WarmupSparseAttentionFunction.apply(_spread_proxy_heads(q_proxy, k_proxy, q, k), k_proxy, q, k, v, int(top_k), float(scale), None,
-                                                sinks)
+    """Dense causal warmup attention with full-sequence proxy KL gradients (top_k is accepted and ignored, as in the
+    reference)."""
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), False, None, sinks)
 
 
 def sparse_attention_warmup_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, scale: float, sinks=None):
     """`sparse_attention_warmup` on packed sequences (see `sparse_attention_varlen`): dense causal attention and the
     full-sequence proxy KL inside every document.  The schedule still visits every causal block pair of the packed
     sequence; pairs that straddle documents are masked."""
-    if q.ndim != 4:
-        raise ValueError("all attention tensors must have shape (B, H, S, D)")
-    _require_cuda(q)
-    doc_start = ops.doc_start_from_cu_seqlens(cu_seqlens, q.shape[0], q.shape[2], q.device)
-    return _WarmupSparseAttentionFunction.apply(_spread_proxy_heads(q_proxy, k_proxy, q, k), k_proxy, q, k, v, int(top_k), float(scale), doc_start,
-                                                sinks)
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), False, _doc_start(q, cu_seqlens), sinks)

@@ -1,0 +1,49 @@
+// Launchers shared by the C-ABI entry points of single stages and the whole-pass entry points (pipeline.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "../../include/flash_msa_b200.h"
+
+namespace fmsa {
+
+// `counter`: one zeroed word.
+int launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                      const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr, const int32_t* col_q,
+                      void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
+                      int32_t* counter, int32_t* status, cudaStream_t st);
+// `sinks`: fp32 [Hq] softmax-bias logits or null; `zero`: a device scalar to clear on the way, or null.
+int launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
+                       const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
+                       int g_begin, int g_count, int dense, cudaStream_t st);
+// `counter`, `counter_proxy`: zeroed here if `zero_counters` (they may then be the same word).
+int launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                      const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const fmsa_tensor* d_out, const float* lse,
+                      const float* lse_proxy, const float* delta, const int32_t* row_ptr, const int32_t* col_q, void* dq_part,
+                      void* dqp_part, int64_t part_slots, int split, float* dkp_acc, float* dk_acc, float* dv_acc, int g_begin,
+                      int g_count, int with_kl, int dense, float* kl_value, int32_t* counter, int32_t* counter_proxy,
+                      bool zero_counters, int32_t* status, cudaStream_t st);
+
+// One (B,H,S,128) gradient from its contiguous fp32 accumulator: dst = 16-bit (src * scale * (*factor or 1)).
+struct CastJob {
+    const float* src;
+    void* dst;
+    const float* factor;
+    int64_t sb, sh, ss;
+    float scale;
+    uint32_t H, n8;      // heads; eighths of the element count
+};
+struct CastJobs {
+    CastJob job[3];
+    uint32_t S;
+};
+int launch_cast_grads(const CastJobs& jobs, int count, bool fp16, cudaStream_t st);
+int launch_sink_grad(const float* lse, const float* delta, const float* sinks, float* dsinks, int B, int S, int Hq, cudaStream_t st);
+
+// `zero`, `nzero`: words to clear on the way, or null.
+int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos, int64_t rows_bh,
+                         int32_t S, int32_t Kb, void* scratch, cudaStream_t st, int32_t* zero = nullptr, int nzero = 0);
+size_t reverse_index_scratch_bytes(int64_t rows_bh, int32_t S);
+
+}  // namespace fmsa

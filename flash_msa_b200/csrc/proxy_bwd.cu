@@ -527,7 +527,6 @@ int launch_proxy_bwd(const fmsa_problem* pb, const fmsa_tensor& q_proxy, const f
                                         proxy_bwd_kernel<true, true>};
     const KernelFn kernel = kernels[(pb->dtype == FMSA_DTYPE_FP16 ? 2 : 0) + (pb->doc_start ? 1 : 0)];
     if (!ensure_smem_attr(reinterpret_cast<const void*>(kernel), kProxySmemBytes)) return FMSA_ERR_CUDA;
-    if (cudaMemsetAsync(units.counter, 0, sizeof(int32_t), stream) != cudaSuccess) return FMSA_ERR_CUDA;
     kernel<<<grid, kProxyThreads, kProxySmemBytes, stream>>>(tqp, tkp, tdqp, P);
     return check_launch();
 }

@@ -15,6 +15,7 @@
 #include <mutex>
 
 #include "host_common.h"
+#include "launch.h"
 #include "sm100.cuh"
 
 namespace fmsa {
@@ -77,7 +78,9 @@ __global__ void rix_colscan_kernel(const uint8_t* __restrict__ counts, int32_t* 
 }
 
 __global__ void __launch_bounds__(1024) rix_rowscan_kernel(const int32_t* __restrict__ totals,
-                                                           int32_t* __restrict__ row_ptr, int64_t n) {
+                                                           int32_t* __restrict__ row_ptr, int64_t n, int32_t* __restrict__ zero, int nzero) {
+    if (zero)   // words a later kernel of the sequence wants to find zeroed
+        for (int i = threadIdx.x; i < nzero; i += 1024) zero[i] = 0;
     __shared__ int64_t part[1024];
     const int tid = threadIdx.x;
     const int64_t per = (n + 1023) / 1024;
@@ -161,7 +164,7 @@ RixWorkspace carve(void* base, int64_t rows_bh, int NB) {
 
 // Launch sequence shared with any other entry point that supplies its own scratch memory.
 int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos,
-                         int64_t rows_bh, int32_t S, int32_t Kb, void* scratch, cudaStream_t st) {
+                         int64_t rows_bh, int32_t S, int32_t Kb, void* scratch, cudaStream_t st, int32_t* zero, int nzero) {
     const int NB = S / kBlock;
     const RixWorkspace w = carve(scratch, rows_bh, NB);
     const dim3 grid(static_cast<unsigned>(NB), static_cast<unsigned>(rows_bh));
@@ -175,7 +178,7 @@ int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t
     rix_count_kernel<<<grid, 128, smem, st>>>(block_indices, w.counts, S, NB, Kb);
     const int64_t cols = rows_bh * NB;
     rix_colscan_kernel<<<static_cast<unsigned>((cols + 127) / 128), 128, 0, st>>>(w.counts, w.blk_off, w.totals, rows_bh, NB);
-    rix_rowscan_kernel<<<1, 1024, 0, st>>>(w.totals, row_ptr, cols);
+    rix_rowscan_kernel<<<1, 1024, 0, st>>>(w.totals, row_ptr, cols, zero, nzero);
     rix_fill_kernel<<<grid, 128, smem, st>>>(block_indices, w.blk_off, row_ptr, col_q, edge_pos, S, NB, Kb);
     return check_launch();
 }

@@ -33,6 +33,7 @@
 #include <type_traits>
 
 #include "host_common.h"
+#include "launch.h"
 #include "msa_common.cuh"
 #include "proxy_bwd.h"
 #include "sm100.cuh"
@@ -896,7 +897,66 @@ __global__ void __launch_bounds__(256) cast_scaled_rows_kernel(const float* __re
     }
 }
 
+// dsinks[h] = -sum over the rows of head h of exp(sink_h - lse') * delta: one CTA per head, in a fixed order.
+__global__ void __launch_bounds__(512) sink_grad_kernel(const float* __restrict__ lse, const float* __restrict__ delta,
+                                                        const float* __restrict__ sinks, float* __restrict__ dsinks, int B, int S, int Hq) {
+    __shared__ float part[16];
+    const int h = blockIdx.x;
+    const float sk = sinks[h];
+    float sum = 0.f;
+    for (int b = 0; b < B; ++b) {
+        const int64_t at = (static_cast<int64_t>(b) * Hq + h) * S;
+        for (int s = threadIdx.x; s < S; s += 512) sum += expf(sk - lse[at + s]) * delta[at + s];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float total = 0.f;
+        for (int i = 0; i < 16; ++i) total += part[i];
+        dsinks[h] = -total;
+    }
+}
+
+// dK, dV and dKp from their fp32 accumulators in one launch (blockIdx.y): 8 elements per thread into (B,H,S,128) views.
+template <bool FP16>
+__global__ void __launch_bounds__(256) cast_grads_kernel(const CastJobs J) {
+    const CastJob& c = J.job[blockIdx.y];
+    const float f = (c.factor ? *c.factor : 1.f) * c.scale;
+    const uint32_t n8 = c.n8, stride = gridDim.x * 256;
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n8; i += stride) {
+        const uint32_t rowi = i >> 4, c8 = (i & 15) * 8;
+        const uint32_t bh = rowi / J.S, sq = rowi - bh * J.S, b = bh / c.H, h = bh - b * c.H;
+        const float4 v0 = reinterpret_cast<const float4*>(c.src)[2 * static_cast<int64_t>(i)];
+        const float4 v1 = reinterpret_cast<const float4*>(c.src)[2 * static_cast<int64_t>(i) + 1];
+        uint4 o;
+        o.x = pack_act<FP16>(v0.x * f, v0.y * f);
+        o.y = pack_act<FP16>(v0.z * f, v0.w * f);
+        o.z = pack_act<FP16>(v1.x * f, v1.y * f);
+        o.w = pack_act<FP16>(v1.z * f, v1.w * f);
+        *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(c.dst) + b * c.sb + h * c.sh + sq * c.ss + c8) = o;
+    }
+}
+
 }  // namespace
+
+int launch_cast_grads(const CastJobs& jobs, int count, bool fp16, cudaStream_t st) {
+    uint32_t most = 0;
+    for (int i = 0; i < count; ++i) most = jobs.job[i].n8 > most ? jobs.job[i].n8 : most;
+    uint32_t grid = (most + 255) / 256;
+    if (grid > 148 * 8) grid = 148 * 8;
+    const dim3 g(grid, static_cast<unsigned>(count));
+    if (fp16) cast_grads_kernel<true><<<g, 256, 0, st>>>(jobs);
+    else cast_grads_kernel<false><<<g, 256, 0, st>>>(jobs);
+    return check_launch();
+}
+
+int launch_sink_grad(const float* lse, const float* delta, const float* sinks, float* dsinks, int B, int S, int Hq, cudaStream_t st) {
+    sink_grad_kernel<<<Hq, 512, 0, st>>>(lse, delta, sinks, dsinks, B, S, Hq);
+    return check_launch();
+}
+
 }  // namespace fmsa
 
 extern "C" int fmsa_cast_scaled_rows(const float* src, const fmsa_tensor* dst, int32_t B, int32_t H, int32_t S,
@@ -965,6 +1025,17 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
                                const int32_t* col_q, void* dq_part, void* dqp_part, int64_t part_slots, int32_t split,
                                float* dkp_acc, float* dk_acc, float* dv_acc, int32_t g_begin, int32_t g_count, int32_t with_kl,
                                int32_t dense, float* kl_value, int32_t* counter, int32_t* status, void* stream) {
+    return fmsa::launch_sparse_bwd(pb, q, k, v, q_proxy, k_proxy, d_out, lse, lse_proxy, delta, row_ptr, col_q, dq_part, dqp_part,
+                                   part_slots, split, dkp_acc, dk_acc, dv_acc, g_begin, g_count, with_kl, dense, kl_value, counter,
+                                   counter, true, status, static_cast<cudaStream_t>(stream));
+}
+
+int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                            const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const fmsa_tensor* d_out, const float* lse,
+                            const float* lse_proxy, const float* delta, const int32_t* row_ptr, const int32_t* col_q, void* dq_part,
+                            void* dqp_part, int64_t part_slots, int split, float* dkp_acc, float* dk_acc, float* dv_acc, int g_begin,
+                            int g_count, int with_kl, int dense, float* kl_value, int32_t* counter, int32_t* counter_proxy,
+                            bool zero_counters, int32_t* status, cudaStream_t st) {
     using namespace fmsa;
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(q && k && v && d_out && q->ptr && k->ptr && v->ptr && d_out->ptr);
@@ -1013,7 +1084,6 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     P.S = pb->S; P.Hq = pb->Hq; P.Hkv = pb->Hkv; P.mpp = pb->Hq / pb->Hp;
     P.scale_log2e = pb->scale * kLog2e;
 
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = device_sm_count();
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
     const bool varlen = P.doc_start != nullptr;
@@ -1025,7 +1095,7 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     const KernelFn kernel = kernels[(fp16 ? 4 : 0) + (varlen ? 2 : 0) + (with_kl ? 1 : 0)];
     const void* kfn = reinterpret_cast<const void*>(kernel);
     if (sms <= 0 || !ensure_smem_attr(kfn, kBwdSmemBytes)) return FMSA_ERR_CUDA;
-    if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
+    if (zero_counters && cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
     UnitSpace& U = P.units;
     U.row_ptr = row_ptr; U.counter = counter;
     U.S = pb->S; U.NB = pb->S / kBlock; U.Hkv = pb->Hkv; U.Hp = pb->Hp; U.ppk = pb->Hp / pb->Hkv;
@@ -1038,6 +1108,8 @@ extern "C" int fmsa_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     const int grid = U.n_subunits < sms ? U.n_subunits : sms;
     kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tk, tv, tdq, P);
     if (with_kl) {
+        if (zero_counters && cudaMemsetAsync(counter_proxy, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
+        U.counter = counter_proxy;
         const int rc = launch_proxy_bwd(pb, *q_proxy, *k_proxy, lse_proxy, U, col_q, dqp_part, part_slots, split, dkp_acc, kl_value, grid, status, st);
         if (rc != FMSA_OK) return rc;
     }

@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "host_common.h"
+#include "launch.h"
 #include "msa_common.cuh"
 #include "sm100.cuh"
 #include "tma_host.h"
@@ -639,6 +640,8 @@ struct CombineParams {
     int S, NB, Hq, Hp, mpp, ppk, Kb;
     int g_begin, G, dense;
     int hgroup;                // main heads per blockIdx.y of the row kernel
+    const float* sinks;        // [Hq] softmax-bias logits or null
+    float* zero;               // a scalar to set to zero, or null
 };
 
 // Two kernels.  The partial rows of all main heads of one edge are contiguous (mpp * 256 bytes), so a warp reads them with
@@ -680,7 +683,11 @@ struct CombineRow {
     }
 };
 
-template <int LPR, bool DENSE>   // lanes per query row: 16 (two rows per warp, at most 16 edges per row) or 32
+// SINKS: one extra logit per main head joins the row's softmax (it takes probability and contributes no value): it is merged
+// into the row's log-sum-exp here, and the row kernel, whose weights come from that, then needs nothing else.  The KL
+// teacher's rows then sum to T = mean_h exp(lse_h - lse'_h) < 1, and the gradient of -sum_k t_k log p_k becomes T p - t: the
+// proxy log-sum-exp is lowered by log T, which scales the proxy probabilities by T.
+template <int LPR, bool DENSE, bool SINKS>   // LPR lanes per query row: 16 (two rows per warp, at most 16 edges per row) or 32
 __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P) {
     constexpr int kMaxHeads = kWideMaxHeads + 1;
     const int lane = threadIdx.x & 31, l = lane % LPR;
@@ -690,42 +697,56 @@ __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P)
     const CombineRow<DENSE> row(P, valid ? w0 : nrows - 1);
     const int lse_stride = P.mpp + 1;
     const float2* stats = reinterpret_cast<const float2*>(P.lse_part);
-    const int h0 = blockIdx.y * kMaxHeads;   // first head of this block's group; head number mpp is the proxy
-    const int nheads = min(kMaxHeads, P.mpp + (P.lse_proxy ? 1 : 0) - h0);
-    float hm[kMaxHeads], hs[kMaxHeads];
-#pragma unroll
-    for (int hh = 0; hh < kMaxHeads; ++hh) {
-        hm[hh] = -INFINITY;
-        hs[hh] = 0.f;
-    }
-    for (int s0 = 0; s0 < row.nslots; s0 += LPR) {
-        const int sl = valid ? row.slot_of(P, s0 + l) : -1;
-        const float2* rec = stats + static_cast<int64_t>(sl) * lse_stride + h0;
+    if (P.zero && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *P.zero = 0.f;
+    float keep = 0.f;   // SINKS: sum over the main heads of exp(lse - lse')
+    // Groups of heads (head number mpp is the proxy): one per blockIdx.y, or with SINKS one after another.
+    for (int h0 = blockIdx.y * kMaxHeads; h0 < P.mpp + (P.lse_proxy ? 1 : 0); h0 += gridDim.y * kMaxHeads) {
+        const int nheads = min(kMaxHeads, P.mpp + (P.lse_proxy ? 1 : 0) - h0);
+        float hm[kMaxHeads], hs[kMaxHeads];
 #pragma unroll
         for (int hh = 0; hh < kMaxHeads; ++hh) {
-            if (hh < nheads && sl >= 0) {
-                const float2 st = rec[hh];
-                const float mn = fmaxf(hm[hh], st.x);
-                hs[hh] = hs[hh] * fast_exp2(hm[hh] - mn) + st.y * fast_exp2(st.x - mn);
-                hm[hh] = mn;
+            hm[hh] = -INFINITY;
+            hs[hh] = 0.f;
+        }
+        for (int s0 = 0; s0 < row.nslots; s0 += LPR) {
+            const int sl = valid ? row.slot_of(P, s0 + l) : -1;
+            const float2* rec = stats + static_cast<int64_t>(sl) * lse_stride + h0;
+#pragma unroll
+            for (int hh = 0; hh < kMaxHeads; ++hh) {
+                if (hh < nheads && sl >= 0) {
+                    const float2 st = rec[hh];
+                    const float mn = fmaxf(hm[hh], st.x);
+                    hs[hh] = hs[hh] * fast_exp2(hm[hh] - mn) + st.y * fast_exp2(st.x - mn);
+                    hm[hh] = mn;
+                }
             }
         }
-    }
-    // Across the row's lanes: first the maximum, then the sums brought to it (half the instructions of merging
-    // (max, sum) pairs in every round; the kernel is bound by instruction issue, not by memory).
+        // Across the row's lanes: first the maximum, then the sums brought to it (half the instructions of merging
+        // (max, sum) pairs in every round; the kernel is bound by instruction issue, not by memory).
 #pragma unroll
-    for (int hh = 0; hh < kMaxHeads; ++hh) {
-        if (hh < nheads) {
-            float m = hm[hh];
+        for (int hh = 0; hh < kMaxHeads; ++hh) {
+            if (hh < nheads) {
+                float m = hm[hh];
 #pragma unroll
-            for (int off = LPR / 2; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-            float sum = (hm[hh] == -INFINITY) ? 0.f : hs[hh] * fast_exp2(hm[hh] - m);
+                for (int off = LPR / 2; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+                float sum = (hm[hh] == -INFINITY) ? 0.f : hs[hh] * fast_exp2(hm[hh] - m);
 #pragma unroll
-            for (int off = LPR / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            if (l == 0 && valid) {
-                const float total = (m + __log2f(sum)) * kLn2;   // natural-log LSE of the whole row
-                if (h0 + hh == P.mpp) P.lse_proxy[row.bp * P.S + row.q] = total;
-                else P.lse[(static_cast<int64_t>(row.b) * P.Hq + row.p * P.mpp + h0 + hh) * P.S + row.q] = total;
+                for (int off = LPR / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+                if (l == 0 && valid) {
+                    float total = (m + __log2f(sum)) * kLn2;   // natural-log LSE of the whole row
+                    if (SINKS) {
+                        if (h0 + hh == P.mpp) {
+                            total -= logf(keep / static_cast<float>(P.mpp));
+                        } else {
+                            const float sk = P.sinks[row.p * P.mpp + h0 + hh];
+                            const float with = fmaxf(total, sk) + log1pf(expf(-fabsf(total - sk)));
+                            keep += expf(total - with);
+                            total = with;
+                        }
+                    }
+                    if (h0 + hh == P.mpp) P.lse_proxy[row.bp * P.S + row.q] = total;
+                    else P.lse[(static_cast<int64_t>(row.b) * P.Hq + row.p * P.mpp + h0 + hh) * P.S + row.q] = total;
+                }
             }
         }
     }
@@ -836,6 +857,16 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
                                const int32_t* col_q, void* o_part, float* lse_part, int64_t part_slots, int32_t g_begin,
                                int32_t g_count, int32_t with_proxy, int32_t dense, int32_t* counter, int32_t* status,
                                void* stream) {
+    if (!counter) return FMSA_ERR_ARGUMENT;
+    if (cudaMemsetAsync(counter, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream)) != cudaSuccess) return FMSA_ERR_CUDA;
+    return fmsa::launch_sparse_fwd(pb, q, k, v, q_proxy, k_proxy, row_ptr, col_q, o_part, lse_part, part_slots, g_begin, g_count,
+                                   with_proxy, dense, counter, status, static_cast<cudaStream_t>(stream));
+}
+
+int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                            const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr, const int32_t* col_q,
+                            void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
+                            int32_t* counter, int32_t* status, cudaStream_t st) {
     using namespace fmsa;
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(q && k && v && q->ptr && k->ptr && v->ptr && o_part && lse_part && counter && status);
@@ -880,14 +911,12 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
     P.g_begin = g_begin; P.G = g_count; P.with_proxy = with_proxy ? 1 : 0; P.dense = dense ? 1 : 0;
     P.scale_log2e = pb->scale * kLog2e;
 
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = device_sm_count();
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
     const bool varlen = P.doc_start != nullptr;
     const void* kfn = fp16 ? (varlen ? reinterpret_cast<const void*>(sparse_fwd_kernel<true, true>) : reinterpret_cast<const void*>(sparse_fwd_kernel<true, false>))
                            : (varlen ? reinterpret_cast<const void*>(sparse_fwd_kernel<false, true>) : reinterpret_cast<const void*>(sparse_fwd_kernel<false, false>));
     if (sms <= 0 || !ensure_smem_attr(kfn, kFwdSmemBytes)) return FMSA_ERR_CUDA;
-    if (cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
     P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
     const int64_t per_group = subunits_per_group(P.NB, P.ppk, P.chunks);
     FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA)
@@ -904,6 +933,13 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
 extern "C" int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part,
                                        const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse,
                                        float* lse_proxy, int32_t g_begin, int32_t g_count, int32_t dense, void* stream) {
+    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, nullptr, g_begin, g_count,
+                                    dense, static_cast<cudaStream_t>(stream));
+}
+
+int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
+                             const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
+                             int g_begin, int g_count, int dense, cudaStream_t cst) {
     using namespace fmsa;
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(o_part && lse_part && out && lse);
@@ -914,21 +950,24 @@ extern "C" int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_par
     P.out = static_cast<__nv_bfloat16*>(out); P.lse = lse; P.lse_proxy = lse_proxy;
     P.S = pb->S; P.NB = pb->S / kBlock; P.Hq = pb->Hq; P.Hp = pb->Hp; P.mpp = pb->Hq / pb->Hp; P.ppk = pb->Hp / pb->Hkv;
     P.Kb = pb->top_k_blocks; P.g_begin = g_begin; P.G = g_count; P.dense = dense ? 1 : 0;
+    P.sinks = sinks; P.zero = zero;
     const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * P.S;
     const int64_t grid = (rows + 7) / 8;
     FMSA_REQUIRE(grid <= 0x7fffffffLL);
-    cudaStream_t cst = static_cast<cudaStream_t>(stream);
     const bool f16 = pb->dtype == FMSA_DTYPE_FP16;
     // Up to eight main heads per proxy head one block takes them all; beyond, groups of (nearly) equal size of at most six
     // heads: the three-sweep form has its loads in flight without spilling.
     const int row_groups = P.mpp <= kWideMaxHeads ? 1 : (P.mpp + 5) / 6;
     P.hgroup = (P.mpp + row_groups - 1) / row_groups;
-    const int lse_groups = (P.mpp + (lse_proxy ? 1 : 0) + kWideMaxHeads) / (kWideMaxHeads + 1);
+    const int lse_groups = sinks ? 1 : (P.mpp + (lse_proxy ? 1 : 0) + kWideMaxHeads) / (kWideMaxHeads + 1);
     const dim3 cg(static_cast<unsigned>(grid), static_cast<unsigned>(row_groups));
-    const dim3 lg(static_cast<unsigned>(grid), static_cast<unsigned>(lse_groups));
-    if (dense) combine_lse_kernel<32, true><<<lg, 256, 0, cst>>>(P);
-    else if (P.Kb <= 16) combine_lse_kernel<16, false><<<dim3(static_cast<unsigned>((rows + 15) / 16), static_cast<unsigned>(lse_groups)), 256, 0, cst>>>(P);
-    else combine_lse_kernel<32, false><<<lg, 256, 0, cst>>>(P);
+    const bool half_warps = !dense && P.Kb <= 16;
+    const dim3 lg(static_cast<unsigned>(half_warps ? (rows + 15) / 16 : grid), static_cast<unsigned>(lse_groups));
+#define FMSA_LSE(L, D) (sinks ? combine_lse_kernel<L, D, true><<<lg, 256, 0, cst>>>(P) : combine_lse_kernel<L, D, false><<<lg, 256, 0, cst>>>(P))
+    if (dense) FMSA_LSE(32, true);
+    else if (half_warps) FMSA_LSE(16, false);
+    else FMSA_LSE(32, false);
+#undef FMSA_LSE
 #define FMSA_ROWS3(K, F, G) (dense ? combine_rows_kernel<K, F, true, G><<<cg, 256, 0, cst>>>(P) : combine_rows_kernel<K, F, false, G><<<cg, 256, 0, cst>>>(P))
 #define FMSA_ROWS(K, G) (f16 ? FMSA_ROWS3(K, true, G) : FMSA_ROWS3(K, false, G))
     if (row_groups > 1) FMSA_ROWS(3, true);

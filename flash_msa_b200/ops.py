@@ -7,6 +7,7 @@ from dataclasses import dataclass
 import ctypes
 import os
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -48,7 +49,8 @@ class _Timed:
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _require_cuda(*tensors):
@@ -221,10 +223,26 @@ def _problem(q, k, q_proxy, k_proxy, top_k_blocks, scale, doc_start=None) -> "_l
                             _dtype_code(q.dtype), doc_start.data_ptr() if doc_start is not None else None)
 
 
+MAX_HOST_BOUNDARIES = 896   # FMSA_MAX_HOST_BOUNDARIES of the header
+
+
 def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> torch.Tensor:
     """int32 [B,S] on `device`: for every token of a packed sequence the position of the first token of its document.
     `cu_seqlens` is [n+1] (one packing for every batch element) or [B,n+1]; it starts at 0 and ends at `seq_len`
     (the FlashAttention varlen convention).  The kernels take this array (`fmsa_problem.doc_start`)."""
+    if not (isinstance(cu_seqlens, torch.Tensor) and cu_seqlens.device.type == "cuda"):
+        # boundaries that the host holds are checked here and travel as a kernel parameter: nothing waits for the device
+        cu = np.asarray(cu_seqlens)
+        if cu.ndim not in (1, 2) or (cu.ndim == 2 and cu.shape[0] != batch) or cu.shape[-1] < 2:
+            raise ValueError("cu_seqlens must have shape [n+1] or [B, n+1]")
+        if (cu[..., 0] != 0).any() or (cu[..., -1] != seq_len).any() or (cu[..., 1:] < cu[..., :-1]).any():
+            raise ValueError("cu_seqlens must rise from 0 to the sequence length")
+        if cu.size <= MAX_HOST_BOUNDARIES and torch.device(device).type == "cuda":
+            cu = np.ascontiguousarray(cu, dtype=np.int32)
+            out = torch.empty(batch, seq_len, dtype=torch.int32, device=device)
+            _launch("fmsa_doc_start", 1, _lib.load().fmsa_doc_start(cu.ctypes.data, cu.shape[-1], int(cu.ndim == 2), batch, seq_len,
+                                                                 out.data_ptr(), _stream(out.device)), out.device)
+            return out
     cu = torch.as_tensor(cu_seqlens).to(device=device, dtype=torch.int64)
     if cu.dim() == 1:
         cu = cu.unsqueeze(0).expand(batch, -1)
@@ -313,8 +331,6 @@ class DeferredStatus:
         """Waits for every queued status word and raises for the first non-zero one."""
         self._poll(block=True)
 
-
-deferred_status = DeferredStatus()
 
 
 def proxy_block_scores(q_proxy: torch.Tensor, k_proxy: torch.Tensor, scale: float, status=None, doc_start=None) -> torch.Tensor:

@@ -1,0 +1,263 @@
+"""Whole forward and backward passes: one C call each (csrc/pipeline.cu) on one workspace.
+
+What depends only on shapes, strides, types and options - the argument block, sizes, layouts - is worked out once and
+kept as a plan; a call then fills in pointers.  (Driven stage by stage the host took 0.65 ms for a training pass of
+B=1 S=1024 Hq=8, six times what the GPU needs.)"""
+from __future__ import annotations
+
+import ctypes
+from ctypes import c_float, c_int32, c_int64, c_void_p
+
+import torch
+
+from . import _lib, ops
+
+_STAGES = ("select_scores", "reverse_index", "attn_fwd", "fwd_combine", "bwd_delta", "attn_bwd", "bwd_combine", "cast")
+
+
+def _tensor_fields(name):
+    return [(name, c_void_p), (name + "_sb", c_int64), (name + "_sh", c_int64), (name + "_ss", c_int64)]
+
+
+_PROBLEM = list(_lib.FmsaProblem._fields_)
+_INPUTS = sum((_tensor_fields(n) for n in ("q", "k", "v", "q_proxy", "k_proxy")), [])
+
+
+class ForwardArgs(ctypes.Structure):
+    """Mirror of ``fmsa_forward_args`` with its nested structs laid out flat (same offsets)."""
+    _fields_ = _PROBLEM + _INPUTS + [
+        ("sinks", c_void_p), ("dense", c_int32), ("with_proxy", c_int32), ("max_partial_bytes", c_int64), ("workspace_bytes", c_int64),
+        ("workspace", c_void_p), ("row_ptr", c_void_p), ("col_q", c_void_p), ("edge_pos", c_void_p), ("out", c_void_p),
+        ("lse", c_void_p), ("lse_proxy", c_void_p), ("kl_loss", c_void_p), ("status", c_void_p)]
+
+
+class BackwardArgs(ctypes.Structure):
+    """Mirror of ``fmsa_backward_args``, flat."""
+    _fields_ = _PROBLEM + _INPUTS + _tensor_fields("d_out") + [
+        ("sinks", c_void_p), ("dense", c_int32), ("with_kl", c_int32), ("split_above", c_int32), ("reserved", c_int32),
+        ("max_partial_bytes", c_int64), ("workspace_bytes", c_int64), ("workspace", c_void_p), ("row_ptr", c_void_p),
+        ("col_q", c_void_p), ("edge_pos", c_void_p), ("out", c_void_p), ("lse", c_void_p), ("lse_proxy", c_void_p),
+        ("grad_kl", c_void_p)] + sum((_tensor_fields(n) for n in ("dq", "dk", "dv", "dq_proxy", "dk_proxy")), []) + [
+        ("dsinks", c_void_p), ("kl_value", c_void_p), ("status", c_void_p)]
+
+
+class Marks(ctypes.Structure):
+    """Mirror of ``fmsa_marks``."""
+    _fields_ = [("events", ctypes.POINTER(c_void_p)), ("stages", ctypes.POINTER(c_int32)), ("capacity", c_int32), ("used", c_int32)]
+
+
+class _Timing:
+    """Events around every stage of one call while `ops.KERNEL_EVENTS` collects them (used by the benchmark)."""
+    CAPACITY = 128
+    _spare = []
+
+    def __init__(self):
+        spare = _Timing._spare
+        while len(spare) < self.CAPACITY:
+            e = torch.cuda.Event(enable_timing=True)
+            e.record()             # creates the CUDA event
+            spare.append(e)
+        self.handles = (c_void_p * self.CAPACITY)(*(e.cuda_event for e in spare[:self.CAPACITY]))
+        self.stages = (c_int32 * self.CAPACITY)()
+        self.marks = Marks(ctypes.cast(self.handles, ctypes.POINTER(c_void_p)), ctypes.cast(self.stages, ctypes.POINTER(c_int32)),
+                           self.CAPACITY, 0)
+
+    def publish(self):
+        n = self.marks.used
+        events, _Timing._spare = _Timing._spare[:n], _Timing._spare[n:]
+        for i in range(0, n - 1, 2):
+            ops.KERNEL_EVENTS.append((_STAGES[self.stages[i]], events[i], events[i + 1]))
+
+
+def _conforms(shape, stride):
+    """What the kernels read in place (see `ops._as_kernel_input`); a dimension of one position may have any stride."""
+    return stride[3] == 1 and all(st % 128 == 0 and st > 0 for st in stride[:3])
+
+
+def _bshd(shape, stride):
+    """Whether the tensor is a (B,H,S,D) view of dense (B,S,H,D) storage: its gradient is then written in that layout."""
+    b, h, s, d = shape
+    return h > 1 and stride == (s * h * d, d, h * d, 1)
+
+
+class Plan:
+    """Everything about a call that shapes, strides, types and options decide."""
+
+    def __init__(self, inputs, top_k_blocks, scale, dense, max_partial_bytes):
+        qp, kp, q, k, v = inputs
+        lib = _lib.load()
+        b, hq, s, d = q.shape
+        hkv, hp, hpkv = k.shape[1], qp.shape[1], kp.shape[1]
+        self.dense, self.shape, self.dtype, self.device = dense, (b, hq, s, d), q.dtype, q.device
+        self.pb = _lib.FmsaProblem(b, s, hq, hkv, hp, hpkv, 1 if dense else int(top_k_blocks), float(scale), ops._dtype_code(q.dtype), None)
+        self.max_partial_bytes = int(max_partial_bytes)
+        self.copies = [i for i, t in enumerate(inputs) if not _conforms(t.shape, t.stride())]
+        self.grad_shapes = [((b, s, t.shape[1], d), True) if _bshd(t.shape, t.stride()) else (tuple(t.shape), False) for t in inputs]
+        self.out_shape = (b, s, hq * d)
+        pbr = ctypes.byref(self.pb)
+        self.forward_bytes = lib.fmsa_forward_workspace_bytes(pbr, int(dense), self.max_partial_bytes)
+        # saved for the backward, one int32 tensor: row_ptr | col_q | edge_pos | lse | lse_proxy, each from a 64-word boundary
+        nb, edges = s // ops.BLOCK_SIZE, 0 if dense else b * hp * s * int(top_k_blocks)
+        sizes = [0 if dense else b * hp * nb + 1, edges, edges, b * hq * s, b * hp * s]
+        self.at, off = [], 0
+        for n in sizes:
+            self.at.append(4 * off)
+            off += (n + 63) // 64 * 64
+        self.saved_words = off
+        self.forward_args = bytes(self._args(ForwardArgs, inputs, workspace_bytes=self.forward_bytes))
+        self._backward = {}
+
+    def _args(self, kind, inputs, **more):
+        a = kind(*(getattr(self.pb, f) for f, _ in _PROBLEM), dense=int(self.dense), max_partial_bytes=self.max_partial_bytes, **more)
+        for name, i in (("q_proxy", 0), ("k_proxy", 1), ("q", 2), ("k", 3), ("v", 4)):
+            self._strides(a, name, inputs[i].contiguous().stride() if i in self.copies else inputs[i].stride())
+        return a
+
+    @staticmethod
+    def _strides(a, name, stride):
+        setattr(a, name + "_sb", stride[0])
+        setattr(a, name + "_sh", stride[1])
+        setattr(a, name + "_ss", stride[2])
+
+    def backward_template(self, inputs, with_kl):
+        """(argument block, workspace bytes) of a backward with or without the KL work."""
+        got = self._backward.get(with_kl)
+        if got is None:
+            nbytes = _lib.load().fmsa_backward_workspace_bytes(ctypes.byref(self.pb), int(self.dense), int(with_kl), ops.SPLIT_PARTIALS_ABOVE,
+                                                               self.max_partial_bytes)
+            a = self._args(BackwardArgs, inputs, with_kl=int(with_kl), split_above=ops.SPLIT_PARTIALS_ABOVE, workspace_bytes=nbytes)
+            for name, (shape, bshd) in zip(("dq_proxy", "dk_proxy", "dq", "dk", "dv"), self.grad_shapes):
+                n1, n2 = shape[1], shape[2]
+                self._strides(a, name, (n1 * n2 * 128, 128, n2 * 128) if bshd else (n1 * n2 * 128, n2 * 128, 128))
+            got = self._backward[with_kl] = (bytes(a), nbytes)
+        return got
+
+    def conform(self, inputs):
+        """The inputs as the kernels can read them: in place, or copied once."""
+        if not self.copies and all(t.data_ptr() % 16 == 0 for t in inputs):
+            return inputs
+        return [t.contiguous() if i in self.copies else (t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.preserve_format))
+                for i, t in enumerate(inputs)]
+
+
+_plans = {}
+_MAX_PLANS = 256
+
+
+def plan(inputs, top_k_blocks, scale, dense) -> Plan:
+    q = inputs[2]
+    key = (top_k_blocks, scale, dense, ops.MAX_PARTIAL_BYTES, ops.SPLIT_PARTIALS_ABOVE, q.dtype, q.device,
+           *[t.shape for t in inputs], *[t.stride() for t in inputs])
+    p = _plans.get(key)
+    if p is None:
+        if len(_plans) >= _MAX_PLANS:
+            _plans.clear()
+        p = _plans[key] = Plan(inputs, top_k_blocks, scale, dense, ops.MAX_PARTIAL_BYTES)
+    return p
+
+
+def _call(fn, what, args, device):
+    timing = _Timing() if ops.KERNEL_EVENTS is not None else None
+    launches = c_int32(0)
+    _lib.check(fn(ctypes.byref(args), ctypes.byref(timing.marks) if timing else None, ctypes.byref(launches), ops._stream(device)), what)
+    ops.LAUNCHES += launches.value
+    if timing:
+        timing.publish()
+
+
+def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
+    """Returns (out [B,S,Hq*128], kl_loss placeholder, saved).  `sinks`: fp32 [Hq] or None."""
+    qp, kp, q, k, v = p.conform(inputs)
+    dev = p.device
+    a = ForwardArgs.from_buffer_copy(p.forward_args)
+    out = torch.empty(p.out_shape, dtype=p.dtype, device=dev)
+    kl = torch.empty((), dtype=torch.float32, device=dev)
+    saved = torch.empty(p.saved_words, dtype=torch.int32, device=dev)
+    ws = torch.empty(p.forward_bytes, dtype=torch.uint8, device=dev)
+    a.q_proxy, a.k_proxy, a.q, a.k, a.v = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
+    base, at = saved.data_ptr(), p.at
+    if not p.dense:
+        a.row_ptr, a.col_q, a.edge_pos = base + at[0], base + at[1], base + at[2]
+    a.lse, a.lse_proxy = base + at[3], base + at[4]
+    a.with_proxy = 1 if with_proxy else 0
+    a.out, a.kl_loss, a.workspace, a.status = out.data_ptr(), kl.data_ptr(), ws.data_ptr(), status_ptr
+    if doc_start is not None:
+        a.doc_start = doc_start.data_ptr()
+    if sinks is not None:
+        a.sinks = sinks.data_ptr()
+    _call(_lib.load().fmsa_forward, "fmsa_forward", a, dev)
+    return out, kl, saved
+
+
+def backward(p: Plan, inputs, out, grad_out, saved, grad_kl, kl_value, doc_start, sinks, status_ptr):
+    """Returns (dq_proxy, dk_proxy, dq, dk, dv, dsinks) in the inputs' type and layout; `grad_kl`, `kl_value`: fp32 scalars or None."""
+    qp, kp, q, k, v = p.conform(inputs)
+    dev = p.device
+    b, hq, s, d = p.shape
+    if grad_out.dtype != p.dtype:
+        grad_out = grad_out.to(p.dtype)
+    st = grad_out.stride()
+    if grad_out.dim() != 3 or st[2] != 1 or st[0] % 128 or st[1] % 128 or st[0] <= 0 or st[1] <= 0 or grad_out.data_ptr() % 16:
+        grad_out = grad_out.reshape(p.out_shape).clone(memory_format=torch.contiguous_format)
+        st = grad_out.stride()
+    template, nbytes = p.backward_template(inputs, grad_kl is not None)
+    a = BackwardArgs.from_buffer_copy(template)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    grads = [torch.empty(shape, dtype=p.dtype, device=dev) for shape, _ in p.grad_shapes]
+    a.q_proxy, a.k_proxy, a.q, a.k, a.v = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
+    a.d_out, a.d_out_sb, a.d_out_sh, a.d_out_ss = grad_out.data_ptr(), st[0], 128, st[1]
+    a.dq_proxy, a.dk_proxy, a.dq, a.dk, a.dv = (g.data_ptr() for g in grads)
+    base, at = saved.data_ptr(), p.at
+    if not p.dense:
+        a.row_ptr, a.col_q, a.edge_pos = base + at[0], base + at[1], base + at[2]
+    a.lse, a.lse_proxy = base + at[3], base + at[4]
+    a.out, a.workspace, a.status = out.data_ptr(), ws.data_ptr(), status_ptr
+    if grad_kl is not None:
+        if grad_kl.dtype != torch.float32 or grad_kl.device != dev:
+            grad_kl = grad_kl.to(device=dev, dtype=torch.float32)
+        a.grad_kl = grad_kl.data_ptr()
+        if kl_value is not None:
+            a.kl_value = kl_value.data_ptr()
+    if doc_start is not None:
+        a.doc_start = doc_start.data_ptr()
+    dsinks = None
+    if sinks is not None:
+        dsinks = torch.empty(hq, dtype=torch.float32, device=dev)
+        a.sinks, a.dsinks = sinks.data_ptr(), dsinks.data_ptr()
+    _call(_lib.load().fmsa_backward, "fmsa_backward", a, dev)
+    return [g.transpose(1, 2) if bshd else g for g, (_, bshd) in zip(grads, p.grad_shapes)] + [dsinks]
+
+
+class StatusBoard:
+    """Status words of the calls of this process, in pinned host memory that the kernels write directly (only ever when
+    something is wrong), so that a call needs no word of its own, no copy and no event.  A word is one of a few kinds of
+    call; trouble raises RuntimeError at the next call of the library or at `drain`."""
+    KINDS = ("flash_msa_func forward", "flash_msa_func backward", "flash_msa_warmup_func forward", "flash_msa_warmup_func backward")
+
+    def __init__(self):
+        self._words = None
+        self._devices = set()
+
+    def pointer(self, kind: int, device) -> int:
+        if self._words is None:
+            self._keep = torch.zeros(16, dtype=torch.int32).pin_memory()
+            self._words = (c_int32 * 16).from_address(self._keep.data_ptr())
+        self._devices.add(device)
+        self.poll()
+        return ctypes.addressof(self._words) + 4 * kind
+
+    def poll(self) -> None:
+        if self._words is not None and any(self._words):
+            for i, what in enumerate(self.KINDS):
+                code = self._words[i]
+                if code:
+                    self._words[i] = 0
+                    raise RuntimeError(f"{what} (reported late): {ops._STATUS_NAMES.get(code, code)}")
+
+    def drain(self) -> None:
+        for device in list(self._devices):
+            torch.cuda.synchronize(device)
+        self.poll()
+
+
+status_board = StatusBoard()

@@ -245,6 +245,69 @@ int fmsa_cast_scaled_rows(const float* src, const fmsa_tensor* dst, int32_t B, i
 int fmsa_copy2d_async(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t rows,
                       void* stream);
 
+/* Whole passes.  One call launches the stages above in order, in as many passes over (batch, KV head) groups as keep the
+ * partial rows of a pass within max_partial_bytes, out of one workspace (256-byte aligned, size from the *_workspace_bytes
+ * functions).  Beside the stages: `sinks`, fp32 [Hq] softmax-bias logits (one per main head: it joins the softmax denominator
+ * and contributes no value; the reference lists it as missing) or NULL.  lse, lse_proxy and out are then those with the
+ * sinks, dsinks [Hq] their gradient.
+ * kl_loss: fp32 scalar set to zero (the reference's placeholder), or NULL.  with_proxy = 0 leaves out the proxy log-sum-exp,
+ * which only a backward needs.  dense ignores row_ptr, col_q and edge_pos.
+ * dq_proxy and dk_proxy are zeroed when with_kl = 0.  All five gradients are dense (B,H,S,128) or (B,S,H,128) storage.
+ * split_above: rows with more edges than this store two planes of partial rows (`split` above).
+ * *launches: number of kernels launched.  marks: NULL, or CUDA events to record before and after every stage. */
+typedef struct {
+    fmsa_problem pb;
+    fmsa_tensor q, k, v, q_proxy, k_proxy;
+    const float* sinks;
+    int32_t dense, with_proxy;
+    int64_t max_partial_bytes, workspace_bytes;
+    void* workspace;
+    int32_t *row_ptr, *col_q, *edge_pos;
+    void* out;
+    float *lse, *lse_proxy, *kl_loss;
+    int32_t* status;
+} fmsa_forward_args;
+
+typedef struct {
+    fmsa_problem pb;
+    fmsa_tensor q, k, v, q_proxy, k_proxy, d_out;
+    const float* sinks;
+    int32_t dense, with_kl, split_above, reserved;
+    int64_t max_partial_bytes, workspace_bytes;
+    void* workspace;
+    const int32_t *row_ptr, *col_q, *edge_pos;
+    const void* out;
+    const float *lse, *lse_proxy, *grad_kl;
+    fmsa_tensor dq, dk, dv, dq_proxy, dk_proxy;
+    float *dsinks, *kl_value;
+    int32_t* status;
+} fmsa_backward_args;
+
+#define FMSA_STAGE_SELECT 0
+#define FMSA_STAGE_REVERSE_INDEX 1
+#define FMSA_STAGE_ATTN_FWD 2
+#define FMSA_STAGE_FWD_COMBINE 3
+#define FMSA_STAGE_DELTA 4
+#define FMSA_STAGE_ATTN_BWD 5
+#define FMSA_STAGE_BWD_COMBINE 6
+#define FMSA_STAGE_CAST 7
+typedef struct {
+    void** events;    /* cudaEvent_t [capacity], recorded in pairs: before and after a stage */
+    int32_t* stages;  /* [capacity], the stage of each recorded event */
+    int32_t capacity, used;
+} fmsa_marks;
+
+int64_t fmsa_forward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int64_t max_partial_bytes);
+int fmsa_forward(const fmsa_forward_args* args, fmsa_marks* marks, int32_t* launches, void* stream);
+int64_t fmsa_backward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int32_t with_kl, int32_t split_above,
+                                      int64_t max_partial_bytes);
+int fmsa_backward(const fmsa_backward_args* args, fmsa_marks* marks, int32_t* launches, void* stream);
+
+/* doc_start [B,S] (see fmsa_problem) from document boundaries in HOST memory: [n], or [B][n] with per_batch = 1; each list
+ * starts at 0, ends at S and does not fall.  At most FMSA_MAX_HOST_BOUNDARIES in all (they travel as a kernel parameter). */
+#define FMSA_MAX_HOST_BOUNDARIES 896
+int fmsa_doc_start(const int32_t* boundaries, int32_t n, int32_t per_batch, int32_t B, int32_t S, int32_t* doc_start, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

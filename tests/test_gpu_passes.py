@@ -1,0 +1,86 @@
+"""The whole-pass entry points where they branch: softmax sinks with one and several groups of heads in the log-sum-exp
+kernel, inputs that have to be copied first, a forward without a backward, document boundaries from host and device
+memory, the status words in host memory."""
+import pytest
+import torch
+
+from oracle import msa_oracle as O
+from tests.gpu_util import SCALE, bf16_inputs, kernel_selection, max_err, yardstick_check
+
+pytestmark = pytest.mark.gpu
+NAMES = ["dq_proxy", "dk_proxy", "dq", "dk", "dv"]
+
+
+@pytest.mark.parametrize("mpp", [1, 8, 9, 12])
+def test_sinks_over_groups_of_heads(mpp):
+    import flash_msa_b200 as fm
+    cfg = dict(b=2, s=384, hq=2 * mpp, hkv=2, hp=2, hpkv=1, kb=2, seed=80 + mpp)
+    qp, kp, q, k, v, do = bf16_inputs(cfg)
+    sinks = (torch.randn(cfg["hq"], generator=torch.Generator().manual_seed(mpp)) + 1.0).cuda().requires_grad_(True)
+    leaves = [t.detach().requires_grad_(True) for t in (qp, kp, q, k, v)]
+    out, kl = fm.flash_msa_func(*leaves, cfg["kb"] * 128, SCALE, sinks=sinks)
+    torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+    idx = kernel_selection(qp, kp, cfg["kb"])
+    args = (qp, kp, q, k, v, cfg["kb"] * 128, SCALE, do, 1.0)
+    r32 = O.sparse_forward_backward(*args, block_indices=idx, sinks=sinks.detach())
+    r16 = O.sparse_forward_backward(*args, block_indices=idx, sinks=sinks.detach(), dtype=torch.bfloat16)
+    yardstick_check("out", out, r32["out"], r16["out"], 2e-3)
+    for n, leaf in zip(NAMES, leaves):
+        yardstick_check(n, leaf.grad, r32[n], r16[n], 2e-3 * r32[n].abs().max().item())
+    # (a sum over all rows of a head of exp(sink - lse) * delta, delta formed from the 16-bit output)
+    assert max_err(sinks.grad, r32["dsinks"]) <= 1e-2 * max(1.0, r32["dsinks"].abs().max().item())
+
+
+@pytest.mark.parametrize("warmup", [False, True])
+def test_copied_inputs_and_forward_alone(warmup):
+    """Strides the kernels cannot read in place (rows 136 elements apart) and a pass without gradients give the plain result."""
+    import flash_msa_b200 as fm
+    cfg = dict(b=2, s=512, hq=6, hkv=2, hp=2, hpkv=2, kb=3, seed=90)
+    *inputs, do = bf16_inputs(cfg)
+    fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
+    res = []
+    for widen in (False, True):
+        base = [torch.nn.functional.pad(t, (0, 8))[..., :128] if widen else t for t in inputs]
+        assert base[0].stride(2) == (136 if widen else 128)
+        leaves = [t.detach().requires_grad_(True) for t in base]
+        out, kl = fn(*leaves, 384, SCALE)
+        torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+        with torch.no_grad():
+            alone, kl0 = fn(*base, 384, SCALE)
+        assert torch.equal(alone, out) and kl0.item() == 0.0 and not alone.requires_grad
+        res.append([out] + [t.grad for t in leaves])
+    for n, a, b in zip(["out"] + NAMES, *res):
+        assert max_err(a, b) <= (0.0 if n in ("out", "dq", "dq_proxy") else 2 ** -7 * a.float().abs().max().item()), n
+
+
+@pytest.mark.parametrize("cu", [[0, 512], [0, 0, 1, 130, 130, 511, 512, 512], [[0, 7, 512], [0, 512, 512]], list(range(0, 513)) + [512] * 500])
+def test_document_boundaries_from_the_host(cu):
+    """Short lists travel as a kernel parameter, long ones and device tensors take the other way: the same array."""
+    from flash_msa_b200 import ops
+    dev = torch.device("cuda", 0)
+    got = ops.doc_start_from_cu_seqlens(cu, 2, 512, dev)
+    assert torch.equal(got, ops.doc_start_from_cu_seqlens(torch.tensor(cu, device=dev), 2, 512, dev))
+    assert torch.equal(got.cpu(), O.doc_start_from_cu_seqlens(cu, 512, 2))
+    for bad in ([0, 5, 3, 512], [1, 512], [0, 511]):
+        with pytest.raises(ValueError):
+            ops.doc_start_from_cu_seqlens(bad, 2, 512, dev)
+
+
+def test_status_words_in_host_memory():
+    """A kernel whose bounded wait ran out writes its status word into pinned host memory; the next look raises once."""
+    from flash_msa_b200 import _lib, passes
+    board = passes.StatusBoard()
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device="cpu").manual_seed(14)
+    src, b = (torch.randn(n, 128, generator=g).to(torch.bfloat16).cuda() for n in (256, 128))
+    rows = torch.arange(128, dtype=torch.int32).cuda()
+    d = torch.zeros(2, 128, 128, device=dev)
+    part = torch.zeros(128, 2, 128, dtype=torch.bfloat16, device=dev)
+    for withhold in (0, 1):
+        _lib.check(_lib.load().fmsa_pipeline_selftest(src.data_ptr(), 256, rows.data_ptr(), b.data_ptr(), d[0].data_ptr(), d[1].data_ptr(),
+                                                      part.data_ptr(), withhold, 2_000_000, board.pointer(1, dev), None), "selftest")
+        if not withhold:
+            board.drain()
+    with pytest.raises(RuntimeError, match="flash_msa_func backward.*timed out"):
+        board.drain()
+    board.drain()
