@@ -459,8 +459,11 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, uint32_t src, int
                  : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Waits until the bulk stores committed so far have finished READING shared memory.
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// Waits until all but the N latest bulk stores committed so far have finished READING shared memory.
+template <int N = 0>
+__device__ __forceinline__ void tma_store_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
 // Waits until they are complete (globally visible at kernel end anyway; used before exit).
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {

@@ -72,11 +72,12 @@ struct UnitDesc {
 constexpr int kFwdQStages = 3;
 constexpr int kUnitRing = 16;
 constexpr int kLimitRing = 8;
+constexpr int kReads = 0, kDraws = 1, kOneThread = 2;   // how a role takes part in the common sequence of sub-units
 
 struct FwdCtrl {
     uint64_t k_full, k_empty, v_full, v_empty, kp_full, kp_empty;
     uint64_t q_full[kFwdQStages], q_empty[kFwdQStages];
-    uint64_t s_full[3], p_full[3], s_free[3];
+    uint64_t s_full[3], p_full[3];
     uint64_t o_full, o_empty;
     uint64_t unit_full[kUnitRing];
     UnitDesc units[kUnitRing];
@@ -107,11 +108,11 @@ static_assert(kFwdSmemBytes <= 232448, "shared memory budget of one CTA");
 // head, then the proxy head.  Hand-offs (all mbarriers, one arrival per warp or per tcgen05.commit):
 //   gather warps  q_full[stage] (TMA bytes)  <- q_empty[stage] (commit after S)
 //   K/V warp      k_full/v_full/kp_full      <- k_empty/kp_empty (commit after the last S of a sub-unit), v_empty
-//   MMA warp      S runs two tiles ahead of P V; s_full[t%3], o_full; s_free[t%3] when tile t no longer needs its S columns
+//   MMA warp      S runs two tiles ahead of P V; s_full[t%3], o_full
 //   softmax       p_full[t%3] when P is in TMEM (or, for a proxy tile, when S has been read)
 //   output group  o_empty when the O accumulator has been read
 // TMEM: three S accumulators at columns 0, 128 and 256 (tile t uses number t%3; P overwrites the first 64 columns of
-// its S), one O accumulator at 384.  With three S accumulators the product S(t+2) does not have to wait for P V(t),
+// its S), one O accumulator at 384.  With three S accumulators the product S(t+2) does not have to wait for P V(t+1),
 // so a softmax group finds its next S finished when it comes back for it; the price is a single O accumulator, i.e.
 // P V(t+1) waits until O(t) has been read out, which takes far less time than a softmax.
 // The register file is re-divided between the warpgroups (setmaxnreg): the softmax and output groups get what the
@@ -151,7 +152,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
         for (int i = 0; i < 3; ++i) {
             mbar_init(BAR(sm->s_full[i]), 1);
             mbar_init(BAR(sm->p_full[i]), 4);
-            mbar_init(BAR(sm->s_free[i]), 1);
         }
         mbar_init(BAR(sm->o_full), 1);
         mbar_init(BAR(sm->o_empty), 4);
@@ -200,6 +200,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
 #endif
         (void)kind;
     };
+    auto wait1 = [&](uint32_t bar, uint32_t parity) {   // the same in a role that a single thread runs
+        if (!bad) bad = !mbar_wait_role(bar, parity);
+    };
     // block barrier of one 128-thread group that also ORs a flag: the roles that use named barriers must
     // leave their loops together
     auto group_or = [&](int id, bool flag) -> bool {
@@ -233,9 +236,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
     // the work and publishes the decoded sub-unit; it passes over sub-units that lie beyond the end of their row, so
     // every published entry has work (or is the end marker).  The roles are at most a handful of tiles apart (Q stages
     // + S and O accumulators), far fewer than the ring has entries.
-    auto next_unit = [&](uint32_t draw, UnitDesc& ud, auto may_draw) -> bool {
+    auto next_unit = [&](uint32_t draw, UnitDesc& ud, auto mode) -> bool {
         const uint32_t uslot = draw & (kUnitRing - 1);
-        if (decltype(may_draw)::value && warp == 12 && lane == 0) {
+        if (decltype(mode)::value == kDraws && warp == 12 && lane == 0) {
             UnitDesc nu;
             nu.chunk1 = -1;
             for (;;) {
@@ -264,7 +267,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
             sm->units[uslot] = nu;
             mbar_arrive(BAR(sm->unit_full[uslot]));
         }
-        wait(BAR(sm->unit_full[uslot]), (draw / kUnitRing) & 1, 7);
+        if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kUnitRing) & 1);
+        else wait(BAR(sm->unit_full[uslot]), (draw / kUnitRing) & 1, 7);
         if (warp >= 8 && warp < 12) bad = group_or(1, bad);
         if (bad) return false;
         ud = sm->units[uslot];
@@ -274,81 +278,63 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
     // Every role has its own loop over the common sequence of sub-units.
     if (warp >= 20) {
         reg_dec<kFwdRegsMisc>();
-        if (warp == 21) {
+        if (warp == 21 && elect_one()) {
             // =========================== MMA issue ===========================
+            // One thread runs the whole role; one loop with one site per product keeps its code small.
             UnitDesc ud;
-            for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
-                const int ntiles = __shfl_sync(0xffffffffu, (ud.chunk1 - ud.chunk0) * hpc, 0);   // (known to be uniform)
-                wait(BAR(sm->k_full), nsub & 1, 5);
-                bool kp_ready = false, v_ready = false;
-                uint32_t gts = gt;            // running index of the next S to issue, its accumulator and phase bit
-                uint32_t ssb = sb, ssph = sph;
-                int hs = 0;                   // its head
-                int s_issued = 0;
-                auto next_s = [&]() {
-                    if (s_issued == ntiles) return;
-                    const bool proxy = hs == P.mpp;
-                    if (proxy && !kp_ready) {
-                        wait(BAR(sm->kp_full), nsub & 1, 5);
-                        kp_ready = true;
-                    }
-                    wait(BAR(sm->q_full[qs]), qph, 1);
-                    if (gts >= 3) wait(BAR(sm->s_free[ssb]), ssph ^ 1, 2);
-                    tc_fence_after_sync();
-                    if (!bad && elect_one()) {
-                        umma_tile_128<false, false, FP16>(tmem_s0 + ssb * 128, tile_q0 + qs * kTileBytes, proxy ? tile_kp : tile_k, false);
+            for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kOneThread>{}); ++draw, ++nsub) {
+                const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
+                wait1(BAR(sm->k_full), nsub & 1);
+                if (P.with_proxy) wait1(BAR(sm->kp_full), nsub & 1);
+                uint32_t ssb = sb;            // accumulator of the next S to issue
+                int hs = 0, hh = 0;           // heads of tile t + 2 (S) and of tile t (P V)
+#pragma unroll 1
+                for (int t = -2; t < ntiles && !bad; ++t) {
+                    if (t + 2 < ntiles) {
+                        // S runs two tiles ahead: the softmax groups never starve.  It overwrites the accumulator of tile t - 1,
+                        // whose scores have been read (p_full) and whose P V has been issued: products execute in order.
+                        wait1(BAR(sm->q_full[qs]), qph);
+                        if (bad) break;
+                        tc_fence_after_sync();
+                        umma_tile_128<false, false, FP16>(tmem_s0 + ssb * 128, tile_q0 + qs * kTileBytes, hs == P.mpp ? tile_kp : tile_k, false);
                         umma_commit(BAR(sm->s_full[ssb]));
                         umma_commit(BAR(sm->q_empty[qs]));
-                    }
-                    if (++qs == kFwdQStages) {
-                        qs = 0;
-                        qph ^= 1;
-                    }
-                    if (++ssb == 3) {
-                        ssb = 0;
-                        ssph ^= 1;
-                    }
-                    ++gts;
-                    if (++hs == hpc) hs = 0;
-                    if (++s_issued == ntiles && !bad && elect_one()) {
-                        umma_commit(BAR(sm->k_empty));    // every S of this sub-unit has been issued
-                        umma_commit(BAR(sm->kp_empty));
-                    }
-                };
-                next_s();
-                next_s();
-                int hh = 0;
-                for (int t = 0; t < ntiles && !bad; ++t, ++gt) {
-                    const bool is_proxy = hh == P.mpp;
-                    next_s();   // S runs two tiles ahead: the softmax groups never starve
-                    wait(BAR(sm->p_full[sb]), sph, 3);
-                    if (!is_proxy) {
-                        if (!v_ready) {
-                            wait(BAR(sm->v_full), nsub & 1, 5);
-                            v_ready = true;
+                        if (++qs == kFwdQStages) {
+                            qs = 0;
+                            qph ^= 1;
                         }
-                        if (mt >= 1) wait(BAR(sm->o_empty), (mt - 1) & 1, 4);
+                        if (++ssb == 3) ssb = 0;
+                        if (++hs == hpc) hs = 0;
+                        if (t + 3 == ntiles) {   // every S of this sub-unit has been issued
+                            umma_commit(BAR(sm->k_empty));
+                            umma_commit(BAR(sm->kp_empty));
+                        }
+                    }
+                    if (t < 0) continue;
+                    wait1(BAR(sm->p_full[sb]), sph);
+                    if (hh != P.mpp) {
+                        if (t == 0) wait1(BAR(sm->v_full), nsub & 1);
+                        if (mt >= 1) wait1(BAR(sm->o_empty), (mt - 1) & 1);
+                        if (bad) break;
                         tc_fence_after_sync();
-                        if (!bad && elect_one()) {
-                            const uint32_t ts = tmem_s0 + sb * 128;
-                            umma_ts<8, 8, FP16>(tmem_o0, ts, tile_v, false);   // O = P V_j
-                            umma_commit(BAR(sm->o_full));
-                        }
+                        umma_ts<8, 8, FP16>(tmem_o0, tmem_s0 + sb * 128, tile_v, false);   // O = P V_j
+                        umma_commit(BAR(sm->o_full));
                         ++mt;
                     }
-                    if (!bad && elect_one()) umma_commit(BAR(sm->s_free[sb]));
+                    if (bad) break;
                     if (++sb == 3) {
                         sb = 0;
                         sph ^= 1;
                     }
                     if (++hh == hpc) hh = 0;
+                    ++gt;
                 }
-                if (!bad && elect_one()) umma_commit(BAR(sm->v_empty));
+                if (!bad) umma_commit(BAR(sm->v_empty));
             }
         } else if (warp == 20) {
             // =========================== K / V / Kp loads ===========================
             UnitDesc ud;
-            for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
+            for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
                 if (nsub > 0) wait(BAR(sm->k_empty), (nsub - 1) & 1);
                 if (!bad && lane == 0) {
                     mbar_arrive_expect_tx(BAR(sm->k_full), kTileBytes);
@@ -377,7 +363,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
         const int g = warp - 12;
         const int quad = (lane >> 1) & 3, panel = lane & 1;
         UnitDesc ud;
-        for (uint32_t draw = 0; next_unit(draw, ud, std::true_type{}); ++draw, ++nsub) {
+        for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kDraws>{}); ++draw, ++nsub) {
             const int64_t q_base = static_cast<int64_t>(ud.b) * P.q_row_b + static_cast<int64_t>(ud.p) * P.mpp * P.q_row_h;
             const int64_t qp_base = static_cast<int64_t>(ud.b) * P.qp_row_b + static_cast<int64_t>(ud.p) * P.qp_row_h;
             for (int chunk = ud.chunk0; chunk < ud.chunk1 && !bad; ++chunk) {
@@ -428,9 +414,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
         // Thread = row of the O accumulator: bf16, staged in the operand layout, one TMA tile store per panel.
         // The last, partial chunk of a reverse-index row is written row by row (its slots end where the next
         // row's begin).
-        const int otid = tid - 8 * 32;
         UnitDesc ud;
-        for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
+        for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
             const int64_t slot_base = ud.e0 - edge_base;   // slot of the first row of the reverse-index row
             int hh = 0, chunk = ud.chunk0;
@@ -439,42 +424,49 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     const int nrows = min(kBlock, ud.n - chunk * kBlock);
                     const int64_t slot0 = slot_base + static_cast<int64_t>(chunk) * kBlock;
                     const bool full = nrows == kBlock;
-                    const uint32_t to = tmem_o0;
-                    if (otid == 0) tma_store_wait_read();   // the staging tile's previous store has read it
+                    // Two panels of 64 columns: while one panel's TMA store still reads its staging half, the other one is
+                    // filled.  (Staged and stored as one tile the group took 2.4 k cycles per tile and held everybody up.)
+                    if (warp == 8 && elect_one()) tma_store_wait_read<1>();   // all but the latest store: panel 0's half is free
+                    __syncwarp();
                     wait(BAR(sm->o_full), mt & 1);
                     bad = group_or(1, bad);
                     if (bad) break;
                     tc_fence_after_sync();
                     __nv_bfloat16* grow = P.o_part + ((slot0 + row) * P.mpp + hh) * kHeadDim;
-#pragma unroll
-                    for (int c = 0; c < 128; c += 32) {
-                        uint32_t v[32];
-                        tmem_ld32(tmem_addr(to, quarter, c), v);
+#pragma unroll 1
+                    for (int c = 0; c < 128; c += 64) {
+                        uint32_t v0[32], v1[32];
+                        tmem_ld32(tmem_addr(tmem_o0, quarter, c), v0);
+                        tmem_ld32(tmem_addr(tmem_o0, quarter, c + 32), v1);
+                        if (c > 0 && warp == 8 && elect_one()) tma_store_wait_read<1>();
                         tmem_ld_wait();
-                        uint32_t pk[16];
+                        if (c > 0) {
+                            tc_fence_before_sync();
+                            warp_arrive(BAR(sm->o_empty));
+                            if (full) named_barrier_sync(1, 128);
+                        }
+                        uint32_t pk[32];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) pk[i] = pack_act<FP16>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                        for (int i = 0; i < 16; ++i) pk[i] = pack_act<FP16>(__uint_as_float(v0[2 * i]), __uint_as_float(v0[2 * i + 1]));
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) pk[16 + i] = pack_act<FP16>(__uint_as_float(v1[2 * i]), __uint_as_float(v1[2 * i + 1]));
                         if (full) {
 #pragma unroll
-                            for (int k8 = 0; k8 < 4; ++k8)
+                            for (int k8 = 0; k8 < 8; ++k8)
                                 st_shared_v4(tile_o + swz_offset(row, (c >> 3) + k8), pk[4 * k8], pk[4 * k8 + 1], pk[4 * k8 + 2],
                                              pk[4 * k8 + 3]);
+                            fence_async_smem();
+                            named_barrier_sync(1, 128);
+                            if (warp == 8 && elect_one()) {
+                                tma_store_3d(&tmap_o, tile_o + (c >> 6) * kPanelBytes, c, hh, static_cast<int>(slot0));
+                                tma_store_commit();
+                            }
+                            __syncwarp();
                         } else if (row < nrows) {
 #pragma unroll
-                            for (int k8 = 0; k8 < 4; ++k8)
+                            for (int k8 = 0; k8 < 8; ++k8)
                                 *reinterpret_cast<uint4*>(grow + c + 8 * k8) =
                                     make_uint4(pk[4 * k8], pk[4 * k8 + 1], pk[4 * k8 + 2], pk[4 * k8 + 3]);
-                        }
-                    }
-                    tc_fence_before_sync();
-                    warp_arrive(BAR(sm->o_empty));
-                    if (full) {
-                        fence_async_smem();
-                        named_barrier_sync(1, 128);
-                        if (otid == 0) {
-                            tma_store_3d(&tmap_o, tile_o, 0, hh, static_cast<int>(slot0));
-                            tma_store_3d(&tmap_o, tile_o + kPanelBytes, 64, hh, static_cast<int>(slot0));
-                            tma_store_commit();
                         }
                     }
                     ++mt;
@@ -485,14 +477,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                 }
             }
         }
-        if (otid == 0) tma_store_wait_all();
+        if (warp == 8 && elect_one()) tma_store_wait_all();
     } else {
         reg_inc<kFwdRegsSoftmax>();
         // =========================== softmax groups ===========================
         const uint32_t wg = static_cast<uint32_t>(warp >> 2);
         const float2 sc2 = make_float2(P.scale_log2e, P.scale_log2e);
         UnitDesc ud;
-        for (uint32_t draw = 0; next_unit(draw, ud, std::false_type{}); ++draw, ++nsub) {
+        for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
             const int64_t slot_base = ud.e0 - edge_base;
             int hh = 0, chunk = ud.chunk0;
@@ -525,8 +517,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     const bool masked = (chunk == 0) || (VARLEN && __any_sync(0xffffffffu, low > 0));
                     const int limit = (chunk == 0) ? sm->limits[(cbase + chunk - ud.chunk0) & (kLimitRing - 1)][row] : 127;
                     float m = 0.f, l = 0.f;
-                    {
-                        const bool kMasked = masked, kProxy = is_proxy;
+                    // Two instances: with the mask as a run-time condition every element paid for its comparison and selection.
+                    auto softmax_row = [&](auto masked_c) __attribute__((always_inline)) {
+                        constexpr bool kMasked = decltype(masked_c)::value;
                         // Two passes over the 128 logits of the row (maximum, then exponentials), software-pipelined over
                         // 32-column pieces: the TMEM load of the next piece is in flight while this one is worked on
                         // (tcgen05.wait::ld waits for every load issued so far, hence the order wait, issue, compute).
@@ -576,7 +569,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                                 pk[i >> 1] = pack_act<FP16>(p0, p1);
                             }
                             // P (bf16, two keys per column) over S columns this thread has already consumed
-                            if (!kProxy) tmem_st16(tmem_addr(ts, quarter, c >> 1), pk);
+                            if (!is_proxy) tmem_st16(tmem_addr(ts, quarter, c >> 1), pk);
                         };
 #pragma unroll 1
                         for (int c = 0; c < 128; c += 64) {
@@ -588,7 +581,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                             piece_exp(bb, c + 32);
                         }
                         l = l2.x + l2.y;
-                    }
+                    };
+                    if (masked) softmax_row(std::true_type{});
+                    else softmax_row(std::false_type{});
                     if (!is_proxy) tmem_st_wait();
                     tc_fence_before_sync();
                     warp_arrive(BAR(sm->p_full[sb]));
@@ -621,6 +616,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 200000) __nanosleep(1000);
     }
+    __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
