@@ -131,7 +131,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                                                                     const __grid_constant__ CUtensorMap tmap_do,
                                                                     const __grid_constant__ CUtensorMap tmap_k,
                                                                     const __grid_constant__ CUtensorMap tmap_v,
-                                                                    const __grid_constant__ CUtensorMap tmap_dq,
                                                                     const BwdParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -172,7 +171,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         prefetch_tmap(&tmap_do);
         prefetch_tmap(&tmap_k);
         prefetch_tmap(&tmap_v);
-        prefetch_tmap(&tmap_dq);
     }
     if (warp == 0) {
         tmem_alloc(smem_u32(&sm->tmem_slot), 512);
@@ -447,7 +445,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     const int nrows = min(64, ud.n - chunk * kBlock - 64 * x);   // <= 0: nothing to write
                     const int nparts = P.split ? 2 : 1;
                     for (int part = 0; part < nparts; ++part) {
-                        if (part > 0) named_barrier_sync(1, 128);   // the staging tile's first part has been read
 #pragma unroll 1
                         for (int i = 0; i < 2; ++i) {   // 16 head-dimension lanes of the warp's 32 at a time
                             uint32_t v[32];
@@ -476,26 +473,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                             for (int j = 0; j < 4; ++j) stmatrix_x4_trans(at + j * 16 * 128, pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
                         }
                         const int64_t pslot0 = slot0 + 64 * x + part * P.part_slots;
-                        fence_async_smem();
+                        // 256 contiguous bytes per row and half-warp.  (A TMA tile store read the staging half some 600 cycles
+                        // longer, which the compute groups waited for at the next tile: 1.22 -> 1.20 ms without KL work.)
                         named_barrier_sync(1, 128);
-                        if (nrows == 64) {
-                            if (warp == 8 && elect_one()) {
-#pragma unroll 1
-                                for (int c = 0; c < 2; ++c)
-                                    tma_store_3d(&tmap_dq, stage + c * (kPanelBytes / 2), 64 * c, hh, static_cast<int>(pslot0));
-                                tma_store_commit();
-                                tma_store_wait_read();
-                            }
-                        } else if (nrows > 0) {
-                            // the ragged end of a reverse-index row (its slots end where the next row's begin)
-                            for (int e = otid; e < nrows * 16; e += 128) {
-                                const int r = e >> 4, c = e & 15;
-                                __nv_bfloat16* grow = P.dq_part + ((pslot0 + r) * P.mpp + hh) * kHeadDim;
-                                *reinterpret_cast<uint4*>(grow + 8 * c) =
-                                    ld_shared_v4(stage + (c >> 3) * (kPanelBytes / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
-                            }
-                            named_barrier_sync(1, 128);
+                        for (int e = otid; e < nrows * 16; e += 128) {
+                            const int r = e >> 4, c = e & 15;
+                            *reinterpret_cast<uint4*>(P.dq_part + ((pslot0 + r) * P.mpp + hh) * kHeadDim + 8 * c) =
+                                ld_shared_v4(stage + (c >> 3) * (kPanelBytes / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
                         }
+                        named_barrier_sync(1, 128);
                     }
                     if (warp == 8) warp_arrive(BAR(sm->ds_free[x]));
                 }
@@ -525,7 +511,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                 }
             }
         }
-        if (warp == 8 && elect_one()) tma_store_wait_all();
     } else {
         reg_inc<kBwdRegsCompute>();
         // =========================== compute groups ===========================
@@ -1063,12 +1048,10 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     FMSA_REQUIRE(part_slots > 0 && part_slots * (split ? 2 : 1) < 0x7fffffffLL);
     const uint64_t q_rows = gather_rows(pb->B, pb->Hq, pb->S, q->stride_b, q->stride_h, q->stride_s);
     const uint64_t do_rows = gather_rows(pb->B, pb->Hq, pb->S, d_out->stride_b, d_out->stride_h, d_out->stride_s);
-    CUtensorMap tq, tdo, tk, tv, tdq;
+    CUtensorMap tq, tdo, tk, tv;
     if (!make_tmap_gather(&tq, q->ptr, q_rows) || !make_tmap_gather(&tdo, d_out->ptr, do_rows) ||
         !make_tmap_bhsd(&tk, k->ptr, pb->B, pb->Hkv, pb->S, k->stride_b, k->stride_h, k->stride_s, 128) ||
-        !make_tmap_bhsd(&tv, v->ptr, pb->B, pb->Hkv, pb->S, v->stride_b, v->stride_h, v->stride_s, 128) ||
-        !make_tmap_partials_swz(&tdq, dq_part, static_cast<uint64_t>(part_slots) * (split ? 2 : 1),
-                                static_cast<uint64_t>(pb->Hq / pb->Hp), 64))
+        !make_tmap_bhsd(&tv, v->ptr, pb->B, pb->Hkv, pb->S, v->stride_b, v->stride_h, v->stride_s, 128))
         return FMSA_ERR_CUDA;
 
     BwdParams P;
@@ -1087,7 +1070,7 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     const int sms = device_sm_count();
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
     const bool varlen = P.doc_start != nullptr;
-    using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
+    using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
     static const KernelFn kernels[8] = {sparse_bwd_kernel<false, false, false>, sparse_bwd_kernel<false, false, true>,
                                         sparse_bwd_kernel<false, true, false>,  sparse_bwd_kernel<false, true, true>,
                                         sparse_bwd_kernel<true, false, false>,  sparse_bwd_kernel<true, false, true>,
@@ -1106,7 +1089,7 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     U.per_group = static_cast<uint32_t>(per_group);
     U.n_subunits = static_cast<int32_t>(per_group * g_count);
     const int grid = U.n_subunits < sms ? U.n_subunits : sms;
-    kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tk, tv, tdq, P);
+    kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tk, tv, P);
     if (with_kl) {
         if (zero_counters && cudaMemsetAsync(counter_proxy, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
         U.counter = counter_proxy;
