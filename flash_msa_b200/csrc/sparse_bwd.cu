@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
             mbar_init(BAR(sm->pds_full[i]), 8);
             mbar_init(BAR(sm->dq_full[i]), 1);
             mbar_init(BAR(sm->dq_free[i]), 4);
-            mbar_init(BAR(sm->ds_free[i]), 1);
+            mbar_init(BAR(sm->ds_free[i]), 4);
         }
         for (int i = 0; i < kBwdUnitRing; ++i) mbar_init(BAR(sm->unit_full[i]), 1);
         fence_mbar_init();
@@ -243,7 +243,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
         }
         if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1);
         else wait(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1, 7);
-        if (warp >= 8 && warp < 12) bad = group_or(1, bad);
         if (bad) return false;
         ud = sm->units[uslot];
         return ud.chunk1 >= 0;
@@ -421,7 +420,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     } else if (warp >= 8) {
         reg_dec<kBwdRegsOutput>();
         // =========================== output group ===========================
-        const int otid = tid - 8 * 32;
         UnitRec ud;
         for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kReads>{}); ++draw, ++nsub) {
             const int ntiles = (ud.chunk1 - ud.chunk0) * hpc;
@@ -432,23 +430,28 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
                     wait(BAR(sm->dq_full[x]), gt & 1, 2);
-                    bad = group_or(1, bad);
                     if (bad) break;
                     tc_fence_after_sync();
                     // dQ^T (lane = head dimension, column = query of the half) -> 16 bit -> transposed into the half's panel of
-                    // the dS^T tile (its products are done): 64 rows of one query each, two 64-column panels in the swizzle of
-                    // the TMA tile store.  With `split` the rows leave twice: rounded, and the remainder of that rounding (a second
+                    // the dS^T tile (its products are done), from where it leaves as rows of one query.  Every warp stages and
+                    // stores its own 32 head dimensions, 64 bytes of a row, so that the four warps meet nowhere (storing whole rows
+                    // of 256 bytes took two barriers per store, during which the panel was held: ... us).
+                    // With `split` the rows leave twice: rounded, and the remainder of that rounding (a second
                     // plane of the partial buffers, `part_slots` slots further on), so that the sum over many edges keeps
                     // fp32-like accuracy.
-                    const uint32_t src = tmem + 128 * x + 64;
-                    const uint32_t stage = tile_ds + x * kPanelBytes;
-                    const int nrows = min(64, ud.n - chunk * kBlock - 64 * x);   // <= 0: nothing to write
+                    const uint32_t src = tmem + 128 * x + 64 + (static_cast<uint32_t>(quarter * 32) << 16);
+                    const uint32_t stage = tile_ds + x * kPanelBytes + quarter * (kPanelBytes / 4);   // 64 rows of 64 bytes, swizzled
+                    const int r0 = lane >> 2;                                                  // the lane stores rows r0 + 8 i
+                    const int nrows = min(64, ud.n - chunk * kBlock - 64 * x) - r0;            // <= 0: nothing to write
+                    __nv_bfloat16* to = P.dq_part + ((slot0 + 64 * x + r0) * P.mpp + hh) * kHeadDim + 32 * quarter + 8 * (lane & 3);
+                    const uint32_t from = stage + r0 * 64 + (((lane ^ (r0 >> 1)) & 3) << 4);
                     const int nparts = P.split ? 2 : 1;
+#pragma unroll 1
                     for (int part = 0; part < nparts; ++part) {
 #pragma unroll 1
                         for (int i = 0; i < 2; ++i) {   // 16 head-dimension lanes of the warp's 32 at a time
                             uint32_t v[32];
-                            tmem_ld_16x256_x8(src + (static_cast<uint32_t>(quarter * 32 + 16 * i) << 16), v);
+                            tmem_ld_16x256_x8(src + (static_cast<uint32_t>(16 * i) << 16), v);
                             tmem_ld_wait();
                             if (i == 1 && part == nparts - 1) {
                                 tc_fence_before_sync();
@@ -466,24 +469,22 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                                 }
                             }
                             // stmatrix: lane l addresses row l%8 of block l/8; blocks are (queries +0, dims +0), (+0, +8), (+8, +0), (+8, +8)
-                            const int cd = quarter * 4 + 2 * i + ((lane >> 3) & 1);   // 16-byte chunk of the 256-byte row
-                            const int q8 = (lane >> 4) * 8 + (lane & 7);
-                            const uint32_t at = stage + (cd >> 3) * (kPanelBytes / 2) + q8 * 128 + (((cd & 7) ^ (lane & 7)) << 4);
+                            const int cd = 2 * i + ((lane >> 3) & 1);   // 16-byte chunk of the warp's 64 bytes
+                            const uint32_t at = stage + ((lane >> 4) * 8 + (lane & 7)) * 64 + ((cd ^ ((lane >> 1) & 3)) << 4);
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) stmatrix_x4_trans(at + j * 16 * 128, pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+                            for (int j = 0; j < 4; ++j) stmatrix_x4_trans(at + j * 16 * 64, pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
                         }
-                        const int64_t pslot0 = slot0 + 64 * x + part * P.part_slots;
-                        // 256 contiguous bytes per row and half-warp.  (A TMA tile store read the staging half some 600 cycles
-                        // longer, which the compute groups waited for at the next tile: 1.22 -> 1.20 ms without KL work.)
-                        named_barrier_sync(1, 128);
-                        for (int e = otid; e < nrows * 16; e += 128) {
-                            const int r = e >> 4, c = e & 15;
-                            *reinterpret_cast<uint4*>(P.dq_part + ((pslot0 + r) * P.mpp + hh) * kHeadDim + 8 * c) =
-                                ld_shared_v4(stage + (c >> 3) * (kPanelBytes / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
-                        }
-                        named_barrier_sync(1, 128);
+                        __syncwarp();
+                        uint4 w[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) w[i] = ld_shared_v4(from + i * 8 * 64);   // row r0 + 8 i
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (8 * i < nrows) *reinterpret_cast<uint4*>(to + static_cast<int64_t>(8 * i) * P.mpp * kHeadDim) = w[i];
+                        to += P.part_slots * P.mpp * kHeadDim;
+                        __syncwarp();   // the rows have been read
                     }
-                    if (warp == 8) warp_arrive(BAR(sm->ds_free[x]));
+                    warp_arrive(BAR(sm->ds_free[x]));
                 }
                 if (++hh == hpc) {
                     hh = 0;
