@@ -35,10 +35,10 @@ inline int device_sm_count() {
     }
     return cached[dev];
 }
-// Raises a kernel's dynamic shared-memory limit once per (kernel, device).  Up to 32 kernels.
+// Raises a kernel's dynamic shared-memory limit once per (kernel, device).  Up to 64 kernels.
 inline bool ensure_smem_attr(const void* func, size_t bytes) {
     struct Entry { const void* f; unsigned long long done; };
-    static Entry table[32] = {};
+    static Entry table[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     for (auto& e : table) {

@@ -59,7 +59,6 @@ struct BwdParams {
     __nv_bfloat16* dq_part;    // [(edge - edge_base) * mpp + head][128]: per-edge dQ contributions (unscaled)
     uint32_t* teacher;         // KL kernels: per edge 256 bytes (the dqp_part buffer), filled by the compute groups below
     int64_t part_slots;        // slots per plane of dq_part
-    int split;                 // 1: every contribution is stored as a bf16 pair (value, rounding remainder) in two planes
     float *dk_acc, *dv_acc;    // fp32, zero-initialised, [B,Hkv,S,128]
     int32_t* status;
     int S, Hq, Hkv, mpp;
@@ -125,8 +124,8 @@ constexpr uint32_t kHalfRowBytes = 64 * 128;   // rows 64.. of a panel: where ha
 // ds_free (the half's panel of the dS^T tile, which doubles as the staging tile of its dQ store, is reusable),
 // acc_full / acc_free (dV, dK flushed at the end of a sub-unit).
 // VARLEN: document masking of packed sequences (P.doc_start given).  A separate instantiation, so that the plain kernel
-// carries none of its registers or code.
-template <bool FP16, bool VARLEN, bool KL>
+// carries none of its registers or code.  SPLIT: two planes of partial rows.
+template <bool FP16, bool VARLEN, bool KL, bool SPLIT>
 __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
                                                                     const __grid_constant__ CUtensorMap tmap_do,
                                                                     const __grid_constant__ CUtensorMap tmap_k,
@@ -208,20 +207,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     };
     auto wait1 = [&](uint32_t bar, uint32_t parity) {   // the same in a role that a single thread runs
         if (!bad) bad = !mbar_wait_role(bar, parity);
-    };
-    auto group_or = [&](int id, bool flag) -> bool {   // 128-thread barrier that also ORs a flag
-        uint32_t r;
-        asm volatile(
-            "{\n"
-            ".reg .pred p, q;\n"
-            "setp.ne.b32 q, %1, 0;\n"
-            "barrier.cta.red.or.pred p, %2, 128, q;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(r)
-            : "r"(flag ? 1u : 0u), "r"(id)
-            : "memory");
-        return r != 0;
     };
     auto warp_arrive = [&](uint32_t bar) {
         __syncwarp();
@@ -435,8 +420,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     // dQ^T (lane = head dimension, column = query of the half) -> 16 bit -> transposed into the half's panel of
                     // the dS^T tile (its products are done), from where it leaves as rows of one query.  Every warp stages and
                     // stores its own 32 head dimensions, 64 bytes of a row, so that the four warps meet nowhere (storing whole rows
-                    // of 256 bytes took two barriers per store, during which the panel was held: ... us).
-                    // With `split` the rows leave twice: rounded, and the remainder of that rounding (a second
+                    // of 256 bytes took two barriers per store, during which the panel was held: 1.17 -> 1.14 ms without KL work).
+                    // With SPLIT the rows leave twice: rounded, and the remainder of that rounding (a second
                     // plane of the partial buffers, `part_slots` slots further on), so that the sum over many edges keeps
                     // fp32-like accuracy.
                     const uint32_t src = tmem + 128 * x + 64 + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -445,32 +430,22 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     const int nrows = min(64, ud.n - chunk * kBlock - 64 * x) - r0;            // <= 0: nothing to write
                     __nv_bfloat16* to = P.dq_part + ((slot0 + 64 * x + r0) * P.mpp + hh) * kHeadDim + 32 * quarter + 8 * (lane & 3);
                     const uint32_t from = stage + r0 * 64 + (((lane ^ (r0 >> 1)) & 3) << 4);
-                    const int nparts = P.split ? 2 : 1;
-#pragma unroll 1
-                    for (int part = 0; part < nparts; ++part) {
+                    // stmatrix: lane l addresses row l%8 of block l/8; blocks are (queries +0, dims +0), (+0, +8), (+8, +0), (+8, +8)
+                    const uint32_t into = stage + ((lane >> 4) * 8 + (lane & 7)) * 64;
+                    const int64_t row8 = static_cast<int64_t>(8 * P.mpp) * kHeadDim;
+                    if constexpr (!SPLIT) {
 #pragma unroll 1
                         for (int i = 0; i < 2; ++i) {   // 16 head-dimension lanes of the warp's 32 at a time
-                            uint32_t v[32];
+                            uint32_t v[32], pk[16];
                             tmem_ld_16x256_x8(src + (static_cast<uint32_t>(16 * i) << 16), v);
                             tmem_ld_wait();
-                            if (i == 1 && part == nparts - 1) {
+                            if (i == 1) {
                                 tc_fence_before_sync();
                                 warp_arrive(BAR(sm->dq_free[x]));
                             }
-                            uint32_t pk[16];
-                            if (part == 0) {
 #pragma unroll
-                                for (int k = 0; k < 16; ++k) pk[k] = pack_act<FP16>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-                            } else {
-#pragma unroll
-                                for (int k = 0; k < 16; ++k) {
-                                    const float x0 = __uint_as_float(v[2 * k]), x1 = __uint_as_float(v[2 * k + 1]);
-                                    pk[k] = pack_act<FP16>(x0 - act_round<FP16>(x0), x1 - act_round<FP16>(x1));
-                                }
-                            }
-                            // stmatrix: lane l addresses row l%8 of block l/8; blocks are (queries +0, dims +0), (+0, +8), (+8, +0), (+8, +8)
-                            const int cd = 2 * i + ((lane >> 3) & 1);   // 16-byte chunk of the warp's 64 bytes
-                            const uint32_t at = stage + ((lane >> 4) * 8 + (lane & 7)) * 64 + ((cd ^ ((lane >> 1) & 3)) << 4);
+                            for (int k = 0; k < 16; ++k) pk[k] = pack_act<FP16>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+                            const uint32_t at = into + (((2 * i + ((lane >> 3) & 1)) ^ ((lane >> 1) & 3)) << 4);   // 16-byte chunk of the row
 #pragma unroll
                             for (int j = 0; j < 4; ++j) stmatrix_x4_trans(at + j * 16 * 64, pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
                         }
@@ -480,9 +455,49 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                         for (int i = 0; i < 8; ++i) w[i] = ld_shared_v4(from + i * 8 * 64);   // row r0 + 8 i
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
-                            if (8 * i < nrows) *reinterpret_cast<uint4*>(to + static_cast<int64_t>(8 * i) * P.mpp * kHeadDim) = w[i];
-                        to += P.part_slots * P.mpp * kHeadDim;
-                        __syncwarp();   // the rows have been read
+                            if (8 * i < nrows) *reinterpret_cast<uint4*>(to + i * row8) = w[i];
+                    } else {
+                        // 32 queries at a time: their rounded values in the first 32 staging rows, the remainders in the others.
+                        // (All 64 queries, one plane after the other, read dQ^T twice and kept it until the first plane had left:
+                        // 1.68 -> 1.58 ms at B=2 S=8192 Hq=32 top-k 16 blocks without KL work.)
+#pragma unroll 1
+                        for (int y = 0; y < 2; ++y) {
+#pragma unroll 1
+                            for (int i = 0; i < 2; ++i) {
+                                uint32_t v[16], hi[8], lo[8];
+                                tmem_ld_16x256_x4(src + 32 * y + (static_cast<uint32_t>(16 * i) << 16), v);
+                                tmem_ld_wait();
+                                if (y + i == 2) {
+                                    tc_fence_before_sync();
+                                    warp_arrive(BAR(sm->dq_free[x]));
+                                }
+#pragma unroll
+                                for (int k = 0; k < 8; ++k) {
+                                    const float x0 = __uint_as_float(v[2 * k]), x1 = __uint_as_float(v[2 * k + 1]);
+                                    hi[k] = pack_act<FP16>(x0, x1);
+                                    lo[k] = pack_act<FP16>(x0 - act_lo<FP16>(hi[k]), x1 - act_hi<FP16>(hi[k]));
+                                }
+                                const uint32_t at = into + (((2 * i + ((lane >> 3) & 1)) ^ ((lane >> 1) & 3)) << 4);
+#pragma unroll
+                                for (int j = 0; j < 2; ++j) {
+                                    stmatrix_x4_trans(at + j * 16 * 64, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
+                                    stmatrix_x4_trans(at + (32 + j * 16) * 64, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
+                                }
+                            }
+                            __syncwarp();
+                            uint4 w[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) w[i] = ld_shared_v4(from + i * 8 * 64);
+                            __nv_bfloat16* to2 = to + P.part_slots * P.mpp * kHeadDim;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (32 * y + 8 * i < nrows) {
+                                    *reinterpret_cast<uint4*>(to + i * row8) = w[i];
+                                    *reinterpret_cast<uint4*>(to2 + i * row8) = w[4 + i];
+                                }
+                            to += 4 * row8;
+                            __syncwarp();   // the rows have been read
+                        }
                     }
                     warp_arrive(BAR(sm->ds_free[x]));
                 }
@@ -1062,7 +1077,7 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     P.lse = lse; P.delta = delta;
     P.col_q = col_q; P.doc_start = pb->doc_start;
     P.dq_part = static_cast<__nv_bfloat16*>(dq_part); P.teacher = static_cast<uint32_t*>(dqp_part);
-    P.part_slots = part_slots; P.split = split ? 1 : 0;
+    P.part_slots = part_slots;
     P.dk_acc = dk_acc; P.dv_acc = dv_acc;
     P.status = status;
     P.S = pb->S; P.Hq = pb->Hq; P.Hkv = pb->Hkv; P.mpp = pb->Hq / pb->Hp;
@@ -1072,11 +1087,12 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     const bool fp16 = pb->dtype == FMSA_DTYPE_FP16;
     const bool varlen = P.doc_start != nullptr;
     using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
-    static const KernelFn kernels[8] = {sparse_bwd_kernel<false, false, false>, sparse_bwd_kernel<false, false, true>,
-                                        sparse_bwd_kernel<false, true, false>,  sparse_bwd_kernel<false, true, true>,
-                                        sparse_bwd_kernel<true, false, false>,  sparse_bwd_kernel<true, false, true>,
-                                        sparse_bwd_kernel<true, true, false>,   sparse_bwd_kernel<true, true, true>};
-    const KernelFn kernel = kernels[(fp16 ? 4 : 0) + (varlen ? 2 : 0) + (with_kl ? 1 : 0)];
+#define FMSA_BWD_KERNELS(F, V) \
+    sparse_bwd_kernel<F, V, false, false>, sparse_bwd_kernel<F, V, false, true>, sparse_bwd_kernel<F, V, true, false>, sparse_bwd_kernel<F, V, true, true>
+    static const KernelFn kernels[16] = {FMSA_BWD_KERNELS(false, false), FMSA_BWD_KERNELS(false, true), FMSA_BWD_KERNELS(true, false),
+                                         FMSA_BWD_KERNELS(true, true)};
+#undef FMSA_BWD_KERNELS
+    const KernelFn kernel = kernels[(fp16 ? 8 : 0) + (varlen ? 4 : 0) + (with_kl ? 2 : 0) + (split ? 1 : 0)];
     const void* kfn = reinterpret_cast<const void*>(kernel);
     if (sms <= 0 || !ensure_smem_attr(kfn, kBwdSmemBytes)) return FMSA_ERR_CUDA;
     if (zero_counters && cudaMemsetAsync(counter, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
