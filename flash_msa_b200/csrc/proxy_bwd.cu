@@ -76,7 +76,6 @@ static_assert(kProxyTileBytes + sizeof(ProxyCtrl) <= kProxySmemBytes, "shared me
 template <bool FP16, bool VARLEN>
 __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qp,
                                                                      const __grid_constant__ CUtensorMap tmap_kp,
-                                                                     const __grid_constant__ CUtensorMap tmap_dqp,
                                                                      const ProxyParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -99,7 +98,7 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
             mbar_init(BAR(sm->st_empty[i]), 8);
             mbar_init(BAR(sm->s_full[i]), 1);
             mbar_init(BAR(sm->ds_full[i]), 8);
-            mbar_init(BAR(sm->ds_free[i]), 1);
+            mbar_init(BAR(sm->ds_free[i]), 4);
         }
         for (int i = 0; i < kProxyQStages; ++i) {
             mbar_init(BAR(sm->q_full[i]), 4);
@@ -113,7 +112,6 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
         fence_mbar_init();
         prefetch_tmap(&tmap_qp);
         prefetch_tmap(&tmap_kp);
-        prefetch_tmap(&tmap_dqp);
     }
     if (warp == 0) {
         tmem_alloc(smem_u32(&sm->tmem_slot), 512);
@@ -138,20 +136,6 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
     auto wait1 = [&](uint32_t bar, uint32_t parity) {   // the same in a role that a single thread runs
         if (!bad) bad = !mbar_wait_role(bar, parity);
     };
-    auto group_or = [&](bool flag) -> bool {   // 128-thread barrier of the output group that also ORs a flag
-        uint32_t r;
-        asm volatile(
-            "{\n"
-            ".reg .pred p, q;\n"
-            "setp.ne.b32 q, %1, 0;\n"
-            "barrier.cta.red.or.pred p, 1, 128, q;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(r)
-            : "r"(flag ? 1u : 0u)
-            : "memory");
-        return r != 0;
-    };
     auto warp_arrive = [&](uint32_t bar) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
@@ -168,7 +152,6 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
         }
         if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kProxyUnitRing) & 1);
         else wait(BAR(sm->unit_full[uslot]), (draw / kProxyUnitRing) & 1);
-        if (warp >= 8 && warp < 12) bad = group_or(bad);
         if (bad) return false;
         ud = sm->units[uslot];
         return ud.chunk1 >= 0;
@@ -312,57 +295,57 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
 #pragma unroll 1
             for (int chunk = ud.chunk0; chunk < ud.chunk1; ++chunk, ++gt) {
                 wait(BAR(sm->dq_full), gt & 1);
-                bad = group_or(bad);
                 if (bad) break;
                 tc_fence_after_sync();
-                const uint32_t stage = tile_ds0 + (gt & 1) * kTileBytes;   // the tile's dSp^T, whose product is done
-                const int nrows = min(kBlock, ud.n - chunk * kBlock);
-                const int nparts = P.split ? 2 : 1;
+                // Thread = row.  A warp stages its 32 rows in the tile's dSp^T (whose product is done), 64 columns at a time, and
+                // stores them itself, 128 contiguous bytes of four rows per instruction: the four warps meet nowhere.  With two planes
+                // the rounding remainders lie in the other panel.
+                const uint32_t rows = tile_ds0 + (gt & 1) * kTileBytes + quarter * 32 * 128;
+                const int r0 = lane >> 3;   // the lane stores rows r0 + 4 i of the warp's
+                const int nrows = ud.n - chunk * kBlock - 32 * quarter - r0;
+                __nv_bfloat16* to = P.dqp_part + (slot_base + static_cast<int64_t>(chunk) * kBlock + 32 * quarter + r0) * kHeadDim + 8 * (lane & 7);
 #pragma unroll 1
-                for (int part = 0; part < nparts; ++part) {
-                    if (part > 0) named_barrier_sync(1, 128);   // the first part has left the staging tile
-                    const int64_t pslot0 = slot_base + static_cast<int64_t>(chunk) * kBlock + part * P.part_slots;
-                    __nv_bfloat16* grow = P.dqp_part + (pslot0 + row) * kHeadDim;
-#pragma unroll 1
-                    for (int c = 0; c < 128; c += 32) {
-                        uint32_t v[32], pk[16];
-                        tmem_ld32(tmem_addr(tmem_dq, quarter, c), v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            float x0 = __uint_as_float(v[2 * i]), x1 = __uint_as_float(v[2 * i + 1]);
-                            if (part > 0) {
-                                x0 -= act_round<FP16>(x0);
-                                x1 -= act_round<FP16>(x1);
-                            }
-                            pk[i] = pack_act<FP16>(x0, x1);
-                        }
-                        if (nrows == kBlock) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                st_shared_v4(stage + swz_offset(row, (c >> 3) + k), pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
-                        } else if (row < nrows) {   // the ragged end of a reverse-index row is written row by row
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                *reinterpret_cast<uint4*>(grow + c + 8 * k) = make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
-                        }
-                    }
-                    if (part == nparts - 1) {
+                for (int c = 0; c < 128; c += 32) {
+                    uint32_t v[32], pk[16];
+                    tmem_ld32(tmem_addr(tmem_dq, quarter, c), v);
+                    tmem_ld_wait();
+                    if (c == 96) {
                         tc_fence_before_sync();
                         warp_arrive(BAR(sm->dq_free));
                     }
-                    if (nrows == kBlock) {
-                        fence_async_smem();
-                        named_barrier_sync(1, 128);
-                        if (warp == 8 && elect_one()) {
-                            tma_store_3d(&tmap_dqp, stage, 0, 0, static_cast<int>(pslot0));
-                            tma_store_3d(&tmap_dqp, stage + kPanelBytes, 64, 0, static_cast<int>(pslot0));
-                            tma_store_commit();
-                            tma_store_wait_read();
-                        }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) pk[i] = pack_act<FP16>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                    uint32_t panel = rows + (P.split ? 0 : c >> 6) * kPanelBytes;
+                    const int k0 = (c >> 3) & 4;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        st_shared_v4(panel + lane * 128 + (((k0 + k) ^ (lane & 7)) << 4), pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
+                    if (P.split) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            pk[i] = pack_act<FP16>(__uint_as_float(v[2 * i]) - act_lo<FP16>(pk[i]), __uint_as_float(v[2 * i + 1]) - act_hi<FP16>(pk[i]));
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            st_shared_v4(panel + kPanelBytes + lane * 128 + (((k0 + k) ^ (lane & 7)) << 4), pk[4 * k], pk[4 * k + 1], pk[4 * k + 2],
+                                         pk[4 * k + 3]);
                     }
+                    if (k0 == 0) continue;
+                    __syncwarp();
+                    __nv_bfloat16* dst = to + (c & 64);
+#pragma unroll 1
+                    for (int part = 0; part <= P.split; ++part) {
+                        uint4 w[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) w[i] = ld_shared_v4(panel + (r0 + 4 * i) * 128 + (((lane ^ (r0 + 4 * i)) & 7) << 4));
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (4 * i < nrows) *reinterpret_cast<uint4*>(dst + 4 * i * kHeadDim) = w[i];
+                        panel += kPanelBytes;
+                        dst += P.part_slots * kHeadDim;
+                    }
+                    __syncwarp();   // the staging rows have been read
                 }
-                if (warp == 8) warp_arrive(BAR(sm->ds_free[gt & 1]));
+                warp_arrive(BAR(sm->ds_free[gt & 1]));
             }
             if (bad) break;
             // dKp of the sub-unit: lane = key row of the block
@@ -383,7 +366,6 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
                 warp_arrive(BAR(sm->acc_free));
             }
         }
-        if (warp == 8 && elect_one()) tma_store_wait_all();
     } else {
         reg_inc<kProxyRegsCompute>();
         // =========================== compute groups ===========================
@@ -507,10 +489,9 @@ int launch_proxy_bwd(const fmsa_problem* pb, const fmsa_tensor& q_proxy, const f
                      const UnitSpace& units, const int32_t* col_q, void* teacher_dqp, int64_t part_slots, int split,
                      float* dkp_acc, float* kl_value, int grid, int32_t* status, cudaStream_t stream) {
     const uint64_t qp_rows = gather_rows(pb->B, pb->Hp, pb->S, q_proxy.stride_b, q_proxy.stride_h, q_proxy.stride_s);
-    CUtensorMap tqp, tkp, tdqp;
+    CUtensorMap tqp, tkp;
     if (!make_tmap_gather(&tqp, q_proxy.ptr, qp_rows) ||
-        !make_tmap_bhsd(&tkp, k_proxy.ptr, pb->B, pb->Hpkv, pb->S, k_proxy.stride_b, k_proxy.stride_h, k_proxy.stride_s, 128) ||
-        !make_tmap_partials_swz(&tdqp, teacher_dqp, static_cast<uint64_t>(part_slots) * (split ? 2 : 1), 1))
+        !make_tmap_bhsd(&tkp, k_proxy.ptr, pb->B, pb->Hpkv, pb->S, k_proxy.stride_b, k_proxy.stride_h, k_proxy.stride_s, 128))
         return FMSA_ERR_CUDA;
     ProxyParams P;
     P.qp_row_b = static_cast<int32_t>(q_proxy.stride_b / 128); P.qp_row_h = static_cast<int32_t>(q_proxy.stride_h / 128);
@@ -522,12 +503,12 @@ int launch_proxy_bwd(const fmsa_problem* pb, const fmsa_tensor& q_proxy, const f
     P.scale_log2e = pb->scale * kLog2e; P.inv_mpp = static_cast<float>(pb->Hp) / static_cast<float>(pb->Hq);
     P.kl_value = kl_value;
     P.kl_value_scale = kLn2 / (static_cast<float>(pb->B) * pb->Hp * pb->S);
-    using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, ProxyParams);
+    using KernelFn = void (*)(CUtensorMap, CUtensorMap, ProxyParams);
     static const KernelFn kernels[4] = {proxy_bwd_kernel<false, false>, proxy_bwd_kernel<false, true>, proxy_bwd_kernel<true, false>,
                                         proxy_bwd_kernel<true, true>};
     const KernelFn kernel = kernels[(pb->dtype == FMSA_DTYPE_FP16 ? 2 : 0) + (pb->doc_start ? 1 : 0)];
     if (!ensure_smem_attr(reinterpret_cast<const void*>(kernel), kProxySmemBytes)) return FMSA_ERR_CUDA;
-    kernel<<<grid, kProxyThreads, kProxySmemBytes, stream>>>(tqp, tkp, tdqp, P);
+    kernel<<<grid, kProxyThreads, kProxySmemBytes, stream>>>(tqp, tkp, P);
     return check_launch();
 }
 
