@@ -286,12 +286,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -349,7 +343,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
 }
 
 // ---------------------------------------------------------------------------------------------
-// cp.async row gather into a swizzled tile
+// cp.async copy into a swizzled tile
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
     const int n = valid ? 16 : 0;   // src-size 0 writes 16 zero bytes
@@ -366,20 +360,6 @@ __device__ __forceinline__ uint32_t swz_offset(int row, int chunk16) {
     return static_cast<uint32_t>((chunk16 >> 3) * kPanelBytes + row * 128 + (((chunk16 & 7) ^ (row & 7)) << 4));
 }
 
-// Every thread of the CTA calls this.  Row r of the tile is copied from `base + rows[r]*stride`
-// (elements); a negative row id produces a row of zeros.  `rows` may live in shared memory.
-template <int NTHREADS>
-__device__ __forceinline__ void gather_tile_async(uint32_t tile, const __nv_bfloat16* base, int64_t stride,
-                                                  const int* rows, int tid) {
-#pragma unroll 4
-    for (int it = tid; it < 128 * 16; it += NTHREADS) {
-        const int r = it >> 4, c16 = it & 15;
-        const int row = rows[r];
-        const bool ok = row >= 0;
-        const __nv_bfloat16* src = base + static_cast<int64_t>(ok ? row : 0) * stride + c16 * 8;
-        cp_async_16(tile + swz_offset(r, c16), src, ok);
-    }
-}
 // Contiguous variant: tile row r comes from `base + (row0 + r)*stride`.
 template <int NTHREADS>
 __device__ __forceinline__ void load_tile_async(uint32_t tile, const __nv_bfloat16* base, int64_t stride, int tid) {
@@ -388,36 +368,6 @@ __device__ __forceinline__ void load_tile_async(uint32_t tile, const __nv_bfloat
         const int r = it >> 4, c16 = it & 15;
         cp_async_16(tile + swz_offset(r, c16), base + static_cast<int64_t>(r) * stride + c16 * 8, true);
     }
-}
-
-// Lean 512-thread variants used by the attention kernels.  Thread `tid` always moves the same
-// 16-byte chunk column of rows tid/16 + 32k (k = 0..3), so its swizzled destination offset is a
-// per-thread constant plus k * 4096 bytes; only the source row changes.
-struct GatherLane {
-    uint32_t dst_off;   // swizzled offset of (row tid/16, chunk tid%16) inside a tile
-    int r0;             // tid / 16
-    int col;            // element offset of the chunk inside the 128-element row
-};
-__device__ __forceinline__ GatherLane make_gather_lane(int tid) {
-    GatherLane g;
-    g.r0 = tid >> 4;
-    g.col = (tid & 15) * 8;
-    g.dst_off = swz_offset(g.r0, tid & 15);
-    return g;
-}
-__device__ __forceinline__ void gather_tile_512(uint32_t tile, const __nv_bfloat16* base, int64_t stride, const int* rows,
-                                                const GatherLane& g) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int row = rows[g.r0 + 32 * k];
-        const bool ok = row >= 0;
-        cp_async_16(tile + g.dst_off + k * 4096, base + static_cast<int64_t>(ok ? row : 0) * stride + g.col, ok);
-    }
-}
-__device__ __forceinline__ void load_tile_512(uint32_t tile, const __nv_bfloat16* base, int64_t stride, const GatherLane& g) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        cp_async_16(tile + g.dst_off + k * 4096, base + static_cast<int64_t>(g.r0 + 32 * k) * stride + g.col, true);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -457,11 +407,6 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const void* tmap, int 
 }
 // TMA tile STORE shared -> global (bulk-group completion).  The source tile must have been made
 // visible to the async proxy (fence_async_smem + a barrier) before the elected thread issues it.
-__device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap), "r"(src), "r"(x),
-                 "r"(y)
-                 : "memory");
-}
 __device__ __forceinline__ void tma_store_3d(const void* tmap, uint32_t src, int x, int y, int z) {
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap), "r"(src),
                  "r"(x), "r"(y), "r"(z)
@@ -514,7 +459,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // The same for the activation type of a kernel instantiation: bf16 (FP16 = false) or fp16.  A packed pair sits in
 // one 32-bit word, the first element in the low half.
@@ -527,10 +471,6 @@ __device__ __forceinline__ uint32_t pack_act(float lo, float hi) {
     return pack_bf16(lo, hi);
 }
 template <bool FP16>
-__device__ __forceinline__ float act_round(float x) {
-    return FP16 ? __half2float(__float2half_rn(x)) : bf16_round(x);
-}
-template <bool FP16>
 __device__ __forceinline__ float act_lo(uint32_t w) {
     if (FP16) return __low2float(*reinterpret_cast<const __half2*>(&w));
     return __low2float(*reinterpret_cast<const __nv_bfloat162*>(&w));   // (a conversion the compiler can fold into the consumer; a shift is not)
@@ -539,23 +479,6 @@ template <bool FP16>
 __device__ __forceinline__ float act_hi(uint32_t w) {
     if (FP16) return __high2float(*reinterpret_cast<const __half2*>(&w));
     return __high2float(*reinterpret_cast<const __nv_bfloat162*>(&w));
-}
-
-// Stores 16 accumulator values of a TRANSPOSED tile (this lane = head-dimension index d, value i =
-// output row row0+i) as bf16: the 32 lanes of a warp write 64 contiguous bytes of one output row per
-// instruction.  `dst` points at (row row0, element d); rows are `rstride` elements apart; rows >=
-// nvalid are skipped (the test is uniform over the warp).  (Exchanging values between lane pairs
-// to write packed 4-byte pairs was measured slower than one bf16 per lane.)
-__device__ __forceinline__ void store_transposed_bf16_16(__nv_bfloat16* dst, int64_t rstride, const uint32_t (&v)[16],
-                                                         int row0, int nvalid) {
-    if (row0 + 16 <= nvalid) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) dst[i * rstride] = __float2bfloat16_rn(__uint_as_float(v[i]));
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (row0 + i < nvalid) dst[i * rstride] = __float2bfloat16_rn(__uint_as_float(v[i]));
-    }
 }
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {

@@ -55,20 +55,6 @@ inline bool make_tmap_bhsd(CUtensorMap* map, const void* base, uint64_t B, uint6
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Partial-row buffer [slots][heads][128] bf16 (heads = 1 gives the 2-D case) for tile STORES of
-// 128 slots x one head x 128 elements from a dense row-major shared-memory tile (no swizzle).
-inline bool make_tmap_partials(CUtensorMap* map, const void* base, uint64_t slots, uint64_t heads) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[3] = {128, heads, slots};
-    const cuuint64_t strides[2] = {256, 256 * heads};
-    const cuuint32_t box[3] = {128, 1, 128};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Row-gather view of a (B, H, S, 128) bf16 activation whose strides are all multiples of 128 elements: a
 // 2-D matrix of 256-byte rows in which element row (b, h, s) has index (b*stride_b + h*stride_h +
 // s*stride_s) / 128.  Box = 64 columns x 1 row, 128-byte swizzle: the form tile::gather4 loads take.
@@ -92,14 +78,14 @@ inline uint64_t gather_rows(int64_t B, int64_t H, int64_t S, int64_t sb, int64_t
     return static_cast<uint64_t>(((B - 1) * sb + (H - 1) * sh + (S - 1) * ss) / 128 + 1);
 }
 
-// Partial-row buffer [slots][heads][128] bf16 for tile STORES of `box_rows` slots x one head from a shared-memory
+// Partial-row buffer [slots][heads][128] bf16 for tile STORES of 128 slots x one head from a shared-memory
 // tile in the operand layout (two 64-column panels, 128-byte swizzle): one store per panel.
-inline bool make_tmap_partials_swz(CUtensorMap* map, const void* base, uint64_t slots, uint64_t heads, uint32_t box_rows = 128) {
+inline bool make_tmap_partials_swz(CUtensorMap* map, const void* base, uint64_t slots, uint64_t heads) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[3] = {128, heads, slots};
     const cuuint64_t strides[2] = {256, 256 * heads};
-    const cuuint32_t box[3] = {64, 1, box_rows};
+    const cuuint32_t box[3] = {64, 1, 128};
     const cuuint32_t estr[3] = {1, 1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
