@@ -36,7 +36,7 @@ __host__ __device__ __forceinline__ int64_t dense_row_offset(int j, int S) {
 // blocks are about equally long, and the sub-units that lie beyond the end of their row cluster
 // together), so both a dynamic work counter and a static round-robin deal stay balanced.
 // -------------------------------------------------------------------------------------------
-constexpr int kMaxChunksPerSubUnit = 8;
+constexpr int kMaxChunksPerSubUnit = 16;
 
 // Key blocks j that can have a sub-unit s: NB - j > C*s, i.e. j < NB - C*s.
 __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int ppk, int C) {
@@ -45,16 +45,20 @@ __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int ppk, 
     return (n * NB - C * (n * (n - 1) / 2)) * ppk;
 }
 
-// C for a launch: the largest power of two up to 8 that still leaves every CTA `kSubUnitsPerCta` sub-units on average.  A
+// C for a launch: the largest power of two up to 8 that still leaves every CTA `kSubUnitsPerCta` sub-units on average, or 16
+// where that leaves it `kLongSubUnitsPerCta`.  A
 // sub-unit loads K and V once and flushes dV and dK once, so long ones save traffic; short ones fill the SMs and bound the
 // tail of the launch: a problem of a few dozen chunks otherwise runs on a handful of SMs (B=1, S=1024, Hq=8, top-k 4 blocks:
 // 64 chunks on 16 CTAs).  `edges` is an upper bound of the selected (row, block) pairs; a row of the reverse index is on
 // average half a chunk longer than its edges.  Drawing and passing over a sub-unit beyond the end of its row costs about a
 // microsecond, so C does not go below what keeps the enumeration at `kDrawsPerCta` per CTA.
-constexpr int kSubUnitsPerCta = 6, kDrawsPerCta = 32;
+// With 16 the rows of a group are gathered in half as many sweeps, which counts where they do not fit L2 (B=1 S=65536 Hq=8
+// top-k 32 blocks, 14 sub-units per CTA: forward 1.70 -> 1.56 ms, backward 3.83 -> 3.49 ms; S=32768, 64 blocks: equal), while
+// at 7 sub-units per CTA (B=2 S=8192 Hq=32 top-k 16 blocks) the tail makes it slower: 0.672 -> 0.692 ms forward.
+constexpr int kSubUnitsPerCta = 6, kLongSubUnitsPerCta = 12, kDrawsPerCta = 32;
 inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int ppk, int sms) {
     const int64_t chunks = (edges + kBlock - 1) / kBlock + groups * ppk * NB / 2;
-    int c = kMaxChunksPerSubUnit;
+    int c = chunks >= static_cast<int64_t>(kMaxChunksPerSubUnit) * kLongSubUnitsPerCta * sms ? kMaxChunksPerSubUnit : kMaxChunksPerSubUnit / 2;
     while (c > 1 && chunks < static_cast<int64_t>(c) * kSubUnitsPerCta * sms &&
            groups * subunits_per_group(NB, ppk, c / 2) <= static_cast<int64_t>(kDrawsPerCta) * sms)
         c >>= 1;
