@@ -146,9 +146,12 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
     float kl_acc = 0.f;
     auto next_unit = [&](uint32_t draw, UnitRec& ud, auto mode) -> bool {   // as in the main kernel
         const uint32_t uslot = draw & (kProxyUnitRing - 1);
-        if (decltype(mode)::value == kDraws && warp == 12 && lane == 0) {
-            sm->units[uslot] = draw_subunit(P.units);
-            mbar_arrive(BAR(sm->unit_full[uslot]));
+        if (decltype(mode)::value == kDraws && warp == 12) {
+            const UnitRec nu = draw_subunit(P.units);
+            if (lane == 0) {
+                sm->units[uslot] = nu;
+                mbar_arrive(BAR(sm->unit_full[uslot]));
+            }
         }
         if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kProxyUnitRing) & 1);
         else wait(BAR(sm->unit_full[uslot]), (draw / kProxyUnitRing) & 1);

@@ -222,9 +222,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     // ring has entries.
     auto next_unit = [&](uint32_t draw, UnitRec& ud, auto mode) -> bool {
         const uint32_t uslot = draw & (kBwdUnitRing - 1);
-        if (decltype(mode)::value == kDraws && warp == 12 && lane == 0) {
-            sm->units[uslot] = draw_subunit(P.units);
-            mbar_arrive(BAR(sm->unit_full[uslot]));
+        if (decltype(mode)::value == kDraws && warp == 12) {
+            const UnitRec nu = draw_subunit(P.units);
+            if (lane == 0) {
+                sm->units[uslot] = nu;
+                mbar_arrive(BAR(sm->unit_full[uslot]));
+            }
         }
         if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1);
         else wait(BAR(sm->unit_full[uslot]), (draw / kBwdUnitRing) & 1, 7);
@@ -1102,7 +1105,7 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     U.g_begin = g_begin; U.dense = dense ? 1 : 0;
     U.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, U.NB, U.ppk, sms);
     const int64_t per_group = subunits_per_group(U.NB, U.ppk, U.chunks);
-    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA)
+    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA and 31)
     U.per_group = static_cast<uint32_t>(per_group);
     U.n_subunits = static_cast<int32_t>(per_group * g_count);
     const int grid = U.n_subunits < sms ? U.n_subunits : sms;

@@ -238,12 +238,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
     // + S and O accumulators), far fewer than the ring has entries.
     auto next_unit = [&](uint32_t draw, UnitDesc& ud, auto mode) -> bool {
         const uint32_t uslot = draw & (kUnitRing - 1);
-        if (decltype(mode)::value == kDraws && warp == 12 && lane == 0) {
+        if (decltype(mode)::value == kDraws && warp == 12) {
             UnitDesc nu;
-            nu.chunk1 = -1;
-            for (;;) {
-                const uint32_t u = static_cast<uint32_t>(atomicAdd(P.counter, 1));
-                if (u >= static_cast<uint32_t>(P.n_subunits)) break;
+            const bool more = draw_work(P.counter, static_cast<uint32_t>(P.n_subunits), [&](uint32_t u) -> bool {
                 const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks, P.units_per_group);
                 const uint32_t g = P.g_begin + su.g;
                 const int b = g / static_cast<uint32_t>(P.Hkv), kvh = g % static_cast<uint32_t>(P.Hkv), p = kvh * P.ppk + su.pp;
@@ -257,15 +254,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     e0 = P.row_ptr[bp * P.NB + su.j];
                     n = P.row_ptr[bp * P.NB + su.j + 1] - static_cast<int>(e0);
                 }
-                if (su.chunk0 * kBlock < n) {
-                    nu.j = su.j; nu.b = b; nu.kvh = kvh; nu.p = p; nu.n = n; nu.e0 = e0;
-                    nu.chunk0 = su.chunk0;
-                    nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + P.chunks);
-                    break;
-                }
+                nu.j = su.j; nu.b = b; nu.kvh = kvh; nu.p = p; nu.n = n; nu.e0 = e0;
+                nu.chunk0 = su.chunk0;
+                nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + P.chunks);
+                return su.chunk0 * kBlock < n;
+            });
+            if (!more) nu.chunk1 = -1;
+            if (lane == 0) {
+                sm->units[uslot] = nu;
+                mbar_arrive(BAR(sm->unit_full[uslot]));
             }
-            sm->units[uslot] = nu;
-            mbar_arrive(BAR(sm->unit_full[uslot]));
         }
         if (decltype(mode)::value == kOneThread) wait1(BAR(sm->unit_full[uslot]), (draw / kUnitRing) & 1);
         else wait(BAR(sm->unit_full[uslot]), (draw / kUnitRing) & 1, 7);
@@ -915,7 +913,7 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     if (sms <= 0 || !ensure_smem_attr(kfn, kFwdSmemBytes)) return FMSA_ERR_CUDA;
     P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
     const int64_t per_group = subunits_per_group(P.NB, P.ppk, P.chunks);
-    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA)
+    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA and 31)
     P.units_per_group = static_cast<uint32_t>(per_group);
     P.n_subunits = static_cast<int32_t>(per_group * g_count);
     const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
