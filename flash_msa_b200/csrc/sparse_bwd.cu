@@ -810,56 +810,46 @@ __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_kernel(
 // -------------------------------------------------------------------------------------------
 // delta[b,h,q] = sum_d out[b,q,h,d] * dout[b,q,h,d]   (flash_msa/flash_msa.py:99)
 // -------------------------------------------------------------------------------------------
-// One CTA per (batch, 32 consecutive query positions): half-warp g takes positions 2g and 2g+1 and walks the heads,
+// One CTA per (batch, 8 consecutive query positions): half-warp g takes position g%8 and every other group of four heads,
 // each lane reading 16 bytes of the `out` row and of the `dout` row (a half-warp covers one 256-byte row per load, four
-// rows in flight); the sums meet in shared memory so that delta leaves in 128-byte runs along the sequence.
+// rows in flight); the sums meet in shared memory so that delta leaves in 32-byte runs along the sequence.  Bound by memory;
+// with 32 positions per CTA there were too few CTAs to hide its latency (B=3 S=1664 Hq=20:
+// 27.9 -> 9.6 us; B=2 S=8192 Hq=32: 52.6 -> 46.9 us).
 template <bool FP16>
 __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                                     int64_t do_sb, int64_t do_ss, int64_t do_sh, float* __restrict__ delta,
                                                     int B, int S, int Hq) {
-    extern __shared__ float sdelta[];   // [Hq][32]
+    extern __shared__ float sdelta[];   // [Hq][8]
     const int lane = threadIdx.x & 31, l16 = lane & 15;
     const int g = threadIdx.x >> 4;   // half-warp 0..15
-    const int qblocks = S >> 5;
-    const int b = blockIdx.x / qblocks, q0 = (blockIdx.x % qblocks) << 5;
+    const int qblocks = S >> 3;
+    const int b = blockIdx.x / qblocks, q0 = (blockIdx.x % qblocks) << 3;
     auto dot8 = [](const uint4& a, const uint4& d) {
         return act_lo<FP16>(a.x) * act_lo<FP16>(d.x) + act_hi<FP16>(a.x) * act_hi<FP16>(d.x) + act_lo<FP16>(a.y) * act_lo<FP16>(d.y) +
                act_hi<FP16>(a.y) * act_hi<FP16>(d.y) + act_lo<FP16>(a.z) * act_lo<FP16>(d.z) + act_hi<FP16>(a.z) * act_hi<FP16>(d.z) +
                act_lo<FP16>(a.w) * act_lo<FP16>(d.w) + act_hi<FP16>(a.w) * act_hi<FP16>(d.w);
     };
+    const int ql = g & 7, q = q0 + ql;
+    const __nv_bfloat16* orow = out + (static_cast<int64_t>(b) * S + q) * Hq * kHeadDim + l16 * 8;
+    const __nv_bfloat16* drow = dout + b * do_sb + q * do_ss + l16 * 8;
+    for (int h = 4 * (g >> 3); h < Hq; h += 8) {
+        uint4 a[4], d[4];
 #pragma unroll
-    for (int qq = 0; qq < 2; ++qq) {
-        const int ql = 2 * g + qq, q = q0 + ql;
-        const __nv_bfloat16* orow = out + (static_cast<int64_t>(b) * S + q) * Hq * kHeadDim + l16 * 8;
-        const __nv_bfloat16* drow = dout + b * do_sb + q * do_ss + l16 * 8;
-        int h = 0;
-        for (; h + 4 <= Hq; h += 4) {
-            uint4 a[4], d[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = *reinterpret_cast<const uint4*>(orow + static_cast<int64_t>(h + i) * kHeadDim);
-                d[i] = *reinterpret_cast<const uint4*>(drow + (h + i) * do_sh);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float sum = dot8(a[i], d[i]);
-#pragma unroll
-                for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-                if (l16 == 0) sdelta[(h + i) * 32 + ql] = sum;
-            }
+        for (int i = 0; i < 4; ++i) {
+            const int hi = min(h + i, Hq - 1);
+            a[i] = *reinterpret_cast<const uint4*>(orow + static_cast<int64_t>(hi) * kHeadDim);
+            d[i] = *reinterpret_cast<const uint4*>(drow + hi * do_sh);
         }
-        for (; h < Hq; ++h) {
-            const uint4 a = *reinterpret_cast<const uint4*>(orow + static_cast<int64_t>(h) * kHeadDim);
-            const uint4 d = *reinterpret_cast<const uint4*>(drow + h * do_sh);
-            float sum = dot8(a, d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float sum = dot8(a[i], d[i]);
 #pragma unroll
             for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            if (l16 == 0) sdelta[h * 32 + ql] = sum;
+            if (l16 == 0 && h + i < Hq) sdelta[(h + i) * 8 + ql] = sum;
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < Hq * 32; i += 256)
-        delta[(static_cast<int64_t>(b) * Hq + (i >> 5)) * S + q0 + (i & 31)] = sdelta[i];
+    for (int i = threadIdx.x; i < Hq * 8; i += 256) delta[(static_cast<int64_t>(b) * Hq + (i >> 3)) * S + q0 + (i & 7)] = sdelta[i];
 }
 
 // dst = bf16(src * const_scale * factor), factor = *scale_ptr when given (the upstream kl gradient lives on the
@@ -990,9 +980,9 @@ extern "C" int fmsa_bwd_delta(const void* out, const fmsa_tensor* d_out, float* 
     FMSA_REQUIRE(dtype == FMSA_DTYPE_BF16 || dtype == FMSA_DTYPE_FP16);
     FMSA_REQUIRE(aligned16(out) && aligned16(d_out->ptr));
     FMSA_REQUIRE(d_out->stride_b % 8 == 0 && d_out->stride_h % 8 == 0 && d_out->stride_s % 8 == 0);
-    const int64_t grid = static_cast<int64_t>(B) * (S / 32);
-    FMSA_REQUIRE(S % 32 == 0 && grid <= 0x7fffffffLL && Hq * 32 * sizeof(float) <= 48 * 1024);
-    const size_t smem = static_cast<size_t>(Hq) * 32 * sizeof(float);
+    const int64_t grid = static_cast<int64_t>(B) * (S / 8);
+    FMSA_REQUIRE(S % 32 == 0 && grid <= 0x7fffffffLL && Hq * 8 * sizeof(float) <= 48 * 1024);
+    const size_t smem = static_cast<size_t>(Hq) * 8 * sizeof(float);
     if (dtype == FMSA_DTYPE_FP16)
         delta_kernel<true><<<static_cast<unsigned>(grid), 256, smem, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out->ptr), d_out->stride_b, d_out->stride_s,
