@@ -21,6 +21,7 @@ def _tensor_fields(name):
 
 _PROBLEM = list(_lib.FmsaProblem._fields_)
 _INPUTS = sum((_tensor_fields(n) for n in ("q", "k", "v", "q_proxy", "k_proxy")), [])
+_ORDER = ("q_proxy", "k_proxy", "q", "k", "v")   # of the inputs in a tuple of tensors
 
 
 class ForwardArgs(ctypes.Structure):
@@ -69,8 +70,8 @@ class _Timing:
             ops.KERNEL_EVENTS.append((_STAGES[self.stages[i]], events[i], events[i + 1]))
 
 
-def _conforms(shape, stride):
-    """What the kernels read in place (see `ops._as_kernel_input`); a dimension of one position may have any stride."""
+def _conforms(stride):
+    """Strides that the kernels read in place (see `ops._as_kernel_input`)."""
     return stride[3] == 1 and all(st % 128 == 0 and st > 0 for st in stride[:3])
 
 
@@ -91,7 +92,7 @@ class Plan:
         self.dense, self.shape, self.dtype, self.device = dense, (b, hq, s, d), q.dtype, q.device
         self.pb = _lib.FmsaProblem(b, s, hq, hkv, hp, hpkv, 1 if dense else int(top_k_blocks), float(scale), ops._dtype_code(q.dtype), None)
         self.max_partial_bytes = int(max_partial_bytes)
-        self.copies = [i for i, t in enumerate(inputs) if not _conforms(t.shape, t.stride())]
+        self.in_place = all(_conforms(t.stride()) for t in inputs)
         self.grad_shapes = [((b, s, t.shape[1], d), True) if _bshd(t.shape, t.stride()) else (tuple(t.shape), False) for t in inputs]
         self.out_shape = (b, s, hq * d)
         pbr = ctypes.byref(self.pb)
@@ -109,8 +110,8 @@ class Plan:
 
     def _args(self, kind, inputs, **more):
         a = kind(*(getattr(self.pb, f) for f, _ in _PROBLEM), dense=int(self.dense), max_partial_bytes=self.max_partial_bytes, **more)
-        for name, i in (("q_proxy", 0), ("k_proxy", 1), ("q", 2), ("k", 3), ("v", 4)):
-            self._strides(a, name, inputs[i].contiguous().stride() if i in self.copies else inputs[i].stride())
+        for name, t in zip(_ORDER, inputs):
+            self._strides(a, name, t.stride())
         return a
 
     @staticmethod
@@ -133,11 +134,21 @@ class Plan:
         return got
 
     def conform(self, inputs):
-        """The inputs as the kernels can read them: in place, or copied once."""
-        if not self.copies and all(t.data_ptr() % 16 == 0 for t in inputs):
+        """The inputs as the kernels can read them: in place, or - other strides, or an address off the 16-byte grid, which is
+        not part of what a plan knows - copied once into (B,H,S,128) order."""
+        if self.in_place and all(t.data_ptr() % 16 == 0 for t in inputs):
             return inputs
-        return [t.contiguous() if i in self.copies else (t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.preserve_format))
-                for i, t in enumerate(inputs)]
+        return [t if _conforms(t.stride()) and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in inputs]
+
+    def point(self, a, inputs):
+        """Points the argument block `a` at the inputs or at their copies, and returns what it points at (to be kept until the
+        launch).  The block's strides are the inputs'; those of a copy are its own, so they are filled in with its address."""
+        given = self.conform(inputs)
+        a.q_proxy, a.k_proxy, a.q, a.k, a.v = (t.data_ptr() for t in given)
+        if given is not inputs:
+            for name, t in zip(_ORDER, given):
+                self._strides(a, name, t.stride())
+        return given
 
 
 _plans = {}
@@ -167,14 +178,13 @@ def _call(fn, what, args, device):
 
 def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
     """Returns (out [B,S,Hq*128], kl_loss placeholder, saved).  `sinks`: fp32 [Hq] or None."""
-    qp, kp, q, k, v = p.conform(inputs)
     dev = p.device
     a = ForwardArgs.from_buffer_copy(p.forward_args)
+    given = p.point(a, inputs)   # noqa: F841 - copies live until the launch
     out = torch.empty(p.out_shape, dtype=p.dtype, device=dev)
     kl = torch.empty((), dtype=torch.float32, device=dev)
     saved = torch.empty(p.saved_words, dtype=torch.int32, device=dev)
     ws = torch.empty(p.forward_bytes, dtype=torch.uint8, device=dev)
-    a.q_proxy, a.k_proxy, a.q, a.k, a.v = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
     base, at = saved.data_ptr(), p.at
     if not p.dense:
         a.row_ptr, a.col_q, a.edge_pos = base + at[0], base + at[1], base + at[2]
@@ -191,9 +201,8 @@ def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
 
 def backward(p: Plan, inputs, out, grad_out, saved, grad_kl, kl_value, doc_start, sinks, status_ptr):
     """Returns (dq_proxy, dk_proxy, dq, dk, dv, dsinks) in the inputs' type and layout; `grad_kl`, `kl_value`: fp32 scalars or None."""
-    qp, kp, q, k, v = p.conform(inputs)
     dev = p.device
-    b, hq, s, d = p.shape
+    hq = p.shape[1]
     if grad_out.dtype != p.dtype:
         grad_out = grad_out.to(p.dtype)
     st = grad_out.stride()
@@ -202,9 +211,9 @@ def backward(p: Plan, inputs, out, grad_out, saved, grad_kl, kl_value, doc_start
         st = grad_out.stride()
     template, nbytes = p.backward_template(inputs, grad_kl is not None)
     a = BackwardArgs.from_buffer_copy(template)
+    given = p.point(a, inputs)   # noqa: F841 - copies live until the launch
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     grads = [torch.empty(shape, dtype=p.dtype, device=dev) for shape, _ in p.grad_shapes]
-    a.q_proxy, a.k_proxy, a.q, a.k, a.v = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
     a.d_out, a.d_out_sb, a.d_out_sh, a.d_out_ss = grad_out.data_ptr(), st[0], 128, st[1]
     a.dq_proxy, a.dk_proxy, a.dq, a.dk, a.dv = (g.data_ptr() for g in grads)
     base, at = saved.data_ptr(), p.at

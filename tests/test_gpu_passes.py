@@ -53,6 +53,31 @@ def test_copied_inputs_and_forward_alone(warmup):
         assert max_err(a, b) <= (0.0 if n in ("out", "dq", "dq_proxy") else 2 ** -7 * a.float().abs().max().item()), n
 
 
+@pytest.mark.parametrize("warmup", [False, True])
+def test_slices_off_the_16_byte_grid(warmup):
+    """Heads of a wider buffer that begins one element late: strides the kernels could read, an address they cannot, so every
+    input is copied and the copy's strides count (tests/test_passes_host.py).  The plain result, bit for bit where sums have a
+    fixed order."""
+    import flash_msa_b200 as fm
+    cfg = dict(b=2, s=512, hq=6, hkv=2, hp=2, hpkv=2, kb=3, seed=91)
+    *inputs, do = bf16_inputs(cfg)
+    fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
+
+    def late(t):
+        b, h, s, d = t.shape
+        view = torch.zeros(b * s * 2 * h * d + 8, dtype=t.dtype, device=t.device)[1:-7].view(b, s, 2 * h, d)[:, :, :h].transpose(1, 2)
+        assert view.data_ptr() % 16 == 2 and view.stride() == (2 * s * h * d, d, 2 * h * d, 1)
+        return view.copy_(t)
+    res = []
+    for base in (inputs, [late(t) for t in inputs]):
+        leaves = [t.detach().requires_grad_(True) for t in base]
+        out, kl = fn(*leaves, 384, SCALE)
+        torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+        res.append([out] + [t.grad for t in leaves])
+    for n, a, b in zip(["out"] + NAMES, *res):
+        assert max_err(a, b) <= (0.0 if n in ("out", "dq", "dq_proxy") else 2 ** -7 * a.float().abs().max().item()), n
+
+
 @pytest.mark.parametrize("cu", [[0, 512], [0, 0, 1, 130, 130, 511, 512, 512], [[0, 7, 512], [0, 512, 512]], list(range(0, 513)) + [512] * 500])
 def test_document_boundaries_from_the_host(cu):
     """Short lists travel as a kernel parameter, long ones and device tensors take the other way: the same array."""

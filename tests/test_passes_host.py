@@ -1,0 +1,78 @@
+"""Host side of the whole-pass calls, without a GPU: what an argument block says about the tensors whose pointers it holds.
+The native call is replaced by a recorder, so that nothing is launched."""
+import pytest
+import torch
+
+from flash_msa_b200 import passes
+
+B, H, HKV, S = 2, 4, 2, 256
+NAMES = ("q_proxy", "k_proxy", "q", "k", "v")
+
+
+def _dense(h, fill):
+    return torch.arange(B * h * S * 128, dtype=torch.float32).remainder_(61).add_(fill).to(torch.bfloat16).view(B, h, S, 128)
+
+
+def _strided(t, kind):
+    """`t`'s values in another layout."""
+    b, h, s, d = t.shape
+    if kind == "dense":
+        return t.clone()
+    if kind == "bshd":
+        return t.transpose(1, 2).contiguous().transpose(1, 2)
+    if kind in ("packed", "packed_shifted"):      # some heads of a (B,S,2H,128) buffer, which may begin one element late
+        shift = 1 if kind == "packed_shifted" else 0
+        buf = torch.zeros(b * s * 2 * h * d + 8, dtype=t.dtype)
+        view = buf[shift:shift + b * s * 2 * h * d].view(b, s, 2 * h, d)[:, :, :h].transpose(1, 2)
+        return view.copy_(t)
+    if kind == "shifted":                          # dense, but not on a 16-byte boundary
+        return torch.empty(t.numel() + 8, dtype=t.dtype)[3:3 + t.numel()].view(t.shape).copy_(t)
+    if kind == "wide":                             # rows 136 elements apart
+        return torch.zeros(b, h, s, d + 8, dtype=t.dtype)[..., :d].copy_(t)
+    if kind == "expanded":                         # every head the same memory
+        return t[:, :1].clone().expand(b, h, s, d)
+    raise ValueError(kind)
+
+
+KINDS = ["dense", "bshd", "packed", "packed_shifted", "shifted", "wide", "expanded"]
+
+
+class _Recorder:
+    """Stands in for the native call; `given` are the tensors that `Plan.conform` hands to it."""
+
+    def __init__(self, monkeypatch):
+        self.blocks, self.given = [], []
+        conform = passes.Plan.conform
+
+        def watch(plan, *args):
+            self.given.append(list(conform(plan, *args)))
+            return self.given[-1]
+        monkeypatch.setattr(passes.Plan, "conform", watch)
+        monkeypatch.setattr(passes, "_call", lambda fn, what, a, device: self.blocks.append(type(a).from_buffer_copy(a)))
+
+    def check(self, block, given, inputs):
+        for name, t, asked in zip(NAMES, given, inputs):
+            assert getattr(block, name) == t.data_ptr() and t.data_ptr() % 16 == 0, name
+            strides = tuple(getattr(block, f"{name}_{x}") for x in ("sb", "sh", "ss"))
+            assert strides + (1,) == t.stride(), name
+            assert all(st > 0 and st % 128 == 0 for st in strides), name
+            assert torch.equal(t, asked), name
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+def test_strides_in_the_argument_block_are_those_of_the_tensors(monkeypatch, kind, dense):
+    """An input that cannot be read in place is copied, and then the copy's strides are what the kernels get: also when its
+    strides alone would do and only its address does not (the clone of a slice does not have the slice's strides)."""
+    rec = _Recorder(monkeypatch)
+    inputs = tuple(_strided(_dense(h, i), kind) for i, h in enumerate((2, 1, H, HKV, HKV)))
+    plan = passes.plan(inputs, 0 if dense else 1, 0.1, dense)
+    out, _, saved = passes.forward(plan, inputs, None, None, 0, True)
+    passes.backward(plan, inputs, out, torch.zeros_like(out), saved, torch.ones(()), None, None, None, 0)
+    for block, given in zip(rec.blocks, rec.given):
+        rec.check(block, given, inputs)
+    # the same shapes and strides on a 16-byte boundary, and then off it again: nothing is remembered of the address
+    again = [_strided(t.contiguous(), "packed") if kind == "packed_shifted" else t for t in inputs]
+    for tensors in (again, inputs):
+        passes.forward(passes.plan(tensors, 0 if dense else 1, 0.1, dense), tensors, None, None, 0, True)
+        rec.check(rec.blocks[-1], rec.given[-1], tensors)
