@@ -167,6 +167,8 @@ def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks):
     if q.device.type != "cuda":
         raise RuntimeError("warmup MSA forward requires CUDA tensors")
     inputs = (q_proxy, k_proxy, q, k, v)
+    if any(t.device != q.device for t in inputs):   # (a host pointer would reach the kernels as it is)
+        raise ValueError("q_proxy, k_proxy, q, k, and v must be on one CUDA device")
     plan = passes.plan(inputs, top_k_blocks, scale, not sparse)
     if torch.is_grad_enabled() and (any(t.requires_grad for t in inputs) or (sinks is not None and sinks.requires_grad)):
         return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, plan)

@@ -76,3 +76,25 @@ def test_strides_in_the_argument_block_are_those_of_the_tensors(monkeypatch, kin
     for tensors in (again, inputs):
         passes.forward(passes.plan(tensors, 0 if dense else 1, 0.1, dense), tensors, None, None, 0, True)
         rec.check(rec.blocks[-1], rec.given[-1], tensors)
+
+
+class _SaysCuda(torch.Tensor):
+    """A CPU tensor that reports `where` as its device (no launch is reached with it)."""
+    where = torch.device("cuda", 0)
+    device = property(lambda self: self.where)
+
+
+@pytest.mark.parametrize("warmup", [False, True])
+@pytest.mark.parametrize("odd", [0, 1, 3, 4])
+@pytest.mark.parametrize("where", ["cpu", "cuda:1"])
+def test_inputs_on_another_device_than_q_are_refused(monkeypatch, where, odd, warmup):
+    import flash_msa_b200 as fm
+    monkeypatch.setattr(passes, "forward", lambda *a, **k: pytest.fail("a call with tensors on two devices went through"))
+    inputs = [_dense(h, i).as_subclass(_SaysCuda) for i, h in enumerate((2, 1, H, HKV, HKV))]
+    inputs[odd].where = torch.device(where)
+    fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
+    with pytest.raises(ValueError, match="device"):
+        fn(*inputs, 128, 0.1)
+    # (a q that is not on a GPU keeps its own error)
+    with pytest.raises(RuntimeError, match="CUDA"):
+        fn(*(_dense(h, i) for i, h in enumerate((2, 1, H, HKV, HKV))), 128, 0.1)
