@@ -92,7 +92,8 @@ class Plan:
         self.dense, self.shape, self.dtype, self.device = dense, (b, hq, s, d), q.dtype, q.device
         self.pb = _lib.FmsaProblem(b, s, hq, hkv, hp, hpkv, 1 if dense else int(top_k_blocks), float(scale), ops._dtype_code(q.dtype), None)
         self.max_partial_bytes = int(max_partial_bytes)
-        self.in_place = all(_conforms(t.stride()) for t in inputs)
+        self.shapes, self.layout = [t.shape for t in inputs], [t.stride() for t in inputs]
+        self.in_place = all(map(_conforms, self.layout))
         self.grad_shapes = [((b, s, t.shape[1], d), True) if _bshd(t.shape, t.stride()) else (tuple(t.shape), False) for t in inputs]
         self.out_shape = (b, s, hq * d)
         pbr = ctypes.byref(self.pb)
@@ -105,13 +106,13 @@ class Plan:
             self.at.append(4 * off)
             off += (n + 63) // 64 * 64
         self.saved_words = off
-        self.forward_args = bytes(self._args(ForwardArgs, inputs, workspace_bytes=self.forward_bytes))
+        self.forward_args = bytes(self._args(ForwardArgs, workspace_bytes=self.forward_bytes))
         self._backward = {}
 
-    def _args(self, kind, inputs, **more):
+    def _args(self, kind, **more):
         a = kind(*(getattr(self.pb, f) for f, _ in _PROBLEM), dense=int(self.dense), max_partial_bytes=self.max_partial_bytes, **more)
-        for name, t in zip(_ORDER, inputs):
-            self._strides(a, name, t.stride())
+        for name, stride in zip(_ORDER, self.layout):
+            self._strides(a, name, stride)
         return a
 
     @staticmethod
@@ -120,35 +121,49 @@ class Plan:
         setattr(a, name + "_sh", stride[1])
         setattr(a, name + "_ss", stride[2])
 
-    def backward_template(self, inputs, with_kl):
+    def backward_template(self, with_kl):
         """(argument block, workspace bytes) of a backward with or without the KL work."""
         got = self._backward.get(with_kl)
         if got is None:
             nbytes = _lib.load().fmsa_backward_workspace_bytes(ctypes.byref(self.pb), int(self.dense), int(with_kl), ops.SPLIT_PARTIALS_ABOVE,
                                                                self.max_partial_bytes)
-            a = self._args(BackwardArgs, inputs, with_kl=int(with_kl), split_above=ops.SPLIT_PARTIALS_ABOVE, workspace_bytes=nbytes)
+            a = self._args(BackwardArgs, with_kl=int(with_kl), split_above=ops.SPLIT_PARTIALS_ABOVE, workspace_bytes=nbytes)
             for name, (shape, bshd) in zip(("dq_proxy", "dk_proxy", "dq", "dk", "dv"), self.grad_shapes):
                 n1, n2 = shape[1], shape[2]
                 self._strides(a, name, (n1 * n2 * 128, 128, n2 * 128) if bshd else (n1 * n2 * 128, n2 * 128, 128))
             got = self._backward[with_kl] = (bytes(a), nbytes)
         return got
 
-    def conform(self, inputs):
+    def conform(self, inputs, as_planned=True):
         """The inputs as the kernels can read them: in place, or - other strides, or an address off the 16-byte grid, which is
         not part of what a plan knows - copied once into (B,H,S,128) order."""
-        if self.in_place and all(t.data_ptr() % 16 == 0 for t in inputs):
+        if as_planned and self.in_place and all(t.data_ptr() % 16 == 0 for t in inputs):
             return inputs
         return [t if _conforms(t.stride()) and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in inputs]
 
-    def point(self, a, inputs):
+    def point(self, a, inputs, as_planned=True):
         """Points the argument block `a` at the inputs or at their copies, and returns what it points at (to be kept until the
-        launch).  The block's strides are the inputs'; those of a copy are its own, so they are filled in with its address."""
-        given = self.conform(inputs)
+        launch).  The block's strides are those the plan was made for; where the tensors have others (`as_planned` False: these
+        inputs; or copies) they are filled in with the addresses."""
+        given = self.conform(inputs, as_planned)
         a.q_proxy, a.k_proxy, a.q, a.k, a.v = (t.data_ptr() for t in given)
         if given is not inputs:
             for name, t in zip(_ORDER, given):
                 self._strides(a, name, t.stride())
         return given
+
+    def check_unpacked(self, inputs, out, saved):
+        """Raises ValueError for tensors that a saved-tensor hook brought back as something else."""
+        dev = self.device
+        if (out.shape != self.out_shape or out.dtype != self.dtype or out.device != dev
+                or saved.shape != (self.saved_words,) or saved.dtype != torch.int32 or saved.device != dev
+                or any(t.shape != sh or t.dtype != self.dtype or t.device != dev for t, sh in zip(inputs, self.shapes))):
+            raise ValueError("the tensors saved for the backward came back with another shape, type or device")
+
+
+def _whole(t):
+    """Contiguous and on the 16-byte grid, as the kernels read `out` and the saved index."""
+    return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
 _plans = {}
@@ -200,8 +215,11 @@ def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
 
 
 def backward(p: Plan, inputs, out, grad_out, saved, grad_kl, kl_value, doc_start, sinks, status_ptr):
-    """Returns (dq_proxy, dk_proxy, dq, dk, dv, dsinks) in the inputs' type and layout; `grad_kl`, `kl_value`: fp32 scalars or None."""
+    """Returns (dq_proxy, dk_proxy, dq, dk, dv, dsinks) in the type and layout of the forward's inputs; `grad_kl`, `kl_value`:
+    fp32 scalars or None.  `inputs`, `out` and `saved` may be other tensors than the forward's (saved-tensor hooks)."""
     dev = p.device
+    p.check_unpacked(inputs, out, saved)
+    out, saved = _whole(out), _whole(saved)
     hq = p.shape[1]
     if grad_out.dtype != p.dtype:
         grad_out = grad_out.to(p.dtype)
@@ -209,9 +227,9 @@ def backward(p: Plan, inputs, out, grad_out, saved, grad_kl, kl_value, doc_start
     if grad_out.dim() != 3 or st[2] != 1 or st[0] % 128 or st[1] % 128 or st[0] <= 0 or st[1] <= 0 or grad_out.data_ptr() % 16:
         grad_out = grad_out.reshape(p.out_shape).clone(memory_format=torch.contiguous_format)
         st = grad_out.stride()
-    template, nbytes = p.backward_template(inputs, grad_kl is not None)
+    template, nbytes = p.backward_template(grad_kl is not None)
     a = BackwardArgs.from_buffer_copy(template)
-    given = p.point(a, inputs)   # noqa: F841 - copies live until the launch
+    given = p.point(a, inputs, [t.stride() for t in inputs] == p.layout)   # noqa: F841 - copies live until the launch
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     grads = [torch.empty(shape, dtype=p.dtype, device=dev) for shape, _ in p.grad_shapes]
     a.d_out, a.d_out_sb, a.d_out_sh, a.d_out_ss = grad_out.data_ptr(), st[0], 128, st[1]

@@ -78,6 +78,28 @@ def test_slices_off_the_16_byte_grid(warmup):
         assert max_err(a, b) <= (0.0 if n in ("out", "dq", "dq_proxy") else 2 ** -7 * a.float().abs().max().item()), n
 
 
+@pytest.mark.parametrize("warmup", [False, True])
+def test_saved_tensors_kept_on_the_host(warmup):
+    """`save_on_cpu` brings the inputs back contiguous although they were views of (B,S,H,D) storage."""
+    import flash_msa_b200 as fm
+    cfg = dict(b=2, s=512, hq=6, hkv=2, hp=2, hpkv=2, kb=3, seed=92)
+    *inputs, do = bf16_inputs(cfg, layout="bshd")
+    fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
+    res = []
+    for offload in (False, True):
+        leaves = [t.detach().requires_grad_(True) for t in inputs]
+        if offload:
+            with torch.autograd.graph.save_on_cpu():
+                out, kl = fn(*leaves, 384, SCALE)
+        else:
+            out, kl = fn(*leaves, 384, SCALE)
+        torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+        res.append([t.grad for t in leaves])
+    for n, a, b in zip(NAMES, *res):
+        assert a.stride() == b.stride()
+        assert max_err(a, b) <= (0.0 if n in ("dq", "dq_proxy") else 2 ** -7 * a.float().abs().max().item()), n
+
+
 @pytest.mark.parametrize("cu", [[0, 512], [0, 0, 1, 130, 130, 511, 512, 512], [[0, 7, 512], [0, 512, 512]], list(range(0, 513)) + [512] * 500])
 def test_document_boundaries_from_the_host(cu):
     """Short lists travel as a kernel parameter, long ones and device tensors take the other way: the same array."""

@@ -78,6 +78,44 @@ def test_strides_in_the_argument_block_are_those_of_the_tensors(monkeypatch, kin
         rec.check(rec.blocks[-1], rec.given[-1], tensors)
 
 
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("first", ["dense", "bshd", "packed"])
+@pytest.mark.parametrize("then", KINDS)
+def test_backward_takes_the_strides_of_what_it_is_given(monkeypatch, first, then, dense):
+    """Saved-tensor hooks hand the backward other tensors than the forward had: `torch.autograd.graph.save_on_cpu` brings
+    every input back contiguous, whatever it was, a hook that packs them into one buffer brings back slices."""
+    if then == "expanded":
+        pytest.skip("an unpacked tensor holds the values of the packed one")
+    rec = _Recorder(monkeypatch)
+    values = [_dense(h, i) for i, h in enumerate((2, 1, H, HKV, HKV))]
+    inputs = tuple(_strided(t, first) for t in values)
+    plan = passes.plan(inputs, 0 if dense else 1, 0.1, dense)
+    out, _, saved = passes.forward(plan, inputs, None, None, 0, True)
+    unpacked = tuple(_strided(t, then) for t in values)
+    odd = torch.empty(out.numel() + 8, dtype=out.dtype)[1:1 + out.numel()].view(out.shape)
+    grads = passes.backward(plan, unpacked, odd, torch.zeros_like(out), saved, torch.ones(()), None, None, None, 0)
+    rec.check(rec.blocks[1], rec.given[1], values)
+    assert rec.blocks[1].out % 16 == 0
+    # the gradients keep the layout of the forward's inputs, which are the leaves
+    for name, g, t in zip(NAMES, grads, inputs):
+        assert getattr(rec.blocks[1], "d" + name) == g.data_ptr() and g.shape == t.shape
+        assert tuple(getattr(rec.blocks[1], f"d{name}_{x}") for x in ("sb", "sh", "ss")) + (1,) == g.stride()
+
+
+@pytest.mark.parametrize("odd", [{"dtype": torch.float16}, {"shape": True}, {"device": "meta"}])
+@pytest.mark.parametrize("which", range(7))
+def test_backward_refuses_tensors_of_another_kind(monkeypatch, which, odd):
+    """What comes back from a hook with another type, shape or device is refused instead of read."""
+    monkeypatch.setattr(passes, "_call", lambda fn, what, a, device: None)
+    inputs = [_dense(h, i) for i, h in enumerate((2, 1, H, HKV, HKV))]
+    plan = passes.plan(inputs, 1, 0.1, False)
+    out, _, saved = passes.forward(plan, inputs, None, None, 0, True)
+    ts = inputs + [out, saved]
+    ts[which] = ts[which][..., :64] if "shape" in odd else ts[which].to(**odd)
+    with pytest.raises(ValueError, match="backward"):
+        passes.backward(plan, ts[:5], ts[5], torch.zeros_like(out), ts[6], None, None, None, None, 0)
+
+
 class _SaysCuda(torch.Tensor):
     """A CPU tensor that reports `where` as its device (no launch is reached with it)."""
     where = torch.device("cuda", 0)
