@@ -57,9 +57,9 @@ def _validate_inputs(q_proxy, k_proxy, q, k, v, top_k, sparse: bool):
     return num_blocks, top_k_blocks
 
 
-def _require_cuda(q):
+def _require_cuda(q, message="flash_msa_b200 requires CUDA tensors (there is no CPU path)"):
     if q.device.type != "cuda":
-        raise RuntimeError("flash_msa_b200 requires CUDA tensors (there is no CPU path)")
+        raise RuntimeError(message)
 
 
 # The reference returns a zero placeholder as kl_loss and users cannot watch the distillation loss
@@ -125,16 +125,34 @@ def _sink_logits(sinks):
     return None if sinks is None else sinks.detach().to(torch.float32).contiguous()
 
 
+def _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, with_proxy):
+    """Checks the call, then runs its forward: (plan, fp32 sink logits or None, out, kl_loss placeholder, saved)."""
+    _, top_k_blocks = _validate_inputs(q_proxy, k_proxy, q, k, v, top_k if sparse else 0, sparse)
+    if sparse:
+        _require_cuda(q)
+    sinks = _check_sinks(sinks, q)
+    if not sparse:
+        _require_cuda(q, "warmup MSA forward requires CUDA tensors")
+    inputs = (q_proxy, k_proxy, q, k, v)
+    if any(t.device != q.device for t in inputs):   # (a host pointer would reach the kernels as it is)
+        raise ValueError("q_proxy, k_proxy, q, k, and v must be on one CUDA device")
+    plan = passes.plan(inputs, top_k_blocks, scale, not sparse)
+    logits = _sink_logits(sinks)
+    status = _Status(0 if sparse else 2, plan.device)
+    out, kl_loss, saved = passes.forward(plan, inputs, doc_start, logits, status.ptr, with_proxy)
+    status.check()
+    return plan, logits, out, kl_loss, saved
+
+
 class _AttentionFunction(torch.autograd.Function):
-    """Sparse (plan.dense False) or dense warmup attention behind autograd.  kl_loss is a placeholder whose gradient
-    switches the KL branch of the backward on (reference: flash_msa/msa_forward_cutedsl.py:69)."""
+    """Sparse or dense warmup attention behind autograd.  kl_loss is a placeholder whose gradient switches the KL branch of
+    the backward on (reference: flash_msa/msa_forward_cutedsl.py:69)."""
 
     @staticmethod
-    def forward(ctx, q_proxy, k_proxy, q, k, v, sinks, doc_start, plan):
-        status = _Status(2 if plan.dense else 0, plan.device)
-        logits = _sink_logits(sinks)
-        out, kl_loss, saved = passes.forward(plan, (q_proxy, k_proxy, q, k, v), doc_start, logits, status.ptr, True)
-        status.check()
+    def forward(ctx, q_proxy, k_proxy, q, k, v, sinks, doc_start, top_k, scale, sparse):
+        # (everything that depends on the inputs is done in here: a trace records this call as one node, which comes back with
+        # tensors of any size when the trace is run)
+        plan, logits, out, kl_loss, saved = _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, True)
         ctx.save_for_backward(q_proxy, k_proxy, q, k, v, out, saved)
         # an output that does not feed the loss arrives as None in backward (not as zeros): no gradient for
         # kl_loss then really skips the proxy work, as the reference intends (flash_msa/flash_msa.py:104-106)
@@ -155,28 +173,18 @@ class _AttentionFunction(torch.autograd.Function):
                                                        ctx.logits, status.ptr)
         _publish_kl(klv)
         status.check()
-        return dqp, dkp, dq, dk, dv, None if dsinks is None else dsinks.to(ctx.sinks_dtype), None, None
+        return dqp, dkp, dq, dk, dv, None if dsinks is None else dsinks.to(ctx.sinks_dtype), None, None, None, None
 
 
 def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks):
     q_proxy = _spread_proxy_heads(q_proxy, k_proxy, q, k)
-    _, top_k_blocks = _validate_inputs(q_proxy, k_proxy, q, k, v, top_k if sparse else 0, sparse)
-    if sparse:
-        _require_cuda(q)
-    sinks = _check_sinks(sinks, q)
-    if q.device.type != "cuda":
-        raise RuntimeError("warmup MSA forward requires CUDA tensors")
-    inputs = (q_proxy, k_proxy, q, k, v)
-    if any(t.device != q.device for t in inputs):   # (a host pointer would reach the kernels as it is)
-        raise ValueError("q_proxy, k_proxy, q, k, and v must be on one CUDA device")
-    plan = passes.plan(inputs, top_k_blocks, scale, not sparse)
-    if torch.is_grad_enabled() and (any(t.requires_grad for t in inputs) or (sinks is not None and sinks.requires_grad)):
-        return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, plan)
-    # no backward will follow: the proxy log-sum-exp, which only the backward needs, is left out
-    status = _Status(0 if sparse else 2, plan.device)
-    out, kl_loss, _ = passes.forward(plan, inputs, doc_start, _sink_logits(sinks), status.ptr, False)
-    status.check()
-    return out, kl_loss
+    with_grad = torch.is_grad_enabled() and (any(t.requires_grad for t in (q_proxy, k_proxy, q, k, v)) or
+                                             (sinks is not None and sinks.requires_grad))
+    if with_grad or torch._C._is_tracing():
+        return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, top_k, scale, sparse)
+    # No backward will follow: the proxy log-sum-exp, which only the backward needs, is left out.  (Under a trace this would
+    # leave nothing but the allocation of `out` in it.)
+    return _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, False)[2:4]
 
 
 def _spread_proxy_heads(q_proxy, k_proxy, q, k):

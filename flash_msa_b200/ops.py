@@ -230,8 +230,9 @@ def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> t
     """int32 [B,S] on `device`: for every token of a packed sequence the position of the first token of its document.
     `cu_seqlens` is [n+1] (one packing for every batch element) or [B,n+1]; it starts at 0 and ends at `seq_len`
     (the FlashAttention varlen convention).  The kernels take this array (`fmsa_problem.doc_start`)."""
-    if not (isinstance(cu_seqlens, torch.Tensor) and cu_seqlens.device.type == "cuda"):
+    if not (isinstance(cu_seqlens, torch.Tensor) and cu_seqlens.device.type == "cuda") and not torch._C._is_tracing():
         # boundaries that the host holds are checked here and travel as a kernel parameter: nothing waits for the device
+        # (a trace would not see that kernel; it records the torch operations below)
         cu = np.asarray(cu_seqlens)
         if cu.ndim not in (1, 2) or (cu.ndim == 2 and cu.shape[0] != batch) or cu.shape[-1] < 2:
             raise ValueError("cu_seqlens must have shape [n+1] or [B, n+1]")

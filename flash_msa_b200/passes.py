@@ -84,17 +84,16 @@ def _bshd(shape, stride):
 class Plan:
     """Everything about a call that shapes, strides, types and options decide."""
 
-    def __init__(self, inputs, top_k_blocks, scale, dense, max_partial_bytes):
-        qp, kp, q, k, v = inputs
+    def __init__(self, shapes, layout, dtype, device, top_k_blocks, scale, dense, max_partial_bytes):
         lib = _lib.load()
-        b, hq, s, d = q.shape
-        hkv, hp, hpkv = k.shape[1], qp.shape[1], kp.shape[1]
-        self.dense, self.shape, self.dtype, self.device = dense, (b, hq, s, d), q.dtype, q.device
-        self.pb = _lib.FmsaProblem(b, s, hq, hkv, hp, hpkv, 1 if dense else int(top_k_blocks), float(scale), ops._dtype_code(q.dtype), None)
+        hp, hpkv, hkv = (shapes[i][1] for i in (0, 1, 3))
+        b, hq, s, d = shapes[2]
+        self.dense, self.shape, self.dtype, self.device = dense, (b, hq, s, d), dtype, device
+        self.pb = _lib.FmsaProblem(b, s, hq, hkv, hp, hpkv, 1 if dense else int(top_k_blocks), float(scale), ops._dtype_code(dtype), None)
         self.max_partial_bytes = int(max_partial_bytes)
-        self.shapes, self.layout = [t.shape for t in inputs], [t.stride() for t in inputs]
+        self.shapes, self.layout = shapes, layout
         self.in_place = all(map(_conforms, self.layout))
-        self.grad_shapes = [((b, s, t.shape[1], d), True) if _bshd(t.shape, t.stride()) else (tuple(t.shape), False) for t in inputs]
+        self.grad_shapes = [((b, s, sh[1], d), True) if _bshd(sh, st) else (sh, False) for sh, st in zip(shapes, layout)]
         self.out_shape = (b, s, hq * d)
         pbr = ctypes.byref(self.pb)
         self.forward_bytes = lib.fmsa_forward_workspace_bytes(pbr, int(dense), self.max_partial_bytes)
@@ -172,13 +171,15 @@ _MAX_PLANS = 256
 
 def plan(inputs, top_k_blocks, scale, dense) -> Plan:
     q = inputs[2]
-    key = (top_k_blocks, scale, dense, ops.MAX_PARTIAL_BYTES, ops.SPLIT_PARTIALS_ABOVE, q.dtype, q.device,
-           *[t.shape for t in inputs], *[t.stride() for t in inputs])
+    shapes, layout = [t.shape for t in inputs], [t.stride() for t in inputs]
+    if torch._C._is_tracing():   # sizes are traced tensors then
+        shapes = [torch.Size(map(int, sh)) for sh in shapes]
+    key = (top_k_blocks, scale, dense, ops.MAX_PARTIAL_BYTES, ops.SPLIT_PARTIALS_ABOVE, q.dtype, q.device, *shapes, *layout)
     p = _plans.get(key)
     if p is None:
         if len(_plans) >= _MAX_PLANS:
             _plans.clear()
-        p = _plans[key] = Plan(inputs, top_k_blocks, scale, dense, ops.MAX_PARTIAL_BYTES)
+        p = _plans[key] = Plan(shapes, layout, q.dtype, q.device, top_k_blocks, scale, dense, ops.MAX_PARTIAL_BYTES)
     return p
 
 

@@ -1,5 +1,7 @@
 """Host side of the whole-pass calls, without a GPU: what an argument block says about the tensors whose pointers it holds.
 The native call is replaced by a recorder, so that nothing is launched."""
+import ctypes
+
 import pytest
 import torch
 
@@ -136,3 +138,52 @@ def test_inputs_on_another_device_than_q_are_refused(monkeypatch, where, odd, wa
     # (a q that is not on a GPU keeps its own error)
     with pytest.raises(RuntimeError, match="CUDA"):
         fn(*(_dense(h, i) for i, h in enumerate((2, 1, H, HKV, HKV))), 128, 0.1)
+
+
+@pytest.fixture
+def on_the_host(monkeypatch):
+    """The public functions on CPU tensors, with a forward that copies q's storage to `out` behind torch's back."""
+    from flash_msa_b200 import api
+
+    def forward(p, inputs, doc_start, sinks, status_ptr, with_proxy):
+        out = torch.empty(p.out_shape, dtype=p.dtype)
+        ctypes.memmove(out.data_ptr(), inputs[2].data_ptr(), 2 * out.numel())
+        if doc_start is not None:
+            ctypes.memmove(out.data_ptr(), doc_start.data_ptr(), 4 * doc_start.numel())
+        return out, torch.zeros(()), torch.zeros(p.saved_words, dtype=torch.int32)
+    monkeypatch.setattr(passes, "forward", forward)
+    monkeypatch.setattr(passes.status_board, "pointer", lambda kind, device: 0)
+    monkeypatch.setattr(api, "_require_cuda", lambda *a: None)
+    return api
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("warmup", [False, True])
+def test_a_trace_calls_the_library(on_the_host, grad, warmup):
+    """A traced function runs the call again on what it is given, also with other sizes, and refuses what the call refuses."""
+    import flash_msa_b200 as fm
+    fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
+
+    def values(seed, b=B):
+        g = torch.Generator().manual_seed(seed)
+        return tuple(torch.randn(b, h, S, 128, generator=g).to(torch.bfloat16) for h in (2, 1, H, HKV, HKV))
+    with torch.set_grad_enabled(grad):
+        first = tuple(t.requires_grad_(grad) for t in values(1))
+        traced = torch.jit.trace(lambda *ts: fn(*ts, 128, 0.1), first, check_trace=False)
+        for ts in (values(2), values(3, b=1)):
+            out, _ = traced(*ts)
+            assert torch.equal(out.detach().flatten(), ts[2].flatten())
+        with pytest.raises((ValueError, RuntimeError), match="divisible by 128"):
+            traced(*(t[:, :, :200] for t in values(4)))
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+def test_a_trace_keeps_document_boundaries(on_the_host):
+    import flash_msa_b200 as fm
+    ts = tuple(_dense(h, i) for i, h in enumerate((2, 1, H, HKV, HKV)))
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda *a: fm.flash_msa_varlen_func(*a, [0, 100, S], 128, 0.1), ts, check_trace=False)
+        out, _ = traced(*ts)
+    doc_start = out.flatten()[:2 * B * S].view(torch.int32).view(B, S)
+    assert torch.equal(doc_start, torch.tensor([0] * 100 + [100] * (S - 100), dtype=torch.int32).expand(B, S))
