@@ -4,6 +4,7 @@ flash_msa/warmup/flash_msa_warmup.py:6-106), on top of the sm_100a kernels."""
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 from . import ops, passes
 
@@ -180,10 +181,10 @@ def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks):
     q_proxy = _spread_proxy_heads(q_proxy, k_proxy, q, k)
     with_grad = torch.is_grad_enabled() and (any(t.requires_grad for t in (q_proxy, k_proxy, q, k, v)) or
                                              (sinks is not None and sinks.requires_grad))
-    if with_grad or torch._C._is_tracing():
+    if with_grad or forward_ad._current_level >= 0 or torch._C._is_tracing():
         return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, top_k, scale, sparse)
-    # No backward will follow: the proxy log-sum-exp, which only the backward needs, is left out.  (Under a trace this would
-    # leave nothing but the allocation of `out` in it.)
+    # No backward will follow: the proxy log-sum-exp, which only the backward needs, is left out.  (Tangents would be lost
+    # here, which the autograd function refuses, and a trace would hold nothing but the allocation of `out`.)
     return _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, False)[2:4]
 
 

@@ -4,6 +4,7 @@ import ctypes
 
 import pytest
 import torch
+from torch.autograd import forward_ad
 
 from flash_msa_b200 import passes
 
@@ -187,3 +188,25 @@ def test_a_trace_keeps_document_boundaries(on_the_host):
         out, _ = traced(*ts)
     doc_start = out.flatten()[:2 * B * S].view(torch.int32).view(B, S)
     assert torch.equal(doc_start, torch.tensor([0] * 100 + [100] * (S - 100), dtype=torch.int32).expand(B, S))
+
+
+@pytest.mark.parametrize("warmup", [False, True])
+def test_transforms_without_a_rule_are_refused(monkeypatch, warmup):
+    """Tangents would be lost without a word, and batched tensors have no memory of their own."""
+    import flash_msa_b200 as fm
+    from flash_msa_b200 import api
+    launched = []
+    monkeypatch.setattr(passes, "_call", lambda *a: launched.append(a))
+    monkeypatch.setattr(passes.status_board, "pointer", lambda kind, device: 0)
+    monkeypatch.setattr(api, "_require_cuda", lambda *a: None)
+    fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
+    inputs = [_dense(h, i) for i, h in enumerate((2, 1, H, HKV, HKV))]
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad), forward_ad.dual_level():
+            q = forward_ad.make_dual(inputs[2], torch.ones_like(inputs[2]))
+            with pytest.raises(NotImplementedError, match="jvp"):
+                fn(*inputs[:2], q, *inputs[3:], 128, 0.1)
+        launched.clear()   # (the autograd function runs its forward before it looks for a rule)
+        with torch.set_grad_enabled(grad), pytest.raises(RuntimeError):
+            torch.func.vmap(lambda *ts: fn(*ts, 128, 0.1))(*(t.unsqueeze(0) for t in inputs))
+        assert not launched
