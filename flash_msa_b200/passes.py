@@ -6,6 +6,7 @@ B=1 S=1024 Hq=8, six times what the GPU needs.)"""
 from __future__ import annotations
 
 import ctypes
+import threading
 from ctypes import c_float, c_int32, c_int64, c_void_p
 
 import torch
@@ -258,18 +259,22 @@ def backward(p: Plan, inputs, out, grad_out, saved, grad_kl, kl_value, doc_start
 
 class StatusBoard:
     """Status words of the calls of this process, in pinned host memory that the kernels write directly (only ever when
-    something is wrong), so that a call needs no word of its own, no copy and no event.  A word is one of a few kinds of
-    call; trouble raises RuntimeError at the next call of the library or at `drain`."""
+    something is wrong), so that a call needs no word of its own, no copy and no event.  There is one word for each of a few
+    kinds of call, shared by all threads, streams and devices: it says what kind of call met trouble, not whose it was, and the
+    RuntimeError is raised by whichever call of the library comes next, or by `drain`."""
     KINDS = ("flash_msa_func forward", "flash_msa_func backward", "flash_msa_warmup_func forward", "flash_msa_warmup_func backward")
 
     def __init__(self):
         self._words = None
         self._devices = set()
+        self._lock = threading.Lock()
 
     def pointer(self, kind: int, device) -> int:
         if self._words is None:
-            self._keep = torch.zeros(16, dtype=torch.int32).pin_memory()
-            self._words = (c_int32 * 16).from_address(self._keep.data_ptr())
+            with self._lock:   # of several first calls one makes the words; kernels hold on to their address
+                if self._words is None:
+                    self._keep = torch.zeros(16, dtype=torch.int32).pin_memory()
+                    self._words = (c_int32 * 16).from_address(self._keep.data_ptr())
         self._devices.add(device)
         self.poll()
         return ctypes.addressof(self._words) + 4 * kind

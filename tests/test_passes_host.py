@@ -1,6 +1,8 @@
 """Host side of the whole-pass calls, without a GPU: what an argument block says about the tensors whose pointers it holds.
 The native call is replaced by a recorder, so that nothing is launched."""
 import ctypes
+import threading
+import time
 
 import pytest
 import torch
@@ -210,3 +212,29 @@ def test_transforms_without_a_rule_are_refused(monkeypatch, warmup):
         with torch.set_grad_enabled(grad), pytest.raises(RuntimeError):
             torch.func.vmap(lambda *ts: fn(*ts, 128, 0.1))(*(t.unsqueeze(0) for t in inputs))
         assert not launched
+
+
+def test_first_calls_of_several_threads_share_one_status_board(monkeypatch):
+    """Pinning takes a while, and every thread that makes its first call meanwhile must end up with the same words."""
+    pinned = []
+
+    def pin(t):
+        time.sleep(0.05)
+        pinned.append(t)
+        return t
+    monkeypatch.setattr(torch.Tensor, "pin_memory", pin)
+    board, start, got = passes.StatusBoard(), threading.Barrier(8), []
+
+    def call(i):
+        start.wait()
+        got.append(board.pointer(i % 4, torch.device("cuda", 0)) - 4 * (i % 4))
+    threads = [threading.Thread(target=call, args=(i,)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(pinned) == 1 and got == [pinned[0].data_ptr()] * 8
+    ctypes.c_int32.from_address(got[0] + 4).value = 2
+    with pytest.raises(RuntimeError, match="flash_msa_func backward.*out-of-range index"):
+        board.pointer(0, torch.device("cuda", 0))
+    assert board.pointer(0, torch.device("cuda", 0)) == got[0]     # raised once
