@@ -114,13 +114,14 @@ constexpr uint32_t kHalfRowBytes = 64 * 128;   // rows 64.. of a panel: where ha
 //                at a time: 8 columns of P^T, then 8 of dS^T); columns 64..127 dP^T, then dQ^T (lane = head dimension).
 //   R2 [256,384) dV, R3 [384,512) dK (lane = key), accumulated over the sub-unit.
 // A step of the issuing warp (half x of main tile t), behind P^T / dS^T of that half:
-//   dQ^T = K^T dS^T -> Rx+64,  dV += P^T dO,  dK += dS^T Q,  S^T(t+1) = K Q^T -> Rx,  [dQ^T read out]  dP^T(t+1) = V dO^T -> Rx+64
+//   dQ^T = K^T dS^T -> Rx+64,  dV += P^T dO,  dK += dS^T Q,  [these complete]  S^T(t+1) = K Q^T -> Rx,  [dQ^T read out]
+//   dP^T(t+1) = V dO^T -> Rx+64
 // so dQ^T is read out under three products, and everything half x needs for tile t+1 is under way before the step of the
 // other half begins.  (As one 128-query tile whose products, arithmetic and hand-offs followed one another, a tile took 8.1 k
 // cycles, 4.0 k of them products: S^T, dP^T, dV and dK of 128 queries fill the 512 columns, and nothing of the next tile
 // could start before dQ had been read out.)
-// Hand-offs (mbarriers; one arrival per warp or per tcgen05.commit): qdo_full (TMA bytes) <- qdo_empty; st_full <- st_empty
-// (row statistics); sdp_full (S^T and dP^T of a half), pds_full (P^T, dS^T written), dq_full -> dq_free (dQ^T read out),
+// Hand-offs (mbarriers; one arrival per warp or per tcgen05.commit): qdo_full (TMA bytes) <- qdo_empty (dV, dK have read the
+// rows, and the half's P^T, dS^T); st_full <- st_empty (row statistics); sdp_full (S^T and dP^T of a half), pds_full (P^T, dS^T written), dq_full -> dq_free (dQ^T read out),
 // ds_free (the half's panel of the dS^T tile, which doubles as the staging tile of its dQ store, is reusable),
 // acc_full / acc_free (dV, dK flushed at the end of a sub-unit).
 // VARLEN: document masking of packed sequences (P.doc_start given).  A separate instantiation, so that the plain kernel
@@ -290,6 +291,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                         for (int fx = u < 0 ? 0 : x; fx <= x; ++fx) {
                             const uint32_t rf = tmem + 128 * fx;
                             wait1(BAR(sm->qdo_full[s][fx]), (g >> 1) & 1);
+                            // dV and dK of the half's previous tile read P^T, dS^T from the columns that S^T overwrites: they must
+                            // have completed, because products are only sure to follow one another where accumulator and shape
+                            // are the same.  (At B=2 S=8192 Hq=32 top-k 16 blocks the wait takes this kernel from 1.161 to
+                            // 1.192 ms without KL work, the two backward kernels from 1.586 to 1.594 ms with it; dQ^T issued behind
+                            // dV and dK, so that the tensor core has work meanwhile, 1.237 and 1.640: dQ^T is read out later.)
+                            if (g >= 1) wait1(BAR(sm->qdo_empty[s ^ 1][fx]), ((g - 1) >> 1) & 1);
                             if (bad) break;
                             tc_fence_after_sync();
                             umma_ss<64, 8, false, false, FP16>(rf, tile_k, tile_q0 + s * kTileBytes + fx * kHalfRowBytes, false);   // S^T = K_j Q_g^T
