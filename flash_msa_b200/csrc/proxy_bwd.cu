@@ -184,6 +184,10 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
                     if (t + 1 < ntiles) {   // Sp^T runs one tile ahead
                         const uint32_t g = gt + (t >= 0 ? 1 : 0);
                         wait1(BAR(sm->q_full[fs]), fph);
+                        // dKp of tile g - 2 (its Qp stage is the one after this) reads dSp^T from the columns that Sp^T overwrites:
+                        // it must have completed, because products are only sure to follow one another where accumulator and
+                        // shape are the same.
+                        if (g >= 2) wait1(BAR(sm->q_empty[fs == kProxyQStages - 1 ? 0 : fs + 1]), ((g - 2) / kProxyQStages) & 1);
                         if (bad) break;
                         tc_fence_after_sync();
                         umma_tile_128<false, false, FP16>(tmem + (g & 1) * 128, kp, tile_q0 + fs * kTileBytes, false);
