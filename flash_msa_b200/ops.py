@@ -276,64 +276,6 @@ def check_status(status: torch.Tensor, what: str) -> None:
         raise RuntimeError(f"{what}: {_STATUS_NAMES.get(code, code)}")
 
 
-class DeferredStatus:
-    """Checks device status words without synchronising: `push` copies the word to a slot of a small pinned
-    ring on the current stream and records an event; every later `push` (and `drain`) looks at the words
-    whose events have completed and raises for a non-zero one, so a timed-out wait or a bad index surfaces
-    at the next call of the library instead of passing silently.  Nothing is queued while the stream is
-    being captured into a graph."""
-    SLOTS = 64
-
-    def __init__(self):
-        self._host = None
-        self._pending = []        # (slot, event, what, status tensor: kept alive until its copy has run)
-        self._next = 0
-
-    def _poll(self, block: bool) -> None:
-        while self._pending:
-            slot, event, what, _ = self._pending[0]
-            if block:
-                event.synchronize()
-            elif not event.query():
-                return
-            self._pending.pop(0)
-            code = int(self._host[slot])
-            if code != 0:
-                raise RuntimeError(f"{what} (reported late): {_STATUS_NAMES.get(code, code)}")
-
-    def push(self, status: torch.Tensor, what: str) -> None:
-        if torch.cuda.is_current_stream_capturing():
-            return
-        if self._host is None:
-            self._host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
-            self._side = {}
-        self._poll(block=len(self._pending) >= self.SLOTS - 1)
-        slot = self._next
-        self._next = (slot + 1) % self.SLOTS
-        # The copy runs on a side stream behind an event of the calling stream: a device-to-host copy on the calling
-        # stream itself would queue behind whatever large copies the application has on the copy engine and hold
-        # the next kernels back (measured: 3.4 ms per step in the host-buffer pipeline).
-        dev = status.device
-        side = self._side.get(dev)
-        if side is None:
-            side = self._side[dev] = torch.cuda.Stream(dev)
-        done = torch.cuda.Event()
-        done.record(torch.cuda.current_stream(dev))
-        side.wait_event(done)
-        event = torch.cuda.Event()
-        with torch.cuda.stream(side):
-            self._host[slot:slot + 1].copy_(status, non_blocking=True)
-            event.record(side)
-        # (the reference held here, not record_stream: the caching allocator then never has to defer the reuse of
-        # the word's block by the side stream's progress, which would make its behaviour depend on host timing)
-        self._pending.append((slot, event, what, status))
-
-    def drain(self) -> None:
-        """Waits for every queued status word and raises for the first non-zero one."""
-        self._poll(block=True)
-
-
-
 def proxy_block_scores(q_proxy: torch.Tensor, k_proxy: torch.Tensor, scale: float, status=None, doc_start=None) -> torch.Tensor:
     """fp32 block scores [B,Hp,S,NB]; entries of future blocks are left unwritten.  With `doc_start` (int32 [B,S]) the
     keys before a row's document are hidden and blocks that lie entirely before it score -inf."""

@@ -75,19 +75,28 @@ def test_bounded_wait_runs_out(ops):
 
 
 def test_status_word_surfaces_without_synchronising(ops):
-    """The status word of a call is copied to pinned memory behind it and raised by a later look: a kernel whose
-    bounded wait ran out (status 1) turns into a RuntimeError at `drain`, a clean call into nothing."""
+    """A kernel writes its status word into pinned host memory, and the next call of the library looks at it without waiting:
+    a bounded wait that ran out (status 1) turns into a RuntimeError there, once, a clean call into nothing."""
+    import flash_msa_b200 as fm
+    from flash_msa_b200 import _lib, passes
     g = torch.Generator(device="cpu").manual_seed(13)
     src = torch.randn(256, 128, generator=g).to(torch.bfloat16).cuda()
     b = torch.randn(128, 128, generator=g).to(torch.bfloat16).cuda()
-    rows = torch.arange(128).cuda()
-    watch = ops.DeferredStatus()
-    watch.push(ops.pipeline_selftest(src, rows, b)[3], "clean call")
-    watch.drain()
-    watch.push(ops.pipeline_selftest(src, rows, b, withhold=True, limit_ns=2_000_000)[3], "withheld signal")
-    with pytest.raises(RuntimeError, match="withheld signal.*timed out"):
-        watch.drain()
-    watch.drain()                                   # the queue is empty again
+    rows = torch.arange(128, dtype=torch.int32).cuda()
+    d = torch.zeros(2, 128, 128, device="cuda")
+    part = torch.zeros(128, 2, 128, dtype=torch.bfloat16, device="cuda")
+    qp, kp, q, k, v = (torch.randn(1, h, 256, 128, generator=g).to(torch.bfloat16).cuda() for h in (1, 1, 2, 1, 1))
+    call = lambda: fm.flash_msa_func(qp, kp, q, k, v, 128, 128 ** -0.5)
+    want = call()[0]
+    for withhold in (0, 1):
+        word = passes.status_board.pointer(0, src.device)
+        _lib.check(_lib.load().fmsa_pipeline_selftest(src.data_ptr(), 256, rows.data_ptr(), b.data_ptr(), d[0].data_ptr(), d[1].data_ptr(),
+                                                      part.data_ptr(), withhold, 2_000_000, word, None), "selftest")
+        torch.cuda.synchronize()
+        if withhold:
+            with pytest.raises(RuntimeError, match="flash_msa_func forward.*timed out"):
+                call()
+        assert torch.equal(call()[0], want)
 
 
 @pytest.mark.parametrize("s,kb", [(128, 1), (512, 2), (1024, 4), (2048, 16), (4096, 32), (8192, 33), (8192, 64), (16384, 128)])
