@@ -100,6 +100,33 @@ def test_saved_tensors_kept_on_the_host(warmup):
         assert max_err(a, b) <= (0.0 if n in ("dq", "dq_proxy") else 2 ** -7 * a.float().abs().max().item()), n
 
 
+@pytest.mark.parametrize("dense,kl,cap,cu", [(False, True, None, None), (False, False, 1, None), (True, True, 1, None),
+                                             (False, True, None, [0, 100, 640]), (True, False, None, [0, 100, 640])])
+def test_single_stages_agree_with_whole_passes(monkeypatch, dense, kl, cap, cu):
+    """The stage entry points, which other bindings call one by one, against the whole-pass calls that drive the same kernels:
+    bit for bit where sums have a fixed order, also over several passes."""
+    import flash_msa_b200 as fm
+    from flash_msa_b200 import ops
+    if cap:
+        monkeypatch.setattr(ops, "MAX_PARTIAL_BYTES", cap)
+    cfg = dict(b=2, s=640, hq=12, hkv=2, hp=4, hpkv=2, kb=2, seed=93)
+    qp, kp, q, k, v, do = bf16_inputs(cfg)
+    gk = torch.ones((), device="cuda") if kl else None
+    leaves = [t.detach().requires_grad_(True) for t in (qp, kp, q, k, v)]
+    fn = {(False, False): fm.flash_msa_func, (True, False): fm.flash_msa_warmup_func, (False, True): fm.flash_msa_varlen_func,
+          (True, True): fm.flash_msa_warmup_varlen_func}[dense, cu is not None]
+    out, kl_loss = fn(*leaves, *([] if cu is None else [cu]), cfg["kb"] * 128, SCALE)
+    torch.autograd.backward([out, kl_loss] if kl else [out], [do, gk] if kl else [do])
+    ds = None if cu is None else ops.doc_start_from_cu_seqlens(cu, cfg["b"], cfg["s"], qp.device)
+    rix = None if dense else ops.build_reverse_index(ops.select_blocks_fused(qp, kp, SCALE, cfg["kb"], doc_start=ds))
+    out2, lse, lse_p = ops.attention_forward(q, k, v, qp, kp, SCALE, rix, dense=dense, doc_start=ds)
+    grads = ops.attention_backward(q, k, v, qp, kp, out2, do, lse, lse_p, SCALE, rix, gk, dense=dense, doc_start=ds)
+    assert torch.equal(out, out2)
+    for n, leaf, b in zip(NAMES, leaves, grads):
+        a = torch.zeros_like(b) if leaf.grad is None else leaf.grad
+        assert max_err(a, b) <= (0.0 if n in ("dq", "dq_proxy") else 2 ** -7 * b.float().abs().max().item()), n
+
+
 @pytest.mark.parametrize("cu", [[0, 512], [0, 0, 1, 130, 130, 511, 512, 512], [[0, 7, 512], [0, 512, 512]], list(range(0, 513)) + [512] * 500])
 def test_document_boundaries_from_the_host(cu):
     """Short lists travel as a kernel parameter, long ones and device tensors take the other way: the same array."""
