@@ -224,7 +224,8 @@ def sparse_attention_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, s
     varlen convention) gives their boundaries, and a query sees only the keys of its own document - in the block scores
     and the selection, in the attention and in every gradient.  Blocks stay 128 positions of the PACKED sequence, so S
     must still be a multiple of 128 (pad the last document).  The reference has no such path (its README lists
-    variable-length batches as missing).  Boundaries in host memory (a list, a CPU tensor) spare the call a wait."""
+    variable-length batches as missing).  Boundaries in host memory (a list, a CPU tensor) are checked there
+    and travel with a kernel launch; those in a CUDA tensor make the call wait for the device, for the same checks."""
     return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, _doc_start(q, cu_seqlens), sinks)
 
 

@@ -230,21 +230,23 @@ def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> t
     """int32 [B,S] on `device`: for every token of a packed sequence the position of the first token of its document.
     `cu_seqlens` is [n+1] (one packing for every batch element) or [B,n+1]; it starts at 0 and ends at `seq_len`
     (the FlashAttention varlen convention).  The kernels take this array (`fmsa_problem.doc_start`)."""
-    if not (isinstance(cu_seqlens, torch.Tensor) and cu_seqlens.device.type == "cuda") and not torch._C._is_tracing():
+    cu_seqlens = torch.as_tensor(cu_seqlens)
+    if cu_seqlens.device.type == "cpu" and not torch._C._is_tracing():
         # boundaries that the host holds are checked here and travel as a kernel parameter: nothing waits for the device
         # (a trace would not see that kernel; it records the torch operations below)
-        cu = np.asarray(cu_seqlens)
+        cu = cu_seqlens.to(torch.int64).numpy()
         if cu.ndim not in (1, 2) or (cu.ndim == 2 and cu.shape[0] != batch) or cu.shape[-1] < 2:
             raise ValueError("cu_seqlens must have shape [n+1] or [B, n+1]")
         if (cu[..., 0] != 0).any() or (cu[..., -1] != seq_len).any() or (cu[..., 1:] < cu[..., :-1]).any():
             raise ValueError("cu_seqlens must rise from 0 to the sequence length")
-        if cu.size <= MAX_HOST_BOUNDARIES and torch.device(device).type == "cuda":
+        if cu.size <= MAX_HOST_BOUNDARIES and batch <= 65535 and torch.device(device).type == "cuda":
             cu = np.ascontiguousarray(cu, dtype=np.int32)
             out = torch.empty(batch, seq_len, dtype=torch.int32, device=device)
             _launch("fmsa_doc_start", 1, _lib.load().fmsa_doc_start(cu.ctypes.data, cu.shape[-1], int(cu.ndim == 2), batch, seq_len,
                                                                  out.data_ptr(), _stream(out.device)), out.device)
             return out
-    cu = torch.as_tensor(cu_seqlens).to(device=device, dtype=torch.int64)
+    # (boundaries in device memory: the checks below wait for the device, three times)
+    cu = cu_seqlens.to(device=device, dtype=torch.int64)
     if cu.dim() == 1:
         cu = cu.unsqueeze(0).expand(batch, -1)
     if cu.dim() != 2 or cu.shape[0] != batch or cu.shape[1] < 2:

@@ -4,11 +4,13 @@ import ctypes
 import threading
 import time
 
+import numpy as np
 import pytest
 import torch
 from torch.autograd import forward_ad
 
 from flash_msa_b200 import passes
+from oracle import msa_oracle as O
 
 B, H, HKV, S = 2, 4, 2, 256
 NAMES = ("q_proxy", "k_proxy", "q", "k", "v")
@@ -238,3 +240,18 @@ def test_first_calls_of_several_threads_share_one_status_board(monkeypatch):
     with pytest.raises(RuntimeError, match="flash_msa_func backward.*out-of-range index"):
         board.pointer(0, torch.device("cuda", 0))
     assert board.pointer(0, torch.device("cuda", 0)) == got[0]     # raised once
+
+
+@pytest.mark.parametrize("form", ["list", "tuple", "range", "int32", "bf16", "scalars", "numpy", "per_batch"])
+def test_forms_of_document_boundaries(form):
+    """Whatever torch.as_tensor takes is taken, from host memory as well."""
+    from flash_msa_b200 import ops
+    cu = [0, 64, 192, 256]
+    given = {"list": cu, "tuple": tuple(cu), "range": range(0, 257, 64), "int32": torch.tensor(cu, dtype=torch.int32),
+             "bf16": torch.tensor(cu).to(torch.bfloat16), "scalars": [torch.tensor(x) for x in cu],
+             "numpy": np.array(cu, dtype=np.int16), "per_batch": [cu, [0, 0, 1, 256]]}[form]
+    got = ops.doc_start_from_cu_seqlens(given, 2, 256, torch.device("cpu"))
+    assert torch.equal(got, O.doc_start_from_cu_seqlens(list(given) if form == "range" else given if form == "per_batch" else cu, 256, 2))
+    for bad in ([0, 5, 3, 256], [1, 256], [0, 255], [0], [[0, 256]] * 3):
+        with pytest.raises(ValueError):
+            ops.doc_start_from_cu_seqlens(bad, 2, 256, torch.device("cpu"))
