@@ -46,12 +46,16 @@ __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int ppk, 
 }
 
 // C for a launch: the largest power of two up to 8 that still leaves every CTA `kSubUnitsPerCta` sub-units on average, or 16
-// where that leaves it `kLongSubUnitsPerCta`.  A
-// sub-unit loads K and V once and flushes dV and dK once, so long ones save traffic; short ones fill the SMs and bound the
-// tail of the launch: a problem of a few dozen chunks otherwise runs on a handful of SMs (B=1, S=1024, Hq=8, top-k 4 blocks:
-// 64 chunks on 16 CTAs).  `edges` is an upper bound of the selected (row, block) pairs; a row of the reverse index is on
-// average half a chunk longer than its edges.  Drawing and passing over sub-units beyond the end of their rows costs about a
-// microsecond (up to 32 at a time), so C does not go below what keeps the enumeration at `kDrawsPerCta` per CTA.
+// where that leaves it `kLongSubUnitsPerCta`.  A sub-unit loads K and V once and flushes dV and dK once, so long ones save
+// traffic; short ones fill the SMs and bound the tail of the launch: a problem of a few dozen chunks otherwise runs on a
+// handful of SMs (B=1, S=1024, Hq=8, top-k 4 blocks: 64 chunks on 16 CTAs).
+// The averages are those of an upper bound: `edges` is what the host knows without a look at the selection, S * top_k_blocks
+// per proxy head in the sparse schedule.  Early rows have fewer blocks to select, and documents hide some: 77 % of it are
+// there at S=4096 top-k 16 blocks, 63 % at S=16384 top-k 96, 48 % with five documents at S=8192 top-k 16, so a launch can
+// have half the sub-units per CTA that the constants say.  Both constants were measured with this bound (and the lengths below
+// chosen by it).  A row of the reverse index is on average half a chunk longer than its edges.  Drawing and passing over
+// sub-units beyond the end of their rows costs about a microsecond (up to 32 at a time), so C does not go below what keeps
+// the enumeration at `kDrawsPerCta` per CTA.
 // With 16 the rows of a group are gathered in half as many sweeps, which counts where they do not fit L2 (B=1 S=65536 Hq=8
 // top-k 32 blocks, 14 sub-units per CTA: forward 1.70 -> 1.56 ms, backward 3.83 -> 3.49 ms; S=32768, 64 blocks: equal), while
 // at 7 sub-units per CTA (B=2 S=8192 Hq=32 top-k 16 blocks) the tail makes it slower: 0.672 -> 0.692 ms forward.
