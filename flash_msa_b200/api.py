@@ -135,7 +135,8 @@ def _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, 
     if not sparse:
         _require_cuda(q, "warmup MSA forward requires CUDA tensors")
     inputs = (q_proxy, k_proxy, q, k, v)
-    if any(t.device != q.device for t in inputs):   # (a host pointer would reach the kernels as it is)
+    dev = q.device
+    if q_proxy.device != dev or k_proxy.device != dev or k.device != dev or v.device != dev:   # (a host pointer would reach the kernels as it is)
         raise ValueError("q_proxy, k_proxy, q, k, and v must be on one CUDA device")
     plan = passes.plan(inputs, top_k_blocks, scale, not sparse)
     logits = _sink_logits(sinks)

@@ -94,7 +94,7 @@ class Plan:
         self.max_partial_bytes = int(max_partial_bytes)
         self.shapes, self.layout = shapes, layout
         self.in_place = all(map(_conforms, self.layout))
-        self.grad_shapes = [((b, s, sh[1], d), True) if _bshd(sh, st) else (sh, False) for sh, st in zip(shapes, layout)]
+        self.grad_shapes = [((b, s, sh[1], d), True) if _bshd(sh, st) else (tuple(sh), False) for sh, st in zip(shapes, layout)]
         self.out_shape = (b, s, hq * d)
         pbr = ctypes.byref(self.pb)
         self.forward_bytes = lib.fmsa_forward_workspace_bytes(pbr, int(dense), self.max_partial_bytes)
@@ -146,7 +146,8 @@ class Plan:
         launch).  The block's strides are those the plan was made for; where the tensors have others (`as_planned` False: these
         inputs; or copies) they are filled in with the addresses."""
         given = self.conform(inputs, as_planned)
-        a.q_proxy, a.k_proxy, a.q, a.k, a.v = (t.data_ptr() for t in given)
+        qp, kp, q, k, v = given
+        a.q_proxy, a.k_proxy, a.q, a.k, a.v = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
         if given is not inputs:
             for name, t in zip(_ORDER, given):
                 self._strides(a, name, t.stride())
@@ -154,11 +155,15 @@ class Plan:
 
     def check_unpacked(self, inputs, out, saved):
         """Raises ValueError for tensors that a saved-tensor hook brought back as something else."""
-        dev = self.device
-        if (out.shape != self.out_shape or out.dtype != self.dtype or out.device != dev
-                or saved.shape != (self.saved_words,) or saved.dtype != torch.int32 or saved.device != dev
-                or any(t.shape != sh or t.dtype != self.dtype or t.device != dev for t, sh in zip(inputs, self.shapes))):
-            raise ValueError("the tensors saved for the backward came back with another shape, type or device")
+        dtype, dev = self.dtype, self.device
+        for t, shape in zip(inputs, self.shapes):
+            if t.shape != shape or t.dtype != dtype or t.device != dev:
+                break
+        else:
+            if (out.shape == self.out_shape and out.dtype == dtype and out.device == dev
+                    and saved.shape == (self.saved_words,) and saved.dtype == torch.int32 and saved.device == dev):
+                return
+        raise ValueError("the tensors saved for the backward came back with another shape, type or device")
 
 
 def _whole(t):
