@@ -412,14 +412,15 @@ def local_problem(name, rank, world):
 
 
 def bwd_traffic_bytes(workload):
-    """DRAM bytes per launch of the dominant kernel from the committed ncu summary (profiles/traffic_c2q.json: a
-    capture of the quarter-size case; traffic is proportional to the (batch, KV group) units processed)."""
+    """DRAM bytes per step of the backward attention kernels (sparse_bwd_kernel, proxy_bwd_kernel) from the committed ncu summary
+    (profiles/traffic_c2q.json: a capture of the quarter-size case; traffic is proportional to the (batch, KV group) units
+    processed)."""
     path = os.path.join(ROOT, "profiles", "traffic_c2q.json")
     if workload != "c2" or not os.path.exists(path):
         return None
     with open(path) as f:
         t = json.load(f)
-    return float(t["scale_to_c2"]) * (float(t["dram_bytes_read"]) + float(t["dram_bytes_write"]))
+    return float(t["scale_to_c2"]) * sum(float(k["dram_bytes_read"]) + float(k["dram_bytes_write"]) for k in t["kernels"].values())
 
 
 class GpuContext:
@@ -622,18 +623,18 @@ def main():
     value = total_flops / (ms_per_step * 1e-3) / 1e12
     tokens = cfg["b"] * cfg["s"] * (world if scaling == "weak" else 1)
 
-    # dominant kernel: the fused backward.  Algorithmic FLOPs per launch = 5 products over the
-    # selected pairs of this rank's problem.
+    # Dominant kernels: the backward's two (main, and the KL part behind it), which one stage times together.  Algorithmic FLOPs
+    # = 5 products over the selected pairs of this rank's problem; the KL part's own products are not counted.
     bwd_times = main_res["per_kernel"].get("attn_bwd", [float("nan")])
     bwd_ms_step = sum(bwd_times) / main_res["steps"]     # all launches of one step (large problems run in passes)
-    bwd_launches = len(bwd_times) / main_res["steps"]
+    bwd_passes = len(bwd_times) / main_res["steps"]
     bwd_flops = flops(local) * 5.0 / 7.0
     achieved = bwd_flops / (bwd_ms_step * 1e-3) / 1e12
-    traffic = bwd_traffic_bytes(args.workload) if bwd_launches == 1 else None
-    roofline = {"kernel": "sparse_bwd_kernel", "bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"],
+    traffic = bwd_traffic_bytes(args.workload) if bwd_passes == 1 else None
+    roofline = {"kernel": "sparse_bwd_kernel + proxy_bwd_kernel", "bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"],
                 "unit": "TFLOP/s", "frac": achieved / peaks["bf16_tflops"], "traffic": traffic,
-                "peak_source": f"{peaks['source']} (burst cuBLAS bf16)", "ms_per_launch": bwd_ms_step / bwd_launches,
-                "launches_per_step": bwd_launches}
+                "peak_source": f"{peaks['source']} (burst cuBLAS bf16)", "ms_per_step": bwd_ms_step,
+                "launches_per_step": 2 * bwd_passes}
 
     line = {
         "metric": "sparse_attn_fwd_bwd_tflops", "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
