@@ -180,8 +180,8 @@ class _AttentionFunction(torch.autograd.Function):
 
 def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks):
     q_proxy = _spread_proxy_heads(q_proxy, k_proxy, q, k)
-    with_grad = torch.is_grad_enabled() and (any(t.requires_grad for t in (q_proxy, k_proxy, q, k, v)) or
-                                             (sinks is not None and sinks.requires_grad))
+    with_grad = torch.is_grad_enabled() and (q_proxy.requires_grad or k_proxy.requires_grad or q.requires_grad or k.requires_grad or
+                                             v.requires_grad or (sinks is not None and sinks.requires_grad))
     if with_grad or forward_ad._current_level >= 0 or torch._C._is_tracing():
         return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, top_k, scale, sparse)
     # No backward will follow: the proxy log-sum-exp, which only the backward needs, is left out.  (Tangents would be lost

@@ -92,7 +92,7 @@ class Plan:
         self.dense, self.shape, self.dtype, self.device = dense, (b, hq, s, d), dtype, device
         self.pb = _lib.FmsaProblem(b, s, hq, hkv, hp, hpkv, 1 if dense else int(top_k_blocks), float(scale), ops._dtype_code(dtype), None)
         self.max_partial_bytes = int(max_partial_bytes)
-        self.shapes, self.layout = shapes, layout
+        self.layout = layout
         self.in_place = all(map(_conforms, self.layout))
         self.grad_shapes = [((b, s, sh[1], d), True) if _bshd(sh, st) else (tuple(sh), False) for sh, st in zip(shapes, layout)]
         self.out_shape = (b, s, hq * d)
@@ -106,6 +106,7 @@ class Plan:
             self.at.append(4 * off)
             off += (n + 63) // 64 * 64
         self.saved_words = off
+        self.saved_shapes = (*shapes, self.out_shape, (off,))
         self.forward_args = bytes(self._args(ForwardArgs, workspace_bytes=self.forward_bytes))
         self._backward = {}
 
@@ -134,36 +135,31 @@ class Plan:
             got = self._backward[with_kl] = (bytes(a), nbytes)
         return got
 
-    def conform(self, inputs, as_planned=True):
-        """The inputs as the kernels can read them: in place, or - other strides, or an address off the 16-byte grid, which is
-        not part of what a plan knows - copied once into (B,H,S,128) order."""
-        if as_planned and self.in_place and all(t.data_ptr() % 16 == 0 for t in inputs):
-            return inputs
-        return [t if _conforms(t.stride()) and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in inputs]
-
     def point(self, a, inputs, as_planned=True):
-        """Points the argument block `a` at the inputs or at their copies, and returns what it points at (to be kept until the
-        launch).  The block's strides are those the plan was made for; where the tensors have others (`as_planned` False: these
-        inputs; or copies) they are filled in with the addresses."""
-        given = self.conform(inputs, as_planned)
-        qp, kp, q, k, v = given
-        a.q_proxy, a.k_proxy, a.q, a.k, a.v = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
-        if given is not inputs:
-            for name, t in zip(_ORDER, given):
-                self._strides(a, name, t.stride())
+        """Points the argument block `a` at the inputs as the kernels can read them: in place, or - other strides, or an address
+        off the 16-byte grid, which is not part of what a plan knows - copied once into (B,H,S,128) order.  Returns what it points
+        at, to be kept until the launch.  The block's strides are those the plan was made for; where the tensors have others
+        (`as_planned` False: these inputs; or copies) they are filled in with the addresses."""
+        qp, kp, q, k, v = inputs
+        pqp, pkp, pq, pk, pv = qp.data_ptr(), kp.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
+        if as_planned and self.in_place and not (pqp | pkp | pq | pk | pv) & 15:
+            a.q_proxy, a.k_proxy, a.q, a.k, a.v = pqp, pkp, pq, pk, pv
+            return inputs
+        given = [t if _conforms(t.stride()) and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in inputs]
+        for name, t in zip(_ORDER, given):
+            setattr(a, name, t.data_ptr())
+            self._strides(a, name, t.stride())
         return given
 
     def check_unpacked(self, inputs, out, saved):
         """Raises ValueError for tensors that a saved-tensor hook brought back as something else."""
-        dtype, dev = self.dtype, self.device
-        for t, shape in zip(inputs, self.shapes):
-            if t.shape != shape or t.dtype != dtype or t.device != dev:
-                break
-        else:
-            if (out.shape == self.out_shape and out.dtype == dtype and out.device == dev
-                    and saved.shape == (self.saved_words,) and saved.dtype == torch.int32 and saved.device == dev):
-                return
-        raise ValueError("the tensors saved for the backward came back with another shape, type or device")
+        qp, kp, q, k, v = inputs
+        dt, dev = self.dtype, self.device
+        if not (qp.dtype is dt and kp.dtype is dt and q.dtype is dt and k.dtype is dt and v.dtype is dt and out.dtype is dt
+                and saved.dtype is torch.int32 and qp.device == dev and kp.device == dev and q.device == dev and k.device == dev
+                and v.device == dev and out.device == dev and saved.device == dev
+                and (qp.shape, kp.shape, q.shape, k.shape, v.shape, out.shape, saved.shape) == self.saved_shapes):
+            raise ValueError("the tensors saved for the backward came back with another shape, type or device")
 
 
 def _whole(t):

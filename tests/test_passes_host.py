@@ -45,16 +45,16 @@ KINDS = ["dense", "bshd", "packed", "packed_shifted", "shifted", "wide", "expand
 
 
 class _Recorder:
-    """Stands in for the native call; `given` are the tensors that `Plan.conform` hands to it."""
+    """Stands in for the native call; `given` are the tensors that `Plan.point` points it at."""
 
     def __init__(self, monkeypatch):
         self.blocks, self.given = [], []
-        conform = passes.Plan.conform
+        point = passes.Plan.point
 
         def watch(plan, *args):
-            self.given.append(list(conform(plan, *args)))
+            self.given.append(list(point(plan, *args)))
             return self.given[-1]
-        monkeypatch.setattr(passes.Plan, "conform", watch)
+        monkeypatch.setattr(passes.Plan, "point", watch)
         monkeypatch.setattr(passes, "_call", lambda fn, what, a, device: self.blocks.append(type(a).from_buffer_copy(a)))
 
     def check(self, block, given, inputs):
