@@ -238,7 +238,7 @@ def test_fewer_proxy_heads_than_kv_heads(fm, heads, warmup):
 @pytest.mark.parametrize("mpp", [5, 7, 8, 12, 16])
 def test_main_heads_per_proxy_head(fm, mpp, warmup):
     """Hq/Hp beyond the BASELINE shapes: 5, 7 and 8 main heads per proxy head take the three- and four-sweep forms of the
-    combine kernels, 12 and 16 the one-head-at-a-time forms; 5 and 7 do not divide 128 (the reference refuses them,
+    combine kernels, 12 and 16 their groups of heads; 5 and 7 do not divide 128 (the reference refuses them,
     flash_msa/flash_msa.py:153-158)."""
     cfg = dict(b=1, s=768, hq=2 * mpp, hkv=2, hp=2, hpkv=1, kb=3, seed=50 + mpp)
     qp, kp, q, k, v, do = bf16_inputs(cfg)
