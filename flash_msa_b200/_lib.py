@@ -78,6 +78,12 @@ def _declare(lib):
     lib.fmsa_sparse_fwd.argtypes = [PB, T, T, T, T, T, P, P, P, P, c_int64, c_int32, c_int32, c_int32, c_int32, P, P, P]
     lib.fmsa_sparse_fwd_combine.restype = c_int
     lib.fmsa_sparse_fwd_combine.argtypes = [PB, P, P, P, P, P, P, P, c_int32, c_int32, c_int32, P]
+    lib.fmsa_forward_tiles.restype = c_int32
+    lib.fmsa_forward_tiles.argtypes = [PB, c_int32]
+    lib.fmsa_tile_fwd_workspace_bytes.restype = c_int64
+    lib.fmsa_tile_fwd_workspace_bytes.argtypes = [PB, c_int32]
+    lib.fmsa_tile_fwd.restype = c_int
+    lib.fmsa_tile_fwd.argtypes = [PB, T, T, T, T, T, P, P, c_int64, P, P, P, c_int32, P, P]
     lib.fmsa_bwd_delta.restype = c_int
     lib.fmsa_bwd_delta.argtypes = [P, T, P, c_int32, c_int32, c_int32, c_int32, P]
     lib.fmsa_sparse_bwd.restype = c_int
@@ -95,6 +101,8 @@ def _declare(lib):
     lib.fmsa_backward_workspace_bytes.argtypes = [PB, c_int32, c_int32, c_int32, c_int64]
     lib.fmsa_forward.restype = c_int
     lib.fmsa_forward.argtypes = [P, P, P, P]
+    lib.fmsa_forward_alone.restype = c_int
+    lib.fmsa_forward_alone.argtypes = [P, c_int32, P, P, P]
     lib.fmsa_backward.restype = c_int
     lib.fmsa_backward.argtypes = [P, P, P, P]
     lib.fmsa_doc_start.restype = c_int

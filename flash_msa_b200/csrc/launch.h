@@ -8,15 +8,21 @@
 
 namespace fmsa {
 
+// Rows of query tiles first_tile .. of the reverse index; `row_start`: where they begin in its rows (first_tile > 0).
 // `counter`: one zeroed word.
 int launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
-                      const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr, const int32_t* col_q,
-                      void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
+                      const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr,
+                      const int32_t* row_start, int first_tile, const int32_t* col_q, void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
                       int32_t* counter, int32_t* status, cudaStream_t st);
 // `sinks`: fp32 [Hq] softmax-bias logits or null; `zero`: a device scalar to clear on the way, or null.
 int launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
                        const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
-                       int g_begin, int g_count, int dense, cudaStream_t st);
+                       int first_tile, int g_begin, int g_count, int dense, cudaStream_t st);
+// Query tiles 0 .. tiles-1 of every (batch, proxy head).  `visits`: from reverse_index_launch or launch_tile_visits (null if dense);
+// lse_proxy null: without the proxy head.  `counter`: one zeroed word.  Returns the number of launches in *launches.
+int launch_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v, const fmsa_tensor* q_proxy,
+                    const fmsa_tensor* k_proxy, const void* visits, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
+                    int tiles, int dense, int32_t* counter, int32_t* status, cudaStream_t st);
 // `counter`, `counter_proxy`: zeroed here if `zero_counters` (they may then be the same word).
 int launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
                       const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const fmsa_tensor* d_out, const float* lse,
@@ -41,9 +47,18 @@ struct CastJobs {
 int launch_cast_grads(const CastJobs& jobs, int count, bool fp16, cudaStream_t st);
 int launch_sink_grad(const float* lse, const float* delta, const float* sinks, float* dsinks, int B, int S, int Hq, cudaStream_t st);
 
-// `zero`, `nzero`: words to clear on the way, or null.
+// What a whole pass has the reverse index do on the way.
+struct RixExtras {
+    void* visits = nullptr;         // [rows_bh][tiles][tiles] 128-bit words: which rows of query tile i selected block j
+    int tiles = 0;
+    int32_t* row_start = nullptr;   // [rows_bh*NB] position of the first row of a query tile >= tiles in every reverse-index row
+    int32_t* zero = nullptr;        // words to clear
+    int nzero = 0;
+};
 int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos, int64_t rows_bh,
-                         int32_t S, int32_t Kb, void* scratch, cudaStream_t st, int32_t* zero = nullptr, int nzero = 0);
+                         int32_t S, int32_t Kb, void* scratch, cudaStream_t st, const RixExtras& x = RixExtras());
+// Nothing but `visits` (and the cleared words).
+int launch_tile_visits(const int32_t* block_indices, int64_t rows_bh, int32_t S, int32_t Kb, const RixExtras& x, cudaStream_t st);
 size_t reverse_index_scratch_bytes(int64_t rows_bh, int32_t S);
 
 }  // namespace fmsa

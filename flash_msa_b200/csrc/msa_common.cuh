@@ -39,9 +39,10 @@ __host__ __device__ __forceinline__ int64_t dense_row_offset(int j, int S) {
 constexpr int kMaxChunksPerSubUnit = 16;
 
 // Key blocks j that can have a sub-unit s: NB - j > C*s, i.e. j < NB - C*s.
-__host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int ppk, int C) {
-    // sum over s = 0 .. n-1 of (NB - C*s), n = ceil(NB / C)
-    const int64_t n = (NB + C - 1) / C;
+// (`depth`: most chunks a row can have; NB, or NB - T where the rows hold query positions of tiles T, T+1, .. only.)
+__host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int depth, int ppk, int C) {
+    // sum over s = 0 .. n-1 of (NB - C*s), n = ceil(depth / C)
+    const int64_t n = (depth + C - 1) / C;
     return (n * NB - C * (n * (n - 1) / 2)) * ppk;
 }
 
@@ -60,13 +61,35 @@ __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int ppk, 
 // top-k 32 blocks, 14 sub-units per CTA: forward 1.70 -> 1.56 ms, backward 3.83 -> 3.49 ms; S=32768, 64 blocks: equal), while
 // at 7 sub-units per CTA (B=2 S=8192 Hq=32 top-k 16 blocks) the tail makes it slower: 0.672 -> 0.692 ms forward.
 constexpr int kSubUnitsPerCta = 6, kLongSubUnitsPerCta = 12, kDrawsPerCta = 32;
-inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int ppk, int sms) {
+inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int depth, int ppk, int sms) {
     const int64_t chunks = (edges + kBlock - 1) / kBlock + groups * ppk * NB / 2;
     int c = chunks >= static_cast<int64_t>(kMaxChunksPerSubUnit) * kLongSubUnitsPerCta * sms ? kMaxChunksPerSubUnit : kMaxChunksPerSubUnit / 2;
     while (c > 1 && chunks < static_cast<int64_t>(c) * kSubUnitsPerCta * sms &&
-           groups * subunits_per_group(NB, ppk, c / 2) <= static_cast<int64_t>(kDrawsPerCta) * sms)
+           groups * subunits_per_group(NB, depth, ppk, c / 2) <= static_cast<int64_t>(kDrawsPerCta) * sms)
         c >>= 1;
     return c;
+}
+
+// -------------------------------------------------------------------------------------------
+// Which query tiles the query-tile stationary forward (tile_fwd.cu) takes: the first `forward_tiles` ones.
+// -------------------------------------------------------------------------------------------
+constexpr int kTileFwdMaxBlocks = 256;   // most blocks that a tile of a sparse call can visit there
+// Query tile i visits up to i + 1 blocks there, against min(i + 1, top_k_blocks) edges per row here, and an edge of the key-block
+// stationary forward and its combine takes as long as about two visits: 18.8 ns against 9.0 ns of the whole GPU per 128 edges, or visit,
+// of a main head (B=2 S=8192 Hq=32 top-k 16 blocks; B=4 S=4096 Hq=32 dense, both with the proxy heads).  So the first 2 top_k_blocks
+// tiles go there; all of them, so that the other forward and its combine need not run, where those would be short (their
+// launches and tails cost as much as some 2800 visits).
+constexpr int kTileFwdVisitsPerEdge = 2, kTileFwdLaunchVisits = 2800;
+inline int forward_tiles(int NB, int top_k_blocks, int64_t main_heads, int dense) {   // main_heads: of all batch elements
+    if (dense) return NB;
+    int t = kTileFwdVisitsPerEdge * top_k_blocks;
+    if (NB <= kTileFwdMaxBlocks) {
+        if (t >= NB) return NB;
+        const int64_t visits = (static_cast<int64_t>(NB) * (NB + 1) - static_cast<int64_t>(t) * (t + 1)) / 2;   // of the tiles from t on
+        const int64_t edges = static_cast<int64_t>(NB - t) * top_k_blocks;
+        if ((visits - kTileFwdVisitsPerEdge * edges) * main_heads <= kTileFwdLaunchVisits) return NB;
+    }
+    return t < kTileFwdMaxBlocks ? t : kTileFwdMaxBlocks;
 }
 
 struct SubUnit {

@@ -6,6 +6,7 @@
 // and no launch that only clears a word leave the autograd machinery as the larger part.
 #include "host_common.h"
 #include "launch.h"
+#include "msa_common.cuh"
 
 namespace fmsa {
 namespace {
@@ -32,29 +33,38 @@ int64_t groups_per_pass(const fmsa_problem* pb, int dense, int64_t bytes_per_slo
 }
 
 struct ForwardSpace {
-    int32_t* counters;
+    int32_t* counters;    // one per pass of the key-block stationary forward, then the query-tile stationary one's
+    int32_t* row_start;
     void* o_part;
     float* stats;
     int32_t* indices;
     float* scores;
-    void* rix;
+    void *rix, *visits;
     int64_t gstep, slots, bytes;
+    int tiles, passes;    // query tiles of the query-tile stationary forward; passes of the other one (0: all tiles are the former's)
 };
-// The selection's buffers and the attention's partial rows are not alive at the same time: they share the space.
+// The selection's buffers and the partial rows of the key-block stationary forward, which comes last, are not alive at the same
+// time: they share the space.
 ForwardSpace carve_forward(const fmsa_problem* pb, int dense, int64_t max_bytes, void* base) {
     ForwardSpace w = {};
+    w.tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense);
     const int mpp = pb->Hq / pb->Hp;
     const int64_t groups = static_cast<int64_t>(pb->B) * pb->Hkv, rows = static_cast<int64_t>(pb->B) * pb->Hp, NB = pb->S / 128;
     w.gstep = groups_per_pass(pb, dense, static_cast<int64_t>(mpp) * 256 + (mpp + 1) * 8, max_bytes);
     w.slots = fmsa_fwd_partial_slots(pb, static_cast<int32_t>(w.gstep), dense);
+    w.passes = w.tiles < NB ? static_cast<int>((groups + w.gstep - 1) / w.gstep) : 0;
     Carver c(base);
-    w.counters = c.take<int32_t>((groups + w.gstep - 1) / w.gstep);
+    w.counters = c.take<int32_t>(w.passes + 1);
+    if (w.passes) w.row_start = c.take<int32_t>(rows * NB);
     Carver a = c;
-    w.o_part = a.take<uint16_t>(w.slots * mpp * 128);
-    w.stats = a.take<float>(w.slots * (mpp + 1) * 2);
+    if (w.passes) {
+        w.o_part = a.take<uint16_t>(w.slots * mpp * 128);
+        w.stats = a.take<float>(w.slots * (mpp + 1) * 2);
+    }
     Carver s = c;
     if (!dense) {
         w.indices = s.take<int32_t>(rows * pb->S * pb->top_k_blocks);
+        w.visits = s.take<char>(rows * w.tiles * w.tiles * 16);
         w.rix = s.take<char>(static_cast<int64_t>(reverse_index_scratch_bytes(rows, pb->S)));
         if (pb->top_k_blocks > FMSA_FUSED_SELECT_MAX_BLOCKS) w.scores = s.take<float>(rows * pb->S * NB);
     }
@@ -120,18 +130,24 @@ extern "C" int64_t fmsa_forward_workspace_bytes(const fmsa_problem* pb, int32_t 
 }
 
 extern "C" int fmsa_forward(const fmsa_forward_args* a, fmsa_marks* marks, int32_t* launches, void* stream) {
+    return fmsa_forward_alone(a, 0, marks, launches, stream);
+}
+
+extern "C" int fmsa_forward_alone(const fmsa_forward_args* a, int32_t alone, fmsa_marks* marks, int32_t* launches, void* stream) {
     using namespace fmsa;
     FMSA_REQUIRE(a && problem_ok(&a->pb) && a->workspace && a->out && a->lse && a->status && launches);
     FMSA_REQUIRE((reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0 && (!a->with_proxy || a->lse_proxy));
     const fmsa_problem* pb = &a->pb;
     const int dense = a->dense ? 1 : 0;
-    FMSA_REQUIRE(dense || (a->row_ptr && a->col_q && a->edge_pos && pb->top_k_blocks >= 1 && pb->top_k_blocks <= pb->S / 128));
+    FMSA_REQUIRE(dense || (pb->top_k_blocks >= 1 && pb->top_k_blocks <= pb->S / 128));
     const ForwardSpace w = carve_forward(pb, dense, a->max_partial_bytes, a->workspace);
+    const bool index = !dense && (!alone || w.passes);   // the reverse index is wanted
+    FMSA_REQUIRE(!index || (a->row_ptr && a->col_q && a->edge_pos));
     if (w.bytes > a->workspace_bytes) return FMSA_ERR_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Marks mark{marks, st};
     int n = 0;
-    const int groups = pb->B * pb->Hkv, step = static_cast<int>(w.gstep), passes = (groups + step - 1) / step;
+    const int groups = pb->B * pb->Hkv, step = static_cast<int>(w.gstep);
     if (!dense) {
         const int64_t rows = static_cast<int64_t>(pb->B) * pb->Hp;
         FMSA_REQUIRE(rows <= 65535 && rows * pb->S * pb->top_k_blocks < 0x7fffffffLL);
@@ -149,28 +165,79 @@ extern "C" int fmsa_forward(const fmsa_forward_args* a, fmsa_marks* marks, int32
         }
         mark(FMSA_STAGE_SELECT);
         mark(FMSA_STAGE_REVERSE_INDEX);
-        // (the work counters lie outside the space that the selection's buffers share with the partial rows)
-        FMSA_TRY(reverse_index_launch(w.indices, a->row_ptr, a->col_q, a->edge_pos, rows, pb->S, pb->top_k_blocks, w.rix, st, w.counters,
-                                      passes));
+        // (the work counters and row_start lie outside the space that the selection's buffers share with the partial rows)
+        RixExtras x;
+        x.visits = w.visits; x.tiles = w.tiles; x.row_start = w.row_start;
+        x.zero = w.counters; x.nzero = w.passes + 1;
+        if (index) {
+            FMSA_TRY(reverse_index_launch(w.indices, a->row_ptr, a->col_q, a->edge_pos, rows, pb->S, pb->top_k_blocks, w.rix, st, x));
+            n += 4;
+        } else {
+            FMSA_TRY(launch_tile_visits(w.indices, rows, pb->S, pb->top_k_blocks, x, st));
+            n += 1;
+        }
         mark(FMSA_STAGE_REVERSE_INDEX);
-        n += 4;
-    } else if (cudaMemsetAsync(w.counters, 0, sizeof(int32_t) * passes, st) != cudaSuccess) {
+    } else if (cudaMemsetAsync(w.counters, 0, sizeof(int32_t) * (w.passes + 1), st) != cudaSuccess) {
         return FMSA_ERR_CUDA;
     }
-    for (int i = 0; i < passes; ++i) {
+    float* lse_proxy = a->with_proxy ? a->lse_proxy : nullptr;
+    mark(FMSA_STAGE_ATTN_FWD);
+    FMSA_TRY(launch_tile_fwd(pb, &a->q, &a->k, &a->v, &a->q_proxy, &a->k_proxy, w.visits, a->out, a->lse, lse_proxy, a->sinks, a->kl_loss,
+                             w.tiles, dense, w.counters + w.passes, a->status, st));
+    mark(FMSA_STAGE_ATTN_FWD);
+    n += a->sinks ? 2 : 1;
+    for (int i = 0; i < w.passes; ++i) {
         const int g0 = i * step, gc = groups - g0 < step ? groups - g0 : step;
         mark(FMSA_STAGE_ATTN_FWD);
-        FMSA_TRY(launch_sparse_fwd(pb, &a->q, &a->k, &a->v, &a->q_proxy, &a->k_proxy, a->row_ptr, a->col_q, w.o_part, w.stats, w.slots, g0,
-                                   gc, a->with_proxy, dense, w.counters + i, a->status, st));
+        FMSA_TRY(launch_sparse_fwd(pb, &a->q, &a->k, &a->v, &a->q_proxy, &a->k_proxy, a->row_ptr, w.row_start, w.tiles, a->col_q, w.o_part,
+                                   w.stats, w.slots, g0, gc, a->with_proxy, dense, w.counters + i, a->status, st));
         mark(FMSA_STAGE_ATTN_FWD);
         mark(FMSA_STAGE_FWD_COMBINE);
-        FMSA_TRY(launch_fwd_combine(pb, w.o_part, w.stats, a->edge_pos, a->row_ptr, a->out, a->lse, a->with_proxy ? a->lse_proxy : nullptr,
-                                    a->sinks, i == 0 ? a->kl_loss : nullptr, g0, gc, dense, st));
+        FMSA_TRY(launch_fwd_combine(pb, w.o_part, w.stats, a->edge_pos, a->row_ptr, a->out, a->lse, lse_proxy, a->sinks, nullptr, w.tiles, g0, gc,
+                                    dense, st));
         mark(FMSA_STAGE_FWD_COMBINE);
         n += 3;
     }
     *launches = n;
     return FMSA_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// The query-tile stationary forward as a stage of its own.
+// ---------------------------------------------------------------------------------------------
+extern "C" int32_t fmsa_forward_tiles(const fmsa_problem* pb, int32_t dense) {
+    using namespace fmsa;
+    return problem_ok(pb) ? forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense) : 0;
+}
+
+extern "C" int64_t fmsa_tile_fwd_workspace_bytes(const fmsa_problem* pb, int32_t dense) {
+    using namespace fmsa;
+    if (!problem_ok(pb)) return 0;
+    const int64_t tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense);
+    return 256 + (dense ? 0 : static_cast<int64_t>(pb->B) * pb->Hp * tiles * tiles * 16);
+}
+
+extern "C" int fmsa_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                             const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* block_indices, void* workspace,
+                             int64_t workspace_bytes, void* out, float* lse, float* lse_proxy, int32_t dense, int32_t* status,
+                             void* stream) {
+    using namespace fmsa;
+    FMSA_REQUIRE(problem_ok(pb) && workspace && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && (dense || block_indices));
+    FMSA_REQUIRE(dense || (pb->top_k_blocks >= 1 && pb->top_k_blocks <= pb->S / kBlock));
+    if (workspace_bytes < fmsa_tile_fwd_workspace_bytes(pb, dense)) return FMSA_ERR_WORKSPACE;
+    const int64_t rows = static_cast<int64_t>(pb->B) * pb->Hp;
+    if (rows > 65535 || pb->S / kBlock > 2048) return FMSA_ERR_UNSUPPORTED;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    RixExtras x;
+    x.tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense);
+    x.zero = static_cast<int32_t*>(workspace); x.nzero = 1;
+    if (!dense) {
+        x.visits = static_cast<char*>(workspace) + 256;
+        FMSA_TRY(launch_tile_visits(block_indices, rows, pb->S, pb->top_k_blocks, x, st));
+    } else if (cudaMemsetAsync(workspace, 0, sizeof(int32_t), st) != cudaSuccess) {
+        return FMSA_ERR_CUDA;
+    }
+    return launch_tile_fwd(pb, q, k, v, q_proxy, k_proxy, x.visits, out, lse, lse_proxy, nullptr, nullptr, x.tiles, dense, x.zero, status, st);
 }
 
 extern "C" int64_t fmsa_backward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int32_t with_kl, int32_t split_above,

@@ -48,13 +48,24 @@ __device__ __forceinline__ void build_bitmap(uint32_t* words, const int32_t* til
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(128) rix_count_kernel(const int32_t* __restrict__ idx, uint8_t* __restrict__ counts,
-                                                        int S, int NB, int Kb) {
+// With `visits` the bitmaps of query tiles below `tiles` also go to memory: tile_fwd.cu walks the blocks in them.  `counts` null:
+// nothing else (the grid then has those query tiles only).
+__global__ void __launch_bounds__(128) rix_count_kernel(const int32_t* __restrict__ idx, uint8_t* __restrict__ counts, uint4* __restrict__ visits,
+                                                        int tiles, int32_t* __restrict__ zero, int nzero, int S, int NB, int Kb) {
     extern __shared__ __align__(16) uint32_t words[];
     const int qblk = blockIdx.x;
     const int64_t bp = blockIdx.y;
     const int32_t* tile = stage_rows(words, idx + (bp * S + static_cast<int64_t>(qblk) * kBlock) * Kb, NB, Kb);
     build_bitmap(words, tile, NB, Kb, qblk);
+    if (visits && qblk < tiles) {
+        uint4* vrow = visits + (bp * tiles + qblk) * tiles;
+        for (int j = threadIdx.x; j <= qblk; j += blockDim.x) vrow[j] = reinterpret_cast<const uint4*>(words)[j];
+    }
+    if (!counts) {
+        if (qblk == 0 && bp == 0)
+            for (int i = threadIdx.x; i < nzero; i += blockDim.x) zero[i] = 0;
+        return;
+    }
     uint8_t* crow = counts + (bp * NB + qblk) * NB;
     for (int j = threadIdx.x; j <= qblk; j += blockDim.x) {
         const int c = __popc(words[j * 4]) + __popc(words[j * 4 + 1]) + __popc(words[j * 4 + 2]) + __popc(words[j * 4 + 3]);
@@ -106,7 +117,8 @@ __global__ void __launch_bounds__(1024) rix_rowscan_kernel(const int32_t* __rest
 
 __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ blk_off,
                                                        const int32_t* __restrict__ row_ptr, int32_t* __restrict__ col_q,
-                                                       int32_t* __restrict__ edge_pos, int S, int NB, int Kb) {
+                                                       int32_t* __restrict__ edge_pos, int32_t* __restrict__ row_start, int tiles,
+                                                       int S, int NB, int Kb) {
     extern __shared__ __align__(16) uint32_t words[];
     const int qblk = blockIdx.x;
     const int64_t bp = blockIdx.y;
@@ -118,6 +130,8 @@ __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict
     int32_t* row = tile + r * Kb;   // the selections of row r; each is replaced by its edge position
     const int32_t* rp = row_ptr + bp * NB;
     const int32_t* bo = blk_off + (bp * NB + qblk) * NB;
+    if (row_start && qblk == tiles)
+        for (int j = r; j < NB; j += kBlock) row_start[bp * NB + j] = rp[j] + (j < tiles ? bo[j] : 0);
     const int w = r >> 5;
     const uint32_t below = (1u << (r & 31)) - 1u;
     for (int s = 0; s < Kb; ++s) {
@@ -138,6 +152,8 @@ __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict
     int4* dst = reinterpret_cast<int4*>(edge_pos + row0 * Kb);
     for (int t = threadIdx.x; t < kBlock * Kb / 4; t += blockDim.x) dst[t] = src[t];
 }
+
+constexpr size_t kRixSmemCap = 160 * 1024;   // NB <= 2048 and Kb <= 128 need 96 KB; the attribute is set once, to the cap
 
 struct RixWorkspace {
     uint8_t* counts;
@@ -164,22 +180,31 @@ RixWorkspace carve(void* base, int64_t rows_bh, int NB) {
 
 // Launch sequence shared with any other entry point that supplies its own scratch memory.
 int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos,
-                         int64_t rows_bh, int32_t S, int32_t Kb, void* scratch, cudaStream_t st, int32_t* zero, int nzero) {
+                         int64_t rows_bh, int32_t S, int32_t Kb, void* scratch, cudaStream_t st, const RixExtras& x) {
     const int NB = S / kBlock;
     const RixWorkspace w = carve(scratch, rows_bh, NB);
     const dim3 grid(static_cast<unsigned>(NB), static_cast<unsigned>(rows_bh));
     const size_t smem = static_cast<size_t>(NB) * 16 + static_cast<size_t>(kBlock) * Kb * sizeof(int32_t);
-    constexpr size_t kSmemCap = 160 * 1024;   // NB <= 2048 and Kb <= 128 need 96 KB; the attribute is set once, to the cap
-    if (smem > kSmemCap || (reinterpret_cast<uintptr_t>(block_indices) & 15u) != 0 || (reinterpret_cast<uintptr_t>(edge_pos) & 15u) != 0)
+    if (smem > kRixSmemCap || (reinterpret_cast<uintptr_t>(block_indices) & 15u) != 0 || (reinterpret_cast<uintptr_t>(edge_pos) & 15u) != 0)
         return FMSA_ERR_UNSUPPORTED;
-    if (!ensure_smem_attr(reinterpret_cast<const void*>(rix_count_kernel), kSmemCap) ||
-        !ensure_smem_attr(reinterpret_cast<const void*>(rix_fill_kernel), kSmemCap))
+    if (!ensure_smem_attr(reinterpret_cast<const void*>(rix_count_kernel), kRixSmemCap) ||
+        !ensure_smem_attr(reinterpret_cast<const void*>(rix_fill_kernel), kRixSmemCap))
         return FMSA_ERR_CUDA;
-    rix_count_kernel<<<grid, 128, smem, st>>>(block_indices, w.counts, S, NB, Kb);
+    rix_count_kernel<<<grid, 128, smem, st>>>(block_indices, w.counts, static_cast<uint4*>(x.visits), x.tiles, nullptr, 0, S, NB, Kb);
     const int64_t cols = rows_bh * NB;
     rix_colscan_kernel<<<static_cast<unsigned>((cols + 127) / 128), 128, 0, st>>>(w.counts, w.blk_off, w.totals, rows_bh, NB);
-    rix_rowscan_kernel<<<1, 1024, 0, st>>>(w.totals, row_ptr, cols, zero, nzero);
-    rix_fill_kernel<<<grid, 128, smem, st>>>(block_indices, w.blk_off, row_ptr, col_q, edge_pos, S, NB, Kb);
+    rix_rowscan_kernel<<<1, 1024, 0, st>>>(w.totals, row_ptr, cols, x.zero, x.nzero);
+    rix_fill_kernel<<<grid, 128, smem, st>>>(block_indices, w.blk_off, row_ptr, col_q, edge_pos, x.row_start, x.tiles, S, NB, Kb);
+    return check_launch();
+}
+
+int launch_tile_visits(const int32_t* block_indices, int64_t rows_bh, int32_t S, int32_t Kb, const RixExtras& x, cudaStream_t st) {
+    const int NB = S / kBlock;
+    const size_t smem = static_cast<size_t>(NB) * 16 + static_cast<size_t>(kBlock) * Kb * sizeof(int32_t);
+    if (smem > kRixSmemCap || (reinterpret_cast<uintptr_t>(block_indices) & 15u) != 0) return FMSA_ERR_UNSUPPORTED;
+    if (!ensure_smem_attr(reinterpret_cast<const void*>(rix_count_kernel), kRixSmemCap)) return FMSA_ERR_CUDA;
+    rix_count_kernel<<<dim3(static_cast<unsigned>(x.tiles), static_cast<unsigned>(rows_bh)), 128, smem, st>>>(
+        block_indices, nullptr, static_cast<uint4*>(x.visits), x.tiles, x.zero, x.nzero, S, NB, Kb);
     return check_launch();
 }
 

@@ -47,6 +47,7 @@ struct FwdParams {
     int64_t qp_row_b, qp_row_h, qp_row_s;
     int32_t q_rows_total, qp_rows_total;   // first row index outside the views (reads as zeros)
     const int32_t* row_ptr;
+    const int32_t* row_start;   // per reverse-index row the first position of a query tile >= first_tile, or null (first_tile = 0)
     const int32_t* col_q;
     const int32_t* doc_start;   // [B,S] first token of each token's document (packed sequences), or null
     __nv_bfloat16* o_part;   // [(edge - edge_base) * mpp + head][128]
@@ -55,7 +56,7 @@ struct FwdParams {
     int32_t* counter;
     int32_t* status;
     int S, NB, Hq, Hkv, Hp, mpp, ppk, pg;
-    int g_begin, G;
+    int g_begin, G, first_tile;
     int with_proxy, dense;
     int32_t n_subunits;
     uint32_t units_per_group;
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     e0 = dense_edge_base(bp, P.S, P.NB) + dense_row_offset(su.j, P.S);
                     n = P.S - su.j * kBlock;
                 } else {
-                    e0 = P.row_ptr[bp * P.NB + su.j];
+                    e0 = (P.row_start ? P.row_start : P.row_ptr)[bp * P.NB + su.j];
                     n = P.row_ptr[bp * P.NB + su.j + 1] - static_cast<int>(e0);
                 }
                 nu.j = su.j; nu.b = b; nu.kvh = kvh; nu.p = p; nu.n = n; nu.e0 = e0;
@@ -516,8 +517,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                     if (bad) break;
                     tc_fence_after_sync();
                     // only the first chunk of a reverse-index row can hold rows of the key block itself
-                    const bool masked = (chunk == 0) || (VARLEN && __any_sync(0xffffffffu, low > 0));
-                    const int limit = (chunk == 0) ? sm->limits[(cbase + chunk - ud.chunk0) & (kLimitRing - 1)][row] : 127;
+                    const bool own = chunk == 0 && ud.j >= P.first_tile;
+                    const bool masked = own || (VARLEN && __any_sync(0xffffffffu, low > 0));
+                    const int limit = own ? sm->limits[(cbase + chunk - ud.chunk0) & (kLimitRing - 1)][row] : 127;
                     float m = 0.f, l = 0.f;
                     // Two instances: with the mask as a run-time condition every element paid for its comparison and selection.
                     auto softmax_row = [&](auto masked_c) __attribute__((always_inline)) {
@@ -637,6 +639,7 @@ struct CombineParams {
     float* lse_proxy;          // [B, Hp, S] or null
     int S, NB, Hq, Hp, mpp, ppk, Kb;
     int g_begin, G, dense;
+    int q0;                    // rows q0 .. S-1 of every (batch, proxy head)
     int hgroup;                // main heads per blockIdx.y of the row kernel
     const float* sinks;        // [Hq] softmax-bias logits or null
     float* zero;               // a scalar to set to zero, or null
@@ -665,8 +668,9 @@ struct CombineRow {
     const int32_t* erow;
     __device__ __forceinline__ CombineRow(const CombineParams& P, int64_t w) {
         const int64_t bp0 = static_cast<int64_t>(P.g_begin) * P.ppk;
-        bp = bp0 + w / P.S;
-        q = static_cast<int>(w % P.S);
+        const int rows = P.S - P.q0;
+        bp = bp0 + w / rows;
+        q = P.q0 + static_cast<int>(w % rows);
         b = static_cast<int>(bp / P.Hp);
         p = static_cast<int>(bp % P.Hp);
         edge_base = DENSE ? dense_edge_base(bp0, P.S, P.NB) : static_cast<int64_t>(P.row_ptr[bp0 * P.NB]);
@@ -689,7 +693,7 @@ template <int LPR, bool DENSE, bool SINKS>   // LPR lanes per query row: 16 (two
 __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P) {
     constexpr int kMaxHeads = kWideMaxHeads + 1;
     const int lane = threadIdx.x & 31, l = lane % LPR;
-    const int64_t nrows = static_cast<int64_t>(P.G) * P.ppk * P.S;
+    const int64_t nrows = static_cast<int64_t>(P.G) * P.ppk * (P.S - P.q0);
     const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * (32 / LPR) + lane / LPR;
     const bool valid = w0 < nrows;   // (lanes of a row beyond the end still take part in the shuffles)
     const CombineRow<DENSE> row(P, valid ? w0 : nrows - 1);
@@ -756,7 +760,7 @@ template <int KITER, bool FP16, bool DENSE, bool GROUPED>
 __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) combine_rows_kernel(const CombineParams P) {
     const int lane = threadIdx.x & 31;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    if (w >= static_cast<int64_t>(P.G) * P.ppk * P.S) return;
+    if (w >= static_cast<int64_t>(P.G) * P.ppk * (P.S - P.q0)) return;
     const CombineRow<DENSE> row(P, w);
     const int lse_stride = P.mpp + 1;
     const float2* stats = reinterpret_cast<const float2*>(P.lse_part);
@@ -857,18 +861,19 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
                                void* stream) {
     if (!counter) return FMSA_ERR_ARGUMENT;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream)) != cudaSuccess) return FMSA_ERR_CUDA;
-    return fmsa::launch_sparse_fwd(pb, q, k, v, q_proxy, k_proxy, row_ptr, col_q, o_part, lse_part, part_slots, g_begin, g_count,
+    return fmsa::launch_sparse_fwd(pb, q, k, v, q_proxy, k_proxy, row_ptr, nullptr, 0, col_q, o_part, lse_part, part_slots, g_begin, g_count,
                                    with_proxy, dense, counter, status, static_cast<cudaStream_t>(stream));
 }
 
 int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
-                            const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr, const int32_t* col_q,
-                            void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
+                            const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr,
+                            const int32_t* row_start, int first_tile, const int32_t* col_q, void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
                             int32_t* counter, int32_t* status, cudaStream_t st) {
     using namespace fmsa;
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(q && k && v && q->ptr && k->ptr && v->ptr && o_part && lse_part && counter && status);
     FMSA_REQUIRE(dense || (row_ptr && col_q));
+    FMSA_REQUIRE(first_tile >= 0 && first_tile < pb->S / kBlock && (first_tile == 0 || (row_start && !dense)));
     FMSA_REQUIRE(!with_proxy || (q_proxy && k_proxy && q_proxy->ptr && k_proxy->ptr));
     FMSA_REQUIRE(g_begin >= 0 && g_count > 0 && g_begin + g_count <= pb->B * pb->Hkv);
     FMSA_REQUIRE(dense || (pb->top_k_blocks >= 1 && pb->top_k_blocks <= pb->S / kBlock));
@@ -901,7 +906,7 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     P.q_row_b = q->stride_b / 128; P.q_row_h = q->stride_h / 128; P.q_row_s = q->stride_s / 128;
     P.qp_row_b = qpx->stride_b / 128; P.qp_row_h = qpx->stride_h / 128; P.qp_row_s = qpx->stride_s / 128;
     P.q_rows_total = static_cast<int32_t>(q_rows); P.qp_rows_total = static_cast<int32_t>(qp_rows);
-    P.row_ptr = row_ptr; P.col_q = col_q; P.doc_start = pb->doc_start;
+    P.row_ptr = row_ptr; P.row_start = row_start; P.first_tile = first_tile; P.col_q = col_q; P.doc_start = pb->doc_start;
     P.o_part = static_cast<__nv_bfloat16*>(o_part); P.stat_part = lse_part;
     P.counter = counter; P.status = status;
     P.S = pb->S; P.NB = pb->S / kBlock; P.Hq = pb->Hq; P.Hkv = pb->Hkv; P.Hp = pb->Hp;
@@ -915,8 +920,9 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     const void* kfn = fp16 ? (varlen ? reinterpret_cast<const void*>(sparse_fwd_kernel<true, true>) : reinterpret_cast<const void*>(sparse_fwd_kernel<true, false>))
                            : (varlen ? reinterpret_cast<const void*>(sparse_fwd_kernel<false, true>) : reinterpret_cast<const void*>(sparse_fwd_kernel<false, false>));
     if (sms <= 0 || !ensure_smem_attr(kfn, kFwdSmemBytes)) return FMSA_ERR_CUDA;
-    P.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, P.NB, P.ppk, sms);
-    const int64_t per_group = subunits_per_group(P.NB, P.ppk, P.chunks);
+    const int depth = P.NB - first_tile;
+    P.chunks = chunks_per_subunit((dense ? fmsa_fwd_partial_slots(pb, g_count, 1) : fmsa_fwd_partial_slots(pb, g_count, 0) / P.NB * depth), g_count, P.NB, depth, P.ppk, sms);
+    const int64_t per_group = subunits_per_group(P.NB, depth, P.ppk, P.chunks);
     FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA and 31)
     P.units_per_group = static_cast<uint32_t>(per_group);
     P.n_subunits = static_cast<int32_t>(per_group * g_count);
@@ -931,13 +937,13 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
 extern "C" int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part,
                                        const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse,
                                        float* lse_proxy, int32_t g_begin, int32_t g_count, int32_t dense, void* stream) {
-    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, nullptr, g_begin, g_count,
+    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, nullptr, 0, g_begin, g_count,
                                     dense, static_cast<cudaStream_t>(stream));
 }
 
 int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
                              const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
-                             int g_begin, int g_count, int dense, cudaStream_t cst) {
+                             int first_tile, int g_begin, int g_count, int dense, cudaStream_t cst) {
     using namespace fmsa;
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(o_part && lse_part && out && lse);
@@ -948,8 +954,8 @@ int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const f
     P.out = static_cast<__nv_bfloat16*>(out); P.lse = lse; P.lse_proxy = lse_proxy;
     P.S = pb->S; P.NB = pb->S / kBlock; P.Hq = pb->Hq; P.Hp = pb->Hp; P.mpp = pb->Hq / pb->Hp; P.ppk = pb->Hp / pb->Hkv;
     P.Kb = pb->top_k_blocks; P.g_begin = g_begin; P.G = g_count; P.dense = dense ? 1 : 0;
-    P.sinks = sinks; P.zero = zero;
-    const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * P.S;
+    P.sinks = sinks; P.zero = zero; P.q0 = first_tile * kBlock;
+    const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * (P.S - P.q0);
     const int64_t grid = (rows + 7) / 8;
     FMSA_REQUIRE(grid <= 0x7fffffffLL);
     const bool f16 = pb->dtype == FMSA_DTYPE_FP16;

@@ -120,6 +120,7 @@ class ReverseIndex:
     n_proxy_heads: int
     seq_len: int
     top_k_blocks: int
+    block_indices: torch.Tensor = None   # the selection it was built from
 
 
 def build_reverse_index(block_indices: torch.Tensor) -> ReverseIndex:
@@ -142,7 +143,7 @@ def build_reverse_index(block_indices: torch.Tensor) -> ReverseIndex:
         _launch("fmsa_reverse_index", 4, lib.fmsa_reverse_index(block_indices.data_ptr(), row_ptr.data_ptr(),
                                                               col_q.data_ptr(), edge_pos.data_ptr(), b * hp, s, kb,
                                                               ws.data_ptr(), ws_bytes, _stream(dev)), dev)
-    return ReverseIndex(row_ptr, col_q, edge_pos, b, hp, s, kb)
+    return ReverseIndex(row_ptr, col_q, edge_pos, b, hp, s, kb, block_indices)
 
 
 STATIC_SCRATCH_BYTES = 8 << 20
@@ -175,7 +176,7 @@ def build_reverse_index_static(block_indices: torch.Tensor, row_ptr: torch.Tenso
         _launch("fmsa_reverse_index_static", 4, lib.fmsa_reverse_index_static(
             block_indices.data_ptr(), row_ptr.data_ptr(), col_q.data_ptr(), edge_pos.data_ptr(), b * hp, s, kb,
             _stream(dev)), dev)
-    return ReverseIndex(row_ptr, col_q, edge_pos.view(b, hp, s, kb), b, hp, s, kb)
+    return ReverseIndex(row_ptr, col_q, edge_pos.view(b, hp, s, kb), b, hp, s, kb, block_indices)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -354,7 +355,8 @@ SPLIT_PARTIALS_ABOVE = 32
 
 def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, with_proxy=True, status=None, doc_start=None):
     """Sparse (or dense warmup) forward.  Returns (out [B,S,Hq*D] bf16, lse [B,Hq,S] fp32,
-    lse_proxy [B,Hp,S] fp32 or None)."""
+    lse_proxy [B,Hp,S] fp32 or None).  The stages of `fmsa_forward`, in its order of sums: the key-block stationary ones, then
+    the query tiles that the query-tile stationary kernel takes (all of them if dense; those need `rix.block_indices`)."""
     _require_cuda(q, k, v)
     lib = _lib.load()
     q, k, v = (_as_kernel_input(t.detach()) for t in (q, k, v))
@@ -370,6 +372,22 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
     lse_proxy = torch.empty(b, hp, s, dtype=torch.float32, device=dev) if with_proxy else None
     if status is None:
         status = torch.zeros(1, dtype=torch.int32, device=dev)
+    indices = None if dense else rix.block_indices
+    tiles = lib.fmsa_forward_tiles(ctypes_byref(pb), int(dense)) if dense or indices is not None else 0
+    st = _stream(dev)
+
+    def leading_tiles():
+        nbytes = lib.fmsa_tile_fwd_workspace_bytes(ctypes_byref(pb), int(dense))
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        with _Timed("attn_fwd", dev):
+            _launch("fmsa_tile_fwd", 1 if dense else 2, lib.fmsa_tile_fwd(
+                ctypes_byref(pb), _tensor_arg(q), _tensor_arg(k), _tensor_arg(v), _tensor_arg(qp), _tensor_arg(kp),
+                0 if dense else indices.data_ptr(), ws.data_ptr(), nbytes, out.data_ptr(), lse.data_ptr(),
+                lse_proxy.data_ptr() if with_proxy else 0, int(dense), status.data_ptr(), st), dev)
+        return out, lse, lse_proxy
+
+    if tiles == s // BLOCK_SIZE:
+        return leading_tiles()
     counter = torch.empty(1, dtype=torch.int32, device=dev)
     groups = b * hkv
     per_group = lib.fmsa_fwd_partial_slots(ctypes_byref(pb), 1, int(dense))
@@ -381,7 +399,6 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
     row_ptr = 0 if dense else rix.row_ptr.data_ptr()
     col_q = 0 if dense else rix.col_q.data_ptr()
     edge_pos = 0 if dense else rix.edge_pos.data_ptr()
-    st = _stream(dev)
     for g0 in range(0, groups, gstep):
         gc = min(gstep, groups - g0)
         with _Timed("attn_fwd", dev):
@@ -393,7 +410,7 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
             _launch("fmsa_sparse_fwd_combine", 2, lib.fmsa_sparse_fwd_combine(   # log-sum-exp kernel + row kernel
                 ctypes_byref(pb), o_part.data_ptr(), lse_part.data_ptr(), edge_pos, row_ptr, out.data_ptr(), lse.data_ptr(),
                 lse_proxy.data_ptr() if with_proxy else 0, g0, gc, int(dense), st), dev)
-    return out, lse, lse_proxy
+    return leading_tiles() if tiles else (out, lse, lse_proxy)
 
 
 def attention_backward(q, k, v, q_proxy, k_proxy, out, grad_out, lse, lse_proxy, scale, rix, grad_kl, *, dense=False,

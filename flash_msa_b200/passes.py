@@ -185,17 +185,18 @@ def plan(inputs, top_k_blocks, scale, dense) -> Plan:
     return p
 
 
-def _call(fn, what, args, device):
+def _call(fn, what, args, device, *more):
     timing = _Timing() if ops.KERNEL_EVENTS is not None else None
     launches = c_int32(0)
-    _lib.check(fn(ctypes.byref(args), ctypes.byref(timing.marks) if timing else None, ctypes.byref(launches), ops._stream(device)), what)
+    _lib.check(fn(ctypes.byref(args), *more, ctypes.byref(timing.marks) if timing else None, ctypes.byref(launches), ops._stream(device)), what)
     ops.LAUNCHES += launches.value
     if timing:
         timing.publish()
 
 
 def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
-    """Returns (out [B,S,Hq*128], kl_loss placeholder, saved).  `sinks`: fp32 [Hq] or None."""
+    """Returns (out [B,S,Hq*128], kl_loss placeholder, saved).  `sinks`: fp32 [Hq] or None.  `with_proxy` False: no backward
+    will follow."""
     dev = p.device
     a = ForwardArgs.from_buffer_copy(p.forward_args)
     given = p.point(a, inputs)   # noqa: F841 - copies live until the launch
@@ -213,7 +214,8 @@ def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
         a.doc_start = doc_start.data_ptr()
     if sinks is not None:
         a.sinks = sinks.data_ptr()
-    _call(_lib.load().fmsa_forward, "fmsa_forward", a, dev)
+    lib = _lib.load()
+    _call(lib.fmsa_forward if with_proxy else lib.fmsa_forward_alone, "fmsa_forward", a, dev, *(() if with_proxy else (1,)))
     return out, kl, saved
 
 

@@ -173,6 +173,17 @@ int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_part, const fl
                             const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse, float* lse_proxy,
                             int32_t g_begin, int32_t g_count, int32_t dense, void* stream);
 
+/* Query-tile stationary forward: query tiles (of 128 positions) 0 .. fmsa_forward_tiles()-1 of every (batch, head), in one kernel
+ * that walks the key blocks any row of a tile selected and keeps the output in tensor memory; out, lse and lse_proxy (or NULL) as
+ * fmsa_sparse_fwd_combine writes them.  fmsa_forward sends the first tiles of a sparse call, whose rows select most of what they
+ * can see, and all tiles of a dense one this way, the others through the two stages above.
+ *   block_indices int32 [B,Hp,S,top_k_blocks] (ignored if dense);  workspace 256-byte aligned, fmsa_tile_fwd_workspace_bytes(). */
+int32_t fmsa_forward_tiles(const fmsa_problem* pb, int32_t dense);
+int64_t fmsa_tile_fwd_workspace_bytes(const fmsa_problem* pb, int32_t dense);
+int fmsa_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                  const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* block_indices, void* workspace,
+                  int64_t workspace_bytes, void* out, float* lse, float* lse_proxy, int32_t dense, int32_t* status, void* stream);
+
 /* delta[b,h,q] = sum_d out[b,q,h,d] * d_out[b,q,h,d], fp32 [B,Hq,S].
  * Replaces the torch expression at flash_msa/flash_msa.py:99.  out is the contiguous
  * [B,S,Hq*128] forward output; d_out is described as a (B,Hq,S,128) view. */
@@ -299,6 +310,9 @@ typedef struct {
 
 int64_t fmsa_forward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int64_t max_partial_bytes);
 int fmsa_forward(const fmsa_forward_args* args, fmsa_marks* marks, int32_t* launches, void* stream);
+/* The same for a forward that no backward follows (alone = 1): row_ptr, col_q and edge_pos are scratch, written only where
+ * the forward itself needs them, and may be NULL where fmsa_forward_tiles() covers the sequence. */
+int fmsa_forward_alone(const fmsa_forward_args* args, int32_t alone, fmsa_marks* marks, int32_t* launches, void* stream);
 int64_t fmsa_backward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int32_t with_kl, int32_t split_above,
                                       int64_t max_partial_bytes);
 int fmsa_backward(const fmsa_backward_args* args, fmsa_marks* marks, int32_t* launches, void* stream);

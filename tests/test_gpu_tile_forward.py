@@ -1,0 +1,105 @@
+"""The query-tile stationary forward against the key-block stationary one (a reverse index without its selection sends every
+tile the general way): sizes at which tiles, words of the visit lists and the ring of items end, every layout, type and mask."""
+import dataclasses
+
+import pytest
+import torch
+
+from oracle import msa_oracle as O
+from tests.gpu_util import SCALE, bf16_inputs, kernel_selection, max_err, yardstick_check
+
+pytestmark = pytest.mark.gpu
+
+
+def _selection(cfg, kind):
+    """int32 [B,Hp,S,Kb]: own block, then `kind` of the others, the sentinel NB where there are no more."""
+    b, hp, s, kb = cfg["b"], cfg["hp"], cfg["s"], cfg["kb"]
+    nb = s // 128
+    own = (torch.arange(s) // 128).view(1, 1, s, 1)
+    g = torch.Generator().manual_seed(s + kb)
+    key = torch.rand(b, hp, s, nb, generator=g)
+    if kind == "alike":    # the rows of a tile agree but for a few, so that most blocks are visited by no row or by all of them
+        key = torch.where(torch.rand(b, hp, s, 1, generator=g) < 0.02, key, key[:, :, ::128].repeat_interleave(128, 2))
+    key = key.masked_fill(torch.arange(nb).view(1, 1, 1, nb) > own, -1.0).scatter(3, own.expand(b, hp, s, 1), 2.0)
+    val, idx = key.sort(dim=-1, descending=True)
+    return torch.where(val >= 0, idx, nb)[..., :kb].to(torch.int32).contiguous().cuda()
+
+
+CFGS = [
+    dict(b=1, s=128, hq=1, hkv=1, hp=1, hpkv=1, kb=1),
+    dict(b=3, s=256, hq=6, hkv=1, hp=2, hpkv=1, kb=1),
+    dict(b=2, s=640, hq=12, hkv=2, hp=4, hpkv=2, kb=3),
+    dict(b=1, s=4224, hq=5, hkv=1, hp=1, hpkv=1, kb=20),     # 33 blocks: a second round of 32 in the list of visited blocks
+    dict(b=1, s=8448, hq=4, hkv=2, hp=2, hpkv=2, kb=40),     # 66 blocks, all tiles
+    dict(b=1, s=8448, hq=4, hkv=1, hp=2, hpkv=1, kb=3),      # the first six tiles, the others the general way
+    dict(b=2, s=4096, hq=24, hkv=2, hp=2, hpkv=1, kb=2),     # ... with twelve heads per proxy head
+]
+
+
+@pytest.mark.parametrize("kind", ["random", "alike"])
+@pytest.mark.parametrize("cfg", CFGS, ids=lambda c: f"s{c['s']}_kb{c['kb']}_mpp{c['hq'] // c['hp']}")
+@pytest.mark.parametrize("form", ["plain", "fp16", "bshd", "docs"])
+def test_agrees_with_the_key_block_stationary_forward(cfg, kind, form):
+    from flash_msa_b200 import _lib, ops
+    dt = torch.float16 if form == "fp16" else torch.bfloat16
+    qp, kp, q, k, v, _ = bf16_inputs(dict(cfg, seed=cfg["s"]), layout="bshd" if form == "bshd" else "bhsd", dtype=dt)
+    qp = qp * 3   # sharper proxy rows: their maxima rise by more than the lazy rescale lets pass
+    if form != "bshd":
+        q = q * 4
+    cu = [0, cfg["s"] // 3, cfg["s"] // 3 + 1, cfg["s"]] if form == "docs" else None
+    ds = None if cu is None else ops.doc_start_from_cu_seqlens(cu, cfg["b"], cfg["s"], q.device)
+    idx = _selection(cfg, kind)
+    if ds is not None:   # a selection never holds blocks that end before the row's document
+        idx = torch.where(idx < (ds // 128).view(cfg["b"], 1, -1, 1), cfg["s"] // 128, idx)
+    rix = ops.build_reverse_index(idx)
+    pb = ops._problem(q, k, qp, kp, cfg["kb"], SCALE)
+    assert 1 <= _lib.load().fmsa_forward_tiles(pb, 0) <= cfg["s"] // 128
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ops.attention_forward(q, k, v, qp, kp, SCALE, rix, doc_start=ds, status=status)
+    want = ops.attention_forward(q, k, v, qp, kp, SCALE, dataclasses.replace(rix, block_indices=None), doc_start=ds, status=status)
+    ops.check_status(status, "forward")
+    # Both round P and the result to 16 bits (u = 2^-9 or 2^-12 of an element, P weighted with |v|), one of them the partial rows as
+    # well: five such errors of at most u max|v|.  The logarithms are those of fp32 sums of the same exponentials (2^-22 each).
+    u = 2.0 ** (-12 if dt == torch.float16 else -9)
+    assert max_err(got[0], want[0]) <= 5 * u * v.float().abs().max().item()
+    assert max_err(got[1], want[1]) <= 1e-4 and max_err(got[2], want[2]) <= 1e-4
+    alone = ops.attention_forward(q, k, v, qp, kp, SCALE, rix, doc_start=ds, with_proxy=False)
+    assert torch.equal(alone[0], got[0]) and torch.equal(alone[1], got[1])
+
+
+@pytest.mark.parametrize("s,kb", [(384, 2), (8192, 1)])
+def test_sinks_in_both_forwards(s, kb):
+    """All tiles, and the first two of 64, whose log-sum-exps take the sinks in different kernels."""
+    import flash_msa_b200 as fm
+    cfg = dict(b=1, s=s, hq=4, hkv=1, hp=1, hpkv=1, kb=kb, seed=5)
+    qp, kp, q, k, v, do = bf16_inputs(cfg)
+    sinks = torch.tensor([-3.0, 0.0, 2.0, 6.0], device="cuda", requires_grad=True)
+    leaves = [t.detach().requires_grad_(True) for t in (qp, kp, q, k, v)]
+    out, kl = fm.flash_msa_func(*leaves, kb * 128, SCALE, sinks=sinks)
+    torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+    with torch.no_grad():
+        alone, _ = fm.flash_msa_func(qp, kp, q, k, v, kb * 128, SCALE, sinks=sinks)
+    assert torch.equal(alone, out)
+    idx = kernel_selection(qp, kp, kb)
+    args = (qp, kp, q, k, v, kb * 128, SCALE, do, 1.0)
+    r32 = O.sparse_forward_backward(*args, block_indices=idx, sinks=sinks.detach())
+    r16 = O.sparse_forward_backward(*args, block_indices=idx, sinks=sinks.detach(), dtype=torch.bfloat16)
+    yardstick_check("out", out, r32["out"], r16["out"], 2e-3)
+    for n, leaf in zip(["dq_proxy", "dk_proxy", "dq", "dk", "dv"], leaves):
+        yardstick_check(n, leaf.grad, r32[n], r16[n], 2e-3 * r32[n].abs().max().item())
+
+
+def test_rows_that_select_nothing():
+    """Not what a selection gives, but what the index accepts: no edge for some rows, for a whole tile of them, or for all."""
+    from flash_msa_b200 import ops
+    cfg = dict(b=1, s=512, hq=4, hkv=2, hp=2, hpkv=1, kb=2, seed=3)
+    qp, kp, q, k, v, _ = bf16_inputs(cfg)
+    idx = _selection(cfg, "random")
+    idx[:, 0, 100:300] = 4
+    idx[:, 1, 384:] = 4
+    out, lse, lse_p = ops.attention_forward(q, k, v, qp, kp, SCALE, ops.build_reverse_index(idx))
+    none = (idx == 4).all(-1)                                    # [B,Hp,S]
+    rows = none.repeat_interleave(2, 1)                          # of the main heads
+    heads = out.view(1, 512, 4, 128).transpose(1, 2)
+    assert (heads[rows] == 0).all() and torch.isneginf(lse[rows]).all() and torch.isneginf(lse_p[none]).all()
+    assert torch.isfinite(lse[~rows]).all() and torch.isfinite(out).all()
