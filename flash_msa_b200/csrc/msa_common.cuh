@@ -58,9 +58,11 @@ __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int depth
 // sub-units beyond the end of their rows costs about a microsecond (up to 32 at a time), so C does not go below what keeps
 // the enumeration at `kDrawsPerCta` per CTA.
 // With 16 the rows of a group are gathered in half as many sweeps, which counts where they do not fit L2 (B=1 S=65536 Hq=8
-// top-k 32 blocks, 14 sub-units per CTA: forward 1.70 -> 1.56 ms, backward 3.83 -> 3.49 ms; S=32768, 64 blocks: equal), while
-// at 7 sub-units per CTA (B=2 S=8192 Hq=32 top-k 16 blocks) the tail makes it slower: 0.672 -> 0.692 ms forward.
-constexpr int kSubUnitsPerCta = 6, kLongSubUnitsPerCta = 12, kDrawsPerCta = 32;
+// top-k 32 blocks, 14 sub-units per CTA: forward 1.70 -> 1.56 ms, backward 3.83 -> 3.49 ms), and K, V, dK and dV move half as often
+// (B=2 S=8192 Hq=32 top-k 16 blocks, 7 per CTA, with the last groups cut finer: backward kernels 1.569 -> 1.516 ms; at two per CTA no
+// better, with four sub-units of 8 as the least elsewhere B=1 S=16384 top-k 96: 5.58 -> 6.18 ms).
+constexpr int kTailFreeGroup = 2;   // (see enumerate_subunits)
+constexpr int kSubUnitsPerCta = 6, kLongSubUnitsPerCta = 4, kDrawsPerCta = 32;
 inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int depth, int ppk, int sms) {
     const int64_t chunks = (edges + kBlock - 1) / kBlock + groups * ppk * NB / 2;
     int c = chunks >= static_cast<int64_t>(kMaxChunksPerSubUnit) * kLongSubUnitsPerCta * sms ? kMaxChunksPerSubUnit : kMaxChunksPerSubUnit / 2;
@@ -92,21 +94,60 @@ inline int forward_tiles(int NB, int top_k_blocks, int64_t main_heads, int dense
     return t < kTileFwdMaxBlocks ? t : kTileFwdMaxBlocks;
 }
 
-struct SubUnit {
-    int g, j, pp, chunk0;
+// The sub-units of a launch.  Those of the last groups are cut finer (a quarter of the chunks): a group of B=2 S=8192 Hq=32 top-k 16
+// blocks has fewer sub-units than there are SMs, so that the launch ended with SMs waiting for one last long sub-unit each: they were
+// busy 95-96 % of the kernels' time, 92 % at B=4 S=4096 Hq=16, 79-85 % with five documents at S=8192.  With the long sub-units above and
+// finer last groups, backward kernels: 1.550 -> 1.516, 0.694 -> 0.677, 0.522 -> 0.487 ms; halves instead of quarters: 0.499 with the
+// documents.
+struct SubUnits {
+    int32_t n;                                  // all of them (an upper bound of those with work)
+    uint32_t n_bulk, per_group, per_group_tail; // indices below n_bulk: per_group for each of the first groups; then per_group_tail each
+    int32_t groups_bulk, NB, ppk, chunks, chunks_tail;
 };
-// (32-bit arithmetic: the entry points require fewer than 2^31 sub-units; 64-bit divisions cost kilobytes of code here.)
-__device__ __forceinline__ SubUnit decode_subunit(uint32_t u, int NB, uint32_t ppk, int C, uint32_t per_group) {
+// False: more sub-units than the work counter can hold (it may run past the end by one per CTA and 31).
+inline bool enumerate_subunits(SubUnits* U, int64_t edges, int64_t groups, int NB, int depth, int ppk, int sms) {
+    U->NB = NB;
+    U->ppk = ppk;
+    U->chunks = chunks_per_subunit(edges, groups, NB, depth, ppk, sms);
+    U->chunks_tail = U->chunks >= 4 ? U->chunks / 4 : 1;
+    // Enough groups that the CTAs have about half a sub-unit's worth of work each left when the finer ones begin (a whole one: 0.705 ms at
+    // S=4096, 0.521 with the documents).  A group of several times as much work ends in enough sub-units of its own, the ends of its
+    // rows (B=1 S=65536 top-k 32: SMs 99.8 % busy).
+    const int64_t tail = static_cast<int64_t>(U->chunks) * sms / 2, per = (edges / groups + kBlock - 1) / kBlock + 1;
+    int64_t fine = per > kTailFreeGroup * tail || U->chunks == 1 ? 0 : (tail + per - 1) / per;
+    if (fine > groups) fine = groups;
+    constexpr int64_t kMost = 0x7f000000LL;
+    if (subunits_per_group(NB, depth, ppk, U->chunks_tail) * groups >= kMost) fine = 0;
+    U->groups_bulk = static_cast<int32_t>(groups - fine);
+    const int64_t pg = subunits_per_group(NB, depth, ppk, U->chunks), pt = subunits_per_group(NB, depth, ppk, U->chunks_tail);
+    if (pg * (groups - fine) + pt * fine >= kMost) return false;
+    U->per_group = static_cast<uint32_t>(pg);
+    U->per_group_tail = static_cast<uint32_t>(pt);
+    U->n_bulk = static_cast<uint32_t>(pg * (groups - fine));
+    U->n = static_cast<int32_t>(U->n_bulk + pt * fine);
+    return true;
+}
+
+struct SubUnit {
+    int g, j, pp, chunk0, chunks;
+};
+// (32-bit arithmetic: 64-bit divisions cost kilobytes of code here.)
+__device__ __forceinline__ SubUnit decode_subunit(uint32_t u, const SubUnits& U) {
     SubUnit su;
+    const bool bulk = u < U.n_bulk;
+    const uint32_t per_group = bulk ? U.per_group : U.per_group_tail;
+    su.chunks = bulk ? U.chunks : U.chunks_tail;
+    if (!bulk) u -= U.n_bulk;
     su.g = static_cast<int>(u / per_group);
-    const uint32_t r = u % per_group;
+    const uint32_t r = u - su.g * per_group, ppk = U.ppk;
+    if (!bulk) su.g += U.groups_bulk;
     su.pp = static_cast<int>(r % ppk);
     int x = static_cast<int>(r / ppk);
-    int left = NB, s = 0;   // key blocks that have a sub-unit s
-    while (x >= left) {   // at most NB/C iterations
+    int left = U.NB, s = 0;   // key blocks that have a sub-unit s
+    while (x >= left) {   // at most NB / chunks iterations
         x -= left;
-        left -= C;
-        s += C;
+        left -= su.chunks;
+        s += su.chunks;
     }
     su.j = x;
     su.chunk0 = s;
@@ -117,9 +158,8 @@ __device__ __forceinline__ SubUnit decode_subunit(uint32_t u, int NB, uint32_t p
 struct UnitSpace {
     const int32_t* row_ptr;
     int32_t* counter;
-    int32_t n_subunits;
-    uint32_t per_group;
-    int S, NB, Hkv, Hp, ppk, g_begin, chunks, dense;
+    SubUnits sub;
+    int S, NB, Hkv, Hp, ppk, g_begin, dense;
 };
 
 // A sub-unit as the drawing thread publishes it to the other roles (kept small: it shares the last 3 KB of shared memory).
@@ -152,8 +192,8 @@ __device__ __forceinline__ bool draw_work(int32_t* counter, uint32_t n_subunits,
 // A warp draws and decodes the next sub-unit; the result is lane 0's.
 __device__ __forceinline__ UnitRec draw_subunit(const UnitSpace& U) {
     UnitRec nu;
-    const bool more = draw_work(U.counter, static_cast<uint32_t>(U.n_subunits), [&](uint32_t u) -> bool {
-        const SubUnit su = decode_subunit(u, U.NB, U.ppk, U.chunks, U.per_group);
+    const bool more = draw_work(U.counter, static_cast<uint32_t>(U.sub.n), [&](uint32_t u) -> bool {
+        const SubUnit su = decode_subunit(u, U.sub);
         const uint32_t g = U.g_begin + su.g;
         const int b = g / static_cast<uint32_t>(U.Hkv), kvh = g % static_cast<uint32_t>(U.Hkv), p = kvh * U.ppk + su.pp;
         const int64_t bp = static_cast<int64_t>(b) * U.Hp + p;
@@ -169,7 +209,7 @@ __device__ __forceinline__ UnitRec draw_subunit(const UnitSpace& U) {
         nu.j = static_cast<uint16_t>(su.j); nu.b = static_cast<uint16_t>(b); nu.kvh = static_cast<uint16_t>(kvh);
         nu.p = static_cast<uint16_t>(p); nu.n = n; nu.e0 = e0;
         nu.chunk0 = static_cast<uint16_t>(su.chunk0);
-        nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + U.chunks));
+        nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + su.chunks));
         return su.chunk0 * kBlock < n;
     });
     if (!more) nu.chunk1 = -1;

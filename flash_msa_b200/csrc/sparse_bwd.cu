@@ -1100,12 +1100,8 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     U.row_ptr = row_ptr; U.counter = counter;
     U.S = pb->S; U.NB = pb->S / kBlock; U.Hkv = pb->Hkv; U.Hp = pb->Hp; U.ppk = pb->Hp / pb->Hkv;
     U.g_begin = g_begin; U.dense = dense ? 1 : 0;
-    U.chunks = chunks_per_subunit(fmsa_fwd_partial_slots(pb, g_count, dense), g_count, U.NB, U.NB, U.ppk, sms);
-    const int64_t per_group = subunits_per_group(U.NB, U.NB, U.ppk, U.chunks);
-    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA and 31)
-    U.per_group = static_cast<uint32_t>(per_group);
-    U.n_subunits = static_cast<int32_t>(per_group * g_count);
-    const int grid = U.n_subunits < sms ? U.n_subunits : sms;
+    FMSA_REQUIRE(enumerate_subunits(&U.sub, fmsa_fwd_partial_slots(pb, g_count, dense), g_count, U.NB, U.NB, U.ppk, sms));
+    const int grid = U.sub.n < sms ? U.sub.n : sms;
     kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tk, tv, P);
     if (with_kl) {
         if (zero_counters && cudaMemsetAsync(counter_proxy, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;

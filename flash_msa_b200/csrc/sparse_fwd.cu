@@ -58,9 +58,7 @@ struct FwdParams {
     int S, NB, Hq, Hkv, Hp, mpp, ppk, pg;
     int g_begin, G, first_tile;
     int with_proxy, dense;
-    int32_t n_subunits;
-    uint32_t units_per_group;
-    int chunks;             // chunks per sub-unit
+    SubUnits sub;
     float scale_log2e;
 };
 
@@ -241,8 +239,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
         const uint32_t uslot = draw & (kUnitRing - 1);
         if (decltype(mode)::value == kDraws && warp == 12) {
             UnitDesc nu;
-            const bool more = draw_work(P.counter, static_cast<uint32_t>(P.n_subunits), [&](uint32_t u) -> bool {
-                const SubUnit su = decode_subunit(u, P.NB, P.ppk, P.chunks, P.units_per_group);
+            const bool more = draw_work(P.counter, static_cast<uint32_t>(P.sub.n), [&](uint32_t u) -> bool {
+                const SubUnit su = decode_subunit(u, P.sub);
                 const uint32_t g = P.g_begin + su.g;
                 const int b = g / static_cast<uint32_t>(P.Hkv), kvh = g % static_cast<uint32_t>(P.Hkv), p = kvh * P.ppk + su.pp;
                 const int64_t bp = static_cast<int64_t>(b) * P.Hp + p;
@@ -257,7 +255,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                 }
                 nu.j = su.j; nu.b = b; nu.kvh = kvh; nu.p = p; nu.n = n; nu.e0 = e0;
                 nu.chunk0 = su.chunk0;
-                nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + P.chunks);
+                nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + su.chunks);
                 return su.chunk0 * kBlock < n;
             });
             if (!more) nu.chunk1 = -1;
@@ -921,12 +919,9 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
                            : (varlen ? reinterpret_cast<const void*>(sparse_fwd_kernel<false, true>) : reinterpret_cast<const void*>(sparse_fwd_kernel<false, false>));
     if (sms <= 0 || !ensure_smem_attr(kfn, kFwdSmemBytes)) return FMSA_ERR_CUDA;
     const int depth = P.NB - first_tile;
-    P.chunks = chunks_per_subunit((dense ? fmsa_fwd_partial_slots(pb, g_count, 1) : fmsa_fwd_partial_slots(pb, g_count, 0) / P.NB * depth), g_count, P.NB, depth, P.ppk, sms);
-    const int64_t per_group = subunits_per_group(P.NB, depth, P.ppk, P.chunks);
-    FMSA_REQUIRE(per_group * g_count < 0x7f000000LL);   // (the work counter may run past the end by one per CTA and 31)
-    P.units_per_group = static_cast<uint32_t>(per_group);
-    P.n_subunits = static_cast<int32_t>(per_group * g_count);
-    const int grid = static_cast<int>(P.n_subunits < sms ? P.n_subunits : sms);
+    const int64_t edges = dense ? fmsa_fwd_partial_slots(pb, g_count, 1) : fmsa_fwd_partial_slots(pb, g_count, 0) / P.NB * depth;
+    FMSA_REQUIRE(enumerate_subunits(&P.sub, edges, g_count, P.NB, depth, P.ppk, sms));
+    const int grid = P.sub.n < sms ? P.sub.n : sms;
     if (fp16 && varlen) sparse_fwd_kernel<true, true><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
     else if (fp16) sparse_fwd_kernel<true, false><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
     else if (varlen) sparse_fwd_kernel<false, true><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);

@@ -1,0 +1,30 @@
+"""How a launch is cut into sub-units must not show in its results: one pass over all (batch, KV head) groups against one pass per
+group, whose launches take other sub-unit lengths and finer last groups."""
+import pytest
+import torch
+
+from tests.gpu_util import SCALE, bf16_inputs, max_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("b,s,kb,docs", [(1, 4096, 16, False), (2, 4096, 16, False), (4, 4096, 16, True), (5, 4096, 16, False), (3, 1664, 5, True)])
+def test_one_pass_against_a_pass_per_group(monkeypatch, b, s, kb, docs):
+    """Sub-units of 2, 4, 8 and 16 chunks at most in the one pass (and 1, rows that end inside a chunk, in the last case)."""
+    import flash_msa_b200 as fm
+    from flash_msa_b200 import ops
+    *inputs, do = bf16_inputs(dict(b=b, s=s, hq=4, hkv=4, hp=4, hpkv=4, seed=b + s))
+    res = []
+    for cap in (None, 1):
+        if cap:
+            monkeypatch.setattr(ops, "MAX_PARTIAL_BYTES", cap)
+        leaves = [t.detach().requires_grad_(True) for t in inputs]
+        if docs:
+            out, kl = fm.flash_msa_varlen_func(*leaves, [0, s // 3, s // 2 + 5, s], kb * 128, SCALE)
+        else:
+            out, kl = fm.flash_msa_func(*leaves, kb * 128, SCALE)
+        torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+        res.append([out] + [t.grad for t in leaves])
+    for n, a, c in zip(["out", "dq_proxy", "dk_proxy", "dq", "dk", "dv"], *res):
+        # (the order in which sub-units add to dK, dV and dKp is free: the last bit of the 16-bit result)
+        assert max_err(a, c) <= (0.0 if n in ("out", "dq", "dq_proxy") else 2 ** -7 * c.float().abs().max().item()), n
