@@ -79,7 +79,7 @@ def _declare(lib):
     lib.fmsa_sparse_fwd_combine.restype = c_int
     lib.fmsa_sparse_fwd_combine.argtypes = [PB, P, P, P, P, P, P, P, c_int32, c_int32, c_int32, P]
     lib.fmsa_forward_tiles.restype = c_int32
-    lib.fmsa_forward_tiles.argtypes = [PB, c_int32]
+    lib.fmsa_forward_tiles.argtypes = [PB, c_int32, c_int32]
     lib.fmsa_tile_fwd_workspace_bytes.restype = c_int64
     lib.fmsa_tile_fwd_workspace_bytes.argtypes = [PB, c_int32]
     lib.fmsa_tile_fwd.restype = c_int
@@ -101,8 +101,10 @@ def _declare(lib):
     lib.fmsa_backward_workspace_bytes.argtypes = [PB, c_int32, c_int32, c_int32, c_int64]
     lib.fmsa_forward.restype = c_int
     lib.fmsa_forward.argtypes = [P, P, P, P]
-    lib.fmsa_forward_alone.restype = c_int
-    lib.fmsa_forward_alone.argtypes = [P, c_int32, P, P, P]
+    lib.fmsa_forward_hinted_workspace_bytes.restype = c_int64
+    lib.fmsa_forward_hinted_workspace_bytes.argtypes = [PB, c_int32, c_int32, c_int64]
+    lib.fmsa_forward_hinted.restype = c_int
+    lib.fmsa_forward_hinted.argtypes = [P, c_int32, c_int32, P, P, P]
     lib.fmsa_backward.restype = c_int
     lib.fmsa_backward.argtypes = [P, P, P, P]
     lib.fmsa_doc_start.restype = c_int

@@ -126,7 +126,7 @@ def _sink_logits(sinks):
     return None if sinks is None else sinks.detach().to(torch.float32).contiguous()
 
 
-def _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, with_proxy):
+def _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, visible, sinks, with_proxy):
     """Checks the call, then runs its forward: (plan, fp32 sink logits or None, out, kl_loss placeholder, saved)."""
     _, top_k_blocks = _validate_inputs(q_proxy, k_proxy, q, k, v, top_k if sparse else 0, sparse)
     if sparse:
@@ -141,7 +141,7 @@ def _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, 
     plan = passes.plan(inputs, top_k_blocks, scale, not sparse)
     logits = _sink_logits(sinks)
     status = _Status(0 if sparse else 2, plan.device)
-    out, kl_loss, saved = passes.forward(plan, inputs, doc_start, logits, status.ptr, with_proxy)
+    out, kl_loss, saved = passes.forward(plan, inputs, doc_start, logits, status.ptr, with_proxy, *((visible,) if visible else ()))
     status.check()
     return plan, logits, out, kl_loss, saved
 
@@ -151,10 +151,10 @@ class _AttentionFunction(torch.autograd.Function):
     the backward on (reference: flash_msa/msa_forward_cutedsl.py:69)."""
 
     @staticmethod
-    def forward(ctx, q_proxy, k_proxy, q, k, v, sinks, doc_start, top_k, scale, sparse):
+    def forward(ctx, q_proxy, k_proxy, q, k, v, sinks, doc_start, visible, top_k, scale, sparse):
         # (everything that depends on the inputs is done in here: a trace records this call as one node, which comes back with
         # tensors of any size when the trace is run)
-        plan, logits, out, kl_loss, saved = _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, True)
+        plan, logits, out, kl_loss, saved = _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, visible, sinks, True)
         ctx.save_for_backward(q_proxy, k_proxy, q, k, v, out, saved)
         # an output that does not feed the loss arrives as None in backward (not as zeros): no gradient for
         # kl_loss then really skips the proxy work, as the reference intends (flash_msa/flash_msa.py:104-106)
@@ -175,18 +175,19 @@ class _AttentionFunction(torch.autograd.Function):
                                                        ctx.logits, status.ptr)
         _publish_kl(klv)
         status.check()
-        return dqp, dkp, dq, dk, dv, None if dsinks is None else dsinks.to(ctx.sinks_dtype), None, None, None, None
+        return dqp, dkp, dq, dk, dv, None if dsinks is None else dsinks.to(ctx.sinks_dtype), None, None, None, None, None
 
 
-def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks):
+def _attend(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, documents, sinks):
+    doc_start, visible = documents
     q_proxy = _spread_proxy_heads(q_proxy, k_proxy, q, k)
     with_grad = torch.is_grad_enabled() and (q_proxy.requires_grad or k_proxy.requires_grad or q.requires_grad or k.requires_grad or
                                              v.requires_grad or (sinks is not None and sinks.requires_grad))
     if with_grad or forward_ad._current_level >= 0 or torch._C._is_tracing():
-        return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, top_k, scale, sparse)
+        return _AttentionFunction.apply(q_proxy, k_proxy, q, k, v, sinks, doc_start, visible, top_k, scale, sparse)
     # No backward will follow: the proxy log-sum-exp, which only the backward needs, is left out.  (Tangents would be lost
     # here, which the autograd function refuses, and a trace would hold nothing but the allocation of `out`.)
-    return _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, sinks, False)[2:4]
+    return _forward(q_proxy, k_proxy, q, k, v, top_k, scale, sparse, doc_start, visible, sinks, False)[2:4]
 
 
 def _spread_proxy_heads(q_proxy, k_proxy, q, k):
@@ -205,18 +206,21 @@ def _spread_proxy_heads(q_proxy, k_proxy, q, k):
     return q_proxy   # (anything else is judged by the shape checks of the call)
 
 
-def _doc_start(q, cu_seqlens):
+_NO_DOCUMENTS = (None, 0)
+
+
+def _documents(q, cu_seqlens):
     if q.ndim != 4:
         raise ValueError("all attention tensors must have shape (B, H, S, D)")
     _require_cuda(q)
-    return ops.doc_start_from_cu_seqlens(cu_seqlens, q.shape[0], q.shape[2], q.device)
+    return ops.document_layout(cu_seqlens, q.shape[0], q.shape[2], q.device)
 
 
 def sparse_attention(q_proxy, k_proxy, q, k, v, top_k: int, scale: float, sinks=None):
     """Block-sparse top-k GQA attention.  Returns ``(attn_out [B,S,Hq*D], kl_loss placeholder)``.
     ``sinks`` (optional, beyond the reference): one softmax-bias logit per main query head that joins the softmax
     denominator and contributes no value."""
-    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, None, sinks)
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, _NO_DOCUMENTS, sinks)
 
 
 def sparse_attention_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, scale: float, sinks=None):
@@ -227,17 +231,17 @@ def sparse_attention_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, s
     must still be a multiple of 128 (pad the last document).  The reference has no such path (its README lists
     variable-length batches as missing).  Boundaries in host memory (a list, a CPU tensor) are checked there
     and travel with a kernel launch; those in a CUDA tensor make the call wait for the device, for the same checks."""
-    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, _doc_start(q, cu_seqlens), sinks)
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), True, _documents(q, cu_seqlens), sinks)
 
 
 def sparse_attention_warmup(q_proxy, k_proxy, q, k, v, top_k: int, scale: float, sinks=None):
     """Dense causal warmup attention with full-sequence proxy KL gradients (top_k is accepted and ignored, as in the
     reference)."""
-    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), False, None, sinks)
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), False, _NO_DOCUMENTS, sinks)
 
 
 def sparse_attention_warmup_varlen(q_proxy, k_proxy, q, k, v, cu_seqlens, top_k: int, scale: float, sinks=None):
     """`sparse_attention_warmup` on packed sequences (see `sparse_attention_varlen`): dense causal attention and the
     full-sequence proxy KL inside every document.  The schedule still visits every causal block pair of the packed
     sequence; pairs that straddle documents are masked."""
-    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), False, _doc_start(q, cu_seqlens), sinks)
+    return _attend(q_proxy, k_proxy, q, k, v, int(top_k), float(scale), False, _documents(q, cu_seqlens), sinks)

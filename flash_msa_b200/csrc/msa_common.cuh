@@ -78,18 +78,22 @@ inline int chunks_per_subunit(int64_t edges, int64_t groups, int NB, int depth, 
 constexpr int kTileFwdMaxBlocks = 256;   // most blocks that a tile of a sparse call can visit there
 // Query tile i visits up to i + 1 blocks there, against min(i + 1, top_k_blocks) edges per row here, and an edge of the key-block
 // stationary forward and its combine takes as long as about two visits: 18.8 ns against 9.0 ns of the whole GPU per 128 edges, or visit,
-// of a main head (B=2 S=8192 Hq=32 top-k 16 blocks; B=4 S=4096 Hq=32 dense, both with the proxy heads).  So the first 2 top_k_blocks
-// tiles go there; all of them, so that the other forward and its combine need not run, where those would be short (their
-// launches and tails cost as much as some 2800 visits).
-constexpr int kTileFwdVisitsPerEdge = 2, kTileFwdLaunchVisits = 2800;
-inline int forward_tiles(int NB, int top_k_blocks, int64_t main_heads, int dense) {   // main_heads: of all batch elements
+// of a main head (B=2 S=8192 Hq=32 top-k 16 blocks; B=4 S=4096 Hq=32 dense, both with the proxy heads), and its scattered rows cost more
+// power, which is what limits the clock.  So the first 2.5 top_k_blocks tiles go there (forward of B=2 S=8192 Hq=32 top-k 16, back to back:
+// 2.0 1127, 2.5 1118, 3.0 1164 us; of B=1 S=32768 top-k 64 12.20, 12.10, 12.30 ms); all of them, so that the other forward and its
+// combine need not run, where those would be short (their launches and tails cost as much as some 2800 visits), and where documents are
+// known to be so short that no tile sees more than that many blocks (`visible`, 0: not known; B=1 S=8192 Hq=32 top-k 16 as five documents:
+// forward 0.333 -> 0.189 ms).  The lists of visited blocks are kept for kTileFwdMaxBlocks, the bit maps behind them for sequences of kTileFwdMaxTiles.
+constexpr int kTileFwdLaunchVisits = 2800, kTileFwdMaxTiles = 512;
+inline int forward_tiles(int NB, int top_k_blocks, int64_t main_heads, int dense, int visible) {   // main_heads: of all batch elements
     if (dense) return NB;
-    int t = kTileFwdVisitsPerEdge * top_k_blocks;
+    int t = 5 * top_k_blocks / 2;
+    if (visible > 0 && visible <= t && visible <= kTileFwdMaxBlocks && NB <= kTileFwdMaxTiles) return NB;
     if (NB <= kTileFwdMaxBlocks) {
         if (t >= NB) return NB;
         const int64_t visits = (static_cast<int64_t>(NB) * (NB + 1) - static_cast<int64_t>(t) * (t + 1)) / 2;   // of the tiles from t on
         const int64_t edges = static_cast<int64_t>(NB - t) * top_k_blocks;
-        if ((visits - kTileFwdVisitsPerEdge * edges) * main_heads <= kTileFwdLaunchVisits) return NB;
+        if ((visits - 2 * edges) * main_heads <= kTileFwdLaunchVisits) return NB;
     }
     return t < kTileFwdMaxBlocks ? t : kTileFwdMaxBlocks;
 }

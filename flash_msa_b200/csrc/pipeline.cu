@@ -45,9 +45,9 @@ struct ForwardSpace {
 };
 // The selection's buffers and the partial rows of the key-block stationary forward, which comes last, are not alive at the same
 // time: they share the space.
-ForwardSpace carve_forward(const fmsa_problem* pb, int dense, int64_t max_bytes, void* base) {
+ForwardSpace carve_forward(const fmsa_problem* pb, int dense, int visible, int64_t max_bytes, void* base) {
     ForwardSpace w = {};
-    w.tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense);
+    w.tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense, visible);
     const int mpp = pb->Hq / pb->Hp;
     const int64_t groups = static_cast<int64_t>(pb->B) * pb->Hkv, rows = static_cast<int64_t>(pb->B) * pb->Hp, NB = pb->S / 128;
     w.gstep = groups_per_pass(pb, dense, static_cast<int64_t>(mpp) * 256 + (mpp + 1) * 8, max_bytes);
@@ -125,22 +125,27 @@ struct Marks {
     } while (0)
 
 extern "C" int64_t fmsa_forward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int64_t max_partial_bytes) {
+    return fmsa_forward_hinted_workspace_bytes(pb, dense, 0, max_partial_bytes);
+}
+
+extern "C" int64_t fmsa_forward_hinted_workspace_bytes(const fmsa_problem* pb, int32_t dense, int32_t visible, int64_t max_partial_bytes) {
     using namespace fmsa;
-    return problem_ok(pb) ? carve_forward(pb, dense, max_partial_bytes, nullptr).bytes : 0;
+    return problem_ok(pb) ? carve_forward(pb, dense, visible, max_partial_bytes, nullptr).bytes : 0;
 }
 
 extern "C" int fmsa_forward(const fmsa_forward_args* a, fmsa_marks* marks, int32_t* launches, void* stream) {
-    return fmsa_forward_alone(a, 0, marks, launches, stream);
+    return fmsa_forward_hinted(a, 0, 0, marks, launches, stream);
 }
 
-extern "C" int fmsa_forward_alone(const fmsa_forward_args* a, int32_t alone, fmsa_marks* marks, int32_t* launches, void* stream) {
+extern "C" int fmsa_forward_hinted(const fmsa_forward_args* a, int32_t alone, int32_t visible, fmsa_marks* marks, int32_t* launches,
+                                   void* stream) {
     using namespace fmsa;
     FMSA_REQUIRE(a && problem_ok(&a->pb) && a->workspace && a->out && a->lse && a->status && launches);
     FMSA_REQUIRE((reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0 && (!a->with_proxy || a->lse_proxy));
     const fmsa_problem* pb = &a->pb;
     const int dense = a->dense ? 1 : 0;
     FMSA_REQUIRE(dense || (pb->top_k_blocks >= 1 && pb->top_k_blocks <= pb->S / 128));
-    const ForwardSpace w = carve_forward(pb, dense, a->max_partial_bytes, a->workspace);
+    const ForwardSpace w = carve_forward(pb, dense, visible, a->max_partial_bytes, a->workspace);
     const bool index = !dense && (!alone || w.passes);   // the reverse index is wanted
     FMSA_REQUIRE(!index || (a->row_ptr && a->col_q && a->edge_pos));
     if (w.bytes > a->workspace_bytes) return FMSA_ERR_WORKSPACE;
@@ -205,15 +210,15 @@ extern "C" int fmsa_forward_alone(const fmsa_forward_args* a, int32_t alone, fms
 // ---------------------------------------------------------------------------------------------
 // The query-tile stationary forward as a stage of its own.
 // ---------------------------------------------------------------------------------------------
-extern "C" int32_t fmsa_forward_tiles(const fmsa_problem* pb, int32_t dense) {
+extern "C" int32_t fmsa_forward_tiles(const fmsa_problem* pb, int32_t dense, int32_t visible) {
     using namespace fmsa;
-    return problem_ok(pb) ? forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense) : 0;
+    return problem_ok(pb) ? forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense, visible) : 0;
 }
 
 extern "C" int64_t fmsa_tile_fwd_workspace_bytes(const fmsa_problem* pb, int32_t dense) {
     using namespace fmsa;
     if (!problem_ok(pb)) return 0;
-    const int64_t tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense);
+    const int64_t tiles = fmsa_forward_tiles(pb, dense, 0);
     return 256 + (dense ? 0 : static_cast<int64_t>(pb->B) * pb->Hp * tiles * tiles * 16);
 }
 
@@ -229,7 +234,7 @@ extern "C" int fmsa_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const
     if (rows > 65535 || pb->S / kBlock > 2048) return FMSA_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RixExtras x;
-    x.tiles = forward_tiles(pb->S / kBlock, pb->top_k_blocks, static_cast<int64_t>(pb->B) * pb->Hq, dense);
+    x.tiles = fmsa_forward_tiles(pb, dense, 0);
     x.zero = static_cast<int32_t*>(workspace); x.nzero = 1;
     if (!dense) {
         x.visits = static_cast<char*>(workspace) + 256;

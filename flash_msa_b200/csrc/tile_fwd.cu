@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                             const uint4 w = j >= 0 ? src[j] : make_uint4(0, 0, 0, 0);
                             const bool some = (w.x | w.y | w.z | w.w) != 0;
                             const uint32_t m = __ballot_sync(0xffffffffu, some);
-                            if (some) {
-                                const int at = n + __popc(m & ((1u << lane) - 1u));
+                            const int at = n + __popc(m & ((1u << lane) - 1u));
+                            if (some && at < kTileFwdMaxBlocks) {
                                 sm->rows[slot][at] = w;
                                 sm->block[slot][at] = static_cast<uint16_t>(j);
                             }
@@ -200,6 +200,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                         if (n == 0 && lane == 0) {   // (not from a selection: every row selects its own block)
                             sm->rows[slot][0] = make_uint4(0, 0, 0, 0);
                             sm->block[slot][0] = static_cast<uint16_t>(it.i);
+                        }
+                        if (n > kTileFwdMaxBlocks) {   // (documents that are longer than the caller said)
+                            n = kTileFwdMaxBlocks;
+                            if (lane == 0) atomicMax(P.status, kStatusBadIndex);
                         }
                         it.steps = max(n, 1);
                     }
@@ -547,7 +551,7 @@ int launch_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_ten
     FMSA_REQUIRE(problem_ok(pb) && q && k && v && q->ptr && k->ptr && v->ptr && out && lse && counter && status);
     FMSA_REQUIRE(dense || visits);
     FMSA_REQUIRE(!lse_proxy || (q_proxy && k_proxy && q_proxy->ptr && k_proxy->ptr));
-    FMSA_REQUIRE(tiles >= 1 && tiles <= pb->S / kBlock && (dense || tiles <= kTileFwdMaxBlocks) && pb->scale > 0.f);
+    FMSA_REQUIRE(tiles >= 1 && tiles <= pb->S / kBlock && (dense || tiles <= kTileFwdMaxTiles) && pb->scale > 0.f);
     FMSA_REQUIRE(aligned16(out) && (reinterpret_cast<uintptr_t>(visits) & 15u) == 0);
     const fmsa_tensor* qp = lse_proxy ? q_proxy : q;
     const fmsa_tensor* kp = lse_proxy ? k_proxy : k;

@@ -231,6 +231,12 @@ def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> t
     """int32 [B,S] on `device`: for every token of a packed sequence the position of the first token of its document.
     `cu_seqlens` is [n+1] (one packing for every batch element) or [B,n+1]; it starts at 0 and ends at `seq_len`
     (the FlashAttention varlen convention).  The kernels take this array (`fmsa_problem.doc_start`)."""
+    return document_layout(cu_seqlens, batch, seq_len, device)[0]
+
+
+def document_layout(cu_seqlens, batch: int, seq_len: int, device):
+    """(`doc_start_from_cu_seqlens`, the most key blocks of one document that a query tile can see, or 0 where only the device
+    knows the boundaries)."""
     cu_seqlens = torch.as_tensor(cu_seqlens)
     if cu_seqlens.device.type == "cpu" and not torch._C._is_tracing():
         # boundaries that the host holds are checked here and travel as a kernel parameter: nothing waits for the device
@@ -245,7 +251,8 @@ def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> t
             out = torch.empty(batch, seq_len, dtype=torch.int32, device=device)
             _launch("fmsa_doc_start", 1, _lib.load().fmsa_doc_start(cu.ctypes.data, cu.shape[-1], int(cu.ndim == 2), batch, seq_len,
                                                                  out.data_ptr(), _stream(out.device)), out.device)
-            return out
+            first, end = cu[..., :-1], cu[..., 1:]   # (an empty document spans no block: its last position lies before its first)
+            return out, int((((end - 1) >> 7) - (first >> 7)).max()) + 1
     # (boundaries in device memory: the checks below wait for the device, three times)
     cu = cu_seqlens.to(device=device, dtype=torch.int64)
     if cu.dim() == 1:
@@ -257,7 +264,7 @@ def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> t
         raise ValueError("cu_seqlens must rise from 0 to the sequence length")
     pos = torch.arange(seq_len, device=device, dtype=torch.int64).unsqueeze(0).expand(batch, -1).contiguous()
     which = torch.searchsorted(cu, pos, right=True) - 1
-    return torch.gather(cu, 1, which).to(torch.int32).contiguous()
+    return torch.gather(cu, 1, which).to(torch.int32).contiguous(), 0
 
 
 def _check_doc_start(doc_start, b, s, dev):
@@ -373,7 +380,7 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
     if status is None:
         status = torch.zeros(1, dtype=torch.int32, device=dev)
     indices = None if dense else rix.block_indices
-    tiles = lib.fmsa_forward_tiles(ctypes_byref(pb), int(dense)) if dense or indices is not None else 0
+    tiles = lib.fmsa_forward_tiles(ctypes_byref(pb), int(dense), 0) if dense or indices is not None else 0
     st = _stream(dev)
 
     def leading_tiles():

@@ -98,6 +98,7 @@ class Plan:
         self.out_shape = (b, s, hq * d)
         pbr = ctypes.byref(self.pb)
         self.forward_bytes = lib.fmsa_forward_workspace_bytes(pbr, int(dense), self.max_partial_bytes)
+        self._short_bytes = None   # of a forward that needs no partial rows because documents are short
         # saved for the backward, one int32 tensor: row_ptr | col_q | edge_pos | lse | lse_proxy, each from a 64-word boundary
         nb, edges = s // ops.BLOCK_SIZE, 0 if dense else b * hp * s * int(top_k_blocks)
         sizes = [0 if dense else b * hp * nb + 1, edges, edges, b * hq * s, b * hp * s]
@@ -134,6 +135,16 @@ class Plan:
                 self._strides(a, name, (n1 * n2 * 128, 128, n2 * 128) if bshd else (n1 * n2 * 128, n2 * 128, 128))
             got = self._backward[with_kl] = (bytes(a), nbytes)
         return got
+
+    def short_documents(self, visible):
+        """Workspace bytes of a forward all of whose tiles go the query-tile stationary way because no tile sees more than
+        `visible` blocks; 0 where they do not, or do anyway."""
+        lib, pbr, nb = _lib.load(), ctypes.byref(self.pb), self.shape[2] // ops.BLOCK_SIZE
+        if self.dense or lib.fmsa_forward_tiles(pbr, 0, visible) < nb or lib.fmsa_forward_tiles(pbr, 0, 0) == nb:
+            return 0
+        if self._short_bytes is None:
+            self._short_bytes = lib.fmsa_forward_hinted_workspace_bytes(pbr, 0, visible, self.max_partial_bytes)
+        return self._short_bytes
 
     def point(self, a, inputs, as_planned=True):
         """Points the argument block `a` at the inputs as the kernels can read them: in place, or - other strides, or an address
@@ -185,25 +196,28 @@ def plan(inputs, top_k_blocks, scale, dense) -> Plan:
     return p
 
 
-def _call(fn, what, args, device, *more):
+def _call(fn, what, args, device):
     timing = _Timing() if ops.KERNEL_EVENTS is not None else None
     launches = c_int32(0)
-    _lib.check(fn(ctypes.byref(args), *more, ctypes.byref(timing.marks) if timing else None, ctypes.byref(launches), ops._stream(device)), what)
+    _lib.check(fn(ctypes.byref(args), ctypes.byref(timing.marks) if timing else None, ctypes.byref(launches), ops._stream(device)), what)
     ops.LAUNCHES += launches.value
     if timing:
         timing.publish()
 
 
-def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
+def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy, visible=0):
     """Returns (out [B,S,Hq*128], kl_loss placeholder, saved).  `sinks`: fp32 [Hq] or None.  `with_proxy` False: no backward
-    will follow."""
+    will follow.  `visible`: the most key blocks a query tile can see with `doc_start`, or 0."""
     dev = p.device
     a = ForwardArgs.from_buffer_copy(p.forward_args)
     given = p.point(a, inputs)   # noqa: F841 - copies live until the launch
     out = torch.empty(p.out_shape, dtype=p.dtype, device=dev)
     kl = torch.empty((), dtype=torch.float32, device=dev)
     saved = torch.empty(p.saved_words, dtype=torch.int32, device=dev)
-    ws = torch.empty(p.forward_bytes, dtype=torch.uint8, device=dev)
+    short = p.short_documents(visible) if visible else 0
+    ws = torch.empty(short or p.forward_bytes, dtype=torch.uint8, device=dev)
+    if short:
+        a.workspace_bytes = short
     base, at = saved.data_ptr(), p.at
     if not p.dense:
         a.row_ptr, a.col_q, a.edge_pos = base + at[0], base + at[1], base + at[2]
@@ -215,7 +229,11 @@ def forward(p: Plan, inputs, doc_start, sinks, status_ptr, with_proxy):
     if sinks is not None:
         a.sinks = sinks.data_ptr()
     lib = _lib.load()
-    _call(lib.fmsa_forward if with_proxy else lib.fmsa_forward_alone, "fmsa_forward", a, dev, *(() if with_proxy else (1,)))
+    fn = lib.fmsa_forward
+    if short or not with_proxy:
+        def fn(args, marks, launches, stream, alone=int(not with_proxy), seen=visible if short else 0):
+            return lib.fmsa_forward_hinted(args, alone, seen, marks, launches, stream)
+    _call(fn, "fmsa_forward", a, dev)
     return out, kl, saved
 
 

@@ -178,7 +178,7 @@ int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_part, const fl
  * fmsa_sparse_fwd_combine writes them.  fmsa_forward sends the first tiles of a sparse call, whose rows select most of what they
  * can see, and all tiles of a dense one this way, the others through the two stages above.
  *   block_indices int32 [B,Hp,S,top_k_blocks] (ignored if dense);  workspace 256-byte aligned, fmsa_tile_fwd_workspace_bytes(). */
-int32_t fmsa_forward_tiles(const fmsa_problem* pb, int32_t dense);
+int32_t fmsa_forward_tiles(const fmsa_problem* pb, int32_t dense, int32_t visible);   /* visible: see fmsa_forward_hinted, 0 for this stage */
 int64_t fmsa_tile_fwd_workspace_bytes(const fmsa_problem* pb, int32_t dense);
 int fmsa_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
                   const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* block_indices, void* workspace,
@@ -310,9 +310,13 @@ typedef struct {
 
 int64_t fmsa_forward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int64_t max_partial_bytes);
 int fmsa_forward(const fmsa_forward_args* args, fmsa_marks* marks, int32_t* launches, void* stream);
-/* The same for a forward that no backward follows (alone = 1): row_ptr, col_q and edge_pos are scratch, written only where
- * the forward itself needs them, and may be NULL where fmsa_forward_tiles() covers the sequence. */
-int fmsa_forward_alone(const fmsa_forward_args* args, int32_t alone, fmsa_marks* marks, int32_t* launches, void* stream);
+/* The same with what the caller knows beyond the arguments.
+ * alone    1: no backward follows: row_ptr, col_q and edge_pos are scratch, written only where the forward itself needs them, and may
+ *          be NULL where fmsa_forward_tiles() covers the sequence.
+ * visible  the most key blocks that the rows of any query tile can see (with doc_start: short documents let all tiles go the
+ *          query-tile stationary way), or 0: not known. */
+int64_t fmsa_forward_hinted_workspace_bytes(const fmsa_problem* pb, int32_t dense, int32_t visible, int64_t max_partial_bytes);
+int fmsa_forward_hinted(const fmsa_forward_args* args, int32_t alone, int32_t visible, fmsa_marks* marks, int32_t* launches, void* stream);
 int64_t fmsa_backward_workspace_bytes(const fmsa_problem* pb, int32_t dense, int32_t with_kl, int32_t split_above,
                                       int64_t max_partial_bytes);
 int fmsa_backward(const fmsa_backward_args* args, fmsa_marks* marks, int32_t* launches, void* stream);

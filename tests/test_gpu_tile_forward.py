@@ -53,7 +53,7 @@ def test_agrees_with_the_key_block_stationary_forward(cfg, kind, form):
         idx = torch.where(idx < (ds // 128).view(cfg["b"], 1, -1, 1), cfg["s"] // 128, idx)
     rix = ops.build_reverse_index(idx)
     pb = ops._problem(q, k, qp, kp, cfg["kb"], SCALE)
-    assert 1 <= _lib.load().fmsa_forward_tiles(pb, 0) <= cfg["s"] // 128
+    assert 1 <= _lib.load().fmsa_forward_tiles(pb, 0, 0) <= cfg["s"] // 128
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     got = ops.attention_forward(q, k, v, qp, kp, SCALE, rix, doc_start=ds, status=status)
     want = ops.attention_forward(q, k, v, qp, kp, SCALE, dataclasses.replace(rix, block_indices=None), doc_start=ds, status=status)
@@ -87,6 +87,27 @@ def test_sinks_in_both_forwards(s, kb):
     yardstick_check("out", out, r32["out"], r16["out"], 2e-3)
     for n, leaf in zip(["dq_proxy", "dk_proxy", "dq", "dk", "dv"], leaves):
         yardstick_check(n, leaf.grad, r32[n], r16[n], 2e-3 * r32[n].abs().max().item())
+
+
+@pytest.mark.parametrize("s,kb,cu", [(8192, 2, list(range(0, 8192, 500)) + [8192]), (8448, 4, [0, 0, 1200, 2400, 3700, 3701, 5000, 6200, 7400, 8448])])
+def test_short_documents(s, kb, cu):
+    """Boundaries that the host knows to be close send all tiles the query-tile stationary way, the same ones in device memory only
+    the first; errors as above."""
+    import flash_msa_b200 as fm
+    cfg = dict(b=2, s=s, hq=8, hkv=2, hp=2, hpkv=1, seed=s)
+    qp, kp, q, k, v, do = bf16_inputs(cfg)
+    res = []
+    for bounds in (cu, torch.tensor(cu, device="cuda")):
+        leaves = [t.detach().requires_grad_(True) for t in (qp, kp, q, k, v)]
+        out, kl = fm.flash_msa_varlen_func(*leaves, bounds, kb * 128, SCALE)
+        torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+        with torch.no_grad():
+            alone, _ = fm.flash_msa_varlen_func(qp, kp, q, k, v, bounds, kb * 128, SCALE)
+        assert torch.equal(alone, out)
+        res.append([out] + [t.grad for t in leaves])
+    assert max_err(res[0][0], res[1][0]) <= 5 * 2.0 ** -9 * v.float().abs().max().item()
+    for n, a, b in zip(["dq_proxy", "dk_proxy", "dq", "dk", "dv"], res[0][1:], res[1][1:]):
+        assert max_err(a, b) <= 2e-2 * b.float().abs().max().item(), n   # (delta is formed from the 16-bit output)
 
 
 def test_rows_that_select_nothing():
