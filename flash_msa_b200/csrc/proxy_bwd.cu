@@ -233,15 +233,30 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
                 }
                 __syncwarp();
                 const float* lse = P.lse_proxy + (static_cast<int64_t>(ud.b) * P.Hp + ud.p) * P.S;
+                // Two dependent loads per row take longer than half a tile: positions are fetched two chunks ahead, the log-sum-exps one.
+                int qid[4], next[4];
+                float nl[4];
+                auto fetch_positions = [&](int chunk) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) next[i] = chunk < ud.chunk1 ? row_qid(ud, chunk * kBlock + 4 * lane + i) : -1;
+                };
+                auto advance = [&](int chunk) {   // to chunk `chunk`
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) qid[i] = next[i];
+                    fetch_positions(chunk + 1);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) nl[i] = qid[i] >= 0 ? lse[qid[i]] : INFINITY;
+                };
+                fetch_positions(ud.chunk0);
+                advance(ud.chunk0);
 #pragma unroll 1
                 for (int chunk = ud.chunk0; chunk < ud.chunk1; ++chunk, ++gt) {
                     const uint32_t s = gt & 1;
-                    float nl[4];
+                    const float4 nl4 = make_float4(-kLog2e * nl[0], -kLog2e * nl[1], -kLog2e * nl[2], -kLog2e * nl[3]);
                     uint32_t lim4 = 0, low4 = 0;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const int q = row_qid(ud, chunk * kBlock + 4 * lane + i);
-                        nl[i] = q >= 0 ? -kLog2e * lse[q] : -INFINITY;
+                        const int q = qid[i];
                         lim4 |= ((q >= 0 && (q >> 7) == ud.j) ? static_cast<uint32_t>(q & 127) : 127u) << (8 * i);
                         if (VARLEN && q >= 0) {
                             const int lo = P.doc_start[static_cast<int64_t>(ud.b) * P.S + q], lb = lo >> 7;
@@ -249,10 +264,11 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
                         }
                     }
                     const bool any_low = VARLEN && __any_sync(0xffffffffu, low4 != 0);
+                    advance(chunk + 1);
                     if (gt >= 2) wait(BAR(sm->st_empty[s]), ((gt >> 1) - 1) & 1);
                     if (bad) break;
                     ProxyRowStats* st = &sm->stats[s];
-                    reinterpret_cast<float4*>(st->neg_lse)[lane] = make_float4(nl[0], nl[1], nl[2], nl[3]);
+                    reinterpret_cast<float4*>(st->neg_lse)[lane] = nl4;
                     reinterpret_cast<uint32_t*>(st->limit)[lane] = lim4;
                     if (VARLEN) {
                         reinterpret_cast<uint32_t*>(st->low)[lane] = low4;
@@ -271,9 +287,11 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
         UnitRec ud;
         for (uint32_t draw = 0; next_unit(draw, ud, std::integral_constant<int, kDraws>{}); ++draw, ++nsub) {
             const int base = ud.b * P.qp_row_b + ud.p * P.qp_row_h;
+            int next = row_qid(ud, ud.chunk0 * kBlock + 32 * g + lane);
 #pragma unroll 1
             for (int chunk = ud.chunk0; chunk < ud.chunk1; ++chunk, ++gt) {
-                const int q = row_qid(ud, chunk * kBlock + 32 * g + lane);
+                const int q = next;
+                if (chunk + 1 < ud.chunk1) next = row_qid(ud, (chunk + 1) * kBlock + 32 * g + lane);
                 int r[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -380,16 +398,33 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
         const int q0 = (warp >> 2) * 64;
         const float2 sc2 = make_float2(P.scale_log2e, P.scale_log2e);
         const float2 nim = make_float2(-P.inv_mpp, -P.inv_mpp);
-        // teacher words of this thread's queries in chunk `chunk` (layout: where the main kernel stores them); 0 beyond the end of the row
+        // teacher words of this thread's queries in chunk `chunk`; 0 beyond the end of the row
         auto load_teacher = [&](const UnitRec& ud, int chunk, uint32_t (&w)[32]) __attribute__((always_inline)) {
             const int64_t slot = ud.e0 - edge_base + static_cast<int64_t>(chunk) * kBlock + q0;
-            const int left = ud.n - chunk * kBlock - q0;
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(P.dqp_part) + slot * 64 + row;
+            int left = ud.n - chunk * kBlock - q0;
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(P.dqp_part) + slot * 64;
+            if (left >= 64) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                w[i] = 0u;
-                if (2 * i + 1 < left) w[i] = src[i * 128];
-                else if (2 * i < left) w[i] = reinterpret_cast<const uint16_t*>(src - row + i * 128)[row];
+                for (int g8 = 0; g8 < 8; ++g8) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(src + g8 * 512 + 4 * row);
+                    w[4 * g8] = v.x; w[4 * g8 + 1] = v.y; w[4 * g8 + 2] = v.z; w[4 * g8 + 3] = v.w;
+                }
+                return;
+            }
+#pragma unroll 1
+            for (int g8 = 0; g8 < 8; ++g8, left -= 8, src += 512) {
+#pragma unroll
+                for (int i = 0; i < 28; ++i) w[i] = w[i + 4];
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (left >= 8) {
+                    v = *reinterpret_cast<const uint4*>(src + 4 * row);
+                } else {
+                    auto pair = [&](int i) -> uint32_t {
+                        return 2 * i + 1 < left ? src[i * 128 + row] : 2 * i < left ? reinterpret_cast<const uint16_t*>(src + i * 128)[row] : 0u;
+                    };
+                    v = make_uint4(pair(0), pair(1), pair(2), pair(3));
+                }
+                w[28] = v.x; w[29] = v.y; w[30] = v.z; w[31] = v.w;
             }
         };
         uint32_t cur[32], nxt[32];

@@ -636,17 +636,23 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
                     warp_arrive(BAR(sm->pds_full[x]));
                     if (KL) {
                         if (hh == hpc - 1) {
-                            // Teacher of the chunk: queries 2i, 2i+1 of the tile as one word per key, so that a pair of edges is 512
-                            // bytes [key][2] and a warp writes 128 consecutive ones; an odd last row of the reverse-index row
-                            // is 256 bytes [key].
+                            // Teacher of the chunk (layout: proxy_bwd.h)
                             const int64_t slot = ud.e0 - edge_base + static_cast<int64_t>(chunk) * kBlock + q0;
-                            const int left = ud.n - chunk * kBlock - q0;   // rows from this thread's first query on
-                            uint32_t* dst = P.teacher + slot * 64 + row;
+                            int left = ud.n - chunk * kBlock - q0;   // rows from this thread's first query on
+                            uint32_t* dst = P.teacher + slot * 64;
+#pragma unroll 1
+                            for (int g8 = 0; g8 < 4; ++g8, left -= 8, dst += 512) {
+                                if (left >= 8) {
+                                    *reinterpret_cast<uint4*>(dst + 4 * row) = *reinterpret_cast<const uint4*>(&teacher[0]);
+                                } else {
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                if (2 * i + 1 < left) dst[i * 128] = *reinterpret_cast<const uint32_t*>(&teacher[i]);
-                                else if (2 * i < left) reinterpret_cast<__half*>(dst - row + i * 128)[row] = __low2half(teacher[i]);
-                                teacher[i] = __floats2half2_rn(0.f, 0.f);
+                                    for (int i = 0; i < 4; ++i) {
+                                        if (2 * i + 1 < left) dst[i * 128 + row] = *reinterpret_cast<const uint32_t*>(&teacher[i]);
+                                        else if (2 * i < left) reinterpret_cast<__half*>(dst + i * 128)[row] = __low2half(teacher[i]);
+                                    }
+                                }
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) teacher[i] = i < 12 ? teacher[i + 4] : __floats2half2_rn(0.f, 0.f);
                             }
                         }
 #pragma unroll
