@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../include/flash_msa_b200.h"
 
 namespace fmsa {
@@ -11,6 +13,24 @@ namespace fmsa {
 inline int check_launch() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FMSA_OK : FMSA_ERR_CUDA;
+}
+
+// Launches a kernel of a pass so that its blocks may take their places, and set up shared and tensor memory, while the last blocks of
+// the kernel before it are still at work ("programmatic dependent launch").  Every such kernel calls wait_for_previous_kernel() before its first
+// access to global memory, so nothing it reads or writes is seen out of order.  (B=3 S=1664 Hq=20 fp16 with sinks, fifteen kernels in a row: REPLACE.)
+template <class... Params, class... Args>
+inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);   // (check_launch reports what goes wrong)
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

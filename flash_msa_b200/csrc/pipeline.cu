@@ -75,7 +75,7 @@ ForwardSpace carve_forward(const fmsa_problem* pb, int dense, int visible, int64
 struct BackwardSpace {
     float *dk, *dv, *dkp;
     int32_t* counters;
-    int64_t zero_bytes;   // dk, dv, dkp and the counters lie in front and are cleared by one memset
+    int64_t zero_bytes;   // dk, dv, dkp and the counters lie in front and are cleared by the delta kernel
     float* delta;
     void *dq_part, *dqp_part;
     int64_t gstep, slots, bytes;
@@ -266,14 +266,13 @@ extern "C" int fmsa_backward(const fmsa_backward_args* a, fmsa_marks* marks, int
     const int64_t tokens = static_cast<int64_t>(pb->B) * pb->S;
     FMSA_REQUIRE(tokens * (pb->Hkv > pb->Hpkv ? pb->Hkv : pb->Hpkv) * 16 < 0xffffffffLL);
     mark(FMSA_STAGE_DELTA);
-    FMSA_TRY(fmsa_bwd_delta(a->out, &a->d_out, w.delta, pb->B, pb->S, pb->Hq, pb->dtype, stream));
+    FMSA_TRY(launch_delta(a->out, &a->d_out, w.delta, pb->B, pb->S, pb->Hq, pb->dtype, a->workspace, w.zero_bytes, st));
     mark(FMSA_STAGE_DELTA);
     ++n;
     if (a->sinks) {
         FMSA_TRY(launch_sink_grad(a->lse, w.delta, a->sinks, a->dsinks, pb->B, pb->S, pb->Hq, st));
         ++n;
     }
-    if (cudaMemsetAsync(a->workspace, 0, static_cast<size_t>(w.zero_bytes), st) != cudaSuccess) return FMSA_ERR_CUDA;
     if (!kl) {   // (the views span their storage exactly: dense (B,H,S,128) or (B,S,H,128))
         if (cudaMemsetAsync(const_cast<void*>(a->dq_proxy.ptr), 0, static_cast<size_t>(tokens * pb->Hp * 256), st) != cudaSuccess ||
             cudaMemsetAsync(const_cast<void*>(a->dk_proxy.ptr), 0, static_cast<size_t>(tokens * pb->Hpkv * 256), st) != cudaSuccess)

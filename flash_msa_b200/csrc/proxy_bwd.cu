@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
         return;
     }
 
+    wait_for_previous_kernel();
     const int64_t edge_base = first_slot(P.units);
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
     auto wait = [&](uint32_t bar, uint32_t parity) {   // every lane of the warp calls it; the result is warp-uniform
@@ -550,7 +551,7 @@ int launch_proxy_bwd(const fmsa_problem* pb, const fmsa_tensor& q_proxy, const f
                                         proxy_bwd_kernel<true, true>};
     const KernelFn kernel = kernels[(pb->dtype == FMSA_DTYPE_FP16 ? 2 : 0) + (pb->doc_start ? 1 : 0)];
     if (!ensure_smem_attr(reinterpret_cast<const void*>(kernel), kProxySmemBytes)) return FMSA_ERR_CUDA;
-    kernel<<<grid, kProxyThreads, kProxySmemBytes, stream>>>(tqp, tkp, P);
+    launch_chained(kernel, grid, kProxyThreads, kProxySmemBytes, stream, tqp, tkp, P);
     return check_launch();
 }
 

@@ -52,6 +52,7 @@ __device__ __forceinline__ void build_bitmap(uint32_t* words, const int32_t* til
 // nothing else (the grid then has those query tiles only).
 __global__ void __launch_bounds__(128) rix_count_kernel(const int32_t* __restrict__ idx, uint8_t* __restrict__ counts, uint4* __restrict__ visits,
                                                         int tiles, int32_t* __restrict__ zero, int nzero, int S, int NB, int Kb) {
+    wait_for_previous_kernel();
     extern __shared__ __align__(16) uint32_t words[];
     const int qblk = blockIdx.x;
     const int64_t bp = blockIdx.y;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(128) rix_count_kernel(const int32_t* __restric
 
 __global__ void rix_colscan_kernel(const uint8_t* __restrict__ counts, int32_t* __restrict__ blk_off,
                                    int32_t* __restrict__ totals, int64_t rows_bh, int NB) {
+    wait_for_previous_kernel();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= rows_bh * NB) return;
     const int64_t bp = t / NB;
@@ -90,6 +92,7 @@ __global__ void rix_colscan_kernel(const uint8_t* __restrict__ counts, int32_t* 
 
 __global__ void __launch_bounds__(1024) rix_rowscan_kernel(const int32_t* __restrict__ totals,
                                                            int32_t* __restrict__ row_ptr, int64_t n, int32_t* __restrict__ zero, int nzero) {
+    wait_for_previous_kernel();
     if (zero)   // words a later kernel of the sequence wants to find zeroed
         for (int i = threadIdx.x; i < nzero; i += 1024) zero[i] = 0;
     __shared__ int64_t part[1024];
@@ -119,6 +122,7 @@ __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict
                                                        const int32_t* __restrict__ row_ptr, int32_t* __restrict__ col_q,
                                                        int32_t* __restrict__ edge_pos, int32_t* __restrict__ row_start, int tiles,
                                                        int S, int NB, int Kb) {
+    wait_for_previous_kernel();
     extern __shared__ __align__(16) uint32_t words[];
     const int qblk = blockIdx.x;
     const int64_t bp = blockIdx.y;
@@ -190,11 +194,11 @@ int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t
     if (!ensure_smem_attr(reinterpret_cast<const void*>(rix_count_kernel), kRixSmemCap) ||
         !ensure_smem_attr(reinterpret_cast<const void*>(rix_fill_kernel), kRixSmemCap))
         return FMSA_ERR_CUDA;
-    rix_count_kernel<<<grid, 128, smem, st>>>(block_indices, w.counts, static_cast<uint4*>(x.visits), x.tiles, nullptr, 0, S, NB, Kb);
+    launch_chained(rix_count_kernel, grid, 128, smem, st, block_indices, w.counts, static_cast<uint4*>(x.visits), x.tiles, static_cast<int32_t*>(nullptr), 0, S, NB, Kb);
     const int64_t cols = rows_bh * NB;
-    rix_colscan_kernel<<<static_cast<unsigned>((cols + 127) / 128), 128, 0, st>>>(w.counts, w.blk_off, w.totals, rows_bh, NB);
-    rix_rowscan_kernel<<<1, 1024, 0, st>>>(w.totals, row_ptr, cols, x.zero, x.nzero);
-    rix_fill_kernel<<<grid, 128, smem, st>>>(block_indices, w.blk_off, row_ptr, col_q, edge_pos, x.row_start, x.tiles, S, NB, Kb);
+    launch_chained(rix_colscan_kernel, static_cast<unsigned>((cols + 127) / 128), 128, 0, st, w.counts, w.blk_off, w.totals, rows_bh, NB);
+    launch_chained(rix_rowscan_kernel, 1, 1024, 0, st, w.totals, row_ptr, cols, x.zero, x.nzero);
+    launch_chained(rix_fill_kernel, grid, 128, smem, st, block_indices, w.blk_off, row_ptr, col_q, edge_pos, x.row_start, x.tiles, S, NB, Kb);
     return check_launch();
 }
 
@@ -203,8 +207,8 @@ int launch_tile_visits(const int32_t* block_indices, int64_t rows_bh, int32_t S,
     const size_t smem = static_cast<size_t>(NB) * 16 + static_cast<size_t>(kBlock) * Kb * sizeof(int32_t);
     if (smem > kRixSmemCap || (reinterpret_cast<uintptr_t>(block_indices) & 15u) != 0) return FMSA_ERR_UNSUPPORTED;
     if (!ensure_smem_attr(reinterpret_cast<const void*>(rix_count_kernel), kRixSmemCap)) return FMSA_ERR_CUDA;
-    rix_count_kernel<<<dim3(static_cast<unsigned>(x.tiles), static_cast<unsigned>(rows_bh)), 128, smem, st>>>(
-        block_indices, nullptr, static_cast<uint4*>(x.visits), x.tiles, x.zero, x.nzero, S, NB, Kb);
+    launch_chained(rix_count_kernel, dim3(static_cast<unsigned>(x.tiles), static_cast<unsigned>(rows_bh)), 128, smem, st,
+        block_indices, static_cast<uint8_t*>(nullptr), static_cast<uint4*>(x.visits), x.tiles, x.zero, x.nzero, S, NB, Kb);
     return check_launch();
 }
 

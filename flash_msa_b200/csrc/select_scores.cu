@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(192) select_scores_kernel(const __grid_constan
     const int b = bp / Hp, p = bp % Hp, kph = p / pg;
     // Blocks before the document of the tile's first row are seen by none of its rows; the list of the fused selection never
     // takes them.  (B=1 S=8192 Hp=8 top-k 16 blocks as five documents: 86 -> 35 us.)
+    wait_for_previous_kernel();
     const int j0 = LK > 0 && doc_start ? min(max(doc_start[static_cast<int64_t>(b) * S + qt * kBlock] >> 7, 0), qt) : 0;
 
     if (tid == 0) {
@@ -217,7 +218,7 @@ int launch_select(const CUtensorMap& tq, const CUtensorMap& tk, float* block_sco
     const size_t smem = 3 * kTileBytes + 1024 + sizeof(ScoreSmem);
     if (!ensure_smem_attr(reinterpret_cast<const void*>(select_scores_kernel<FP16, LK>), smem)) return FMSA_ERR_CUDA;
     const dim3 grid(static_cast<unsigned>(B * Hp), static_cast<unsigned>(NB));
-    select_scores_kernel<FP16, LK><<<grid, 192, smem, st>>>(tq, tk, block_scores, Hp, Hp / Hpkv, S, NB, scale, doc_start,
+    launch_chained(select_scores_kernel<FP16, LK>, grid, 192, smem, st, tq, tk, block_scores, Hp, Hp / Hpkv, S, NB, scale, doc_start,
                                                            block_indices, Kb, status);
     return check_launch();
 }

@@ -20,6 +20,7 @@ __device__ __forceinline__ bool beats(float av, int ai, float bv, int bi) {
 template <int KPL>
 __global__ void __launch_bounds__(256) topk_rows_kernel(const float* __restrict__ scores, int32_t* __restrict__ out,
                                                         int64_t total_rows, int S, int NB, int Kb) {
+    wait_for_previous_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (row >= total_rows) return;
@@ -148,10 +149,10 @@ extern "C" int fmsa_select_topk(const float* block_scores, int32_t* block_indice
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const dim3 g(static_cast<unsigned>(grid));
     if (top_k_blocks <= 32)
-        topk_rows_kernel<1><<<g, 256, 0, st>>>(block_scores, block_indices, total, S, NB, top_k_blocks);
+        launch_chained(topk_rows_kernel<1>, g, 256, 0, st, block_scores, block_indices, total, S, NB, top_k_blocks);
     else if (top_k_blocks <= 64)
-        topk_rows_kernel<2><<<g, 256, 0, st>>>(block_scores, block_indices, total, S, NB, top_k_blocks);
+        launch_chained(topk_rows_kernel<2>, g, 256, 0, st, block_scores, block_indices, total, S, NB, top_k_blocks);
     else
-        topk_rows_kernel<4><<<g, 256, 0, st>>>(block_scores, block_indices, total, S, NB, top_k_blocks);
+        launch_chained(topk_rows_kernel<4>, g, 256, 0, st, block_scores, block_indices, total, S, NB, top_k_blocks);
     return check_launch();
 }

@@ -42,6 +42,10 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     return t;
 }
 
+// Kernels launched by launch_chained (host_common.h): the kernels before this one in its stream have completed and their writes are
+// visible.  All threads call it before their first access to global memory.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------

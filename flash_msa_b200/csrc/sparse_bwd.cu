@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     const uint32_t r2 = tmem + 256, r3 = tmem + 384;   // (Rx = tmem + 128 * x)
 
     const int hpc = P.mpp;   // tiles per chunk
+    wait_for_previous_kernel();
     const int64_t edge_base = first_slot(P.units);
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
 #ifdef FMSA_TRACE
@@ -716,6 +717,7 @@ struct BwdCombineParams {
 // two planes, B=1 S=16384 Hq=24, one head at a time with 8-byte loads took 4.26 ms, groups of six heads 2.48 ms.
 template <int KITER, bool SPLIT, bool FP16, bool GROUPED>   // heads of a group <= 2*KITER: few accumulators, high occupancy (latency bound)
 __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) bwd_combine_kernel(const BwdCombineParams P) {
+    wait_for_previous_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     const int64_t bp0 = static_cast<int64_t>(P.g_begin) * P.ppk;
@@ -832,6 +834,7 @@ template <bool FP16>
 __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                                     int64_t do_sb, int64_t do_ss, int64_t do_sh, float* __restrict__ delta,
                                                     int B, int S, int Hq) {
+    wait_for_previous_kernel();
     extern __shared__ float sdelta[];   // [Hq][8]
     const int lane = threadIdx.x & 31, l16 = lane & 15;
     const int g = threadIdx.x >> 4;   // half-warp 0..15
@@ -907,6 +910,7 @@ __global__ void __launch_bounds__(256) cast_scaled_rows_kernel(const float* __re
 // dsinks[h] = -sum over the rows of head h of exp(sink_h - lse') * delta: one CTA per head, in a fixed order.
 __global__ void __launch_bounds__(512) sink_grad_kernel(const float* __restrict__ lse, const float* __restrict__ delta,
                                                         const float* __restrict__ sinks, float* __restrict__ dsinks, int B, int S, int Hq) {
+    wait_for_previous_kernel();
     __shared__ float part[16];
     const int h = blockIdx.x;
     const float sk = sinks[h];
@@ -929,6 +933,7 @@ __global__ void __launch_bounds__(512) sink_grad_kernel(const float* __restrict_
 // dK, dV and dKp from their fp32 accumulators in one launch (blockIdx.y): 8 elements per thread into (B,H,S,128) views.
 template <bool FP16>
 __global__ void __launch_bounds__(256) cast_grads_kernel(const CastJobs J) {
+    wait_for_previous_kernel();
     const CastJob& c = J.job[blockIdx.y];
     const float f = (c.factor ? *c.factor : 1.f) * c.scale;
     const uint32_t n8 = c.n8, stride = gridDim.x * 256;
@@ -954,13 +959,12 @@ int launch_cast_grads(const CastJobs& jobs, int count, bool fp16, cudaStream_t s
     uint32_t grid = (most + 255) / 256;
     if (grid > 148 * 8) grid = 148 * 8;
     const dim3 g(grid, static_cast<unsigned>(count));
-    if (fp16) cast_grads_kernel<true><<<g, 256, 0, st>>>(jobs);
-    else cast_grads_kernel<false><<<g, 256, 0, st>>>(jobs);
+    launch_chained(fp16 ? cast_grads_kernel<true> : cast_grads_kernel<false>, g, 256, 0, st, jobs);
     return check_launch();
 }
 
 int launch_sink_grad(const float* lse, const float* delta, const float* sinks, float* dsinks, int B, int S, int Hq, cudaStream_t st) {
-    sink_grad_kernel<<<Hq, 512, 0, st>>>(lse, delta, sinks, dsinks, B, S, Hq);
+    launch_chained(sink_grad_kernel, Hq, 512, 0, st, lse, delta, sinks, dsinks, B, S, Hq);
     return check_launch();
 }
 
@@ -996,14 +1000,9 @@ extern "C" int fmsa_bwd_delta(const void* out, const fmsa_tensor* d_out, float* 
     const int64_t grid = static_cast<int64_t>(B) * (S / 8);
     FMSA_REQUIRE(S % 32 == 0 && grid <= 0x7fffffffLL && Hq * 8 * sizeof(float) <= 48 * 1024);
     const size_t smem = static_cast<size_t>(Hq) * 8 * sizeof(float);
-    if (dtype == FMSA_DTYPE_FP16)
-        delta_kernel<true><<<static_cast<unsigned>(grid), 256, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out->ptr), d_out->stride_b, d_out->stride_s,
-        d_out->stride_h, delta, B, S, Hq);
-    else
-        delta_kernel<false><<<static_cast<unsigned>(grid), 256, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out->ptr), d_out->stride_b, d_out->stride_s,
-        d_out->stride_h, delta, B, S, Hq);
+    launch_chained(dtype == FMSA_DTYPE_FP16 ? delta_kernel<true> : delta_kernel<false>, static_cast<unsigned>(grid), 256, smem,
+                   static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out->ptr),
+                   d_out->stride_b, d_out->stride_s, d_out->stride_h, delta, B, S, Hq);
     return check_launch();
 }
 
@@ -1108,7 +1107,7 @@ int fmsa::launch_sparse_bwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     U.g_begin = g_begin; U.dense = dense ? 1 : 0;
     FMSA_REQUIRE(enumerate_subunits(&U.sub, fmsa_fwd_partial_slots(pb, g_count, dense), g_count, U.NB, U.NB, U.ppk, sms));
     const int grid = U.sub.n < sms ? U.sub.n : sms;
-    kernel<<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tdo, tk, tv, P);
+    launch_chained(kernel, grid, kBwdThreads, kBwdSmemBytes, st, tq, tdo, tk, tv, P);
     if (with_kl) {
         if (zero_counters && cudaMemsetAsync(counter_proxy, 0, sizeof(int32_t), st) != cudaSuccess) return FMSA_ERR_CUDA;
         U.counter = counter_proxy;
@@ -1160,11 +1159,11 @@ extern "C" int fmsa_sparse_bwd_combine(const fmsa_problem* pb, const void* dq_pa
 #define FMSA_BWD_COMBINE(K, G)                                                                          \
     do {                                                                                             \
         if (fp16) {                                                                                  \
-            if (P.split) bwd_combine_kernel<K, true, true, G><<<cg, 256, 0, cst>>>(P);             \
-            else bwd_combine_kernel<K, false, true, G><<<cg, 256, 0, cst>>>(P);                    \
+            if (P.split) launch_chained(bwd_combine_kernel<K, true, true, G>, cg, 256, 0, cst, P); \
+            else launch_chained(bwd_combine_kernel<K, false, true, G>, cg, 256, 0, cst, P); \
         } else {                                                                                     \
-            if (P.split) bwd_combine_kernel<K, true, false, G><<<cg, 256, 0, cst>>>(P);            \
-            else bwd_combine_kernel<K, false, false, G><<<cg, 256, 0, cst>>>(P);                   \
+            if (P.split) launch_chained(bwd_combine_kernel<K, true, false, G>, cg, 256, 0, cst, P); \
+            else launch_chained(bwd_combine_kernel<K, false, false, G>, cg, 256, 0, cst, P); \
         }                                                                                            \
     } while (0)
     if (groups > 1) FMSA_BWD_COMBINE(3, true);

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
 
     const int hpc = P.mpp + (P.with_proxy ? 1 : 0);   // tiles per chunk
     const int lse_stride = P.mpp + 1;
+    wait_for_previous_kernel();
     const int64_t edge_base = P.dense ? dense_edge_base(static_cast<int64_t>(P.g_begin) * P.ppk, P.S, P.NB)
                                       : static_cast<int64_t>(P.row_ptr[static_cast<int64_t>(P.g_begin) * P.ppk * P.NB]);
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
@@ -689,6 +690,7 @@ struct CombineRow {
 // proxy log-sum-exp is lowered by log T, which scales the proxy probabilities by T.
 template <int LPR, bool DENSE, bool SINKS>   // LPR lanes per query row: 16 (two rows per warp, at most 16 edges per row) or 32
 __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P) {
+    wait_for_previous_kernel();
     constexpr int kMaxHeads = kWideMaxHeads + 1;
     const int lane = threadIdx.x & 31, l = lane % LPR;
     const int64_t nrows = static_cast<int64_t>(P.G) * P.ppk * (P.S - P.q0);
@@ -756,6 +758,7 @@ __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P)
 // 64-register budget of four CTAs per SM just holds; the group's offsets would spill there (0.34 -> 0.77 ms at Hq/Hp = 4).
 template <int KITER, bool FP16, bool DENSE, bool GROUPED>
 __global__ void __launch_bounds__(256, (KITER <= 2) ? 4 : 2) combine_rows_kernel(const CombineParams P) {
+    wait_for_previous_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (w >= static_cast<int64_t>(P.G) * P.ppk * (P.S - P.q0)) return;
@@ -922,10 +925,10 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
     const int64_t edges = dense ? fmsa_fwd_partial_slots(pb, g_count, 1) : fmsa_fwd_partial_slots(pb, g_count, 0) / P.NB * depth;
     FMSA_REQUIRE(enumerate_subunits(&P.sub, edges, g_count, P.NB, depth, P.ppk, sms));
     const int grid = P.sub.n < sms ? P.sub.n : sms;
-    if (fp16 && varlen) sparse_fwd_kernel<true, true><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
-    else if (fp16) sparse_fwd_kernel<true, false><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
-    else if (varlen) sparse_fwd_kernel<false, true><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
-    else sparse_fwd_kernel<false, false><<<grid, kFwdThreads, kFwdSmemBytes, st>>>(tq, tqp, tk, tv, tkp, to, P);
+    if (fp16 && varlen) launch_chained(sparse_fwd_kernel<true, true>, grid, kFwdThreads, kFwdSmemBytes, st, tq, tqp, tk, tv, tkp, to, P);
+    else if (fp16) launch_chained(sparse_fwd_kernel<true, false>, grid, kFwdThreads, kFwdSmemBytes, st, tq, tqp, tk, tv, tkp, to, P);
+    else if (varlen) launch_chained(sparse_fwd_kernel<false, true>, grid, kFwdThreads, kFwdSmemBytes, st, tq, tqp, tk, tv, tkp, to, P);
+    else launch_chained(sparse_fwd_kernel<false, false>, grid, kFwdThreads, kFwdSmemBytes, st, tq, tqp, tk, tv, tkp, to, P);
     return check_launch();
 }
 
@@ -962,12 +965,12 @@ int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const f
     const dim3 cg(static_cast<unsigned>(grid), static_cast<unsigned>(row_groups));
     const bool half_warps = !dense && P.Kb <= 16;
     const dim3 lg(static_cast<unsigned>(half_warps ? (rows + 15) / 16 : grid), static_cast<unsigned>(lse_groups));
-#define FMSA_LSE(L, D) (sinks ? combine_lse_kernel<L, D, true><<<lg, 256, 0, cst>>>(P) : combine_lse_kernel<L, D, false><<<lg, 256, 0, cst>>>(P))
+#define FMSA_LSE(L, D) (sinks ? launch_chained(combine_lse_kernel<L, D, true>, lg, 256, 0, cst, P) : launch_chained(combine_lse_kernel<L, D, false>, lg, 256, 0, cst, P))
     if (dense) FMSA_LSE(32, true);
     else if (half_warps) FMSA_LSE(16, false);
     else FMSA_LSE(32, false);
 #undef FMSA_LSE
-#define FMSA_ROWS3(K, F, G) (dense ? combine_rows_kernel<K, F, true, G><<<cg, 256, 0, cst>>>(P) : combine_rows_kernel<K, F, false, G><<<cg, 256, 0, cst>>>(P))
+#define FMSA_ROWS3(K, F, G) (dense ? launch_chained(combine_rows_kernel<K, F, true, G>, cg, 256, 0, cst, P) : launch_chained(combine_rows_kernel<K, F, false, G>, cg, 256, 0, cst, P))
 #define FMSA_ROWS(K, G) (f16 ? FMSA_ROWS3(K, true, G) : FMSA_ROWS3(K, false, G))
     if (row_groups > 1) FMSA_ROWS(3, true);
     else if (P.mpp <= 2) FMSA_ROWS(1, false);

@@ -128,7 +128,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
         prefetch_tmap(&tmap_v);
         prefetch_tmap(&tmap_qp);
         prefetch_tmap(&tmap_kp);
-        if (P.zero && blockIdx.x == 0) *P.zero = 0.f;
     }
     if (warp == 0) {
         tmem_alloc(smem_u32(&sm->tmem_slot), 512);
@@ -144,6 +143,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
         if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);
         return;
     }
+
+    wait_for_previous_kernel();
+    if (P.zero && blockIdx.x == 0 && tid == 0) *P.zero = 0.f;
 
     bool bad = false;   // a bounded wait gave up (here or in another role): the thread stops taking work
     auto wait = [&](uint32_t bar, uint32_t parity) {   // every lane of the warp calls it; the result is warp-uniform
@@ -527,6 +529,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
 // One thread per (batch, proxy head, query position).
 __global__ void __launch_bounds__(256) sink_lse_kernel(float* __restrict__ lse, float* __restrict__ lse_proxy, const float* __restrict__ sinks,
                                                        int B, int Hp, int mpp, int S, int rows) {
+    wait_for_previous_kernel();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
     if (t >= static_cast<int64_t>(B) * Hp * rows) return;
     const int q = static_cast<int>(t % rows);
@@ -583,10 +586,10 @@ int launch_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_ten
     const KernelFn kernel = kernels[(fp16 ? 2 : 0) + (varlen ? 1 : 0)];
     if (sms <= 0 || !ensure_smem_attr(reinterpret_cast<const void*>(kernel), kTileSmemBytes)) return FMSA_ERR_CUDA;
     const int grid = P.n_items < sms ? P.n_items : sms;
-    kernel<<<grid, kTileThreads, kTileSmemBytes, st>>>(tq, tk, tv, tqp, tkp, P);
+    launch_chained(kernel, grid, kTileThreads, kTileSmemBytes, st, tq, tk, tv, tqp, tkp, P);
     if (sinks) {
         const int64_t threads = bps * tiles * kBlock;
-        sink_lse_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(lse, lse_proxy, sinks, pb->B, pb->Hp, P.mpp, pb->S, tiles * kBlock);
+        launch_chained(sink_lse_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, st, lse, lse_proxy, sinks, pb->B, pb->Hp, P.mpp, pb->S, tiles * kBlock);
     }
     return check_launch();
 }
