@@ -45,6 +45,9 @@ struct CastJobs {
     uint32_t S;
 };
 int launch_cast_grads(const CastJobs& jobs, int count, bool fp16, cudaStream_t st);
+// delta; `zero`, `zero_bytes`: 16-byte aligned memory to clear on the way (a multiple of 16 bytes), or null and 0.
+int launch_delta(const void* out, const fmsa_tensor* d_out, float* delta, int B, int S, int Hq, int dtype, void* zero, int64_t zero_bytes,
+                 cudaStream_t st);
 int launch_sink_grad(const float* lse, const float* delta, const float* sinks, float* dsinks, int B, int S, int Hq, cudaStream_t st);
 
 // What a whole pass has the reverse index do on the way.
