@@ -51,7 +51,15 @@ int launch_delta(const void* out, const fmsa_tensor* d_out, float* delta, int B,
 int launch_sink_grad(const float* lse, const float* delta, const float* sinks, float* dsinks, int B, int S, int Hq, cudaStream_t st);
 
 // What a whole pass has the reverse index do on the way.
+struct RixWorkspace {       // scratch of the reverse index
+    uint8_t* counts;        // [rows_bh][NB][NB] edges of (query tile, key block)
+    int32_t* blk_off;       // [rows_bh][NB][NB] their offsets inside the reverse-index row
+    int32_t* totals;        // [rows_bh][NB]
+    size_t bytes;
+};
+RixWorkspace carve_reverse_index(void* base, int64_t rows_bh, int NB);
 struct RixExtras {
+    bool counted = false;           // the selection has filled `counts` and `visits` (select_fused_launch)
     void* visits = nullptr;         // [rows_bh][tiles][tiles] 128-bit words: which rows of query tile i selected block j
     int tiles = 0;
     int32_t* row_start = nullptr;   // [rows_bh*NB] position of the first row of a query tile >= tiles in every reverse-index row
@@ -60,8 +68,13 @@ struct RixExtras {
 };
 int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos, int64_t rows_bh,
                          int32_t S, int32_t Kb, void* scratch, cudaStream_t st, const RixExtras& x = RixExtras());
+// The fused selection, and what the first step of the reverse index would read its result for: `counts` (see RixWorkspace) and
+// x.visits, each where not null, and the words x.zero to clear.  `block_indices` null: only those.
+int select_fused_launch(const fmsa_problem* pb, const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, int32_t* block_indices,
+                        uint8_t* counts, const RixExtras& x, int32_t* status, cudaStream_t st);
 // Nothing but `visits` (and the cleared words).
 int launch_tile_visits(const int32_t* block_indices, int64_t rows_bh, int32_t S, int32_t Kb, const RixExtras& x, cudaStream_t st);
+int reverse_index_launches(int64_t rows_bh, int32_t S, const RixExtras& x);   // how many kernels that is
 size_t reverse_index_scratch_bytes(int64_t rows_bh, int32_t S);
 
 }  // namespace fmsa

@@ -157,6 +157,10 @@ extern "C" int fmsa_forward_hinted(const fmsa_forward_args* a, int32_t alone, in
         const int64_t rows = static_cast<int64_t>(pb->B) * pb->Hp;
         FMSA_REQUIRE(rows <= 65535 && rows * pb->S * pb->top_k_blocks < 0x7fffffffLL);
         if (pb->S / 128 > 2048) return FMSA_ERR_UNSUPPORTED;
+        // (the work counters and row_start lie outside the space that the selection's buffers share with the partial rows)
+        RixExtras x;
+        x.visits = w.visits; x.tiles = w.tiles; x.row_start = w.row_start;
+        x.zero = w.counters; x.nzero = w.passes + 1;
         mark(FMSA_STAGE_SELECT);
         if (w.scores) {
             FMSA_TRY(fmsa_select_scores(&a->q_proxy, &a->k_proxy, w.scores, pb->B, pb->Hp, pb->Hpkv, pb->S, pb->scale, pb->dtype,
@@ -164,20 +168,17 @@ extern "C" int fmsa_forward_hinted(const fmsa_forward_args* a, int32_t alone, in
             FMSA_TRY(fmsa_select_topk(w.scores, w.indices, rows, pb->S, pb->top_k_blocks, stream));
             n += 2;
         } else {
-            FMSA_TRY(fmsa_select_fused(&a->q_proxy, &a->k_proxy, w.indices, pb->B, pb->Hp, pb->Hpkv, pb->S, pb->top_k_blocks, pb->scale,
-                                       pb->dtype, pb->doc_start, a->status, stream));
+            x.counted = true;
+            FMSA_TRY(select_fused_launch(pb, &a->q_proxy, &a->k_proxy, index ? w.indices : nullptr,
+                                         index ? carve_reverse_index(w.rix, rows, pb->S / 128).counts : nullptr, x, a->status, st));
             n += 1;
         }
         mark(FMSA_STAGE_SELECT);
         mark(FMSA_STAGE_REVERSE_INDEX);
-        // (the work counters and row_start lie outside the space that the selection's buffers share with the partial rows)
-        RixExtras x;
-        x.visits = w.visits; x.tiles = w.tiles; x.row_start = w.row_start;
-        x.zero = w.counters; x.nzero = w.passes + 1;
         if (index) {
             FMSA_TRY(reverse_index_launch(w.indices, a->row_ptr, a->col_q, a->edge_pos, rows, pb->S, pb->top_k_blocks, w.rix, st, x));
-            n += 4;
-        } else {
+            n += reverse_index_launches(rows, pb->S, x);
+        } else if (!x.counted) {
             FMSA_TRY(launch_tile_visits(w.indices, rows, pb->S, pb->top_k_blocks, x, st));
             n += 1;
         }

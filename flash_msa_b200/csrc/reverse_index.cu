@@ -4,6 +4,7 @@
 // Four small kernels, no global atomics and no host synchronisation:
 //   1. count : one CTA per (batch*proxy head, query block) builds a shared-memory bitmap
 //              "row r selected key block j" and writes the per-(query block, key block) counts;
+//   (2 and 3 in one launch where that is enough; 1 is left to the selection in a whole pass)
 //   2. colscan: one thread per (batch*proxy head, key block) turns the counts of its column into
 //              exclusive offsets over the query blocks and records the column total;
 //   3. rowscan: a single CTA turns the totals into row_ptr;
@@ -118,6 +119,42 @@ __global__ void __launch_bounds__(1024) rix_rowscan_kernel(const int32_t* __rest
     if (tid == 1023) row_ptr[n] = static_cast<int32_t>(part[1023]);
 }
 
+// Both scans in one launch where a single CTA has a thread for every column and the columns are short (B=3 S=1664 Hp=4, 156 columns of
+// 13: the index 15.6 -> 10.7 us, with the count left to the selection).
+constexpr int kRixOneScanCounts = 16384;   // (1024 columns of 64: 39 us for the index instead of 32)
+inline bool one_scan(int64_t cols, int NB) { return cols <= 1024 && cols * NB <= kRixOneScanCounts; }
+__global__ void __launch_bounds__(1024) rix_scan_kernel(const uint8_t* __restrict__ counts, int32_t* __restrict__ blk_off,
+                                                        int32_t* __restrict__ row_ptr, int cols, int NB, int32_t* __restrict__ zero, int nzero) {
+    wait_for_previous_kernel();
+    if (zero)
+        for (int i = threadIdx.x; i < nzero; i += 1024) zero[i] = 0;
+    __shared__ int32_t part[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int run = 0;
+    if (t < cols) {
+        const int bp = t / NB, j = t % NB;
+#pragma unroll 8
+        for (int i = j; i < NB; ++i) {
+            const int at = (bp * NB + i) * NB + j;
+            blk_off[at] = run;
+            run += counts[at];
+        }
+    }
+    // exclusive scan of the totals over the CTA (fewer than 2^31 edges: checked at the entry)
+    int incl = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+    }
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += part[w];
+    if (t < cols) row_ptr[t] = before + incl - run;
+    if (t == cols - 1) row_ptr[cols] = before + incl;
+}
+
 __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ blk_off,
                                                        const int32_t* __restrict__ row_ptr, int32_t* __restrict__ col_q,
                                                        int32_t* __restrict__ edge_pos, int32_t* __restrict__ row_start, int tiles,
@@ -159,14 +196,9 @@ __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict
 
 constexpr size_t kRixSmemCap = 160 * 1024;   // NB <= 2048 and Kb <= 128 need 96 KB; the attribute is set once, to the cap
 
-struct RixWorkspace {
-    uint8_t* counts;
-    int32_t* blk_off;
-    int32_t* totals;
-    size_t bytes;
-};
+}  // namespace
 
-RixWorkspace carve(void* base, int64_t rows_bh, int NB) {
+RixWorkspace carve_reverse_index(void* base, int64_t rows_bh, int NB) {
     RixWorkspace w;
     const size_t n2 = static_cast<size_t>(rows_bh) * NB * NB;
     size_t off = 0;
@@ -180,13 +212,11 @@ RixWorkspace carve(void* base, int64_t rows_bh, int NB) {
     return w;
 }
 
-}  // namespace
-
 // Launch sequence shared with any other entry point that supplies its own scratch memory.
 int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos,
                          int64_t rows_bh, int32_t S, int32_t Kb, void* scratch, cudaStream_t st, const RixExtras& x) {
     const int NB = S / kBlock;
-    const RixWorkspace w = carve(scratch, rows_bh, NB);
+    const RixWorkspace w = carve_reverse_index(scratch, rows_bh, NB);
     const dim3 grid(static_cast<unsigned>(NB), static_cast<unsigned>(rows_bh));
     const size_t smem = static_cast<size_t>(NB) * 16 + static_cast<size_t>(kBlock) * Kb * sizeof(int32_t);
     if (smem > kRixSmemCap || (reinterpret_cast<uintptr_t>(block_indices) & 15u) != 0 || (reinterpret_cast<uintptr_t>(edge_pos) & 15u) != 0)
@@ -194,12 +224,22 @@ int reverse_index_launch(const int32_t* block_indices, int32_t* row_ptr, int32_t
     if (!ensure_smem_attr(reinterpret_cast<const void*>(rix_count_kernel), kRixSmemCap) ||
         !ensure_smem_attr(reinterpret_cast<const void*>(rix_fill_kernel), kRixSmemCap))
         return FMSA_ERR_CUDA;
-    launch_chained(rix_count_kernel, grid, 128, smem, st, block_indices, w.counts, static_cast<uint4*>(x.visits), x.tiles, static_cast<int32_t*>(nullptr), 0, S, NB, Kb);
+    if (!x.counted)
+        launch_chained(rix_count_kernel, grid, 128, smem, st, block_indices, w.counts, static_cast<uint4*>(x.visits), x.tiles, static_cast<int32_t*>(nullptr), 0, S, NB, Kb);
     const int64_t cols = rows_bh * NB;
-    launch_chained(rix_colscan_kernel, static_cast<unsigned>((cols + 127) / 128), 128, 0, st, w.counts, w.blk_off, w.totals, rows_bh, NB);
-    launch_chained(rix_rowscan_kernel, 1, 1024, 0, st, w.totals, row_ptr, cols, x.zero, x.nzero);
+    if (one_scan(cols, NB))
+        launch_chained(rix_scan_kernel, 1, 1024, 0, st, w.counts, w.blk_off, row_ptr, static_cast<int>(cols), NB, x.zero, x.nzero);
+    else
+        launch_chained(rix_colscan_kernel, static_cast<unsigned>((cols + 127) / 128), 128, 0, st, w.counts, w.blk_off, w.totals, rows_bh, NB);
+    if (!one_scan(cols, NB))
+        launch_chained(rix_rowscan_kernel, 1, 1024, 0, st, w.totals, row_ptr, cols, x.zero, x.nzero);
     launch_chained(rix_fill_kernel, grid, 128, smem, st, block_indices, w.blk_off, row_ptr, col_q, edge_pos, x.row_start, x.tiles, S, NB, Kb);
     return check_launch();
+}
+
+int reverse_index_launches(int64_t rows_bh, int32_t S, const RixExtras& x) {
+    const int NB = S / kBlock;
+    return (x.counted ? 0 : 1) + (one_scan(rows_bh * NB, NB) ? 1 : 2) + 1;
 }
 
 int launch_tile_visits(const int32_t* block_indices, int64_t rows_bh, int32_t S, int32_t Kb, const RixExtras& x, cudaStream_t st) {
@@ -213,7 +253,7 @@ int launch_tile_visits(const int32_t* block_indices, int64_t rows_bh, int32_t S,
 }
 
 size_t reverse_index_scratch_bytes(int64_t rows_bh, int32_t S) {
-    return carve(nullptr, rows_bh, S / kBlock).bytes;
+    return carve_reverse_index(nullptr, rows_bh, S / kBlock).bytes;
 }
 
 // -------------------------------------------------------------------------------------------

@@ -18,6 +18,7 @@
 // the top-k kernel (score descending, equal scores by ascending block index, own block first, sentinel NB): a new
 // score goes behind every entry that is at least as large, and the own block is put in front at the end.
 #include "host_common.h"
+#include "launch.h"
 #include "sm100.cuh"
 #include "tma_host.h"
 
@@ -25,6 +26,17 @@ namespace fmsa {
 namespace {
 
 constexpr int kScoreStageCols = 16;   // key blocks staged per flush
+
+// Where the fused selection leaves what the reverse index and the query-tile stationary forward need of it, so that no kernel has to read
+// block_indices for that (see RixExtras).  Selection and index, us: B=2 S=8192 Hp=8 top-k 16 blocks
+// 118 + 32 -> 121 + 27; B=1 S=32768 Hp=8 top-k 64 2009 + 260 -> 2012 + 219; forward of B=1 S=512, now two kernels, 34.3 -> 31.2 a call.
+struct SelectExtras {
+    uint8_t* counts;
+    uint4* visits;
+    int tiles;
+    int32_t* zero;
+    int nzero;
+};
 
 struct ScoreSmem {
     uint64_t q_full, k_full[2], k_empty[2], s_full[2], s_empty[2];
@@ -38,7 +50,7 @@ __global__ void __launch_bounds__(192) select_scores_kernel(const __grid_constan
                                                             float* __restrict__ block_scores, int Hp, int pg, int S,
                                                             int NB, float scale, const int32_t* __restrict__ doc_start,
                                                             int32_t* __restrict__ block_indices, int Kb,
-                                                            int* __restrict__ status) {
+                                                            const SelectExtras X, int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t tile_q = tiles, tile_k0 = tiles + kTileBytes;
@@ -190,13 +202,40 @@ __global__ void __launch_bounds__(192) select_scores_kernel(const __grid_constan
                 __syncwarp();
             }
         }
-        if (LK > 0 && ok) {
+        if (LK > 0) {
             // the row's own block always comes first (flash_msa/tests/testing_model.py:90-94)
             list_insert(INFINITY, qt);
-            int32_t* orow = block_indices + (static_cast<int64_t>(bp) * S + qt * kBlock + r) * Kb;
+            if (block_indices && ok) {
+                int32_t* orow = block_indices + (static_cast<int64_t>(bp) * S + qt * kBlock + r) * Kb;
 #pragma unroll
-            for (int i = 0; i < kList; ++i)
-                if (i < Kb) orow[i] = li[i];
+                for (int i = 0; i < kList; ++i)
+                    if (i < Kb) orow[i] = li[i];
+            }
+            if (X.counts || X.visits) {
+                // words[4 j + w]: rows 32 w .. 32 w + 31 that selected block j.  They lie over the K stages, whose products have completed (or
+                // are left alone after a wait that ran out).
+                const int t = static_cast<int>(threadIdx.x) - 64;   // 0..127
+                uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (tile_k0 - smem_u32(smem_raw)));
+                if (ok)
+                    for (int i = t; i < 4 * (qt + 1); i += 128) words[i] = 0u;
+                named_barrier_sync(1, 128);
+                if (ok) {
+#pragma unroll
+                    for (int i = 0; i < kList; ++i)
+                        if (i < Kb && li[i] <= qt) atomicOr(&words[4 * li[i] + quarter], 1u << lane);
+                }
+                named_barrier_sync(1, 128);
+                if (ok) {
+                    for (int j = t; j <= qt; j += 128) {
+                        const uint4 w = reinterpret_cast<const uint4*>(words)[j];
+                        if (X.counts) X.counts[(static_cast<int64_t>(bp) * NB + qt) * NB + j] =
+                            static_cast<uint8_t>(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w));   // <= 128
+                        if (X.visits && qt < X.tiles) X.visits[(static_cast<int64_t>(bp) * X.tiles + qt) * X.tiles + j] = w;
+                    }
+                    if (qt == 0 && bp == 0)
+                        for (int i = t; i < X.nzero; i += 128) X.zero[i] = 0;
+                }
+            }
         }
     }
     if (!ok) atomicMax(status, kStatusWaitTimeout);
@@ -213,19 +252,19 @@ namespace {
 
 template <bool FP16, int LK>
 int launch_select(const CUtensorMap& tq, const CUtensorMap& tk, float* block_scores, int32_t* block_indices, int B, int Hp,
-                  int Hpkv, int S, int Kb, float scale, const int32_t* doc_start, int32_t* status, cudaStream_t st) {
+                  int Hpkv, int S, int Kb, float scale, const int32_t* doc_start, const SelectExtras& X, int32_t* status, cudaStream_t st) {
     const int NB = S / kBlock;
     const size_t smem = 3 * kTileBytes + 1024 + sizeof(ScoreSmem);
     if (!ensure_smem_attr(reinterpret_cast<const void*>(select_scores_kernel<FP16, LK>), smem)) return FMSA_ERR_CUDA;
     const dim3 grid(static_cast<unsigned>(B * Hp), static_cast<unsigned>(NB));
     launch_chained(select_scores_kernel<FP16, LK>, grid, 192, smem, st, tq, tk, block_scores, Hp, Hp / Hpkv, S, NB, scale, doc_start,
-                                                           block_indices, Kb, status);
+                                                           block_indices, Kb, X, status);
     return check_launch();
 }
 
 int select_common(const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, float* block_scores, int32_t* block_indices,
                   int32_t B, int32_t Hp, int32_t Hpkv, int32_t S, int32_t Kb, float scale, int32_t dtype,
-                  const int32_t* doc_start, int32_t* status, void* stream) {
+                  const int32_t* doc_start, int32_t* status, void* stream, const SelectExtras& X = SelectExtras()) {
     FMSA_REQUIRE(q_proxy && k_proxy && q_proxy->ptr && k_proxy->ptr && status);
     FMSA_REQUIRE(B > 0 && Hp > 0 && Hpkv > 0 && Hp % Hpkv == 0 && S > 0 && S % kBlock == 0);
     FMSA_REQUIRE(dtype == FMSA_DTYPE_BF16 || dtype == FMSA_DTYPE_FP16);
@@ -240,8 +279,8 @@ int select_common(const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, float*
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool fp16 = dtype == FMSA_DTYPE_FP16;
 #define FMSA_SELECT(LKV)                                                                                              \
-    (fp16 ? launch_select<true, LKV>(tq, tk, block_scores, block_indices, B, Hp, Hpkv, S, Kb, scale, doc_start, status, st) \
-          : launch_select<false, LKV>(tq, tk, block_scores, block_indices, B, Hp, Hpkv, S, Kb, scale, doc_start, status, st))
+    (fp16 ? launch_select<true, LKV>(tq, tk, block_scores, block_indices, B, Hp, Hpkv, S, Kb, scale, doc_start, X, status, st) \
+          : launch_select<false, LKV>(tq, tk, block_scores, block_indices, B, Hp, Hpkv, S, Kb, scale, doc_start, X, status, st))
     if (Kb == 0) return FMSA_SELECT(0);
     if (Kb <= 8) return FMSA_SELECT(8);
     if (Kb <= 16) return FMSA_SELECT(16);
@@ -269,4 +308,13 @@ extern "C" int fmsa_select_fused(const fmsa_tensor* q_proxy, const fmsa_tensor* 
     if (top_k_blocks > FMSA_FUSED_SELECT_MAX_BLOCKS) return FMSA_ERR_UNSUPPORTED;
     return select_common(q_proxy, k_proxy, nullptr, block_indices, B, Hp, Hpkv, S, top_k_blocks, scale, dtype, doc_start, status,
                          stream);
+}
+
+int fmsa::select_fused_launch(const fmsa_problem* pb, const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, int32_t* block_indices,
+                              uint8_t* counts, const RixExtras& x, int32_t* status, cudaStream_t st) {
+    FMSA_REQUIRE(pb->top_k_blocks >= 1 && pb->top_k_blocks <= pb->S / kBlock && pb->S / kBlock <= kTileBytes / 8);   // (the bit map)
+    if (pb->top_k_blocks > FMSA_FUSED_SELECT_MAX_BLOCKS) return FMSA_ERR_UNSUPPORTED;
+    const SelectExtras X = {counts, static_cast<uint4*>(x.visits), x.tiles, x.zero, x.nzero};
+    return select_common(q_proxy, k_proxy, nullptr, block_indices, pb->B, pb->Hp, pb->Hpkv, pb->S, pb->top_k_blocks, pb->scale, pb->dtype,
+                         pb->doc_start, status, st, X);
 }
