@@ -122,6 +122,13 @@ inline bool enumerate_subunits(SubUnits* U, int64_t edges, int64_t groups, int N
     if (fine > groups) fine = groups;
     constexpr int64_t kMost = 0x7f000000LL;
     if (subunits_per_group(NB, depth, ppk, U->chunks_tail) * groups >= kMost) fine = 0;
+    // (As above, they stay coarser where there would be too many to draw: B=4 S=3968 Hq=16 top-k 2 blocks 735 -> 717 us, B=1 S=41216 Hq=32
+    // top-k 3 2993 -> 2907.  A limit of 64 per CTA has the former at 754 and the latter as it is.)
+    while (fine > 0 && subunits_per_group(NB, depth, ppk, U->chunks) * (groups - fine) + subunits_per_group(NB, depth, ppk, U->chunks_tail) * fine >
+                           static_cast<int64_t>(kDrawsPerCta) * sms) {
+        U->chunks_tail *= 2;
+        if (U->chunks_tail >= U->chunks) fine = 0;
+    }
     U->groups_bulk = static_cast<int32_t>(groups - fine);
     const int64_t pg = subunits_per_group(NB, depth, ppk, U->chunks), pt = subunits_per_group(NB, depth, ppk, U->chunks_tail);
     if (pg * (groups - fine) + pt * fine >= kMost) return false;
@@ -158,6 +165,26 @@ __device__ __forceinline__ SubUnit decode_subunit(uint32_t u, const SubUnits& U)
     return su;
 }
 
+// The first sub-unit from `u` on that has work if it lies in u's group, else the first one of the next group; a warp's job, and every lane
+// gets the result.  One look at the lengths of the rows finds it: a row can have work in u's sweep, at a place not before u's, or else in the
+// next one (work in a later sweep means work in this one too).
+template <class RowLength>
+__device__ __forceinline__ uint32_t next_subunit(uint32_t u, const SubUnits& U, int g_begin, RowLength&& row_length) {
+    const SubUnit su = decode_subunit(u, U);
+    const uint32_t lane = threadIdx.x & 31, ppk = U.ppk, g = g_begin + su.g;
+    const uint32_t here = su.j * ppk + su.pp, rows = (U.NB - su.chunk0) * ppk;   // u's place in its sweep, and the sweep's size
+    const uint32_t group_end = u < U.n_bulk ? (su.g + 1) * U.per_group : U.n_bulk + (su.g + 1 - U.groups_bulk) * U.per_group_tail;
+    uint32_t best = group_end - (u - here);   // from the beginning of u's sweep
+#pragma unroll 4
+    for (uint32_t i = lane; i < rows; i += 32) {
+        const uint32_t j = i / ppk;
+        const int chunks = (row_length((g * ppk + (i - j * ppk)) * U.NB + j) + kBlock - 1) / kBlock;
+        if (chunks > su.chunk0 && i >= here) best = min(best, i);
+        else if (chunks > su.chunk0 + su.chunks) best = min(best, rows + i);
+    }
+    return u - here + __reduce_min_sync(0xffffffffu, best);
+}
+
 // What a launch needs to enumerate its sub-units; a member of the parameters of the backward kernels.
 struct UnitSpace {
     const int32_t* row_ptr;
@@ -178,8 +205,11 @@ struct UnitRec {
 // lane 0 keeps what it fetched.  When the drawn one lies beyond the end of its row the lanes have looked at the 31 behind
 // it as well, and the counter moves past those of them that are empty too.  (With a draw for each empty one, about half of
 // them at B=2 S=8192 Hq=32 top-k 16 blocks: forward 0.674 -> 0.669 ms, backward kernels 1.539 -> 1.527 ms.)
-template <class Load>
-__device__ __forceinline__ bool draw_work(int32_t* counter, uint32_t n_subunits, Load&& load) {
+// Where all 32 are empty it moves on to `next(u)`: the windows of the CTAs overlap, so with a few blocks selected from a long sequence
+// they spent most of the time on passing over empty sub-units, each round for a few dozen (B=1 S=52736 Hq=12 top-k 2 blocks, six
+// documents: forward 816 -> 247 us, backward kernels 1585 -> 433; B=1 S=65536 Hq=8 top-k 32: 1605 -> 1560, 3445 -> 3388).
+template <class Load, class Next>
+__device__ __forceinline__ bool draw_work(int32_t* counter, uint32_t n_subunits, Load&& load, Next&& next) {
     const uint32_t lane = threadIdx.x & 31;
     for (;;) {
         uint32_t u = 0;
@@ -189,7 +219,8 @@ __device__ __forceinline__ bool draw_work(int32_t* counter, uint32_t n_subunits,
         const bool has = u + lane < n_subunits && load(u + lane);
         const uint32_t work = __ballot_sync(0xffffffffu, has);
         if (work & 1u) return true;
-        if (lane == 0) atomicMax(counter, static_cast<int32_t>(u + (work ? __ffs(work) - 1 : 32)));
+        const uint32_t to = work ? u + __ffs(work) - 1 : max(u + 32, next(u));
+        if (lane == 0) atomicMax(counter, static_cast<int32_t>(to));
     }
 }
 
@@ -215,6 +246,8 @@ __device__ __forceinline__ UnitRec draw_subunit(const UnitSpace& U) {
         nu.chunk0 = static_cast<uint16_t>(su.chunk0);
         nu.chunk1 = static_cast<int16_t>(min((n + kBlock - 1) / kBlock, su.chunk0 + su.chunks));
         return su.chunk0 * kBlock < n;
+    }, [&](uint32_t u) -> uint32_t {
+        return next_subunit(u, U.sub, U.g_begin, [&](uint32_t row) { return U.row_ptr[row + 1] - U.row_ptr[row]; });
     });
     if (!more) nu.chunk1 = -1;
     return nu;

@@ -258,6 +258,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
                 nu.chunk0 = su.chunk0;
                 nu.chunk1 = min((n + kBlock - 1) / kBlock, su.chunk0 + su.chunks);
                 return su.chunk0 * kBlock < n;
+            }, [&](uint32_t u) -> uint32_t {
+                return next_subunit(u, P.sub, P.g_begin, [&](uint32_t row) { return P.row_ptr[row + 1] - (P.row_start ? P.row_start : P.row_ptr)[row]; });
             });
             if (!more) nu.chunk1 = -1;
             if (lane == 0) {

@@ -28,3 +28,23 @@ def test_one_pass_against_a_pass_per_group(monkeypatch, b, s, kb, docs):
     for n, a, c in zip(["out", "dq_proxy", "dk_proxy", "dq", "dk", "dv"], *res):
         # (the order in which sub-units add to dK, dV and dKp is free: the last bit of the 16-bit result)
         assert max_err(a, c) <= (0.0 if n in ("out", "dq", "dq_proxy") else 2 ** -7 * c.float().abs().max().item()), n
+
+
+@pytest.mark.parametrize("b,s,hkv,kb,docs", [(1, 12544, 2, 2, True), (2, 12544, 1, 3, False), (1, 33024, 1, 1, False)])
+def test_few_blocks_of_a_long_sequence(b, s, hkv, kb, docs):
+    """Most sub-units lie beyond the end of their rows, more than the 32 that a draw looks at.  With values and dO of one every output is
+    one, and a (batch, KV head)'s dV sums to its number of query rows; a chunk left out or taken twice would move that by more than
+    64 / s >= 2^-9 of it.  Rounded weights and results, each off by 2^-9 at most and in no direction, move the sum of 128 kb terms per row
+    and s rows by 2^-9 / sqrt(s) of it."""
+    import flash_msa_b200 as fm
+    (qp, kp, q, k, v), do = (lambda x: (x[:-1], x[-1]))(bf16_inputs(dict(b=b, s=s, hq=2 * hkv, hkv=hkv, hp=hkv, hpkv=hkv, seed=s + kb)))
+    leaves = [t.detach().requires_grad_(True) for t in (qp, kp, q, k, torch.ones_like(v))]
+    if docs:
+        out, kl = fm.flash_msa_varlen_func(*leaves, [0, s // 3, s // 2 + 5, s], kb * 128, SCALE)
+    else:
+        out, kl = fm.flash_msa_func(*leaves, kb * 128, SCALE)
+    out.backward(torch.ones_like(do))
+    # weights and partial outputs rounded to 16 bits, 2^-9 each, then the result, half of bf16's step of 2^-7 above one: 2^-7
+    assert (out.float() - 1).abs().max().item() <= 2 ** -7
+    total = leaves[4].grad.double().sum(-2 if leaves[4].shape[2] == s else 1)
+    assert (total / (2 * s) - 1).abs().max().item() <= 2 ** -11
