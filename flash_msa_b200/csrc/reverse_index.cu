@@ -183,7 +183,9 @@ __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict
             int rank = __popc(words[j * 4 + w] & below);
             for (int ww = 0; ww < w; ++ww) rank += __popc(words[j * 4 + ww]);
             pos = rp[j] + bo[j] + rank;
-            col_q[pos] = q;
+            // (inside the row wherever the counts are those of these selections; no other index may lead out of col_q)
+            if (pos < rp[j + 1]) col_q[pos] = q;
+            else pos = -1;
         }
         row[at] = pos;
     }

@@ -41,6 +41,7 @@ struct SelectExtras {
 struct ScoreSmem {
     uint64_t q_full, k_full[2], k_empty[2], s_full[2], s_empty[2];
     uint32_t tmem_slot;
+    int32_t gave_up;   // a wait of a warp that owns rows ran out
     float stage[128][kScoreStageCols + 1];
 };
 
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(192) select_scores_kernel(const __grid_constan
             mbar_init(smem_u32(&sm->s_full[i]), 1);
             mbar_init(smem_u32(&sm->s_empty[i]), 128);
         }
+        sm->gave_up = 0;
         fence_mbar_init();
         prefetch_tmap(&tmap_q);
         prefetch_tmap(&tmap_k);
@@ -146,8 +148,8 @@ __global__ void __launch_bounds__(192) select_scores_kernel(const __grid_constan
         };
         for (int j = j0; j <= qt; ++j) {
             const int st = (j - j0) & 1;
-            ok = mbar_wait(smem_u32(&sm->s_full[st]), ((j - j0) >> 1) & 1);
-            if (!ok) break;   // every lane of the warp waits on the same phase: uniform
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sm->s_full[st]), ((j - j0) >> 1) & 1));
+            if (!ok) break;   // (the whole warp, also when a limit ran out in some of its lanes only)
             tc_fence_after_sync();
             // The factor `scale` is positive, so it is applied once to the row maximum instead of to every logit
             // (rounding is monotone: the result is the same bit for bit).  Only the diagonal block needs the causal
@@ -205,40 +207,48 @@ __global__ void __launch_bounds__(192) select_scores_kernel(const __grid_constan
         if (LK > 0) {
             // the row's own block always comes first (flash_msa/tests/testing_model.py:90-94)
             list_insert(INFINITY, qt);
-            if (block_indices && ok) {
+            // words[4 j + w]: rows 32 w .. 32 w + 31 that selected block j.  They lie over the K stages, whose products have completed (or
+            // are left alone after a wait that ran out).
+            const int t = static_cast<int>(threadIdx.x) - 64;   // 0..127
+            uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (tile_k0 - smem_u32(smem_raw)));
+            const bool extras = X.counts || X.visits;
+            if (!ok) sm->gave_up = 1;
+            else if (extras)
+                for (int i = t; i < 4 * (qt + 1); i += 128) words[i] = 0u;
+            named_barrier_sync(1, 128);
+            // A tile that could not be finished selects nothing, in its indices and in what is counted from them alike: the kernels behind
+            // this one size and place the reverse index by the counts.
+            const bool whole = sm->gave_up == 0;
+            if (block_indices) {
                 int32_t* orow = block_indices + (static_cast<int64_t>(bp) * S + qt * kBlock + r) * Kb;
 #pragma unroll
                 for (int i = 0; i < kList; ++i)
-                    if (i < Kb) orow[i] = li[i];
+                    if (i < Kb) orow[i] = whole ? li[i] : NB;
             }
-            if (X.counts || X.visits) {
-                // words[4 j + w]: rows 32 w .. 32 w + 31 that selected block j.  They lie over the K stages, whose products have completed (or
-                // are left alone after a wait that ran out).
-                const int t = static_cast<int>(threadIdx.x) - 64;   // 0..127
-                uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (tile_k0 - smem_u32(smem_raw)));
-                if (ok)
-                    for (int i = t; i < 4 * (qt + 1); i += 128) words[i] = 0u;
-                named_barrier_sync(1, 128);
-                if (ok) {
+            if (extras) {
+                if (whole) {
 #pragma unroll
                     for (int i = 0; i < kList; ++i)
                         if (i < Kb && li[i] <= qt) atomicOr(&words[4 * li[i] + quarter], 1u << lane);
                 }
                 named_barrier_sync(1, 128);
-                if (ok) {
-                    for (int j = t; j <= qt; j += 128) {
-                        const uint4 w = reinterpret_cast<const uint4*>(words)[j];
-                        if (X.counts) X.counts[(static_cast<int64_t>(bp) * NB + qt) * NB + j] =
-                            static_cast<uint8_t>(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w));   // <= 128
-                        if (X.visits && qt < X.tiles) X.visits[(static_cast<int64_t>(bp) * X.tiles + qt) * X.tiles + j] = w;
-                    }
-                    if (qt == 0 && bp == 0)
-                        for (int i = t; i < X.nzero; i += 128) X.zero[i] = 0;
+                for (int j = t; j <= qt; j += 128) {
+                    const uint4 w = whole ? reinterpret_cast<const uint4*>(words)[j] : make_uint4(0, 0, 0, 0);
+                    if (X.counts) X.counts[(static_cast<int64_t>(bp) * NB + qt) * NB + j] =
+                        static_cast<uint8_t>(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w));   // <= 128
+                    if (X.visits && qt < X.tiles) X.visits[(static_cast<int64_t>(bp) * X.tiles + qt) * X.tiles + j] = w;
                 }
             }
+            if (qt == 0 && bp == 0)
+                for (int i = t; i < X.nzero; i += 128) X.zero[i] = 0;
         }
     }
-    if (!ok) atomicMax(status, kStatusWaitTimeout);
+    if (!ok) {
+        atomicMax(status, kStatusWaitTimeout);
+        // Give loads and products that are still in flight time to finish before shared memory and TMEM are released.
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 200000) __nanosleep(1000);
+    }
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 256);
