@@ -265,6 +265,28 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a, uint32_t b_
             : "memory");
 }
 
+// The same where the rows (TMEM lanes) set in `off` keep what D holds: their A is not looked at, so that nothing - not the NaN of
+// 0 * Inf either - reaches them.
+template <int STEPS, int ASTRIDE, bool FP16>
+__device__ __forceinline__ void umma_ts_rows(uint32_t d_tmem, uint32_t a, uint32_t b_tile, bool accumulate, uint4 off) {
+    constexpr uint32_t idesc = umma_idesc(128, false, true, FP16);
+    const uint64_t b0 = desc_mnmajor(b_tile, 0);
+    const uint32_t b_lo = static_cast<uint32_t>(b0), b_hi = static_cast<uint32_t>(b0 >> 32);
+#pragma unroll
+    for (int ks = 0; ks < STEPS; ++ks)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            ".reg .b64 b;\n"
+            "mov.b64 b, {%2, %3};\n"
+            "setp.ne.b32 p, %5, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, {%6, %7, %8, %9}, p;\n"
+            "}\n" ::"r"(d_tmem),
+            "r"(a + ASTRIDE * ks), "r"(b_lo + umma_kstep(true, ks)), "r"(b_hi), "r"(idesc), "r"(ks > 0 || accumulate ? 1u : 0u),
+            "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w)
+            : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMEM loads: warp w of a warpgroup reads lanes 32*(w%4)..+31; thread i gets lane 32*(w%4)+i
 // and 32 consecutive fp32 columns.

@@ -9,8 +9,9 @@
 //
 // Work item = (batch, query tile, main head), or (batch, query tile, proxy head), which needs the log-sum-exp only.  Persistent CTAs
 // draw items from a global counter, longest first.  A step of an item is one visited block: S = Q K_j^T into one of three S buffers in
-// TMEM, P = exp2(S*c - m) over it (16 bit), O += P V_j.  Roles (warp index): 0-3 and 4-7 two softmax groups on alternating steps, 8 tile
-// loads, 9 issue of S, 10 draws the items and lists the blocks they visit, 11 issue of P V.
+// TMEM, P = exp2(S*c - m) over it (16 bit), O += P V_j in the lanes of the rows that selected the block (leaving the others' lanes out,
+// instead of multiplying zeros, keeps a value that is not finite away from them).  Roles (warp index): 0-3 and 4-7 two softmax groups on
+// alternating steps, 8 tile loads, 9 issue of S, 10 draws the items and lists the blocks they visit, 11 issue of P V.
 // TMEM: S buffer n at columns 128 n (P over its first 64), O at 384.
 //
 // B=4 S=4096 Hq=32 dense, with the proxy heads: 0.607 ms against 0.767 + 0.492 ms of the key-block stationary kernel and its combine;
@@ -70,6 +71,7 @@ struct TileCtrl {
     uint16_t block[kTileRing][kTileFwdMaxBlocks];             // the visited blocks, descending
     float top[128];                                           // running maximum of every row (log2 domain)
     float2 part[2][128];                                      // [group] (max, sum) at the end of an item
+    alignas(16) uint32_t off[kTileBuffers][4];                // per S buffer: the rows that did not select the step's block
     uint32_t tmem_slot;
 };
 constexpr size_t kTileFwdTileBytes = static_cast<size_t>(1 + kTileKvStages) * kTileBytes;
@@ -294,11 +296,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                         wait1(BAR(sm->kv_full[st]), ph);
                         if (bad) break;
                         tc_fence_after_sync();
-                        umma_ts<4, 8, FP16>(tmem_o, sbuf, at, t > 0);   // O += P V_j
+                        const uint4 off = *reinterpret_cast<const uint4*>(sm->off[buf]);
+                        // O += P V_j; where the first block is not every row's, O has been cleared
+                        umma_ts_rows<4, 8, FP16>(tmem_o, sbuf, at, t > 0 || (off.x | off.y | off.z | off.w) != 0, off);
                         wait1(BAR(sm->p_full[buf][1]), bph);
                         if (bad) break;
                         tc_fence_after_sync();
-                        umma_ts<4, 8, FP16>(tmem_o, sbuf + 32, at + kHalfRowBytes, true);
+                        umma_ts_rows<4, 8, FP16>(tmem_o, sbuf + 32, at + kHalfRowBytes, true, off);
                         umma_commit(BAR(sm->pv_done[buf]));
                         umma_commit(BAR(sm->kv_empty[st]));
                         skip(t + kTileBuffers < steps ? 2 : 1);
@@ -347,10 +351,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                     const uint32_t word = P.visits ? reinterpret_cast<const uint32_t*>(&sm->rows[slot][t])[quarter]
                                                    : (VARLEN ? __ballot_sync(0xffffffffu, (lo >> 7) <= j) : 0xffffffffu);
                     const bool sel = word >> lane & 1;
+                    bool clear = false;   // the first block is not every row's (not from a selection): such rows start from zeros
+                    if (P.visits && t == 0 && !px) {
+                        const uint4 w = sm->rows[slot][0];
+                        clear = (w.x & w.y & w.z & w.w) != 0xffffffffu;
+                    }
                     const int lowc = VARLEN && (lo >> 7) == j ? lo & 127 : 0;   // first visible key inside the block
                     wait(BAR(sm->s_full[buf]), bph);
                     if (bad) break;
                     tc_fence_after_sync();
+                    if (lane == 0) sm->off[buf][quarter] = ~word;   // (the product that read the buffer's last ones has completed)
                     if (j == diag || (VARLEN && __any_sync(0xffffffffu, lowc > 0))) {   // the causal edge, or the start of the row's document:
                         const int limit = j == diag ? row : 127;                        // hidden logits become -inf
 #pragma unroll 1
@@ -416,7 +426,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                     }
                     const float nm = m == -INFINITY ? 0.f : -m;   // (a row that has not selected anything yet)
                     const float2 nm2 = make_float2(nm, nm);
-                    const uint32_t keep = sel ? 0xffffffffu : 0u;
                     float2 l2a = make_float2(0.f, 0.f), l2b = make_float2(0.f, 0.f);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
@@ -431,18 +440,20 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                             pk[y >> 1] = pack_act<FP16>(pa.x, pa.y);
                             pk[(y >> 1) + 1] = pack_act<FP16>(pb.x, pb.y);
                         }
-                        if (!px) {
-                            if (word != 0xffffffffu) {
-#pragma unroll
-                                for (int y = 0; y < 16; ++y) pk[y] &= keep;
-                            }
-                            tmem_st16(tmem_addr(ts, quarter, 16 * c), pk);
-                        }
+                        if (!px) tmem_st16(tmem_addr(ts, quarter, 16 * c), pk);
                         if (c & 1) {
+                            // the first product of an item overwrites O: the rows of the item before must have been read
+                            if (c == 1 && t == 0) {
+                                if (draw > 0) wait(BAR(sm->o_free), (draw - 1) & 1);
+                                if (clear) {
+                                    tc_fence_after_sync();
+                                    const uint32_t zero[16] = {};
+#pragma unroll 1
+                                    for (int o = 0; o < 128; o += 16) tmem_st16(tmem_addr(tmem_o, quarter, o), zero);
+                                }
+                            }
                             if (!px) tmem_st_wait();
                             tc_fence_before_sync();
-                            // the first product of an item overwrites O: the rows of the item before must have been read
-                            if (c == 1 && t == 0 && draw > 0) wait(BAR(sm->o_free), (draw - 1) & 1);
                             warp_arrive(BAR(sm->p_full[buf][c >> 1]));
                         }
                     }
