@@ -81,6 +81,14 @@ static_assert(kTileSmemBytes <= 232448, "shared memory budget of one CTA");
 // Rows whose maximum grows by less than this (log2) keep the old one: P is then at most 256 times larger than with the
 // new one, the sum is the same, and O need not be rescaled.
 constexpr float kLazyRescale = 8.f;
+// fp16 P (and with it O and the sum) are 2^7 times larger, at most 2^15, so that the P of a block far below the row's maximum become
+// subnormal later.  (The key-block stationary forward takes P relative to the block's own maximum.  One dominant key of value zero in the
+// block visited first, S=4096, 12 / 14 / 16 / 18 nats above N(0,1) logits, error of the row against 64 bits: 2.9e-4 / 2.9e-4 / 4.9e-4 /
+// 3.2e-3; without the factor 1.0e-3 / 7.5e-3 / 5.7e-2 / 0.38; in the key-block stationary forward 3.9e-4 / 1.4e-3 / 1.0e-2 / 6.6e-2.  That one
+// is the better one beyond 22 nats, where such a row of values up to 256 is below fp16's normal numbers itself.  2^11 with a limit of 2^4
+// moves this to 25 nats and rescales more often: forward of B=1 S=16384 Hq=24 top-k 96, logits of four times the width, 1.96 -> 2.11 ms.)
+template <bool FP16>
+constexpr float kLiftP = FP16 ? 7.f : 0.f;
 
 // K and V tiles pass through one ring in the order in which they are needed: K_0 K_1 K_2 V_0 K_3 V_1 .. (proxy head: K_0 K_1 ..).
 //   S thread      S of a step, behind the completion of the P V that read P from the same buffer three steps before (products are only
@@ -424,7 +432,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                             tmem_st16(tmem_addr(tmem_o, quarter, c), o);
                         }
                     }
-                    const float nm = m == -INFINITY ? 0.f : -m;   // (a row that has not selected anything yet)
+                    const float nm = m == -INFINITY ? 0.f : kLiftP<FP16> - m;   // (a row that has not selected anything yet)
                     const float2 nm2 = make_float2(nm, nm);
                     float2 l2a = make_float2(0.f, 0.f), l2b = make_float2(0.f, 0.f);
 #pragma unroll
@@ -481,13 +489,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
                 const float2 a = sm->part[other][row];
                 // (maxima only rise: this group's is the latest)
                 l += a.x == -INFINITY ? 0.f : a.y * fast_exp2(a.x - m);
-                const float lse = l > 0.f ? (m + __log2f(l)) * kLn2 : (l == 0.f ? -INFINITY : l);   // (a NaN stays one)
+                const float lse = l > 0.f ? (m + (__log2f(l) - kLiftP<FP16>)) * kLn2 : (l == 0.f ? -INFINITY : l);   // (a NaN stays one)
                 if (px) {
                     P.lse_proxy[(static_cast<int64_t>(it.b) * P.Hp + it.p) * P.S + q] = lse;
                 } else {
                     const int head = it.p * P.mpp + it.h;
                     P.lse[(static_cast<int64_t>(it.b) * P.Hq + head) * P.S + q] = lse;
-                    if (P.sinks) l += fast_exp2(P.sinks[head] * kLog2e - (m == -INFINITY ? 0.f : m));
+                    if (P.sinks) l += fast_exp2(P.sinks[head] * kLog2e + (m == -INFINITY ? 0.f : kLiftP<FP16> - m));
                     const float inv = l == 0.f ? 0.f : 1.f / l;
                     const float2 inv2 = make_float2(inv, inv);
                     wait(BAR(sm->pv_done[last]), last_ph);

@@ -124,3 +124,41 @@ def test_rows_that_select_nothing():
     heads = out.view(1, 512, 4, 128).transpose(1, 2)
     assert (heads[rows] == 0).all() and torch.isneginf(lse[rows]).all() and torch.isneginf(lse_p[none]).all()
     assert torch.isfinite(lse[~rows]).all() and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("sinks", [False, True])
+@pytest.mark.parametrize("gap", [-5.7, -5.4, 12.0, 14.0, 16.0])
+def test_fp16_probabilities_far_below_the_maximum(gap, sinks):
+    """One key of the block visited first lies `gap` above the N(0,1) logits of the others and has a value of zero, so that the rows of
+    that tile are sums of small probabilities; the other way round (-5.4, 7.8 in the log2 domain, and -5.7), all of the second block
+    just below and above the line at which O is rescaled.  Independent roundings of P, normal (2^-11) or of the subnormals below 2^-21 of the
+    maximum (2^-25 at most, against a root mean square of e 2^-16 at a gap of 16: 4e-4), and of the result (2^-11) add up to less than
+    1e-3 in the 2-norm."""
+    import flash_msa_b200 as fm
+    s, h = 4096, 2
+    g = torch.Generator().manual_seed(21)
+    qp, kp = (torch.randn(1, 1, s, 128, generator=g).half().cuda() for _ in range(2))
+    q, k, v = (torch.randn(1, h, s, 128, generator=g) for _ in range(3))
+    v *= 256   # (no subnormal results)
+    q[..., 0], k[..., 0] = 4.0, 0.0
+    if gap > 0:
+        k[:, :, s - 128] = 0
+        k[:, :, s - 128, 0] = gap / (4.0 * SCALE)
+        v[:, :, s - 128] = 0
+    else:
+        k.zero_()
+        k[:, :, s - 256:s - 128, 0] = -gap / (4.0 * SCALE)
+    q, k, v = (t.half().cuda() for t in (q, k, v))
+    bias = torch.tensor([2.0, gap + 1.0], device="cuda") if sinks else None
+    with torch.no_grad():
+        out, _ = fm.flash_msa_warmup_func(qp, kp, q, k, v, s, SCALE, sinks=bias)
+    rows = slice(s - 128, s)
+    logits = q[:, :, rows].double() @ k.double().transpose(2, 3) * SCALE
+    hidden = torch.arange(s, device="cuda") > torch.arange(s - 128, s, device="cuda").view(-1, 1)
+    logits = logits.masked_fill(hidden, -torch.inf)
+    norm = logits.logsumexp(-1, keepdim=True)
+    if sinks:
+        norm = torch.logaddexp(norm, bias.double().view(1, h, 1, 1))
+    want = (logits - norm).exp() @ v.double()
+    got = out.view(1, s, h, 128).transpose(1, 2)[:, :, rows].double()
+    assert ((got - want).norm(dim=(2, 3)) / want.norm(dim=(2, 3))).max() < 1e-3
