@@ -196,6 +196,20 @@ __global__ void __launch_bounds__(128) rix_fill_kernel(const int32_t* __restrict
     for (int t = threadIdx.x; t < kBlock * Kb / 4; t += blockDim.x) dst[t] = src[t];
 }
 
+// Where query tiles first_tile .. begin in every row, for an index that was built without (one thread per row).
+__global__ void __launch_bounds__(128) rix_row_start_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ col_q,
+                                                            int32_t* __restrict__ row_start, int64_t rows, int q0) {
+    const int64_t r = static_cast<int64_t>(blockIdx.x) * 128 + threadIdx.x;
+    if (r >= rows) return;
+    int lo = row_ptr[r], hi = row_ptr[r + 1];   // query positions ascend inside a row
+    while (lo < hi) {
+        const int mid = lo + (hi - lo) / 2;
+        if (col_q[mid] < q0) lo = mid + 1;
+        else hi = mid;
+    }
+    row_start[r] = lo;
+}
+
 constexpr size_t kRixSmemCap = 160 * 1024;   // NB <= 2048 and Kb <= 128 need 96 KB; the attribute is set once, to the cap
 
 }  // namespace
@@ -303,6 +317,17 @@ extern "C" int fmsa_reverse_index_static(const int32_t* block_indices, int32_t* 
     // was written earlier in the same call, so stale contents of a previous call are never seen.
     return reverse_index_launch(block_indices, row_ptr, col_q, edge_pos, rows_bh, S, top_k_blocks, scratch,
                                 static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int fmsa_row_start(const int32_t* row_ptr, const int32_t* col_q, int64_t rows_bh, int32_t S, int32_t first_tile,
+                              int32_t* row_start, void* stream) {
+    using namespace fmsa;
+    FMSA_REQUIRE(row_ptr && col_q && row_start && rows_bh > 0 && rows_bh <= 65535 && S > 0 && S % kBlock == 0 && first_tile >= 0);
+    const int64_t rows = rows_bh * (S / kBlock);
+    FMSA_REQUIRE(first_tile <= S / kBlock);
+    rix_row_start_kernel<<<static_cast<unsigned>((rows + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(row_ptr, col_q, row_start,
+                                                                                                            rows, first_tile * kBlock);
+    return check_launch();
 }
 
 extern "C" size_t fmsa_reverse_index_workspace_bytes(int64_t rows_bh, int32_t S) {

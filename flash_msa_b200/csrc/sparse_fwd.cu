@@ -862,10 +862,19 @@ extern "C" int fmsa_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, con
                                const int32_t* col_q, void* o_part, float* lse_part, int64_t part_slots, int32_t g_begin,
                                int32_t g_count, int32_t with_proxy, int32_t dense, int32_t* counter, int32_t* status,
                                void* stream) {
+    return fmsa_sparse_fwd_from(pb, q, k, v, q_proxy, k_proxy, row_ptr, nullptr, 0, col_q, o_part, lse_part, part_slots, g_begin, g_count,
+                                with_proxy, dense, counter, status, stream);
+}
+
+extern "C" int fmsa_sparse_fwd_from(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                                    const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr,
+                                    const int32_t* row_start, int32_t first_tile, const int32_t* col_q, void* o_part, float* lse_part,
+                                    int64_t part_slots, int32_t g_begin, int32_t g_count, int32_t with_proxy, int32_t dense,
+                                    int32_t* counter, int32_t* status, void* stream) {
     if (!counter) return FMSA_ERR_ARGUMENT;
     if (cudaMemsetAsync(counter, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream)) != cudaSuccess) return FMSA_ERR_CUDA;
-    return fmsa::launch_sparse_fwd(pb, q, k, v, q_proxy, k_proxy, row_ptr, nullptr, 0, col_q, o_part, lse_part, part_slots, g_begin, g_count,
-                                   with_proxy, dense, counter, status, static_cast<cudaStream_t>(stream));
+    return fmsa::launch_sparse_fwd(pb, q, k, v, q_proxy, k_proxy, row_ptr, row_start, first_tile, col_q, o_part, lse_part, part_slots, g_begin,
+                                   g_count, with_proxy, dense, counter, status, static_cast<cudaStream_t>(stream));
 }
 
 int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
@@ -937,8 +946,14 @@ int fmsa::launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const 
 extern "C" int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part,
                                        const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse,
                                        float* lse_proxy, int32_t g_begin, int32_t g_count, int32_t dense, void* stream) {
-    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, nullptr, 0, g_begin, g_count,
-                                    dense, static_cast<cudaStream_t>(stream));
+    return fmsa_sparse_fwd_combine_from(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, 0, g_begin, g_count, dense, stream);
+}
+
+extern "C" int fmsa_sparse_fwd_combine_from(const fmsa_problem* pb, const void* o_part, const float* lse_part,
+                                            const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse, float* lse_proxy,
+                                            int32_t first_tile, int32_t g_begin, int32_t g_count, int32_t dense, void* stream) {
+    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, nullptr, first_tile, g_begin,
+                                    g_count, dense, static_cast<cudaStream_t>(stream));
 }
 
 int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
@@ -948,6 +963,7 @@ int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const f
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(o_part && lse_part && out && lse);
     FMSA_REQUIRE(dense || (edge_pos && row_ptr));
+    FMSA_REQUIRE(first_tile >= 0 && first_tile < pb->S / kBlock && (first_tile == 0 || !dense));
     FMSA_REQUIRE(g_begin >= 0 && g_count > 0 && g_begin + g_count <= pb->B * pb->Hkv);
     CombineParams P;
     P.o_part = static_cast<const __nv_bfloat16*>(o_part); P.lse_part = lse_part; P.edge_pos = edge_pos; P.row_ptr = row_ptr;

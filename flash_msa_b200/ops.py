@@ -366,8 +366,8 @@ SPLIT_PARTIALS_ABOVE = 32
 
 def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, with_proxy=True, status=None, doc_start=None):
     """Sparse (or dense warmup) forward.  Returns (out [B,S,Hq*D] bf16, lse [B,Hq,S] fp32,
-    lse_proxy [B,Hp,S] fp32 or None).  The stages of `fmsa_forward`, in its order of sums: the key-block stationary ones, then
-    the query tiles that the query-tile stationary kernel takes (all of them if dense; those need `rix.block_indices`)."""
+    lse_proxy [B,Hp,S] fp32 or None).  The stages of `fmsa_forward`, in its order of sums: the query-tile stationary kernel for
+    its tiles (all of them if dense; they need `rix.block_indices`), then the key-block stationary ones for the others."""
     _require_cuda(q, k, v)
     lib = _lib.load()
     q, k, v = (_as_kernel_input(t.detach()) for t in (q, k, v))
@@ -386,8 +386,7 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
     indices = None if dense else rix.block_indices
     tiles = lib.fmsa_forward_tiles(ctypes_byref(pb), int(dense), 0) if dense or indices is not None else 0
     st = _stream(dev)
-
-    def leading_tiles():
+    if tiles:
         nbytes = lib.fmsa_tile_fwd_workspace_bytes(ctypes_byref(pb), int(dense))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
         with _Timed("attn_fwd", dev):
@@ -395,10 +394,14 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
                 ctypes_byref(pb), _tensor_arg(q), _tensor_arg(k), _tensor_arg(v), _tensor_arg(qp), _tensor_arg(kp),
                 0 if dense else indices.data_ptr(), ws.data_ptr(), nbytes, out.data_ptr(), lse.data_ptr(),
                 lse_proxy.data_ptr() if with_proxy else 0, int(dense), status.data_ptr(), st), dev)
-        return out, lse, lse_proxy
-
     if tiles == s // BLOCK_SIZE:
-        return leading_tiles()
+        return out, lse, lse_proxy
+    row_start = None
+    if tiles:
+        row_start = torch.empty(b * hp * (s // BLOCK_SIZE), dtype=torch.int32, device=dev)
+        with _Timed("reverse_index", dev):
+            _launch("fmsa_row_start", 1, lib.fmsa_row_start(rix.row_ptr.data_ptr(), rix.col_q.data_ptr(), b * hp, s, tiles,
+                                                          row_start.data_ptr(), st), dev)
     counter = torch.empty(1, dtype=torch.int32, device=dev)
     groups = b * hkv
     per_group = lib.fmsa_fwd_partial_slots(ctypes_byref(pb), 1, int(dense))
@@ -413,15 +416,15 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
     for g0 in range(0, groups, gstep):
         gc = min(gstep, groups - g0)
         with _Timed("attn_fwd", dev):
-            _launch("fmsa_sparse_fwd", 1, lib.fmsa_sparse_fwd(
+            _launch("fmsa_sparse_fwd_from", 1, lib.fmsa_sparse_fwd_from(
                 ctypes_byref(pb), _tensor_arg(q), _tensor_arg(k), _tensor_arg(v), _tensor_arg(qp), _tensor_arg(kp), row_ptr,
-                col_q, o_part.data_ptr(), lse_part.data_ptr(), slots, g0, gc, int(with_proxy), int(dense),
+                row_start.data_ptr() if tiles else 0, tiles, col_q, o_part.data_ptr(), lse_part.data_ptr(), slots, g0, gc, int(with_proxy), int(dense),
                 counter.data_ptr(), status.data_ptr(), st), dev)
         with _Timed("fwd_combine", dev):
-            _launch("fmsa_sparse_fwd_combine", 2, lib.fmsa_sparse_fwd_combine(   # log-sum-exp kernel + row kernel
+            _launch("fmsa_sparse_fwd_combine_from", 2, lib.fmsa_sparse_fwd_combine_from(   # log-sum-exp kernel + row kernel
                 ctypes_byref(pb), o_part.data_ptr(), lse_part.data_ptr(), edge_pos, row_ptr, out.data_ptr(), lse.data_ptr(),
-                lse_proxy.data_ptr() if with_proxy else 0, g0, gc, int(dense), st), dev)
-    return leading_tiles() if tiles else (out, lse, lse_proxy)
+                lse_proxy.data_ptr() if with_proxy else 0, tiles, g0, gc, int(dense), st), dev)
+    return out, lse, lse_proxy
 
 
 def attention_backward(q, k, v, q_proxy, k_proxy, out, grad_out, lse, lse_proxy, scale, rix, grad_kl, *, dense=False,

@@ -173,6 +173,19 @@ int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_part, const fl
                             const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse, float* lse_proxy,
                             int32_t g_begin, int32_t g_count, int32_t dense, void* stream);
 
+/* The two stages above for query tiles first_tile .. only, where fmsa_tile_fwd (below) takes the tiles before them (not if dense; the
+ * buffers are sized and placed as for all tiles).  row_start int32 [B*Hp*S/128]: where they begin in the rows of the reverse index, from
+ * fmsa_row_start, which works on all rows of an index (rows_bh = B*Hp); with first_tile = 0 it may be NULL. */
+int fmsa_row_start(const int32_t* row_ptr, const int32_t* col_q, int64_t rows_bh, int32_t S, int32_t first_tile, int32_t* row_start,
+                   void* stream);
+int fmsa_sparse_fwd_from(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v,
+                         const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr, const int32_t* row_start,
+                         int32_t first_tile, const int32_t* col_q, void* o_part, float* lse_part, int64_t part_slots, int32_t g_begin,
+                         int32_t g_count, int32_t with_proxy, int32_t dense, int32_t* counter, int32_t* status, void* stream);
+int fmsa_sparse_fwd_combine_from(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
+                                 const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, int32_t first_tile, int32_t g_begin,
+                                 int32_t g_count, int32_t dense, void* stream);
+
 /* Query-tile stationary forward: query tiles (of 128 positions) 0 .. fmsa_forward_tiles()-1 of every (batch, head), in one kernel
  * that walks the key blocks any row of a tile selected and keeps the output in tensor memory; out, lse and lse_proxy (or NULL) as
  * fmsa_sparse_fwd_combine writes them.  fmsa_forward sends the first tiles of a sparse call, whose rows select most of what they

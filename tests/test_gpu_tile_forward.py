@@ -162,3 +162,42 @@ def test_fp16_probabilities_far_below_the_maximum(gap, sinks):
     want = (logits - norm).exp() @ v.double()
     got = out.view(1, s, h, 128).transpose(1, 2)[:, :, rows].double()
     assert ((got - want).norm(dim=(2, 3)) / want.norm(dim=(2, 3))).max() < 1e-3
+
+
+@pytest.mark.parametrize("cap", [None, 1])
+@pytest.mark.parametrize("cfg", [CFGS[0], *CFGS[-2:], dict(b=2, s=5120, hq=4, hkv=2, hp=4, hpkv=2, kb=1)], ids=lambda c: f"s{c['s']}_kb{c['kb']}")
+def test_stages_of_the_tiles_behind(monkeypatch, cfg, cap):
+    """The key-block stationary stages work on the query tiles behind the others' only, from the right place of every reverse-index
+    row, and together they give the whole pass's output bit for bit, in one pass over the groups or several."""
+    import flash_msa_b200 as fm
+    from flash_msa_b200 import _lib, ops
+    if cap:
+        monkeypatch.setattr(ops, "MAX_PARTIAL_BYTES", cap)
+    qp, kp, q, k, v, _ = bf16_inputs(dict(cfg, seed=7))
+    b, hp, nb, s = cfg["b"], cfg["hp"], cfg["s"] // 128, cfg["s"]
+    rix = ops.build_reverse_index(ops.select_blocks_fused(qp, kp, SCALE, cfg["kb"]))
+    tiles = _lib.load().fmsa_forward_tiles(ops._problem(q, k, qp, kp, cfg["kb"], SCALE), 0, 0)
+    lib, calls = _lib.load(), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            def call(*args):
+                calls.append((name, args))
+                return getattr(lib, name)(*args)
+            return call
+    monkeypatch.setattr(_lib, "load", Recorder)
+    out, _, _ = ops.attention_forward(q, k, v, qp, kp, SCALE, rix)
+    monkeypatch.undo()
+    first = [a[8] for n, a in calls if n in ("fmsa_sparse_fwd_from", "fmsa_sparse_fwd_combine_from")]
+    assert not any(n in ("fmsa_sparse_fwd", "fmsa_sparse_fwd_combine") for n, _ in calls)
+    assert first == [] if tiles == nb else first and set(first) == {tiles}
+    with torch.no_grad():
+        want, _ = fm.flash_msa_func(qp, kp, q, k, v, cfg["kb"] * 128, SCALE)
+    assert torch.equal(out, want)
+    row_ptr, col_q = rix.row_ptr.cpu(), rix.col_q.cpu()
+    for t in {0, 1, tiles, nb}:
+        start = torch.empty(b * hp * nb, dtype=torch.int32, device="cuda")
+        _lib.check(lib.fmsa_row_start(rix.row_ptr.data_ptr(), rix.col_q.data_ptr(), b * hp, s, t, start.data_ptr(),
+                                      torch.cuda.current_stream().cuda_stream), "fmsa_row_start")
+        ends = torch.tensor([int((col_q[row_ptr[r]:row_ptr[r + 1]] < 128 * t).sum()) for r in range(b * hp * nb)])
+        assert torch.equal(start.cpu(), row_ptr[:-1] + ends)
