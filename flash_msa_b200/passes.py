@@ -98,7 +98,7 @@ class Plan:
         self.out_shape = (b, s, hq * d)
         pbr = ctypes.byref(self.pb)
         self.forward_bytes = lib.fmsa_forward_workspace_bytes(pbr, int(dense), self.max_partial_bytes)
-        self._short_bytes = None   # of a forward that needs no partial rows because documents are short
+        self._short_bytes = {}   # see short_documents: by `visible`, of which there are at most S/128
         # saved for the backward, one int32 tensor: row_ptr | col_q | edge_pos | lse | lse_proxy, each from a 64-word boundary
         nb, edges = s // ops.BLOCK_SIZE, 0 if dense else b * hp * s * int(top_k_blocks)
         sizes = [0 if dense else b * hp * nb + 1, edges, edges, b * hq * s, b * hp * s]
@@ -139,12 +139,15 @@ class Plan:
     def short_documents(self, visible):
         """Workspace bytes of a forward all of whose tiles go the query-tile stationary way because no tile sees more than
         `visible` blocks; 0 where they do not, or do anyway."""
-        lib, pbr, nb = _lib.load(), ctypes.byref(self.pb), self.shape[2] // ops.BLOCK_SIZE
-        if self.dense or lib.fmsa_forward_tiles(pbr, 0, visible) < nb or lib.fmsa_forward_tiles(pbr, 0, 0) == nb:
-            return 0
-        if self._short_bytes is None:
-            self._short_bytes = lib.fmsa_forward_hinted_workspace_bytes(pbr, 0, visible, self.max_partial_bytes)
-        return self._short_bytes
+        got = self._short_bytes.get(visible)
+        if got is None:
+            lib, pbr, nb = _lib.load(), ctypes.byref(self.pb), self.shape[2] // ops.BLOCK_SIZE
+            if self.dense or lib.fmsa_forward_tiles(pbr, 0, visible) < nb or lib.fmsa_forward_tiles(pbr, 0, 0) == nb:
+                got = 0
+            else:
+                got = lib.fmsa_forward_hinted_workspace_bytes(pbr, 0, visible, self.max_partial_bytes)
+            self._short_bytes[visible] = got
+        return got
 
     def point(self, a, inputs, as_planned=True):
         """Points the argument block `a` at the inputs as the kernels can read them: in place, or - other strides, or an address

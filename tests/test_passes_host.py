@@ -253,3 +253,28 @@ def test_forms_of_document_boundaries(form):
     for bad in ([0, 5, 3, 256], [1, 256], [0, 255], [0], [[0, 256]] * 3):
         with pytest.raises(ValueError):
             ops.doc_start_from_cu_seqlens(bad, 2, 256, torch.device("cpu"))
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_short_documents_are_asked_for_once(monkeypatch, dense):
+    """What a plan's forward needs for documents that span so many blocks depends on nothing else: the library is asked once, and
+    the answers are those that it gives."""
+    from flash_msa_b200 import _lib
+    s, kb = 128 * 40, 3
+    inputs = [torch.empty(1, h, s, 128, dtype=torch.bfloat16) for h in (2, 1, 8, 2, 2)]
+    plan = passes.Plan([t.shape for t in inputs], [t.stride() for t in inputs], torch.bfloat16, inputs[0].device, kb, 0.1, dense, 1 << 32)
+    lib, pb, asked = _lib.load(), ctypes.byref(plan.pb), []
+
+    class Counting:
+        def __getattr__(self, name):
+            asked.append(name)
+            return getattr(lib, name)
+    monkeypatch.setattr(_lib, "load", Counting)
+    counts = []
+    for _ in range(2):
+        for visible in range(1, 41):
+            all_tiles = not dense and lib.fmsa_forward_tiles(pb, 0, visible) == 40
+            assert all_tiles == (not dense and visible <= 5 * kb // 2)
+            assert plan.short_documents(visible) == (lib.fmsa_forward_hinted_workspace_bytes(pb, 0, visible, 1 << 32) if all_tiles else 0)
+        counts.append(len(asked))
+    assert counts[0] == counts[1]
