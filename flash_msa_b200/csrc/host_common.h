@@ -15,10 +15,12 @@ inline int check_launch() {
     return e == cudaSuccess ? FMSA_OK : FMSA_ERR_CUDA;
 }
 
-// Launches a kernel of a pass so that its blocks may take their places, and set up shared and tensor memory, while the last blocks of
-// the kernel before it are still at work ("programmatic dependent launch").  Every such kernel calls wait_for_previous_kernel() before its first
-// access to global memory, so nothing it reads or writes is seen out of order.  (Passes back to back: B=3 S=1664 Hq=20 fp16 with sinks,
-// fifteen kernels, 285.5 -> 259.6 us; B=1 S=8192 Hq=32 as five documents 982 -> 966; forward of B=1 S=512 35.0 -> 33.2.)
+// Launches a kernel of a pass as a programmatic dependent launch: it is made ready while the kernel before it still runs, and its blocks
+// start when the last block of that one has left (no kernel signals its dependents earlier), without waiting for the flush of what it
+// wrote.  What this takes off the way from kernel to kernel is the launch and the flush; set-up is not overlapped with work.  Every such
+// kernel calls wait_for_previous_kernel() before its first access to global memory, and before it leaves, so nothing it reads or writes is
+// seen out of order.  (Passes back to back: B=3 S=1664 Hq=20 fp16 with sinks, fifteen kernels, 285.5 -> 259.6 us; B=1 S=8192 Hq=32 as five
+// documents 982 -> 966; forward of B=1 S=512 35.0 -> 33.2.)
 template <class... Params, class... Args>
 inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchAttribute attr[1];

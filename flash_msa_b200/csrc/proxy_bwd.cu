@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
     if ((tiles - smem_u32(smem_raw)) + kProxyTileBytes + sizeof(ProxyCtrl) > kProxySmemBytes) {
+        wait_for_previous_kernel();   // (a kernel that has left counts as complete for those behind it)
         if (threadIdx.x == 0) atomicMax(P.status, kStatusBadSmem);
         return;
     }
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(kProxyThreads, 1) proxy_bwd_kernel(const __gri
     tc_fence_after_sync();
     constexpr uint32_t tmem = 0, tmem_dq = 256, tmem_dkp = 384;   // all 512 columns: the allocation starts at column 0
     if (sm->tmem_slot != tmem) {
+        wait_for_previous_kernel();   // (a kernel that has left counts as complete for those behind it)
         if (tid == 0) atomicMax(P.status, kStatusBadSmem);
         __syncthreads();
         if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);

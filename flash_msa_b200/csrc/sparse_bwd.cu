@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
     if ((tiles - smem_u32(smem_raw)) + kBwdTileBytes + sizeof(BwdCtrl) > kBwdSmemBytes) {
+        wait_for_previous_kernel();   // (a kernel that has left counts as complete for those behind it)
         if (threadIdx.x == 0) atomicMax(P.status, kStatusBadSmem);
         return;
     }
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) sparse_bwd_kernel(const __grid
     // All 512 columns are this CTA's, so the allocation starts at column 0 and every TMEM address is a constant.
     constexpr uint32_t tmem = 0;
     if (sm->tmem_slot != tmem) {
+        wait_for_previous_kernel();   // (a kernel that has left counts as complete for those behind it)
         if (tid == 0) atomicMax(P.status, kStatusBadSmem);
         __syncthreads();
         if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);

@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sparse_fwd_kernel(const __grid
     // All 512 columns are this CTA's, so the allocation starts at column 0 and every TMEM address is a constant.
     constexpr uint32_t tmem = 0;
     if (sm->tmem_slot != tmem) {
+        wait_for_previous_kernel();   // (a kernel that has left counts as complete for those behind it)
         if (tid == 0) atomicMax(P.status, kStatusBadSmem);
         __syncthreads();
         if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);

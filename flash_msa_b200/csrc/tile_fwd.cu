@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_fwd_kernel(const __grid_
     tc_fence_after_sync();
     constexpr uint32_t tmem = 0, tmem_o = 128 * kTileBuffers;   // all 512 columns: the allocation starts at column 0
     if (sm->tmem_slot != tmem) {
+        wait_for_previous_kernel();   // (a kernel that has left counts as complete for those behind it)
         if (tid == 0) atomicMax(P.status, kStatusBadSmem);
         __syncthreads();
         if (warp == 0) tmem_dealloc(sm->tmem_slot, 512);
