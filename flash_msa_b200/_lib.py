@@ -78,6 +78,8 @@ def _declare(lib):
     lib.fmsa_sparse_fwd.argtypes = [PB, T, T, T, T, T, P, P, P, P, c_int64, c_int32, c_int32, c_int32, c_int32, P, P, P]
     lib.fmsa_sparse_fwd_combine.restype = c_int
     lib.fmsa_sparse_fwd_combine.argtypes = [PB, P, P, P, P, P, P, P, c_int32, c_int32, c_int32, P]
+    lib.fmsa_reverse_index_launches.restype = c_int32
+    lib.fmsa_reverse_index_launches.argtypes = [c_int64, c_int32]
     lib.fmsa_row_start.restype = c_int
     lib.fmsa_row_start.argtypes = [P, P, c_int64, c_int32, c_int32, P, P]
     lib.fmsa_sparse_fwd_from.restype = c_int

@@ -319,6 +319,10 @@ extern "C" int fmsa_reverse_index_static(const int32_t* block_indices, int32_t* 
                                 static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int32_t fmsa_reverse_index_launches(int64_t rows_bh, int32_t S) {
+    return rows_bh > 0 && S > 0 ? fmsa::reverse_index_launches(rows_bh, S, fmsa::RixExtras()) : 0;
+}
+
 extern "C" int fmsa_row_start(const int32_t* row_ptr, const int32_t* col_q, int64_t rows_bh, int32_t S, int32_t first_tile,
                               int32_t* row_start, void* stream) {
     using namespace fmsa;

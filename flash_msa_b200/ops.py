@@ -123,10 +123,6 @@ class ReverseIndex:
     block_indices: torch.Tensor = None   # the selection it was built from
 
 
-def _index_kernels(rows, nb):   # count, scan of columns and rows (one kernel for small ones), fill
-    return 3 if rows * nb <= 1024 and rows * nb * nb <= 16384 else 4
-
-
 def build_reverse_index(block_indices: torch.Tensor) -> ReverseIndex:
     _require_cuda(block_indices)
     if block_indices.dtype != torch.int32 or block_indices.ndim != 4:
@@ -144,7 +140,7 @@ def build_reverse_index(block_indices: torch.Tensor) -> ReverseIndex:
     ws_bytes = lib.fmsa_reverse_index_workspace_bytes(b * hp, s)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     with _Timed("reverse_index", dev):
-        _launch("fmsa_reverse_index", _index_kernels(b * hp, nb), lib.fmsa_reverse_index(block_indices.data_ptr(), row_ptr.data_ptr(),
+        _launch("fmsa_reverse_index", lib.fmsa_reverse_index_launches(b * hp, s), lib.fmsa_reverse_index(block_indices.data_ptr(), row_ptr.data_ptr(),
                                                               col_q.data_ptr(), edge_pos.data_ptr(), b * hp, s, kb,
                                                               ws.data_ptr(), ws_bytes, _stream(dev)), dev)
     return ReverseIndex(row_ptr, col_q, edge_pos, b, hp, s, kb, block_indices)
@@ -177,7 +173,7 @@ def build_reverse_index_static(block_indices: torch.Tensor, row_ptr: torch.Tenso
                          "bytes built into the library; use build_reverse_index (caller-provided workspace)")
     dev = block_indices.device
     with _Timed("reverse_index", dev):
-        _launch("fmsa_reverse_index_static", _index_kernels(b * hp, nb), lib.fmsa_reverse_index_static(
+        _launch("fmsa_reverse_index_static", lib.fmsa_reverse_index_launches(b * hp, s), lib.fmsa_reverse_index_static(
             block_indices.data_ptr(), row_ptr.data_ptr(), col_q.data_ptr(), edge_pos.data_ptr(), b * hp, s, kb,
             _stream(dev)), dev)
     return ReverseIndex(row_ptr, col_q, edge_pos.view(b, hp, s, kb), b, hp, s, kb, block_indices)

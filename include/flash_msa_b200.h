@@ -104,6 +104,7 @@ size_t fmsa_reverse_index_workspace_bytes(int64_t rows_bh, int32_t S);
 int fmsa_reverse_index(const int32_t* block_indices, int32_t* row_ptr, int32_t* col_q, int32_t* edge_pos,
                        int64_t rows_bh, int32_t S, int32_t top_k_blocks, void* workspace, size_t workspace_bytes,
                        void* stream);
+int32_t fmsa_reverse_index_launches(int64_t rows_bh, int32_t S);   /* how many kernels that is */
 
 /* Reverse index for callers that cannot hand the library any device memory of their own.
  * (No counterpart in the reference, whose wrappers allocate their workspaces with torch.)

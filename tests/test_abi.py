@@ -2,6 +2,7 @@
 the public header declares (no kernel is launched here)."""
 import ctypes
 import os
+import re
 
 from flash_msa_b200 import _lib, build
 
@@ -15,6 +16,24 @@ def test_library_builds_and_exports_declared_symbols():
     for name in names:
         assert hasattr(lib, name), name
     assert lib.fmsa_abi_version() == 8          # 8: fmsa_select_fused (block scores and top-k in one kernel)
+
+
+def test_constants_of_the_header():
+    """Limits that the Python side checks ahead of a call are the header's."""
+    from flash_msa_b200 import ops
+    with open(_lib.HEADER_PATH) as f:
+        text = f.read()
+    for name, value in [("FMSA_MAX_HOST_BOUNDARIES", ops.MAX_HOST_BOUNDARIES), ("FMSA_FUSED_SELECT_MAX_BLOCKS", ops.FUSED_SELECT_MAX_BLOCKS),
+                        ("FMSA_STATIC_SCRATCH_BYTES", ops.STATIC_SCRATCH_BYTES), ("FMSA_DTYPE_BF16", _lib.FMSA_DTYPE_BF16),
+                        ("FMSA_DTYPE_FP16", _lib.FMSA_DTYPE_FP16), ("FMSA_OK", _lib.FMSA_OK)]:
+        given = re.search(rf"#define {name}\s+(.+)", text).group(1).split("/*")[0]
+        assert eval(given) == value, name
+
+
+def test_kernels_of_a_reverse_index():
+    lib = _lib.load()   # count, scan of columns and rows (one kernel up to 1024 columns and 16384 counts), fill
+    for rows, s, n in [(1, 128, 3), (64, 2048, 3), (65, 2048, 4), (128, 1024, 3), (129, 1024, 4), (1, 16384, 3), (1, 16512, 4), (0, 128, 0)]:
+        assert lib.fmsa_reverse_index_launches(rows, s) == n
 
 
 def test_argument_errors_do_not_launch():
