@@ -18,8 +18,9 @@ int launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_t
 int launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
                        const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
                        int first_tile, int g_begin, int g_count, int dense, cudaStream_t st);
-// Query tiles 0 .. tiles-1 of every (batch, proxy head).  `visits`: from reverse_index_launch or launch_tile_visits (null if dense);
-// lse_proxy null: without the proxy head.  `counter`: one zeroed word.  Returns the number of launches in *launches.
+// Query tiles 0 .. tiles-1 of every (batch, proxy head).  `visits`: from select_fused_launch, or where the selection is another one from
+// reverse_index_launch or launch_tile_visits (null if dense); lse_proxy null: without the proxy head.  `counter`: one zeroed word.  One
+// launch, and one more with sinks.
 int launch_tile_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_tensor* k, const fmsa_tensor* v, const fmsa_tensor* q_proxy,
                     const fmsa_tensor* k_proxy, const void* visits, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
                     int tiles, int dense, int32_t* counter, int32_t* status, cudaStream_t st);

@@ -1,13 +1,14 @@
 // Deterministic reverse index: a CSR that lists, for every (batch, proxy head, key block), the
 // query positions that selected that block, in ascending order.
 //
-// Four small kernels, no global atomics and no host synchronisation:
+// Small kernels, no global atomics and no host synchronisation:
 //   1. count : one CTA per (batch*proxy head, query block) builds a shared-memory bitmap
-//              "row r selected key block j" and writes the per-(query block, key block) counts;
-//   (2 and 3 in one launch where that is enough; 1 is left to the selection in a whole pass)
+//              "row r selected key block j" and writes the per-(query block, key block) counts
+//              (as a stage; in a whole pass the fused selection leaves them);
 //   2. colscan: one thread per (batch*proxy head, key block) turns the counts of its column into
 //              exclusive offsets over the query blocks and records the column total;
-//   3. rowscan: a single CTA turns the totals into row_ptr;
+//   3. rowscan: a single CTA turns the totals into row_ptr
+//              (2 and 3 are one kernel where that is enough: one_scan);
 //   4. fill  : the bitmap is rebuilt and every edge gets position
 //              row_ptr + block offset + (number of lower rows of its block that chose the key block).
 // The edge rule `0 <= kb < NB && kb <= q/128` is the reference's

@@ -235,8 +235,8 @@ def doc_start_from_cu_seqlens(cu_seqlens, batch: int, seq_len: int, device) -> t
 
 
 def document_layout(cu_seqlens, batch: int, seq_len: int, device):
-    """(`doc_start_from_cu_seqlens`, the most key blocks of one document that a query tile can see, or 0 where only the device
-    knows the boundaries)."""
+    """(`doc_start_from_cu_seqlens`, the most key blocks of one document that a query tile can see, or 0 where that is not worked
+    out: boundaries in device memory, more than MAX_HOST_BOUNDARIES of them, or under a trace)."""
     cu_seqlens = torch.as_tensor(cu_seqlens)
     if cu_seqlens.device.type == "cpu" and not torch._C._is_tracing():
         # boundaries that the host holds are checked here and travel as a kernel parameter: nothing waits for the device
