@@ -14,10 +14,9 @@ int launch_sparse_fwd(const fmsa_problem* pb, const fmsa_tensor* q, const fmsa_t
                       const fmsa_tensor* q_proxy, const fmsa_tensor* k_proxy, const int32_t* row_ptr,
                       const int32_t* row_start, int first_tile, const int32_t* col_q, void* o_part, float* lse_part, int64_t part_slots, int g_begin, int g_count, int with_proxy, int dense,
                       int32_t* counter, int32_t* status, cudaStream_t st);
-// `sinks`: fp32 [Hq] softmax-bias logits or null; `zero`: a device scalar to clear on the way, or null.
+// `sinks`: fp32 [Hq] softmax-bias logits or null.
 int launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
-                       const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
-                       int first_tile, int g_begin, int g_count, int dense, cudaStream_t st);
+                       const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, int first_tile, int g_begin, int g_count, int dense, cudaStream_t st);
 // Query tiles 0 .. tiles-1 of every (batch, proxy head).  `visits`: from select_fused_launch, or where the selection is another one from
 // reverse_index_launch or launch_tile_visits (null if dense); lse_proxy null: without the proxy head.  `counter`: one zeroed word.  One
 // launch, and one more with sinks.

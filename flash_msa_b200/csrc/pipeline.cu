@@ -199,8 +199,7 @@ extern "C" int fmsa_forward_hinted(const fmsa_forward_args* a, int32_t alone, in
                                    w.stats, w.slots, g0, gc, a->with_proxy, dense, w.counters + i, a->status, st));
         mark(FMSA_STAGE_ATTN_FWD);
         mark(FMSA_STAGE_FWD_COMBINE);
-        FMSA_TRY(launch_fwd_combine(pb, w.o_part, w.stats, a->edge_pos, a->row_ptr, a->out, a->lse, lse_proxy, a->sinks, nullptr, w.tiles, g0, gc,
-                                    dense, st));
+        FMSA_TRY(launch_fwd_combine(pb, w.o_part, w.stats, a->edge_pos, a->row_ptr, a->out, a->lse, lse_proxy, a->sinks, w.tiles, g0, gc, dense, st));
         mark(FMSA_STAGE_FWD_COMBINE);
         n += 3;
     }

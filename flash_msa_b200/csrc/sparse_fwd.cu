@@ -644,7 +644,6 @@ struct CombineParams {
     int q0;                    // rows q0 .. S-1 of every (batch, proxy head)
     int hgroup;                // main heads per blockIdx.y of the row kernel
     const float* sinks;        // [Hq] softmax-bias logits or null
-    float* zero;               // a scalar to set to zero, or null
 };
 
 // Two kernels.  The partial rows of all main heads of one edge are contiguous (mpp * 256 bytes), so a warp reads them with
@@ -702,7 +701,6 @@ __global__ void __launch_bounds__(256) combine_lse_kernel(const CombineParams P)
     const CombineRow<DENSE> row(P, valid ? w0 : nrows - 1);
     const int lse_stride = P.mpp + 1;
     const float2* stats = reinterpret_cast<const float2*>(P.lse_part);
-    if (P.zero && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *P.zero = 0.f;
     float keep = 0.f;   // SINKS: sum over the main heads of exp(lse - lse')
     // Groups of heads (head number mpp is the proxy): one per blockIdx.y, or with SINKS one after another.
     for (int h0 = blockIdx.y * kMaxHeads; h0 < P.mpp + (P.lse_proxy ? 1 : 0); h0 += gridDim.y * kMaxHeads) {
@@ -953,13 +951,13 @@ extern "C" int fmsa_sparse_fwd_combine(const fmsa_problem* pb, const void* o_par
 extern "C" int fmsa_sparse_fwd_combine_from(const fmsa_problem* pb, const void* o_part, const float* lse_part,
                                             const int32_t* edge_pos, const int32_t* row_ptr, void* out, float* lse, float* lse_proxy,
                                             int32_t first_tile, int32_t g_begin, int32_t g_count, int32_t dense, void* stream) {
-    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, nullptr, first_tile, g_begin,
-                                    g_count, dense, static_cast<cudaStream_t>(stream));
+    return fmsa::launch_fwd_combine(pb, o_part, lse_part, edge_pos, row_ptr, out, lse, lse_proxy, nullptr, first_tile, g_begin, g_count,
+                                    dense, static_cast<cudaStream_t>(stream));
 }
 
 int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const float* lse_part, const int32_t* edge_pos,
-                             const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, float* zero,
-                             int first_tile, int g_begin, int g_count, int dense, cudaStream_t cst) {
+                             const int32_t* row_ptr, void* out, float* lse, float* lse_proxy, const float* sinks, int first_tile,
+                             int g_begin, int g_count, int dense, cudaStream_t cst) {
     using namespace fmsa;
     FMSA_REQUIRE(problem_ok(pb));
     FMSA_REQUIRE(o_part && lse_part && out && lse);
@@ -971,7 +969,7 @@ int fmsa::launch_fwd_combine(const fmsa_problem* pb, const void* o_part, const f
     P.out = static_cast<__nv_bfloat16*>(out); P.lse = lse; P.lse_proxy = lse_proxy;
     P.S = pb->S; P.NB = pb->S / kBlock; P.Hq = pb->Hq; P.Hp = pb->Hp; P.mpp = pb->Hq / pb->Hp; P.ppk = pb->Hp / pb->Hkv;
     P.Kb = pb->top_k_blocks; P.g_begin = g_begin; P.G = g_count; P.dense = dense ? 1 : 0;
-    P.sinks = sinks; P.zero = zero; P.q0 = first_tile * kBlock;
+    P.sinks = sinks; P.q0 = first_tile * kBlock;
     const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * (P.S - P.q0);
     const int64_t grid = (rows + 7) / 8;
     FMSA_REQUIRE(grid <= 0x7fffffffLL);

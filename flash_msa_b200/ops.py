@@ -390,7 +390,7 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
                 ctypes_byref(pb), _tensor_arg(q), _tensor_arg(k), _tensor_arg(v), _tensor_arg(qp), _tensor_arg(kp),
                 0 if dense else indices.data_ptr(), ws.data_ptr(), nbytes, out.data_ptr(), lse.data_ptr(),
                 lse_proxy.data_ptr() if with_proxy else 0, int(dense), status.data_ptr(), st), dev)
-    if tiles == s // BLOCK_SIZE:
+    if tiles == s // BLOCK_SIZE:   # (all dense calls)
         return out, lse, lse_proxy
     row_start = None
     if tiles:
@@ -400,26 +400,24 @@ def attention_forward(q, k, v, q_proxy, k_proxy, scale, rix, *, dense=False, wit
                                                           row_start.data_ptr(), st), dev)
     counter = torch.empty(1, dtype=torch.int32, device=dev)
     groups = b * hkv
-    per_group = lib.fmsa_fwd_partial_slots(ctypes_byref(pb), 1, int(dense))
+    per_group = lib.fmsa_fwd_partial_slots(ctypes_byref(pb), 1, 0)
     bytes_per_slot = mpp * d * 2 + (mpp + 1) * 8
     gstep = max(1, min(groups, MAX_PARTIAL_BYTES // max(1, per_group * bytes_per_slot)))
     slots = per_group * gstep
     o_part = torch.empty(slots * mpp * d, dtype=q.dtype, device=dev)
     lse_part = torch.empty(slots * (mpp + 1) * 2, dtype=torch.float32, device=dev)
-    row_ptr = 0 if dense else rix.row_ptr.data_ptr()
-    col_q = 0 if dense else rix.col_q.data_ptr()
-    edge_pos = 0 if dense else rix.edge_pos.data_ptr()
+    row_ptr, col_q, edge_pos = rix.row_ptr.data_ptr(), rix.col_q.data_ptr(), rix.edge_pos.data_ptr()
     for g0 in range(0, groups, gstep):
         gc = min(gstep, groups - g0)
         with _Timed("attn_fwd", dev):
             _launch("fmsa_sparse_fwd_from", 1, lib.fmsa_sparse_fwd_from(
                 ctypes_byref(pb), _tensor_arg(q), _tensor_arg(k), _tensor_arg(v), _tensor_arg(qp), _tensor_arg(kp), row_ptr,
-                row_start.data_ptr() if tiles else 0, tiles, col_q, o_part.data_ptr(), lse_part.data_ptr(), slots, g0, gc, int(with_proxy), int(dense),
+                row_start.data_ptr() if tiles else 0, tiles, col_q, o_part.data_ptr(), lse_part.data_ptr(), slots, g0, gc, int(with_proxy), 0,
                 counter.data_ptr(), status.data_ptr(), st), dev)
         with _Timed("fwd_combine", dev):
             _launch("fmsa_sparse_fwd_combine_from", 2, lib.fmsa_sparse_fwd_combine_from(   # log-sum-exp kernel + row kernel
                 ctypes_byref(pb), o_part.data_ptr(), lse_part.data_ptr(), edge_pos, row_ptr, out.data_ptr(), lse.data_ptr(),
-                lse_proxy.data_ptr() if with_proxy else 0, tiles, g0, gc, int(dense), st), dev)
+                lse_proxy.data_ptr() if with_proxy else 0, tiles, g0, gc, 0, st), dev)
     return out, lse, lse_proxy
 
 
