@@ -44,6 +44,14 @@ def kernel_selection(q_proxy, k_proxy, kb):
     return ops.select_blocks(q_proxy, k_proxy, scale=SCALE, num_blocks=q_proxy.shape[2] // 128, top_k_blocks=kb)
 
 
+def forward_tiles(inputs, kb, cu_seqlens=None, dense=False):
+    """How many query tiles of a call the query-tile stationary forward takes; the key-block stationary one takes the others."""
+    from flash_msa_b200 import _lib, ops
+    qp, kp, q, k, _ = inputs
+    visible = 0 if cu_seqlens is None else ops.document_layout(cu_seqlens, q.shape[0], q.shape[2], q.device)[1]
+    return _lib.load().fmsa_forward_tiles(ops._problem(q, k, qp, kp, kb, SCALE), int(dense), visible)
+
+
 _REPORT = {}
 
 

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import msa_oracle as O
-from tests.gpu_util import SCALE, bf16_inputs, kernel_selection, max_err, yardstick_check
+from tests.gpu_util import SCALE, bf16_inputs, forward_tiles, kernel_selection, max_err, yardstick_check
 
 pytestmark = pytest.mark.gpu
 NAMES = ["dq_proxy", "dk_proxy", "dq", "dk", "dv"]
@@ -182,15 +182,16 @@ def test_gradients_in_caller_layout(fm, warmup):
             assert max_err(g_view, g_plain) <= 2 ** -7 * g_plain.float().abs().max().item() + 1e-6, n
 
 
-@pytest.mark.parametrize("warmup", [False, True])
-def test_passes_over_groups_give_the_same_result(fm, warmup):
-    """When the per-edge partial rows of a call would exceed `ops.MAX_PARTIAL_BYTES` the forward and the backward run in
-    several passes over (batch, KV head) groups, reusing one partial buffer.  One group per pass must give what one
-    pass over everything gives: out, lse and dQ bit for bit (they are sums in a fixed order), dK / dV / dKp up to the
-    order of their fp32 reductions."""
+@pytest.mark.parametrize("warmup,s", [(False, 1024), (True, 1024), (False, 5120)])
+def test_passes_over_groups_give_the_same_result(fm, warmup, s):
+    """When the per-edge partial rows of a call would exceed `ops.MAX_PARTIAL_BYTES` the backward, and the forward where it writes
+    partial rows (5120: behind the first seven query tiles), run in several passes over (batch, KV head) groups, reusing one partial
+    buffer.  One group per pass must give what one pass over everything gives: out, lse and dQ bit for bit (they are sums in a fixed
+    order), dK / dV / dKp up to the order of their fp32 reductions."""
     from flash_msa_b200 import ops
-    cfg = dict(b=2, s=1024, hq=12, hkv=3, hp=6, hpkv=3, kb=3, seed=31)
+    cfg = dict(b=2, s=s, hq=12, hkv=3, hp=6, hpkv=3, kb=3, seed=31)
     qp, kp, q, k, v, do = bf16_inputs(cfg)
+    assert forward_tiles((qp, kp, q, k, v), cfg["kb"], dense=warmup) == (7 if s == 5120 else 8)
     fn = fm.flash_msa_warmup_func if warmup else fm.flash_msa_func
     saved = ops.MAX_PARTIAL_BYTES
     results = []

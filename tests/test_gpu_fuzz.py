@@ -3,14 +3,15 @@ functions, against the oracle (selection bit-exact on the kernel's own scores; t
 yardstick).  The shapes are small enough for the eager restatement; what varies is everything the index arithmetic
 depends on: heads per proxy head (also values that do not divide 128), proxy heads per KV head, proxy-K sharing,
 ragged reverse-index rows, top-k larger than the number of visible blocks, documents that start inside blocks, fewer
-proxy heads than KV heads, softmax sinks."""
+proxy heads than KV heads, softmax sinks.  The query-tile stationary forward takes nearly all of these calls whole; a second
+family of draws is long enough, with few enough blocks selected, for tiles that the key-block stationary one works on."""
 import random
 
 import pytest
 import torch
 
 from oracle import msa_oracle as O
-from tests.gpu_util import SCALE, bf16_inputs, yardstick_check
+from tests.gpu_util import SCALE, bf16_inputs, forward_tiles, yardstick_check
 
 pytestmark = pytest.mark.gpu
 NAMES = ["dq_proxy", "dk_proxy", "dq", "dk", "dv"]
@@ -40,11 +41,42 @@ def _draw(seed):
     return cfg, mode, dtype, layout, cu, grad_kl, rng.random() < 0.3
 
 
+def _draw_with_tiles_left(seed):
+    rng = random.Random(3000 + seed)
+    hkv = rng.choice([1, 2, 3])
+    hp = hkv * rng.choice([1, 1, 2])
+    hq = hp * rng.choice([m for m in (1, 2, 3, 5, 9) if hp * m <= 12])
+    s, b = 128 * rng.choice([26, 29, 33]), 1
+    while b * hq < 10:   # (fewer heads go the query-tile stationary way whole)
+        b += 1
+    cfg = dict(b=b, s=s, hq=hq, hkv=hkv, hp=hp, hpkv=rng.choice([d for d in range(1, hp + 1) if hp % d == 0]),
+               kb=1 if s < 3500 else rng.choice([1, 2]), seed=700 + seed)
+    cu = None
+    if rng.random() < 0.5:   # a document of more than a quarter of the sequence
+        cuts = sorted(rng.sample(range(1, 2 * s // 3), k=rng.randint(1, 4)))
+        cu = [0] + cuts + [s]
+    return (cfg, "sparse", rng.choice([torch.bfloat16, torch.float16]), rng.choice(["bhsd", "bshd"]), cu,
+            rng.choice([float(s), 0.4 * s, None]), rng.random() < 0.4)   # (proxy gradients above fp16's subnormals)
+
+
 @pytest.mark.parametrize("seed", range(48))
 def test_random_configuration(seed):
+    _compare_with_the_oracle(_draw(seed), seed, "cpu")
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_random_configuration_with_tiles_left(seed):
+    draw = _draw_with_tiles_left(seed)
+    cfg, _, dtype, _, cu, _, _ = draw
+    assert 1 <= forward_tiles(bf16_inputs(cfg, dtype=dtype)[:5], cfg["kb"], cu) < cfg["s"] // 128
+    _compare_with_the_oracle(draw, seed, "cuda")
+
+
+def _compare_with_the_oracle(draw, seed, where):
+    """`where`: the device that the oracle works on."""
     import flash_msa_b200 as fm
     from flash_msa_b200 import api, ops
-    cfg, mode, dtype, layout, cu, grad_kl, with_sinks = _draw(seed)
+    cfg, mode, dtype, layout, cu, grad_kl, with_sinks = draw
     sinks = None
     if with_sinks:
         sinks = (torch.randn(cfg["hq"], generator=torch.Generator().manual_seed(seed)) * 0.7 + 0.5).cuda().requires_grad_(True)
@@ -66,36 +98,36 @@ def test_random_configuration(seed):
     finally:
         api.DEBUG_CHECK_STATUS = False
     ds = None if cu is None else ops.doc_start_from_cu_seqlens(cu, cfg["b"], cfg["s"], qp.device)
-    ds_cpu = None if ds is None else ds.cpu()
-    cpu16 = [t.cpu() for t in (qp, kp, q, k, v)]
-    cpu32 = [t.float() for t in cpu16]
-    sk32 = None if sinks is None else sinks.detach().float().cpu()
-    sk16 = None if sinks is None else sinks.detach().to(dtype).cpu().requires_grad_(True)
+    ds_o = None if ds is None else ds.to(where)
+    x16 = [t.to(where) for t in (qp, kp, q, k, v)]
+    x32 = [t.float() for t in x16]
+    sk32 = None if sinks is None else sinks.detach().float().to(where)
+    sk16 = None if sinks is None else sinks.detach().to(dtype).to(where).requires_grad_(True)
     extra = [] if sinks is None else [sk16]
     if mode == "warmup":
-        r32 = O.warmup_forward_backward(*cpu32, SCALE, do.float().cpu(), grad_kl, doc_start=ds_cpu, sinks=sk32)
-        o16, _, g16 = O.eager_forward_backward(lambda *t: O.eager_warmup(*t, SCALE, doc_start=ds_cpu, sinks=sk16), cpu16, do.cpu(),
+        r32 = O.warmup_forward_backward(*x32, SCALE, do.float().to(where), grad_kl, doc_start=ds_o, sinks=sk32)
+        o16, _, g16 = O.eager_forward_backward(lambda *t: O.eager_warmup(*t, SCALE, doc_start=ds_o, sinks=sk16), x16, do.to(where),
                                                grad_kl, extra=extra)
     else:
         idx, scores = ops.select_blocks(qp, kp, scale=SCALE, num_blocks=cfg["s"] // 128, top_k_blocks=cfg["kb"],
                                         return_scores=True, doc_start=ds)
         nb = cfg["s"] // 128
-        vis = torch.arange(nb).view(1, 1, 1, nb) <= (torch.arange(cfg["s"]) // 128).view(1, 1, -1, 1)
-        mine = torch.where(vis.expand_as(scores.cpu()), scores.cpu(), torch.full_like(scores.cpu(), float("-inf")))
-        assert torch.equal(idx.cpu(), O.stable_topk(mine, cfg["kb"]))
-        r32 = O.sparse_forward_backward(*cpu32, top_k, SCALE, do.float().cpu(), grad_kl, block_indices=idx.cpu(), doc_start=ds_cpu,
+        vis = torch.arange(nb, device=where).view(1, 1, 1, nb) <= (torch.arange(cfg["s"], device=where) // 128).view(1, 1, -1, 1)
+        mine = torch.where(vis.expand_as(scores.to(where)), scores.to(where), torch.full_like(scores.to(where), float("-inf")))
+        assert torch.equal(idx.to(where), O.stable_topk(mine, cfg["kb"]))
+        r32 = O.sparse_forward_backward(*x32, top_k, SCALE, do.float().to(where), grad_kl, block_indices=idx.to(where), doc_start=ds_o,
                                         sinks=sk32)
         o16, _, g16 = O.eager_forward_backward(
-            lambda *t: O.eager_sparse(*t, top_k, SCALE, block_indices=idx.cpu(), doc_start=ds_cpu, sinks=sk16), cpu16, do.cpu(),
+            lambda *t: O.eager_sparse(*t, top_k, SCALE, block_indices=idx.to(where), doc_start=ds_o, sinks=sk16), x16, do.to(where),
             grad_kl, extra=extra)
     assert out.dtype == dtype
-    yardstick_check("out", out.cpu(), r32["out"], o16, 2e-3 if sinks is not None else 1e-3)
+    yardstick_check("out", out.to(where), r32["out"], o16, 2e-3 if sinks is not None else 1e-3)
     if sinks is not None:
         # (a sum over all rows of exp(sink - lse) * delta: the log-sum-exp is held to 2e-3 absolute elsewhere, i.e. the
         # sink's probability to 0.2 %, and that error is systematic over the rows of a head)
-        yardstick_check("dsinks", sinks.grad.cpu(), r32["dsinks"], g16[5].float(), 5e-3 * max(1.0, r32["dsinks"].abs().max().item()))
+        yardstick_check("dsinks", sinks.grad.to(where), r32["dsinks"], g16[5].float(), 5e-3 * max(1.0, r32["dsinks"].abs().max().item()))
     for n, leaf, y in zip(NAMES, leaves, g16[:5]):
-        got = leaf.grad.cpu()
+        got = leaf.grad.to(where)
         if grad_kl is None and n in ("dq_proxy", "dk_proxy"):
             assert got.abs().max().item() == 0.0
             continue

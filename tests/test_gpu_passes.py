@@ -5,17 +5,20 @@ import pytest
 import torch
 
 from oracle import msa_oracle as O
-from tests.gpu_util import SCALE, bf16_inputs, kernel_selection, max_err, yardstick_check
+from tests.gpu_util import SCALE, bf16_inputs, forward_tiles, kernel_selection, max_err, yardstick_check
 
 pytestmark = pytest.mark.gpu
 NAMES = ["dq_proxy", "dk_proxy", "dq", "dk", "dv"]
 
 
-@pytest.mark.parametrize("mpp", [1, 8, 9, 12])
-def test_sinks_over_groups_of_heads(mpp):
+@pytest.mark.parametrize("mpp,s,kb", [(1, 384, 2), (8, 384, 2), (9, 384, 2), (12, 384, 2), (1, 5120, 1), (8, 3072, 1), (9, 3072, 2), (12, 3072, 1)])
+def test_sinks_over_groups_of_heads(mpp, s, kb):
+    """The query-tile stationary forward alone (384), whose log-sum-exps take the sinks in a kernel of their own, and with the key-block
+    stationary one behind it, whose combine takes them."""
     import flash_msa_b200 as fm
-    cfg = dict(b=2, s=384, hq=2 * mpp, hkv=2, hp=2, hpkv=1, kb=2, seed=80 + mpp)
+    cfg = dict(b=2, s=s, hq=2 * mpp, hkv=2, hp=2, hpkv=1, kb=kb, seed=80 + mpp)
     qp, kp, q, k, v, do = bf16_inputs(cfg)
+    assert forward_tiles((qp, kp, q, k, v), kb) == (3 if s == 384 else 5 * kb // 2)
     sinks = (torch.randn(cfg["hq"], generator=torch.Generator().manual_seed(mpp)) + 1.0).cuda().requires_grad_(True)
     leaves = [t.detach().requires_grad_(True) for t in (qp, kp, q, k, v)]
     out, kl = fm.flash_msa_func(*leaves, cfg["kb"] * 128, SCALE, sinks=sinks)

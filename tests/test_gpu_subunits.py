@@ -3,17 +3,26 @@ group, whose launches take other sub-unit lengths and finer last groups."""
 import pytest
 import torch
 
-from tests.gpu_util import SCALE, bf16_inputs, max_err
+from tests.gpu_util import SCALE, bf16_inputs, forward_tiles, max_err
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("b,s,kb,docs", [(1, 4096, 16, False), (2, 4096, 16, False), (4, 4096, 16, True), (5, 4096, 16, False), (3, 1664, 5, True)])
-def test_one_pass_against_a_pass_per_group(monkeypatch, b, s, kb, docs):
-    """Sub-units of 2, 4, 8 and 16 chunks at most in the one pass (and 1, rows that end inside a chunk, in the last case)."""
+@pytest.mark.parametrize("b,s,kb,docs,form", [
+    (1, 4096, 16, False, None), (2, 4096, 16, False, None), (4, 4096, 16, True, None), (5, 4096, 16, False, None), (3, 1664, 5, True, None),
+    (2, 8192, 2, False, "four"), (2, 8192, 3, False, "shared"), (2, 8192, 3, True, "four"), (1, 12544, 4, True, "shared fp16")])
+def test_one_pass_against_a_pass_per_group(monkeypatch, b, s, kb, docs, form):
+    """The backward with sub-units of 2, 4, 8 and 16 chunks at most in the one pass (and 1, rows that end inside a chunk, in the case of
+    1664); in the cases with a `form` (four KV heads, or three with two proxy heads each) also the forward, whose key-block stationary
+    kernels then work on the tiles that the other one leaves."""
     import flash_msa_b200 as fm
     from flash_msa_b200 import ops
-    *inputs, do = bf16_inputs(dict(b=b, s=s, hq=4, hkv=4, hp=4, hpkv=4, seed=b + s))
+    heads = dict(hq=12, hkv=3, hp=6, hpkv=3) if form and form.startswith("shared") else dict(hq=4, hkv=4, hp=4, hpkv=4)
+    dt = torch.float16 if form == "shared fp16" else torch.bfloat16
+    *inputs, do = bf16_inputs(dict(b=b, s=s, seed=b + s, **heads), dtype=dt)
+    tiles = forward_tiles(inputs, kb, [0, s // 3, s // 2 + 5, s] if docs else None)
+    assert 1 <= tiles < s // 128 if form else tiles == s // 128
+    kl_weight = torch.tensor(float(s if dt == torch.float16 else 1), device="cuda")   # (proxy gradients above fp16's subnormals)
     res = []
     for cap in (None, 1):
         if cap:
@@ -23,7 +32,7 @@ def test_one_pass_against_a_pass_per_group(monkeypatch, b, s, kb, docs):
             out, kl = fm.flash_msa_varlen_func(*leaves, [0, s // 3, s // 2 + 5, s], kb * 128, SCALE)
         else:
             out, kl = fm.flash_msa_func(*leaves, kb * 128, SCALE)
-        torch.autograd.backward([out, kl], [do, torch.ones((), device="cuda")])
+        torch.autograd.backward([out, kl], [do, kl_weight])
         res.append([out] + [t.grad for t in leaves])
     for n, a, c in zip(["out", "dq_proxy", "dk_proxy", "dq", "dk", "dv"], *res):
         # (the order in which sub-units add to dK, dV and dKp is free: the last bit of the 16-bit result)

@@ -201,3 +201,34 @@ def test_stages_of_the_tiles_behind(monkeypatch, cfg, cap):
                                       torch.cuda.current_stream().cuda_stream), "fmsa_row_start")
         ends = torch.tensor([int((col_q[row_ptr[r]:row_ptr[r + 1]] < 128 * t).sum()) for r in range(b * hp * nb)])
         assert torch.equal(start.cpu(), row_ptr[:-1] + ends)
+
+
+@pytest.mark.parametrize("b,s,heads,form", [(2, 640, dict(hq=12, hkv=2, hp=4, hpkv=2), "docs"), (1, 1664, dict(hq=9, hkv=1, hp=1, hpkv=1), "plain"),
+                                            (1, 2048, dict(hq=4, hkv=2, hp=2, hpkv=1), "fp16")])
+def test_dense_schedule_of_the_key_block_stationary_stages(b, s, heads, form):
+    """No call of the package takes a dense forward this way, but the two stages accept it: a pass over all groups and one per group against
+    the query-tile stationary stage, with the errors of the first test above."""
+    from flash_msa_b200 import _lib, ops
+    dt = torch.float16 if form == "fp16" else torch.bfloat16
+    qp, kp, q, k, v, _ = bf16_inputs(dict(b=b, s=s, seed=s, **heads), dtype=dt)
+    ds = ops.doc_start_from_cu_seqlens([0, s // 3, s // 3 + 1, s], b, s, q.device) if form == "docs" else None
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = ops.attention_forward(q, k, v, qp, kp, SCALE, None, dense=True, doc_start=ds, status=status)
+    lib, pb, st = _lib.load(), ops._problem(q, k, qp, kp, 1, SCALE, ds), torch.cuda.current_stream().cuda_stream
+    args = [ops._tensor_arg(t) for t in (q, k, v, qp, kp)]
+    mpp, groups = heads["hq"] // heads["hp"], b * heads["hkv"]
+    u = 2.0 ** (-12 if dt == torch.float16 else -9)
+    for step in (groups, 1):
+        got = [torch.full_like(t, float("nan")) for t in want]
+        slots = lib.fmsa_fwd_partial_slots(pb, step, 1)
+        o_part = torch.empty(slots * mpp * 128, dtype=dt, device="cuda")
+        stats = torch.empty(slots * (mpp + 1) * 2, dtype=torch.float32, device="cuda")
+        counter = torch.empty(1, dtype=torch.int32, device="cuda")
+        for g0 in range(0, groups, step):
+            _lib.check(lib.fmsa_sparse_fwd(pb, *args, 0, 0, o_part.data_ptr(), stats.data_ptr(), slots, g0, step, 1, 1, counter.data_ptr(),
+                                           status.data_ptr(), st), "fmsa_sparse_fwd")
+            _lib.check(lib.fmsa_sparse_fwd_combine(pb, o_part.data_ptr(), stats.data_ptr(), 0, 0, *(t.data_ptr() for t in got), g0, step, 1, st),
+                       "fmsa_sparse_fwd_combine")
+        ops.check_status(status, "forward")
+        assert max_err(got[0], want[0]) <= 5 * u * v.float().abs().max().item()
+        assert max_err(got[1], want[1]) <= 1e-4 and max_err(got[2], want[2]) <= 1e-4
