@@ -54,9 +54,11 @@ __host__ __device__ __forceinline__ int64_t subunits_per_group(int NB, int depth
 // per proxy head in the sparse schedule.  Early rows have fewer blocks to select, and documents hide some: 77 % of it are
 // there at S=4096 top-k 16 blocks, 63 % at S=16384 top-k 96, 48 % with five documents at S=8192 top-k 16, so a launch can
 // have half the sub-units per CTA that the constants say.  Both constants were measured with this bound (and the lengths below
-// chosen by it).  A row of the reverse index is on average half a chunk longer than its edges.  Drawing and passing over
-// sub-units beyond the end of their rows costs about a microsecond (up to 32 at a time), so C does not go below what keeps
-// the enumeration at `kDrawsPerCta` per CTA.
+// chosen by it).  A row of the reverse index is on average half a chunk longer than its edges.  Where most
+// sub-units lie beyond the end of their rows (they are passed over 32 at a time, or to the next one with work: draw_work), C does
+// not go below what keeps the enumeration at `kDrawsPerCta` per CTA: shorter ones gain nothing there and flush dV and dK more often.
+// Backward kernels with a limit of 16 / 32 / 64 / none: B=4 S=3968 Hq=16 top-k 2 blocks 210 / 209 / 246 / 247 us, B=1 S=52736 Hq=12 top-k 2 with six
+// documents 578 / 578 / 601 / 625, B=1 S=41216 Hq=32 top-k 3 and S=65536 Hq=8 top-k 32 equal within the spread of 3 %.
 // With 16 the rows of a group are gathered in half as many sweeps, which counts where they do not fit L2 (B=1 S=65536 Hq=8
 // top-k 32 blocks, 14 sub-units per CTA: forward 1.70 -> 1.56 ms, backward 3.83 -> 3.49 ms), and K, V, dK and dV move half as often
 // (B=2 S=8192 Hq=32 top-k 16 blocks, 7 per CTA, with the last groups cut finer: backward kernels 1.569 -> 1.516 ms; at two per CTA no

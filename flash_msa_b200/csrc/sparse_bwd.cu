@@ -715,7 +715,7 @@ struct BwdCombineParams {
     int64_t part_slots;
 };
 
-constexpr int64_t kLastFirstBytes = 512ll << 20;
+constexpr int64_t kLastFirstBytes = 512ll << 20;   // (figures: fmsa_sparse_bwd_combine)
 
 // One sweep over the contiguous mpp*256-byte record of each edge; with more than eight main heads per proxy head blockIdx.y
 // takes groups of heads, each a contiguous piece of the record (and group 0 the proxy row): at Hq/Hp = 12, 96 edges per row,
@@ -1165,8 +1165,10 @@ extern "C" int fmsa_sparse_bwd_combine(const fmsa_problem* pb, const void* dq_pa
     const int64_t rows = static_cast<int64_t>(g_count) * P.ppk * P.S;
     const int64_t grid = (rows + 7) / 8;
     FMSA_REQUIRE(grid <= 0x7fffffffLL);
-    // Partial rows that are not much more than L2 holds: those written last are still there (B=3 S=1664 Hq=20 top-k 5 blocks, 154 MB:
-    // 43.5 -> 41.5 us).  Of gigabytes too little is, and the other order is the faster one (B=1 S=16384 top-k 96: 2.53 -> 2.61 ms).
+    // Up to a few times L2 (126 MB) a good part of the partial rows, those written last, is still there.  B=1 Hq=16 Hp=4 top-k 16 blocks, one
+    // plane: 160 MB 29.2 -> 27.1 us, 240 MB 45.6 -> 42.4, 320 MB 59.9 -> 57.9, 480 MB 88.6 both ways; top-k 4: 160 MB 47.5 -> 45.5, 320 MB 84.4 ->
+    // 82.4, 480 MB 119.3 -> 117.2.  From there to 1.3 GB the two orders are within 1 to 3 %, of 5 GB in two planes too little is left and the other
+    // order is the faster one (B=1 S=16384 top-k 96: 2.53 -> 2.61 ms), so the line is at the end of the clear gain.
     const int64_t part_bytes = fmsa_fwd_partial_slots(pb, g_count, dense) * (P.mpp + (dq_proxy ? 1 : 0)) * kHeadDim * 2 * (split ? 2 : 1);
     P.last_first = part_bytes <= kLastFirstBytes ? 1 : 0;
     const int groups = P.mpp <= 8 ? 1 : (P.mpp + 5) / 6;   // as in the forward combine

@@ -15,9 +15,10 @@
 // TMEM: S buffer n at columns 128 n (P over its first 64), O at 384.
 //
 // B=4 S=4096 Hq=32 dense, with the proxy heads: 0.607 ms against 0.767 + 0.492 ms of the key-block stationary kernel and its combine;
-// B=1 S=16384 Hq=24 top-k 96 blocks: 1.49 against 2.11 + 1.54 ms.  A step takes 1860 cycles, of which the tensor core works 1050 and the
-// special function unit 1024.  It is bound by the way from a finished P through P V, S and three hand-offs to the next S in the same
-// buffer (about 2000 cycles), shared by three buffers, and by the softmax of a step (about 2300 beside the other group's).  Measured in
+// B=1 S=16384 Hq=24 top-k 96 blocks: 1.49 against 2.11 + 1.54 ms.  A step takes 1656 cycles (dense, main heads only, one launch under a
+// profiler), of which the tensor core and the special function unit work 1024 each.  It is bound by the way from a finished P through P V,
+// S and three hand-offs to the next S in the same buffer, shared by three buffers, and by the softmax of a step beside the other
+// group's (about 2000 and 2300 cycles when a step took 1860).  Measured in
 // its place, same problem: two heads per CTA with an O and one S buffer each 0.68 ms; the same with two half-block S buffers each
 // 0.62; with twice the softmax warps, one set per half block 0.75; one head, a softmax group per half block 0.72; one issuing
 // thread for all products 1.00 (it needs 1100 to 2000 cycles for a half block's waits, products and commits).
